@@ -246,9 +246,9 @@ int shape_of(negf_b200_ctx* ctx, int npts, const int32_t* ids, LaunchShape& sh) 
   return NEGF_B200_OK;
 }
 
-int grid_for(negf_b200_ctx* ctx, int npts) {
-  int per_sm = ctx->opt.ctas_per_sm > 0 ? ctx->opt.ctas_per_sm : 2;
-  return std::max(1, std::min(npts, per_sm * ctx->sms));
+int max_ctas(negf_b200_ctx* ctx) {
+  const int per_sm = ctx->opt.ctas_per_sm > 0 ? ctx->opt.ctas_per_sm : 2;
+  return std::max(1, per_sm * ctx->sms);
 }
 
 // Runs one launch with device-resident inputs/outputs (all pointers device).
@@ -258,25 +258,25 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
                                                 std::to_string(negf::kMaxOrder));
   int st = sync_descs(ctx);
   if (st) return st;
-  int grid = grid_for(ctx, a.npts);
+  negf::TeamShape ts = negf::team_shape(a.npts, sh.nmax, max_ctas(ctx), std::max(1, ctx->sms));
   const int64_t per = negf::engine_ws_elems(a.mode, sh.nbl_max, sh.ncont_max, sh.nmax);
   if (ctx->ws_limit > 0) {
-    // fewer resident CTAs when the workspace would exceed the limit (the persistent
-    // kernel still runs every point); not even one CTA: refuse
+    // fewer resident teams when the workspace would exceed the limit (the persistent
+    // kernel still runs every point); not even one: refuse
     const size_t per_bytes = (size_t)per * sizeof(double2);
     const size_t fit = ctx->ws_limit > 256 ? (ctx->ws_limit - 256) / per_bytes : 0;
     if (fit < 1)
-      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one CTA's workspace (" + std::to_string(per_bytes) +
+      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(per_bytes) +
                                                     " bytes) exceeds the workspace limit");
-    grid = (int)std::min<size_t>(grid, fit);
+    if ((size_t)ts.teams > fit) ts = negf::team_shape((int)fit, sh.nmax, max_ctas(ctx), std::max(1, ctx->sms));
   }
   // counter lives at the start of the workspace allocation
-  const size_t need = 256 + (size_t)grid * per * sizeof(double2);
+  const size_t need = 256 + (size_t)ts.teams * per * sizeof(double2);
   st = grow(ctx, &ctx->ws, &ctx->ws_bytes, need);
   if (st) return st;
   a.counter = reinterpret_cast<int*>(ctx->ws);
   a.ws = reinterpret_cast<double2*>(reinterpret_cast<char*>(ctx->ws) + 256);
-  a.ws_per_cta = per;
+  a.ws_per_team = per;
   a.Q = (int64_t)sh.nmax * sh.nmax;
   a.nmax = sh.nmax;
   a.nbl_max = sh.nbl_max;
@@ -284,7 +284,7 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
   a.devs = ctx->d_descs;
   a.trace = ctx->trace ? ctx->d_trace : nullptr;
   CK(cudaMemsetAsync(a.counter, 0, sizeof(int), s));
-  cudaError_t e = negf::launch_engine(a, grid, s);
+  cudaError_t e = negf::launch_engine(a, ts.teams, ts.team, s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
   ++ctx->launches;
   return NEGF_B200_OK;

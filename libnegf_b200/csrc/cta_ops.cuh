@@ -1,10 +1,10 @@
 // CTA-level complex128 block operations for sm_100a.
 //
-// Every routine here is executed cooperatively by all threads of one CTA on
-// blocks that live in global memory (HBM, L2-resident while hot).  They are
-// the building blocks of the persistent per-energy-point engine: one CTA
-// owns one (energy, k) point at a time and runs its whole recursive
-// Green's-function solve with these operations.
+// Every routine here is executed cooperatively by all threads of one CTA, or
+// of a team of CTAs (a thread-block cluster), on blocks that live in global
+// memory (HBM, L2-resident while hot).  They are the building blocks of the
+// persistent per-energy-point engine: one team owns one (energy, k) point at
+// a time and runs its whole recursive Green's-function solve with them.
 //
 //   cta_gemm  C = epilogue(op(A) op(B)) on the FP64 tensor pipe
 //             (mma.sync m16n8k4 .f64, 4 real products per complex product),
@@ -62,6 +62,73 @@ __device__ __forceinline__ double2 crecip(double2 z) {
 }
 __device__ __forceinline__ double cabs1(double2 z) { return fabs(z.x) + fabs(z.y); }
 __device__ __forceinline__ double cabs(double2 z) { return hypot(z.x, z.y); }
+
+// ---------------------------------------------------------------- teams
+// A team is the thread-block cluster that works on one problem (one CTA
+// without a cluster launch).  Every CTA of a team runs the same control code
+// with the same values; the routines below split the elements or output
+// tiles of an operation over the team's CTAs, and each operation ends with
+// team_sync(), which also publishes its global-memory writes to the team
+// (cluster-scope release / acquire).  How an element is computed never
+// depends on the team's size, so results are the same bits for every size.
+__device__ __forceinline__ int team_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+__device__ __forceinline__ int team_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return (int)r;
+}
+// All threads of the team; a __syncthreads() for a team of one.
+__device__ __forceinline__ void team_sync() {
+  if (team_size() == 1) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+// First element and stride of this thread in a loop split over the team.
+__device__ __forceinline__ int team_tid() { return team_rank() * (int)blockDim.x + (int)threadIdx.x; }
+__device__ __forceinline__ int team_threads() { return team_size() * (int)blockDim.x; }
+// Shared memory of team member `rank` at this CTA's address p (every CTA of a
+// kernel has the same shared-memory layout).
+__device__ __forceinline__ uint32_t team_addr(const void* p, int rank) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ int team_ld_int(const int* p, int rank) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(team_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ double team_ld_double(const double* p, int rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(team_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void team_st_double2(double2* p, int rank, double2 v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(team_addr(p, rank)), "d"(v.x), "d"(v.y) : "memory");
+}
+// The largest *v (>= 0) over the team, left in every member's *v.  Members may
+// overwrite *v with the result while others still read it: the maximum of
+// the values only grows to the result.  Callers pass a team_sync() before *v
+// is next reset.
+__device__ __forceinline__ void team_max(double* v) {
+  if (team_size() == 1) return;
+  team_sync();
+  if (threadIdx.x == 0) {
+    double m = *v;
+    const int G = team_size(), me = team_rank();
+    for (int r = 0; r < G; ++r)
+      if (r != me) m = fmax(m, team_ld_double(v, r));
+    *v = m;
+  }
+  __syncthreads();
+}
 
 // ---------------------------------------------------------------- async copy
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -235,6 +302,7 @@ struct GemmDesc {
   double* maxabs;
   double2 alpha, beta;
   int M, N, K, lda, ldb, ldc, ldx, k0, jb, tilesM, nk, total;
+  int tile0, tstep;   // first output tile of this CTA and the team's size
   int amode, bmode, emode;
 };
 constexpr int kGemmDescOffset = kStages * kStageElems;   // in double2 units, after the staging ring
@@ -317,7 +385,8 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
   const int total = d->total;
   double lmax = 0.0;
   double accR[2][2][4], accI[2][2][4];
-  int ld_tile = 0, ld_kt = 0, ld_step = 0;   // (tile, K-tile) and index of the next step to load
+  const int tile0 = d->tile0;
+  int ld_tile = tile0, ld_kt = 0, ld_step = 0;   // (tile, K-tile) and index of the next step to load
 
   // the first kStages - 1 steps in flight (an empty group keeps the count when
   // there are fewer steps)
@@ -325,13 +394,13 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
   for (int q = 0; q < kStages - 1; ++q) {
     if (ld_step < total) {
       gemm_issue<AM, BM>(d, ld_tile, ld_kt, smem + q * kStageElems);
-      if (++ld_kt == d->nk) { ld_kt = 0; ++ld_tile; }
+      if (++ld_kt == d->nk) { ld_kt = 0; ld_tile += d->tstep; }
       ++ld_step;
     } else {
       cp_async_commit();
     }
   }
-  int tile = 0, kt = 0;
+  int tile = tile0, kt = 0;
   for (int step = 0; step < total; ++step) {
     if (kt == 0) {
 #pragma unroll
@@ -346,7 +415,7 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
     // refill the buffer of step - 1 with step + kStages - 1
     if (ld_step < total) {
       gemm_issue<AM, BM>(d, ld_tile, ld_kt, smem + (ld_step % kStages) * kStageElems);
-      if (++ld_kt == d->nk) { ld_kt = 0; ++ld_tile; }
+      if (++ld_kt == d->nk) { ld_kt = 0; ld_tile += d->tstep; }
       ++ld_step;
     } else {
       cp_async_commit();
@@ -413,7 +482,7 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
           }
       }
     }
-    if (++kt == d->nk) { kt = 0; ++tile; }
+    if (++kt == d->nk) { kt = 0; tile += d->tstep; }
   }
   if (d->maxabs) {
     // warp max then one atomic per warp on the shared accumulator
@@ -423,8 +492,10 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
       unsigned long long* a = reinterpret_cast<unsigned long long*>(d->maxabs);
       atomicMax(a, (unsigned long long)__double_as_longlong(lmax));  // lmax >= 0: bit order == value order
     }
+    __syncthreads();
+    team_max(d->maxabs);
   }
-  __syncthreads();
+  team_sync();
 }
 
 // The product loop compiled out of line in its own translation unit
@@ -435,8 +506,10 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
 // inversion leaf) was added.
 __device__ void gemm_run(const GemmDesc* d, double2* smem);
 
+// Publishes the descriptor of one product in shared memory; this CTA takes
+// the output tiles rank, rank + size, ...
 __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, const Operand& A, const Operand& B,
-                                                       const Epilogue& e, double2* smem) {
+                                                       const Epilogue& e, double2* smem, int rank, int size) {
   GemmDesc* d = reinterpret_cast<GemmDesc*>(smem + kGemmDescOffset);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -449,15 +522,23 @@ __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, cons
     d->amode = A.mode; d->bmode = B.mode; d->emode = e.mode;
     d->tilesM = (M + TM - 1) / TM;
     d->nk = max(1, (K + TK - 1) / TK);
-    d->total = d->tilesM * ((N + TN - 1) / TN) * d->nk;
+    const int tiles = d->tilesM * ((N + TN - 1) / TN);
+    d->tile0 = rank;
+    d->tstep = size;
+    d->total = rank < tiles ? ((tiles - rank + size - 1) / size) * d->nk : 0;   // tiles rank, rank + size, ...
   }
   __syncthreads();
   return d;
 }
 
+__device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, const Operand& A, const Operand& B,
+                                                       const Epilogue& e, double2* smem) {
+  return gemm_desc_publish(M, N, K, A, B, e, smem, team_rank(), team_size());
+}
+
 // C(MxN) = epilogue( op(A)(MxK) * op(B)(KxN) ).  All threads of the CTA must
-// call it.  `smem` must hold kGemmSmemBytes + sizeof(GemmDesc).  Ends with
-// __syncthreads().
+// call it (all CTAs of the team).  `smem` must hold kGemmSmemBytes +
+// sizeof(GemmDesc).  Ends with team_sync().
 //
 // The operand pipeline runs over the flattened sequence of (output tile,
 // K-tile) steps, so the next output tile's first operands are in flight
@@ -469,7 +550,8 @@ __device__ __forceinline__ void cta_gemm(int M, int N, int K, const Operand& A, 
 }
 
 // ---------------------------------------------------------------- elementwise
-// All loops stride by blockDim; callers __syncthreads() between dependent ops.
+// Loops run over the team (team_tid, team_threads) unless said otherwise;
+// callers team_sync() between dependent ops.
 
 // D(r,c) = s_e * S(r,c) - H(r,c)  (S == nullptr: identity if diag else zero)
 // optionally minus a full block `sub` (contact self-energy) and minus a
@@ -479,12 +561,13 @@ static __device__ __noinline__ void cta_esh(double2* D, int rows, int cols, cons
                         bool diag, const double2* sub, const double2* subdiag, int op) {
   const int n = rows * cols;
   const int sld = (op == OP_C) ? cols : rows;
+  const int tstep = team_threads();
   constexpr int U = 4;  // elements per thread per round: loads of a round are in flight together
-  for (int base = threadIdx.x; base < n; base += U * blockDim.x) {
+  for (int base = team_tid(); base < n; base += U * tstep) {
     double2 hv[U], sv[U], bv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = base + u * blockDim.x;
+      const int idx = base + u * tstep;
       if (idx < n) {
         const int r = idx % rows, c = idx / rows;
         // source element of the un-transposed matrix
@@ -498,7 +581,7 @@ static __device__ __noinline__ void cta_esh(double2* D, int rows, int cols, cons
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = base + u * blockDim.x;
+      const int idx = base + u * tstep;
       if (idx < n) {
         double2 v = csub(cmul(s_e, sv[u]), hv[u]);
         if (op == OP_C) v = cconj(v);
@@ -508,46 +591,51 @@ static __device__ __noinline__ void cta_esh(double2* D, int rows, int cols, cons
   }
 }
 
-__device__ __forceinline__ void cta_copy(double2* D, const double2* S, int n) {
+__device__ __forceinline__ void copy_strided(double2* D, const double2* S, int n, int first, int step) {
   constexpr int U = 4;
-  for (int base = threadIdx.x; base < n; base += U * blockDim.x) {
+  for (int base = first; base < n; base += U * step) {
     double2 v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (base + u * (int)blockDim.x < n) v[u] = S[base + u * blockDim.x];
+      if (base + u * step < n) v[u] = S[base + u * step];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (base + u * (int)blockDim.x < n) D[base + u * blockDim.x] = v[u];
+      if (base + u * step < n) D[base + u * step] = v[u];
   }
 }
+// by one CTA / by the team
+__device__ __forceinline__ void cta_copy(double2* D, const double2* S, int n) {
+  copy_strided(D, S, n, threadIdx.x, blockDim.x);
+}
+__device__ __forceinline__ void team_copy(double2* D, const double2* S, int n) {
+  copy_strided(D, S, n, team_tid(), team_threads());
+}
 
-// D(r, c) = S(r, cperm[c]) for an n x n matrix (column gather)
-__device__ __forceinline__ void cta_copy_colperm(double2* D, const double2* S, int n, const int* cperm) {
+// D(r, c) = S(r, cperm[c]) for an n x n matrix (column gather); this thread's
+// elements are first, first + step, ...
+__device__ __forceinline__ void copy_colperm(double2* D, const double2* S, int n, const int* cperm, int first,
+                                             int step) {
   constexpr int U = 4;
   const int nn = n * n;
-  for (int base = threadIdx.x; base < nn; base += U * blockDim.x) {
+  for (int base = first; base < nn; base += U * step) {
     double2 v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = base + u * blockDim.x;
+      const int idx = base + u * step;
       if (idx < nn) v[u] = S[(size_t)(idx % n) + (size_t)cperm[idx / n] * n];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int idx = base + u * blockDim.x;
+      const int idx = base + u * step;
       if (idx < nn) D[idx] = v[u];
     }
   }
 }
 
-// D (n x w, ld n) = columns [k0, k0+w) of S (ld n)
-__device__ __forceinline__ void cta_copy_cols(double2* D, const double2* S, int n, int k0, int w) {
-  cta_copy(D, S + (size_t)k0 * n, n * w);
-}
-
 // D = i*(A - A^dag)   (zspectral_dns), A square n x n
 __device__ __forceinline__ void cta_spectral(double2* D, const double2* A, int n) {
-  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
+  const int tstep = team_threads();
+  for (int idx = team_tid(); idx < n * n; idx += tstep) {
     const int r = idx % n, c = idx / n;
     double2 a = A[idx], b = cconj(A[(size_t)c + (size_t)r * n]);
     double2 d = csub(a, b);
@@ -603,35 +691,90 @@ __device__ __forceinline__ double2 probe_v(int k) { return make_double2(1.0 + 0.
 // max_i |(A (X v))_i - v_i| for the fixed vector v above (|v_k| ~ 1): of the
 // order of the rounding of the product for an inverse that is backward
 // stable, far above it where the inversion lost accuracy (Gauss-Jordan on a
-// nearly singular matrix).  Two matrix-vector products; y is an n-element
-// shared-memory buffer.  NaN or Inf anywhere gives +Inf.
-// *kappa (optional): max_i sum_j |A_ij| |(Xv)_j|, an estimate of the
-// condition number of A (|v_k| ~ 1; it reads 0.3 .. 1 decade below the
-// 2-norm condition): about 1e3 .. 1e6 for the decimation's Ao away from a
-// lead resonance, above 1e8 near one.
-__device__ __forceinline__ double cta_inv_probe(int n, const double2* A, const double2* X, double2* y, double* red,
-                                                double* kappa = nullptr) {
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+// nearly singular matrix).  Two matrix-vector products; y holds n elements
+// and part kProbeGroups * kThreads elements of shared memory, red 2 doubles.
+// NaN or Inf anywhere gives +Inf.
+// *kappa: max_i sum_j |A_ij| |(Xv)_j|, an estimate of the condition number
+// of A (|v_k| ~ 1; it reads 0.3 .. 1 decade below the 2-norm condition):
+// about 1e3 .. 1e6 for the decimation's Ao away from a lead resonance, above
+// 1e8 near one.
+//
+// Each row sum is kProbeGroups partial sums (columns g, g + kProbeGroups,
+// ...) added in order, each partial sum by one thread: the team's CTAs split
+// the rows, a CTA's threads the partial sums, so that a row is a chain of
+// n / kProbeGroups loads instead of n.
+constexpr int kProbeGroups = 8;
+
+__device__ __forceinline__ double team_inv_probe(int n, const double2* A, const double2* X, double2* y, double2* part,
+                                                 double* red, double* kappa) {
+  const int G = team_size(), rank = team_rank(), tid = threadIdx.x;
+  const int per = (n + G - 1) / G;                       // rows of a CTA, in passes of rp rows
+  const int r0 = min(n, rank * per), r1 = min(n, r0 + per);
+  constexpr int rp = kThreads / kProbeGroups;
+  const int rl = tid % rp, g = tid / rp;
+  if (tid < 2) red[tid] = 0.0;
+  for (int rb = r0; rb < r1; rb += rp) {
+    const int r = rb + rl;
     double2 acc = make_double2(0.0, 0.0);
-    for (int c = 0; c < n; ++c) acc = cadd(acc, cmul(X[(size_t)r + (size_t)c * n], probe_v(c)));
-    y[r] = acc;
+    if (r < r1)
+#pragma unroll 4
+      for (int c = g; c < n; c += kProbeGroups) acc = cadd(acc, cmul(X[(size_t)r + (size_t)c * n], probe_v(c)));
+    part[tid] = acc;
+    __syncthreads();
+    if (g == 0 && r < r1) {
+      for (int q = 1; q < kProbeGroups; ++q) acc = cadd(acc, part[rl + q * rp]);
+      if (G == 1) y[r] = acc;
+      else
+        for (int m = 0; m < G; ++m) team_st_double2(y + r, m, acc);
+    }
+    __syncthreads();
   }
-  __syncthreads();
+  team_sync();
   double e = 0.0, k = 0.0;
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+  for (int rb = r0; rb < r1; rb += rp) {
+    const int r = rb + rl;
     double2 acc = make_double2(0.0, 0.0);
     double sa = 0.0;
-    for (int c = 0; c < n; ++c) {
-      const double2 a = A[(size_t)r + (size_t)c * n];
-      acc = cadd(acc, cmul(a, y[c]));
-      sa += cabs1(a) * cabs1(y[c]);
+    if (r < r1)
+#pragma unroll 4
+      for (int c = g; c < n; c += kProbeGroups) {
+        const double2 a = A[(size_t)r + (size_t)c * n];
+        acc = cadd(acc, cmul(a, y[c]));
+        sa += cabs1(a) * cabs1(y[c]);
+      }
+    part[tid] = acc;
+    part[kThreads + tid] = make_double2(sa, 0.0);
+    __syncthreads();
+    if (g == 0 && r < r1) {
+      for (int q = 1; q < kProbeGroups; ++q) {
+        acc = cadd(acc, part[rl + q * rp]);
+        sa += part[kThreads + rl + q * rp].x;
+      }
+      const double d = cabs(csub(acc, probe_v(r)));
+      e = (d <= 1.7976931348623157e308) ? fmax(e, d) : __longlong_as_double(0x7ff0000000000000LL);
+      k = fmax(k, sa);
     }
-    const double d = cabs(csub(acc, probe_v(r)));
-    e = (d <= 1.7976931348623157e308) ? fmax(e, d) : __longlong_as_double(0x7ff0000000000000LL);
-    k = fmax(k, sa);
+    __syncthreads();
   }
-  if (kappa) *kappa = cta_max(k, red);
-  return cta_max(e, red);
+  if (g == 0) {   // rp threads: whole warps
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      e = fmax(e, __shfl_xor_sync(0xffffffffu, e, o));
+      k = fmax(k, __shfl_xor_sync(0xffffffffu, k, o));
+    }
+    static_assert(rp == 32, "one warp holds the row results");
+    if (tid == 0) {
+      red[0] = e;
+      red[1] = k;
+    }
+  }
+  __syncthreads();
+  team_max(red);
+  team_max(red + 1);
+  *kappa = red[1];
+  const double r = red[0];
+  team_sync();
+  return r;
 }
 
 // A decimation whose Ao reaches this estimated condition number is sensitive
@@ -795,14 +938,35 @@ __host__ __device__ inline size_t zinv_ws_elems(int n, int smem_bytes) {
 
 // Row permutation of the pivots of columns [c0, c1), composed in order
 // (position i of the transformed block holds row perm[i] of the input).
+// perm = the exchanges (j, piv[j]) applied to the identity one after the
+// other, so perm[i] is i taken through them from the last to the first:
+// every thread walks its own positions (measured at n = 256, 128 pivots: a
+// single thread exchanging entries one after the other took 5 times as long).
 __device__ __forceinline__ void gj_block_perm(int* perm, const int* piv, int n, int c0, int c1) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int j = c0; j < c1; ++j) {
+  __syncthreads();   // the last pivots written, every reader done with the old permutation
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    int x = i;
+#pragma unroll 8
+    for (int j = c1 - 1; j >= c0; --j) {
       const int p = piv[j];
-      const int t = perm[j]; perm[j] = perm[p]; perm[p] = t;
+      x = (x == j) ? p : ((x == p) ? j : x);
     }
+    perm[i] = x;
+  }
+  __syncthreads();
+}
+
+// The exchanges composed the other way round (columns of the inverse).
+__device__ __forceinline__ void gj_col_perm(int* perm, const int* piv, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    int x = i;
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) {
+      const int p = piv[j];
+      x = (x == j) ? p : ((x == p) ? j : x);
+    }
+    perm[i] = x;
+  }
   __syncthreads();
 }
 
@@ -1144,6 +1308,50 @@ __device__ __forceinline__ void gj_rows_update(const double2* X, double2* Y, con
   }
 }
 
+// The same update split over the CTAs of a team: CTA `rank` takes a band of
+// rows and every column.  The W rows of the band and the K pivot rows of X
+// are staged in shared memory (K <= kRowsMax; passes of kRowsBand rows and
+// kRowsCols columns bound the stage), then each thread computes whole
+// elements with the arithmetic of gj_rows_update.  With few rows per CTA its
+// row owners would leave most threads idle.
+constexpr int kRowsBand = 64, kRowsCols = 64;
+
+__device__ __forceinline__ void gj_rows_update_team(const double2* X, double2* Y, const double2* Wm, int n, int N,
+                                                    int k0, int K, const int* perm, double2* stage) {
+  const int G = team_size(), tid = threadIdx.x, nt = blockDim.x;
+  const int per = (n + G - 1) / G, r0 = min(n, team_rank() * per), r1 = min(n, r0 + per);
+  double2* sw = stage;                        // [K][kRowsBand]
+  double2* sx = stage + kRowsMax * kRowsBand; // [kRowsCols][K]
+  for (int cc = 0; cc < N; cc += kRowsCols) {
+    const int cw = min(kRowsCols, N - cc);
+    for (int rb = r0; rb < r1; rb += kRowsBand) {
+      const int rw = min(kRowsBand, r1 - rb);
+      for (int q = tid; q < K * cw; q += nt) {
+        const int c = q / K, k = q - c * K;
+        sx[q] = X[perm[k0 + k] + (size_t)(cc + c) * n];
+      }
+      for (int q = tid; q < K * rw; q += nt) {
+        const int k = q / rw, r = q - k * rw;
+        sw[k * kRowsBand + r] = Wm[rb + r + (size_t)k * n];
+      }
+      __syncthreads();
+      for (int q = tid; q < rw * cw; q += nt) {
+        const int c = q / rw, r = q - c * rw, i = rb + r;
+        const bool masked = (i >= k0 && i < k0 + K);
+        double2 acc = masked ? make_double2(0.0, 0.0) : X[perm[i] + (size_t)(cc + c) * n];
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+          const double2 wv = sw[k * kRowsBand + r], t = sx[c * K + k];
+          acc.x = fma(wv.x, t.x, fma(-wv.y, t.y, acc.x));
+          acc.y = fma(wv.x, t.y, fma(wv.y, t.x, acc.y));
+        }
+        Y[i + (size_t)(cc + c) * n] = acc;
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // gj_leaf4 for 1, 2 and 4 rows per thread, each compiled out of line in
 // leaf_dev.cu (see gemm_run); gj_rows_update likewise (rows_run_*: n <= 128
 // two threads per row, n <= 256 one, n <= 512 two rows per thread, n <= 1024
@@ -1159,6 +1367,8 @@ __device__ void rows_run_r2(const double2* X, double2* Y, const double2* Wm, int
                             const int* perm, double2* stage);
 __device__ void rows_run_r4(const double2* X, double2* Y, const double2* Wm, int n, int N, int k0, int K,
                             const int* perm, double2* stage);
+__device__ void rows_run_team(const double2* X, double2* Y, const double2* Wm, int n, int N, int k0, int K,
+                              const int* perm, double2* stage);
 
 // ---------------------------------------------------------------- inversion driver
 // out = A^-1 (n x n).  A is read only (out may alias A).  `ws` holds
@@ -1195,6 +1405,7 @@ struct InvProg {
   double2* out;
   double2* buf[2];
   int n, d, nl, k, l, phase, rpt;
+  int leaf_open;            // a leaf was handed out: its pivots are still to be shared with the team
   int flip_ta, flip_half;   // parity flip owed by the last update
   double2* X;               // leaf step: panel base, first column, width
   int c0, w;
@@ -1218,6 +1429,12 @@ static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* 
   __syncthreads();
   ip.A = A; ip.out = out; ip.n = n;
   if (n <= kSmallInvMax) {
+    if (team_rank() != 0) {   // one CTA holds the whole matrix; the others take over its info
+      team_sync();
+      if (threadIdx.x == 0) *s.flag = team_ld_int(s.flag, 0);
+      __syncthreads();
+      return 1;
+    }
     double2* P = smem;
     double2* f = smem + (size_t)n * n;
     double2* rowj = f + n;
@@ -1232,16 +1449,9 @@ static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* 
     __syncthreads();
     s.tr.stop(TR_INV_PANEL, t0);
     t0 = s.tr.start();
-    if (threadIdx.x == 0) {
-      for (int c = 0; c < n; ++c) s.cperm[c] = c;
-      for (int j = n - 1; j >= 0; --j) {
-        int p = s.piv[j];
-        int tmp = s.cperm[j]; s.cperm[j] = s.cperm[p]; s.cperm[p] = tmp;
-      }
-    }
-    __syncthreads();
-    cta_copy_colperm(out, P, n, s.cperm);
-    __syncthreads();
+    gj_col_perm(s.cperm, s.piv, n);
+    copy_colperm(out, P, n, s.cperm, threadIdx.x, blockDim.x);
+    team_sync();
     s.tr.stop(TR_INV_OTHER, t0);
     return 1;
   }
@@ -1256,7 +1466,7 @@ static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* 
   ip.nl = 1 << d;
   ip.buf[0] = ws;
   ip.buf[1] = ws + (size_t)n * n;
-  ip.k = 0; ip.l = 0; ip.phase = 0; ip.flip_half = 0;
+  ip.k = 0; ip.l = 0; ip.phase = 0; ip.flip_half = 0; ip.leaf_open = 0;
   // per-leaf location (nl <= n): 0 / 1 = buffer, kInA = still only in A (read in place, never written)
   unsigned char* par = reinterpret_cast<unsigned char*>(s.cperm);
   for (int k = threadIdx.x; k < ip.nl; k += blockDim.x) par[k] = kInA;
@@ -1269,6 +1479,17 @@ static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* 
 static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScratch& s) {
   unsigned char* par = reinterpret_cast<unsigned char*>(s.cperm);
   const int n = ip.n, d = ip.d;
+  if (ip.leaf_open) {   // CTA 0 has factorised a leaf: its panel and pivots reach the team
+    ip.leaf_open = 0;
+    if (team_size() > 1) {
+      team_sync();
+      if (team_rank() != 0) {
+        for (int j = threadIdx.x; j < ip.w; j += blockDim.x) s.piv[ip.c0 + j] = team_ld_int(s.piv + ip.c0 + j, 0);
+        if (threadIdx.x == 0) *s.flag = team_ld_int(s.flag, 0);
+      }
+      __syncthreads();
+    }
+  }
   if (ip.flip_half) {   // the update just run moved its target leaves to the other buffer
     for (int q = threadIdx.x; q < ip.flip_half; q += blockDim.x) {
       const unsigned char b = par[ip.flip_ta + q];
@@ -1286,7 +1507,8 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
       ip.w = (((k + 1) * n) >> d) - ip.c0;
       if (par[k] == kInA) {   // only leaf 0: every later leaf is the target of an update first
         const long long t0 = s.tr.start();
-        cta_copy(ip.buf[0] + (size_t)ip.c0 * n, ip.A + (size_t)ip.c0 * n, n * ip.w);
+        // CTA 0 alone reads it before the next team_sync
+        if (team_rank() == 0) cta_copy(ip.buf[0] + (size_t)ip.c0 * n, ip.A + (size_t)ip.c0 * n, n * ip.w);
         __syncthreads();
         if (threadIdx.x == 0) par[k] = 0;
         __syncthreads();
@@ -1295,6 +1517,7 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
       ip.X = ip.buf[par[k]];
       ip.phase = 1;
       ip.l = 1;
+      ip.leaf_open = 1;
       return INV_LEAF;
     }
     // delayed updates of the tree nodes leaf k closes, level ip.l upwards
@@ -1343,23 +1566,27 @@ static __device__ __noinline__ int inv_end(InvProg& ip, InvScratch& s) {
   long long t0 = s.tr.start();
   const double2* X = ip.buf[par[0]];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int c = 0; c < n; ++c) s.perm[c] = c;
-    for (int j = n - 1; j >= 0; --j) {
-      int p = s.piv[j];
-      int tmp = s.perm[j]; s.perm[j] = s.perm[p]; s.perm[p] = tmp;
-    }
-  }
-  __syncthreads();
-  cta_copy_colperm(ip.out, X, n, s.perm);
-  __syncthreads();
+  gj_col_perm(s.perm, s.piv, n);
+  copy_colperm(ip.out, X, n, s.perm, team_tid(), team_threads());
+  team_sync();
   s.tr.stop(TR_INV_OTHER, t0);
   return 0;
 }
 
-// The row-owner update step of ip (INV_ROWS), by rows per thread.
+// The leaf step of ip (INV_LEAF): CTA 0 of the team.
+__device__ __forceinline__ void leaf_run(const InvProg& ip, double2* smem, InvScratch& s) {
+  if (team_rank() != 0) return;
+  if (ip.rpt == 1) leaf_run_r1(ip.X, ip.n, ip.c0, ip.w, smem, s);
+  else if (ip.rpt == 2) leaf_run_r2(ip.X, ip.n, ip.c0, ip.w, smem, s);
+  else leaf_run_r4(ip.X, ip.n, ip.c0, ip.w, smem, s);
+}
+
+// The row-owner update step of ip (INV_ROWS), by team size and rows per thread.
 __device__ __forceinline__ void rows_run(const InvProg& ip, double2* smem, const InvScratch& s) {
-  if (2 * ip.n <= (int)blockDim.x) rows_run_t2(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
+  if (team_size() > 1) {
+    rows_run_team(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
+    team_sync();
+  } else if (2 * ip.n <= (int)blockDim.x) rows_run_t2(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
   else if (ip.rpt == 1) rows_run_r1(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
   else if (ip.rpt == 2) rows_run_r2(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
   else rows_run_r4(ip.rX, ip.rY, ip.rW, ip.n, ip.rN, ip.rk0, ip.rK, s.perm, smem);
@@ -1377,9 +1604,7 @@ __device__ __forceinline__ int cta_zinv(int n, const double2* A, double2* out, d
       if (step == INV_DONE) break;
       if (step == INV_LEAF) {
         const long long t0 = s.tr.start();
-        if (ip.rpt == 1) leaf_run_r1(ip.X, ip.n, ip.c0, ip.w, smem, s);
-        else if (ip.rpt == 2) leaf_run_r2(ip.X, ip.n, ip.c0, ip.w, smem, s);
-        else leaf_run_r4(ip.X, ip.n, ip.c0, ip.w, smem, s);
+        leaf_run(ip, smem, s);
         s.tr.stop(TR_INV_PANEL, t0);
       } else if (step == INV_ROWS) {
         rows_run(ip, smem, s);

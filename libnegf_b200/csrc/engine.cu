@@ -1,11 +1,12 @@
 // Persistent per-energy-point engine for sm_100a.
 //
-// One CTA owns one (energy, k) point at a time and runs its complete solve:
+// One team (a CTA, or a cluster of up to 16 CTAs when a call has few points)
+// owns one (energy, k) point at a time and runs its complete solve:
 // Sancho-Rubio decimation per contact, contact self-energies, the backward
 // gsmr sweep, Gr(1,1), then (by mode) the Caroli transmission, the full
 // retarded sweep with the diagonal spectral density, or the elastic
 // dephasing SCBA loop with the lesser sweep, Meir-Wingreen and layer
-// currents.  CTAs pull points from a global queue, so all energy x k points
+// currents.  Teams pull points from a global queue, so all energy x k points
 // of a call (and all SCBA iterations of each point) run in one launch with
 // no host synchronisation; per-point convergence (decimation, SCBA) is
 // decided on the device.
@@ -16,7 +17,10 @@
 // DOS src/iterative.F90:1821-1952, elastic SCBA :289-363 with
 // src/elphdd.F90:108-276 and src/scba.F90:120-147, Meir-Wingreen and layer
 // current src/iterative.F90:382-461.
+#include <algorithm>
 #include <mutex>
+#include <set>
+#include <utility>
 
 #include "program.cuh"
 
@@ -60,22 +64,22 @@ __device__ __noinline__ int zinv_refined(int n, const double2* A, double2* X, do
   const int nn = n * n;
   for (int k = 0; k < 2 && R; ++k) {
     double kap = 0.0;
-    const double e = cta_inv_probe(n, A, X, sm.main, sm.red, &kap);
+    const double e = team_inv_probe(n, A, X, sm.main, sm.main + n, sm.maxv, &kap);
     if (k == 0 && nearly_singular && kap > kSensitiveCond) *nearly_singular = true;
     if (!(e > kInvProbeTol) || !(e <= 1.7976931348623157e308)) break;
-    for (int q = threadIdx.x; q < nn; q += blockDim.x) R[q] = make_double2((q % n) == (q / n) ? 1.0 : 0.0, 0.0);
-    __syncthreads();
+    for (int q = team_tid(); q < nn; q += team_threads()) R[q] = make_double2((q % n) == (q / n) ? 1.0 : 0.0, 0.0);
+    team_sync();
     gemm(n, n, n, opN(A, n), opN(X, n), R, n, mone, one, sm);     // R = I - A X
-    cta_copy(Xn, X, nn);
-    __syncthreads();
+    team_copy(Xn, X, nn);
+    team_sync();
     gemm(n, n, n, opN(X, n), opN(R, n), Xn, n, one, one, sm);     // X + X R
-    cta_copy(X, Xn, nn);
-    __syncthreads();
+    team_copy(X, Xn, nn);
+    team_sync();
   }
   return bad;
 }
 
-// Sancho-Rubio decimation (src/contselfenergy.F90:271-340), CTA-cooperative.
+// Sancho-Rubio decimation (src/contselfenergy.F90:271-340) by one team.
 // In: Ao, Bo, Co in slot 0, 2, 3 (consumed).  Out: surface GF in *go_out
 // (one of the slots).  Returns a status.
 __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int max_iter, int& ncyc, double2** go_out,
@@ -90,8 +94,8 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
   double2* C1 = w.slot(7);
   const int nn = L * L;
   int st = ST_OK;
-  cta_copy(Aos, Ao, nn);
-  __syncthreads();
+  team_copy(Aos, Ao, nn);
+  team_sync();
   bool ok = false, done = false;
   int it;
   const double2 one = cz(1, 0), zero = cz(0, 0), mone = cz(-1, 0);
@@ -108,11 +112,11 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
       ok = false;
     }
     gemm(L, L, L, opN(Bo, L), opN(X, L), Sf, L, one, zero, sm);            // Self = Bo GoXCo
-    for (int q = threadIdx.x; q < nn; q += blockDim.x) {
+    for (int q = team_tid(); q < nn; q += team_threads()) {
       Aos[q] = csub(Aos[q], Sf[q]);
       Ao[q] = csub(Ao[q], Sf[q]);
     }
-    __syncthreads();
+    team_sync();
     gemm(L, L, L, opN(Go, L), opN(Bo, L), Sf, L, one, zero, sm);            // GoXBo
     gemm(L, L, L, opN(Bo, L), opN(Sf, L), X, L, one, zero, sm);             // B1 = Bo GoXBo
     gemm(L, L, L, opN(Co, L), opN(Sf, L), Ao, L, mone, one, sm);            // Ao -= Co GoXBo
@@ -127,7 +131,7 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
 }
 
 // ---------------------------------------------------------------- engine kernel
-// Persistent: each CTA pulls points from the queue inside engine_step() and
+// Persistent: each team pulls points from the queue inside engine_step() and
 // runs the heavy steps it returns.  The product loop is inlined here and the
 // kernel keeps nothing in registers across engine_step() (its state is in
 // local memory, the shared-memory map in shared memory), so the loop is
@@ -156,14 +160,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_engine(EngineArgs a) {
       cta_gemm_body<OP_RT, OP_RT, EPI_RT>(reinterpret_cast<const GemmDesc*>(smap.main + kGemmDescOffset), smap.main);
     } else if (st == STEP_ROWS) {
       rows_run(c.ip, smap.main, smap.inv);
-    } else if (c.ip.rpt == 1) {
-      leaf_run_r1(c.ip.X, c.ip.n, c.ip.c0, c.ip.w, smap.main, smap.inv);
-    } else if (c.ip.rpt == 2) {
-      leaf_run_r2(c.ip.X, c.ip.n, c.ip.c0, c.ip.w, smap.main, smap.inv);
     } else {
-      leaf_run_r4(c.ip.X, c.ip.n, c.ip.c0, c.ip.w, smap.main, smap.inv);
+      leaf_run(c.ip, smap.main, smap.inv);
     }
   }
+  team_sync();   // no member's shared memory is read any more
   if (a.trace) {
     if (threadIdx.x == 0) smap.tr.acc[TR_TOTAL] += clock64() - t_all;
     __syncthreads();
@@ -186,106 +187,192 @@ int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax) {
   return e;
 }
 
-cudaError_t launch_engine(const EngineArgs& a, int grid, cudaStream_t s) {
-  // the shared-memory opt-in is raised once per device and size (not per launch), so
-  // a launch is a stream operation only and can be captured into a CUDA graph
+// Raises a team kernel's shared-memory limit to that of the largest block
+// order and allows clusters of 16, once per device (not per launch), so that
+// a launch is a stream operation only and can be captured into a CUDA graph.
+cudaError_t team_opt_in(const void* kernel) {
   static std::mutex mu;
-  static int set_bytes[64] = {0};
-  const size_t smem = engine_smem_bytes(a.nmax);
+  static std::set<std::pair<const void*, int>> done;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (dev < 0 || dev >= 64 || set_bytes[dev] < (int)smem) {
-      // every size up to the largest block order, so that later launches never need it
-      const int want = (int)engine_smem_bytes(kMaxOrder);
-      e = cudaFuncSetAttribute(k_engine, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
-      if (e != cudaSuccess) return e;
-      if (dev >= 0 && dev < 64) set_bytes[dev] = want;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({kernel, dev})) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)engine_smem_bytes(kMaxOrder));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) done.insert({kernel, dev});
+  return e;
+}
+
+cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(teams * team);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  if (team > 1) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = team;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  return cfg;
+}
+
+cudaError_t launch_engine(const EngineArgs& a, int teams, int team, cudaStream_t s) {
+  cudaError_t e = team_opt_in((const void*)k_engine);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = team_config(teams, team, engine_smem_bytes(a.nmax), s, &attr);
+  return cudaLaunchKernelEx(&cfg, k_engine, a);
+}
+
+// Clusters of `team` CTAs of the engine that run at once on the current
+// device (0: none), queried once per device and size.
+static int resident_teams(int team) {
+  static std::mutex mu;
+  static int known[64][5];   // count + 1
+  int dev = 0, lg = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  while ((1 << lg) < team) ++lg;
+  std::lock_guard<std::mutex> lk(mu);
+  if (known[dev][lg] == 0) {
+    int n = 0;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = team_config(1, team, engine_smem_bytes(kMaxOrder), nullptr, &attr);
+    if (team_opt_in((const void*)k_engine) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, k_engine, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known[dev][lg] = n + 1;
+  }
+  return known[dev][lg] - 1;
+}
+
+// A team of G CTAs speeds up a problem's products by its output tiles over G;
+// the elimination's leaves stay with one CTA.  So few problems take large
+// teams (T of n = 384, 6 layers, 12 points: 825 -> 194 ms in teams of 16;
+// n = 97, 48 points: 47 -> 33 ms in teams of 4), a full GPU takes one CTA per
+// problem (n = 256, 296 points: teams of 2 lose the overlap of two problems'
+// phases on an SM), and a call just above a whole number of waves takes a team size
+// that splits its last wave (n = 256, 320 points with DOS: 773 -> 693 ms).
+// The cost: waves x time of a point, with the share of an SM that a second CTA
+// costs the first (measured 1.7 for two products at n >= 256).
+TeamShape team_shape(int work, int n, int max_ctas, int sms) {
+  TeamShape best{1, std::max(1, std::min(work, max_ctas))};
+  const int tile = (n + TM - 1) / TM, tiles = tile * tile;
+  double best_cost = 0.0;
+  for (int team = 1; team <= 16; team *= 2) {
+    if (team > 1 && team > tiles) break;
+    int teams = std::min(max_ctas / team, team > 1 ? resident_teams(team) : max_ctas);
+    if (teams < 1) break;
+    teams = std::min(teams, std::max(1, work));
+    const double share = teams * team <= sms ? 1.0 : 1.0 + 0.7 * (std::min(teams * team, 2 * sms) - sms) / sms;
+    const double serial = n <= 64 ? 0.6 : 0.15;
+    const double point = serial + (1.0 - serial) * ((tiles + team - 1) / team) / tiles;
+    const double cost = (double)((work + teams - 1) / teams) * share * point;
+    if (team == 1 || cost < 0.95 * best_cost) {
+      best = TeamShape{team, teams};
+      best_cost = cost;
     }
   }
-  k_engine<<<grid, kThreads, smem, s>>>(a);
-  return cudaGetLastError();
+  return best;
 }
 
 // ---------------------------------------------------------------- primitives
+// CTA (x, b) of the grid: output tiles x, x + gridDim.x, ... of product b.
 __global__ void __launch_bounds__(kThreads, 2)
     k_zgemm_batched(int m, int n, int k, double2 alpha, const double2* A, int64_t sA, const double2* B,
                     int64_t sB, double2 beta, double2* C, int64_t sC, int dagger) {
   extern __shared__ __align__(16) char smem_raw[];
   SmemMap sm = map_smem(smem_raw, 1);
   sm.tr.acc = nullptr;
-  const int b = blockIdx.x;
+  const int64_t b = blockIdx.y;
   Operand Ao = (dagger == 1) ? opC(A + b * sA, k) : opN(A + b * sA, m);
   Operand Bo = (dagger == 2) ? opC(B + b * sB, n) : opN(B + b * sB, k);
-  const GemmDesc* d = gemm_desc_publish(m, n, k, Ao, Bo, epi_store(C + b * sC, m, alpha, beta), sm.main);
+  const GemmDesc* d = gemm_desc_publish(m, n, k, Ao, Bo, epi_store(C + b * sC, m, alpha, beta), sm.main, blockIdx.x,
+                                        gridDim.x);
   cta_gemm_body<OP_RT, OP_RT, EPI_RT>(d, sm.main);
+}
+
+// SMs of the current device, asked once per device.
+static int device_sms() {
+  static std::mutex mu;
+  static int known[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  std::lock_guard<std::mutex> lk(mu);
+  if (known[dev] == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    known[dev] = n;
+  return known[dev] > 0 ? known[dev] : 148;
 }
 
 cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                  const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC,
                                  int dagger, cudaStream_t s) {
   const size_t smem = engine_smem_bytes(1);
-  cudaError_t e = cudaFuncSetAttribute(k_zgemm_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = team_opt_in((const void*)k_zgemm_batched);
   if (e != cudaSuccess) return e;
-  k_zgemm_batched<<<batch, kThreads, smem, s>>>(m, n, k, alpha, A, sA, B, sB, beta, C, sC, dagger);
-  return cudaGetLastError();
+  // A product's tiles over enough CTAs for four waves of the whole batch: one
+  // CTA per product left all but `batch` SMs idle (6 products of order 300:
+  // 1604 -> 111 us); with 1184 products and more one CTA runs through all
+  // tiles of a product, loading the next tile's operands behind this one's
+  // epilogue.
+  const int64_t tiles = (int64_t)((m + TM - 1) / TM) * ((n + TN - 1) / TN);
+  const int64_t want = (8LL * device_sms() + batch - 1) / batch;
+  const int split = (int)std::max<int64_t>(1, std::min(tiles, want));
+  for (int b0 = 0; b0 < batch; b0 += 65535) {   // gridDim.y limit
+    const int nb = std::min(65535, batch - b0);
+    k_zgemm_batched<<<dim3(split, nb), kThreads, smem, s>>>(m, n, k, alpha, A + b0 * sA, sA, B + b0 * sB, sB, beta,
+                                                            C + b0 * sC, sC, dagger);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // per matrix: the inversion's own buffers, then two n x n refinement buffers
 size_t zinv_batched_work_elems(int n) { return zinv_ws_elems(n, kSmemMain) + 2 * (size_t)n * n; }
 
-__global__ void __launch_bounds__(kThreads, 2)
-    k_zinv_batched(int n, const double2* A, double2* Ainv, int* info, double2* work, int64_t wstride) {
-  extern __shared__ __align__(16) char smem_raw[];
-  SmemMap sm = map_smem(smem_raw, n);
-  sm.tr.acc = nullptr;
-  const int b = blockIdx.x;
-  const int64_t nn = (int64_t)n * n;
-  double2* wb = work ? work + b * wstride : nullptr;
-  double2* R = work ? wb + zinv_ws_elems(n, kSmemMain) : nullptr;
-  int inf = zinv_refined(n, A + b * nn, Ainv + b * nn, wb, R, R ? R + nn : nullptr, sm);
-  if (threadIdx.x == 0 && info) info[b] = inf;
-}
-
-cudaError_t launch_zinv_batched(int batch, int n, const double2* A, double2* Ainv, int* info, double2* work,
-                                cudaStream_t s) {
-  const size_t smem = engine_smem_bytes(n);
-  cudaError_t e = cudaFuncSetAttribute(k_zinv_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_zinv_batched<<<batch, kThreads, smem, s>>>(n, A, Ainv, info, work, (int64_t)zinv_batched_work_elems(n));
-  return cudaGetLastError();
-}
-
-// Inverses of the problems map[b], b < batch (map null: b), matrices sA / sX
-// complex elements apart; work holds batch slots of zinv_batched_work_elems(n).
-// info[map[b]] gets the zgetrf-style singular column (0 = none).
+// One team per matrix: the inverses of the problems map[b], b < batch (map
+// null: b), matrices sA / sX complex elements apart; work (may be null where
+// the inversion needs no buffers: then no residual probe) holds batch slots
+// of wstride.  info[p] gets the zgetrf-style singular column (0 = none).
 __global__ void __launch_bounds__(kThreads, 2)
     k_zinv_mapped(int n, const double2* A, int64_t sA, double2* X, int64_t sX, const int* map, int* info,
                   double2* work, int64_t wstride, int* sens) {
   extern __shared__ __align__(16) char smem_raw[];
   SmemMap sm = map_smem(smem_raw, n);
   sm.tr.acc = nullptr;
-  const int b = blockIdx.x;
-  const int p = map ? map[b] : b;
-  double2* wb = work + (int64_t)b * wstride;
-  double2* R = wb + zinv_ws_elems(n, kSmemMain);
+  const int b = blockIdx.x / team_size();
+  const int64_t p = map ? map[b] : b;
+  double2* wb = work ? work + (int64_t)b * wstride : nullptr;
+  double2* R = work ? wb + zinv_ws_elems(n, kSmemMain) : nullptr;
   bool near_sing = false;
-  int inf = zinv_refined(n, A + (int64_t)p * sA, X + (int64_t)p * sX, wb, R, R + (int64_t)n * n, sm, &near_sing);
-  if (threadIdx.x == 0 && info) info[p] = inf;
-  if (threadIdx.x == 0 && sens && near_sing) sens[p] = 1;
+  int inf = zinv_refined(n, A + p * sA, X + p * sX, wb, R, R ? R + (int64_t)n * n : nullptr, sm, &near_sing);
+  if (lead() && info) info[p] = inf;
+  if (lead() && sens && near_sing) sens[p] = 1;
+  team_sync();   // no member's shared memory is read any more
 }
 
 cudaError_t launch_zinv_mapped(int batch, int n, const double2* A, int64_t sA, double2* X, int64_t sX,
                                const int* map, int* info, double2* work, cudaStream_t s, int* sens) {
   if (batch <= 0) return cudaSuccess;
-  const size_t smem = engine_smem_bytes(n);
-  cudaError_t e = cudaFuncSetAttribute(k_zinv_mapped, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = team_opt_in((const void*)k_zinv_mapped);
   if (e != cudaSuccess) return e;
-  k_zinv_mapped<<<batch, kThreads, smem, s>>>(n, A, sA, X, sX, map, info, work,
-                                              (int64_t)zinv_batched_work_elems(n), sens);
-  return cudaGetLastError();
+  const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
+  return cudaLaunchKernelEx(&cfg, k_zinv_mapped, n, A, sA, X, sX, map, info, work,
+                            (int64_t)zinv_batched_work_elems(n), sens);
+}
+
+cudaError_t launch_zinv_batched(int batch, int n, const double2* A, double2* Ainv, int* info, double2* work,
+                                cudaStream_t s) {
+  const int64_t nn = (int64_t)n * n;
+  return launch_zinv_mapped(batch, n, A, nn, Ainv, nn, nullptr, info, work, s, nullptr);
 }
 
 __host__ __device__ inline size_t dec_work_elems(int n) { return (size_t)(S_INV + 3) * n * n; }
@@ -297,32 +384,33 @@ __global__ void __launch_bounds__(kThreads, 2)
   extern __shared__ __align__(16) char smem_raw[];
   SmemMap sm = map_smem(smem_raw, n);
   sm.tr.acc = nullptr;
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / team_size();
   const int64_t nn = (int64_t)n * n;
   Ws w;
   w.base = work + (int64_t)b * dec_work_elems(n);
   w.Q = nn;
   w.ncont = 0;
-  cta_copy(w.slot(0), Ao + b * nn, (int)nn);
-  cta_copy(w.slot(2), Bo + b * nn, (int)nn);
-  cta_copy(w.slot(3), Co + b * nn, (int)nn);
-  __syncthreads();
+  team_copy(w.slot(0), Ao + b * nn, (int)nn);
+  team_copy(w.slot(2), Bo + b * nn, (int)nn);
+  team_copy(w.slot(3), Co + b * nn, (int)nn);
+  team_sync();
   int nc = 0;
   double2* gs = nullptr;
   cta_decimation(n, w, tol, max_iter, nc, &gs, sm);
-  cta_copy(Go + b * nn, gs, (int)nn);
-  if (threadIdx.x == 0 && ncyc) ncyc[b] = nc;
+  team_copy(Go + b * nn, gs, (int)nn);
+  if (lead() && ncyc) ncyc[b] = nc;
+  team_sync();   // no member's shared memory is read any more
 }
 
 cudaError_t launch_decimation_batched(int batch, int n, const double2* Ao, const double2* Bo, const double2* Co,
                                       double2* Go, int* ncyc, double tol, int max_iter, double2* work,
                                       cudaStream_t s) {
-  const size_t smem = engine_smem_bytes(n);
-  cudaError_t e =
-      cudaFuncSetAttribute(k_decimation_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = team_opt_in((const void*)k_decimation_batched);
   if (e != cudaSuccess) return e;
-  k_decimation_batched<<<batch, kThreads, smem, s>>>(n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work);
-  return cudaGetLastError();
+  const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
+  return cudaLaunchKernelEx(&cfg, k_decimation_batched, n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work);
 }
 
 }  // namespace negf

@@ -95,7 +95,7 @@ struct EngineArgs {
   double* ldens; int ldens_stride;
   int* scba_iter; double* scba_err;
   // workspace
-  double2* ws; int64_t ws_per_cta; int64_t Q;  // slot size in complex elements
+  double2* ws; int64_t ws_per_team; int64_t Q;  // slot size in complex elements
   int nmax;                      // max PL/contact PL order over the launch
   int nbl_max;
   int ncont_max;                 // contacts per device, max over the launch
@@ -108,7 +108,16 @@ int64_t engine_slots(int mode, int nbl_max, int ncont_max);
 int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax);
 size_t engine_smem_bytes(int nmax);
 
-cudaError_t launch_engine(const EngineArgs& a, int grid, cudaStream_t s);
+// `teams` teams of `team` CTAs (a thread-block cluster; 1, 2, 4, 8 or 16), one
+// point at a time each
+cudaError_t launch_engine(const EngineArgs& a, int teams, int team, cudaStream_t s);
+
+// The team size for `work` independent problems of block order n, and how
+// many teams of that size run at once (at most max_ctas CTAs on sms SMs).
+struct TeamShape {
+  int team, teams;
+};
+TeamShape team_shape(int work, int n, int max_ctas, int sms);
 
 // CSR -> dense blocks (csr.cu).  Indices 1-based as libNEGF's z_CSR; the
 // outputs are zero-filled staging arrays in the negf_b200_device layout.

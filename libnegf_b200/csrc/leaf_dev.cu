@@ -31,5 +31,9 @@ __device__ void rows_run_r4(const double2* X, double2* Y, const double2* Wm, int
                             const int* perm, double2* stage) {
   gj_rows_update<4, 1, 8>(X, Y, Wm, n, N, k0, K, perm, stage);
 }
+__device__ void rows_run_team(const double2* X, double2* Y, const double2* Wm, int n, int N, int k0, int K,
+                              const int* perm, double2* stage) {
+  gj_rows_update_team(X, Y, Wm, n, N, k0, K, perm, stage);
+}
 
 }  // namespace negf

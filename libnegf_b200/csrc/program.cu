@@ -13,7 +13,7 @@ __device__ int engine_step(const EngineArgs& a, EngineCtl& c, SmemMap& sm) {
     c.open = -1;
   }
   Ws w;
-  w.base = a.ws + (int64_t)blockIdx.x * a.ws_per_cta;
+  w.base = a.ws + (int64_t)(blockIdx.x / team_size()) * a.ws_per_team;
   w.Q = a.Q;
   w.ncont = a.ncont_max;
   w.nbl_max = a.nbl_max;

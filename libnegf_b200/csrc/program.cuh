@@ -173,22 +173,25 @@ __device__ __forceinline__ void set_simple(Op& o, int kind, int m, const double2
 
 // ---------------------------------------------------------------- executor
 // The light operations (everything but products and inversions), executed
-// inside engine_step.
+// inside engine_step.  Elementwise operations are split over the team; sums
+// and maxima over whole blocks are formed by every CTA of the team for
+// itself (the same bits in each, and no exchange).
 __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
   const int tid = threadIdx.x;
+  const int q0 = team_tid(), qs = team_threads();   // elements split over the team
   long long t0 = sm.tr.start();
   switch (o.kind) {
     case K_ESH:
       cta_esh(o.C, o.m, o.n, o.A, o.X, o.alpha, o.flag != 0, o.Y, o.V, o.opa);
       break;
     case K_COPY:
-      cta_copy(o.C, o.A, o.m);
+      team_copy(o.C, o.A, o.m);
       break;
     case K_SUB:
-      for (int q = tid; q < o.m; q += blockDim.x) o.C[q] = csub(o.C[q], o.A[q]);
+      for (int q = q0; q < o.m; q += qs) o.C[q] = csub(o.C[q], o.A[q]);
       break;
     case K_DECUPD:
-      for (int q = tid; q < o.m; q += blockDim.x) {
+      for (int q = q0; q < o.m; q += qs) {
         const double2 s = o.A[q];
         o.C[q] = csub(o.C[q], s);
         o.D[q] = csub(o.D[q], s);
@@ -231,11 +234,11 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
     }
     case K_DOS: {
       const double pi = 3.14159265358979323846;
-      for (int k = tid; k < o.m; k += blockDim.x) o.out[k] = -(1.0 / pi) * o.A[(size_t)k * (o.m + 1)].y;
+      for (int k = q0; k < o.m; k += qs) o.out[k] = -(1.0 / pi) * o.A[(size_t)k * (o.m + 1)].y;
       break;
     }
     case K_SIGDIAG:
-      for (int k = tid; k < o.m; k += blockDim.x) {
+      for (int k = q0; k < o.m; k += qs) {
         const double c = o.cpl[k];
         const double2 v = cscale(c * c, o.A[(size_t)k * (o.m + 1)]);
         if (o.flag == 0) o.C[k] = v;
@@ -244,13 +247,13 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       }
       break;
     case K_SNINIT:
-      for (int q = tid; q < o.m * o.m; q += blockDim.x) {
+      for (int q = q0; q < o.m * o.m; q += qs) {
         const int r = q % o.m, c = q / o.m;
         o.C[q] = (o.A && r == c) ? o.A[r] : cz(0.0, 0.0);
       }
       break;
     case K_SNGAMMA:
-      for (int q = tid; q < o.m * o.m; q += blockDim.x) {
+      for (int q = q0; q < o.m * o.m; q += qs) {
         const int r = q % o.m, c = q / o.m;
         const double2 a1 = o.A[q], b1 = cconj(o.A[(size_t)c + (size_t)r * o.m]);
         const double2 gam = cz(-(a1.y - b1.y), a1.x - b1.x);   // i (S - S^dag)
@@ -258,7 +261,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       }
       break;
     case K_DAGGER:
-      for (int q = tid; q < o.m * o.n; q += blockDim.x) {
+      for (int q = q0; q < o.m * o.n; q += qs) {
         const int r = q % o.m, c = q / o.m;
         o.C[q] = cconj(o.A[(size_t)c + (size_t)r * o.n]);
       }
@@ -305,7 +308,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       // set k summed in its index order, as the reference's accumulation
       // loop (src/iterative.F90:1931-1945); indices past the device skipped
       const double* dos = reinterpret_cast<const double*>(o.A);
-      for (int k = tid; k < o.dd->nldos; k += blockDim.x) {
+      for (int k = q0; k < o.dd->nldos; k += qs) {
         double acc = 0.0;
         for (int q = o.dd->ldos_ptr[k]; q < o.dd->ldos_ptr[k + 1]; ++q) {
           const int i2 = o.dd->ldos_idx[q];
@@ -316,14 +319,14 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       break;
     }
     case K_SUBCOPY:
-      for (int q = tid; q < o.m * o.m; q += blockDim.x) {
+      for (int q = q0; q < o.m * o.m; q += qs) {
         const int r = q % o.m, c = q / o.m;
         o.C[(int64_t)(o.flag + r) + (int64_t)(o.flag + c) * o.ldc] = o.A[q];
       }
       break;
     case K_RESPROBE: {
       double k = 0.0;
-      const double e = cta_inv_probe(o.m, o.A, o.B, sm.main, sm.red, &k);
+      const double e = team_inv_probe(o.m, o.A, o.B, sm.main, sm.main + o.m, sm.maxv, &k);
       if (tid == 0) {
         sm.res[o.slot] = e;
         sm.res[8] = k;
@@ -331,7 +334,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       break;
     }
     case K_EYE:
-      for (int q = tid; q < o.m * o.m; q += blockDim.x)
+      for (int q = q0; q < o.m * o.m; q += qs)
         o.C[q] = make_double2((q % o.m) == (q / o.m) ? 1.0 : 0.0, 0.0);
       break;
     case K_RETCHECK: {
@@ -365,7 +368,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       break;
     }
     case K_ACCUM:
-      for (int q = tid; q < o.m; q += blockDim.x) {
+      for (int q = q0; q < o.m; q += qs) {
         const double2 v = cmul(o.alpha, o.A[q]);
         atomicAdd(&o.C[q].x, v.x);
         atomicAdd(&o.C[q].y, v.y);
@@ -374,7 +377,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
     default:
       break;
   }
-  __syncthreads();
+  team_sync();
   sm.tr.stop(TR_ELEM, t0);
 }
 
@@ -476,7 +479,10 @@ __device__ __forceinline__ const unsigned char* tun_mask_of(const DevDesc* d, in
   return d->tun_mask ? d->tun_mask + d->pstart[bl - 1] : nullptr;
 }
 
-// Fills `o` with the next block operation of this CTA and returns true, or
+// the thread that writes a point's results
+__device__ __forceinline__ bool lead() { return threadIdx.x == 0 && team_rank() == 0; }
+
+// Fills `o` with the next block operation of this team and returns true, or
 // returns false when the work queue is exhausted.
 __device__ __forceinline__ bool next_op(const EngineArgs& a, Prog& s, SmemMap& sm, const Ws& w, Op& o) {
   const double2 one = cz(1, 0), zero = cz(0, 0), mone = cz(-1, 0);
@@ -486,10 +492,10 @@ dispatch:
     case 0:
     for (;;) {
       // ---------------------------------------------------------- next point
-      if (threadIdx.x == 0) *sm.item = atomicAdd(a.counter, 1);
-      __syncthreads();
-      s.p = *sm.item;
-      __syncthreads();
+      if (lead()) *sm.item = atomicAdd(a.counter, 1);
+      team_sync();
+      s.p = team_ld_int(sm.item, 0);
+      team_sync();
       if (s.p >= a.npts) break;
       s.d = a.devs + a.dev_id[s.p];
       s.E = a.energy[s.p];
@@ -502,7 +508,7 @@ dispatch:
         s.ec = cz(s.E, a.energy_im[s.p]);
         s.ecs = s.ec;
       }
-      if (threadIdx.x == 0 && sm.tr.acc) sm.tr.acc[TR_POINTS] += 1;
+      if (lead() && sm.tr.acc) sm.tr.acc[TR_POINTS] += 1;
 
       // ------------------------------------------ contacts (compute_contacts_dns)
       for (s.c = 0; s.c < s.d->ncont; ++s.c) {
@@ -660,7 +666,7 @@ dispatch:
       s.q = 0;                              // pair_of(0) is in effect
       s.fast = (a.mode == MODE_T) && s.d->ncont == 2 && s.npairs == 1 && s.bl1 == 1;
       if (a.mode == MODE_T && s.d->ncont == 1) {
-        if (threadIdx.x == 0 && a.T)
+        if (lead() && a.T)
           for (int q = 0; q < s.npairs; ++q) a.T[(int64_t)s.p * s.npairs + q] = 0.0;
         goto point_done;
       }
@@ -933,7 +939,7 @@ dispatch:
             s.T = fabs(sm.res[1] - sm.res[0]);
           pair_done:
             if (!isfinite(s.T)) put_status(s.st, ST_NONFINITE);
-            if (threadIdx.x == 0 && a.T) a.T[(int64_t)s.p * s.npairs + s.q] = s.T;
+            if (lead() && a.T) a.T[(int64_t)s.p * s.npairs + s.q] = s.T;
             __syncthreads();
           }
           goto point_done;
@@ -1160,7 +1166,7 @@ dispatch:
           o.kind = K_TRACE; o.m = s.d->pl[s.d->cblk[s.c] - 1]; o.A = w.slot(7); o.B = w.slot(8); o.opb = OP_N;
           o.slot = 3; o.mask = nullptr;
           PT_EMIT(s);
-          if (threadIdx.x == 0)
+          if (lead())
             a.curr[(int64_t)s.p * a.curr_stride + s.c] =
                 -(sm.res[2] - a.frm[(int64_t)s.p * a.frm_stride + s.c] * sm.res[3]);
           __syncthreads();
@@ -1171,7 +1177,7 @@ dispatch:
           if (a.ldens) {
             o.kind = K_TRDIAG; o.m = s.d->pl[s.i]; o.A = w.layer(4 + s.par, s.i, s.d->nbl); o.slot = 2;
             PT_EMIT(s);
-            if (threadIdx.x == 0) a.ldens[(int64_t)s.p * a.ldens_stride + s.i] = sm.res[2];
+            if (lead()) a.ldens[(int64_t)s.p * a.ldens_stride + s.i] = sm.res[2];
             __syncthreads();
           }
           if (a.lcurr && s.i + 1 < s.d->nbl) {
@@ -1185,18 +1191,18 @@ dispatch:
             o.kind = K_TRACEC; o.m = s.d->pl[s.i]; o.n = s.d->pl[s.i + 1]; o.A = w.layer(6 + s.par, s.i, s.d->nbl);
             o.B = w.slot(9); o.opb = OP_N; o.slot = 4;                           // Tr(Gn(i,i+1) ESH(i+1,i))
             PT_EMIT(s);
-            if (threadIdx.x == 0) a.lcurr[(int64_t)s.p * a.lcurr_stride + s.i] = -(sm.res[3] - sm.res[5]);
+            if (lead()) a.lcurr[(int64_t)s.p * a.lcurr_stride + s.i] = -(sm.res[3] - sm.res[5]);
             __syncthreads();
           }
         }
-      if (threadIdx.x == 0) {
+      if (lead()) {
         if (a.scba_iter) a.scba_iter[s.p] = s.sit;
         if (a.scba_err) a.scba_err[s.p] = s.err;
       }
       goto point_done;
 
     point_done:
-      if (threadIdx.x == 0) {
+      if (lead()) {
         if (a.ncyc) a.ncyc[s.p] = s.ncyc;
         if (a.status) a.status[s.p] = s.st;
       }

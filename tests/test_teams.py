@@ -1,0 +1,89 @@
+"""Team sizes: a problem is solved by one CTA or by a cluster of up to 16 (few
+problems in a call), and the results are the same bits either way; products
+split over CTAs by output tiles."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from libnegf_b200 import generators as G
+from libnegf_b200 import native
+
+pytestmark = pytest.mark.gpu
+
+
+def _dp(t):
+    return ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_double))
+
+
+def _ip(t):
+    return ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_int32))
+
+
+@pytest.mark.parametrize("dev", [
+    lambda: G.transport_c0(nbl=3, n=33, seed=1),
+    lambda: G.transport_c0(nbl=3, n=65, seed=1),                  # first order with leaves
+    lambda: G.transport_c1(nbl=3, n=129, seed=2),                 # one row and column past two tiles
+    lambda: G.uneven([40, 90, 17, 70], seed=3),
+], ids=["n33", "n65", "n129_S", "uneven"])
+def test_engine_results_do_not_depend_on_the_team_size(gpu_ctx, dev):
+    did = gpu_ctx.upload(dev())
+    E = np.linspace(-1.5, 1.5, 300)                                # more points than CTAs: teams of one
+    try:
+        T, nc, st = gpu_ctx.transmission(did, E, eta=1e-3)
+        Td, dos, _, _ = gpu_ctx.transmission_dos(did, E, eta=1e-3, dos_delta=1e-3)
+        for m in (1, 30, 80):                                      # teams of up to 16, 8 and 2 .. 4
+            a = gpu_ctx.transmission(did, E[:m], eta=1e-3)
+            b = gpu_ctx.transmission_dos(did, E[:m], eta=1e-3, dos_delta=1e-3)
+            assert np.array_equal(a[0], T[:m]) and np.array_equal(a[1], nc[:m]) and np.array_equal(a[2], st[:m])
+            assert np.array_equal(b[0], Td[:m]) and np.array_equal(b[1], dos[:m])
+    finally:
+        gpu_ctx.release(did)
+
+
+@pytest.mark.parametrize("n", [64, 65, 96, 127, 129, 256, 257, 513])
+def test_inverse_bits_do_not_depend_on_the_team_size(n):
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    batch = 300 if n <= 256 else 60
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.randn((batch, n, n), dtype=torch.complex128, device="cuda", generator=g)
+    X, X1 = torch.zeros_like(A), torch.zeros_like(A[:1])
+    info = torch.full((batch,), -1, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.negf_b200_zinv_work_bytes(batch, n), dtype=torch.uint8, device="cuda")
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    w = ctypes.c_void_p(work.data_ptr())
+    assert L.negf_b200_zinv_batched(batch, n, _dp(A), _dp(X), _ip(info), w, s) == 0
+    assert int(info.abs().max()) == 0
+    assert L.negf_b200_zinv_batched(1, n, _dp(A), _dp(X1), _ip(info), w, s) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(X1[0], X[0])
+    A[0, :, 3] = 0.0                                               # a zero row: an exact zero pivot, seen by every member
+    assert L.negf_b200_zinv_batched(1, n, _dp(A), _dp(X1), _ip(info), w, s) == 0
+    torch.cuda.synchronize()
+    assert int(info[0]) > 0
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(1, 1, 1, 1), (64, 65, 17, 2), (63, 130, 64, 1), (300, 20, 33, 5),
+                                         (129, 129, 129, 200)])
+@pytest.mark.parametrize("dagger", [0, 1, 2])
+def test_split_products(m, n, k, batch, dagger):
+    """Against torch: each side's rounding of a K-term complex sum is within
+    2 (K + 2) u |A||B| elementwise."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    r = lambda *s: torch.randn(s, dtype=torch.complex128, device="cuda", generator=g)
+    A = r(batch, m, k) if dagger == 1 else r(batch, k, m)         # column major: reversed index order
+    B = r(batch, k, n) if dagger == 2 else r(batch, n, k)
+    C = torch.zeros((batch, n, m), dtype=torch.complex128, device="cuda")
+    one, zero = (ctypes.c_double * 2)(1, 0), (ctypes.c_double * 2)(0, 0)
+    rc = L.negf_b200_zgemm_batched(batch, m, n, k, one, _dp(A), 2 * m * k, _dp(B), 2 * k * n, zero, _dp(C),
+                                   2 * m * n, dagger, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    a = A.conj() if dagger == 1 else A.transpose(1, 2)
+    b = B.conj() if dagger == 2 else B.transpose(1, 2)
+    err = (C.transpose(1, 2) - a @ b).abs()
+    bound = 4 * (k + 2) * 2.0 ** -53 * (a.abs() @ b.abs())
+    torch.cuda.synchronize()
+    assert bool((err <= bound).all())
