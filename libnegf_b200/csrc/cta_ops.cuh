@@ -37,10 +37,8 @@ constexpr int kStages = NEGF_GEMM_STAGES;   // cp.async ring depth
 static_assert(TK == 8 || TK == 16, "K tile of 8 or 16");
 constexpr int kStageElems = TK * A_LD + TN * B_LD;
 constexpr int kGemmSmemBytes = kStages * kStageElems * 16;
-#ifndef NEGF_SMALL_INV_MAX
-#define NEGF_SMALL_INV_MAX 64
-#endif
-constexpr int kSmallInvMax = NEGF_SMALL_INV_MAX;   // n <= kSmallInvMax: whole matrix in shared memory
+constexpr int kSmallInvMax = 64;       // n <= kSmallInvMax: the whole matrix in one register panel
+constexpr int kPanelMax = 256;         // largest order of the register panels
 
 // ---------------------------------------------------------------- complex
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -59,6 +57,19 @@ __device__ __forceinline__ double2 crecip(double2 z) {
     double r = z.x / z.y, den = z.y + z.x * r;
     return make_double2(r / den, -1.0 / den);
   }
+}
+// 1/z as conj(z) / |z|^2 with z scaled by a power of two to |z| ~ 1 (no
+// overflow or underflow of the square): one reciprocal in the dependent
+// chain where Smith's algorithm has two divisions, for the pivots, whose
+// latency every elimination step waits for.
+__device__ __forceinline__ double2 crecip_scaled(double2 z) {
+  const int hx = __double2hiint(z.x) & 0x7ff00000, hy = __double2hiint(z.y) & 0x7ff00000;
+  if (max(hx, hy) == 0x7ff00000) return crecip(z);                       // Inf, NaN: 1/Inf = 0 as ever
+  const int e = min(max(max(hx, hy) >> 20, 23), 2023);                   // biased exponent
+  const double sc = __hiloint2double((2046 - e) << 20, 0);               // 2^(1023 - e)
+  const double x = z.x * sc, y = z.y * sc;
+  const double r = __drcp_rn(fma(x, x, y * y)) * sc;
+  return make_double2(x * r, -y * r);
 }
 __device__ __forceinline__ double cabs1(double2 z) { return fabs(z.x) + fabs(z.y); }
 __device__ __forceinline__ double cabs(double2 z) { return hypot(z.x, z.y); }
@@ -828,10 +839,6 @@ struct InvScratch {
   Trace tr;
 };
 
-// Pivot search on a column in shared memory: rows [j, n) of col[] -> index
-// of max |Re|+|Im| (first occurrence, as izamax).  All threads call; the
-// caller puts a barrier between two calls (s.redv / s.redi are reused):
-// gj_step's capture and update barriers do.
 // (key, row) of the warp's best candidate: the largest key, the lowest row
 // among equal keys.  Keys are the bits of |Re|+|Im| plus one (that value is
 // >= 0, so its bit pattern orders like it; 0 = no candidate, NaN never
@@ -842,90 +849,6 @@ __device__ __forceinline__ void warp_argmax_key(unsigned long long& key, int& bi
   const unsigned long long wkey = ((unsigned long long)hi << 32) | lo;
   bi = (int)__reduce_min_sync(0xffffffffu, (key == wkey) ? (unsigned)bi : 0xffffffffu);
   key = wkey;
-}
-
-__device__ __forceinline__ int cta_pivot(const double2* col, int j, int n, InvScratch& s) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long key = 0ull;
-  int bi = n;
-  for (int i = j + threadIdx.x; i < n; i += blockDim.x) {
-    const double v = cabs1(col[i]);
-    const unsigned long long kk = (v >= 0.0) ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
-    if (kk > key) { key = kk; bi = i; }
-  }
-  warp_argmax_key(key, bi);
-  unsigned long long* redk = reinterpret_cast<unsigned long long*>(s.redv);
-  if (lane == 0) { redk[warp] = key; s.redi[warp] = bi; }
-  __syncthreads();
-  // every warp reduces the per-warp candidates itself (no second barrier)
-  const int nw = (int)(blockDim.x >> 5);
-  key = (lane < nw) ? redk[lane] : 0ull;
-  bi = (lane < nw) ? s.redi[lane] : n;
-  warp_argmax_key(key, bi);
-  return bi;
-}
-
-// One Gauss-Jordan step on a column panel P (n rows x w cols, ld = n) held in
-// shared memory: pivot row j (global row index), panel column jj.
-// f[] (n) and rowj[] (2w + 1) are shared scratch.  Returns the pivot row chosen.
-// Three barriers per step: pivot search (1), exchange + capture (1),
-// scale + rank-1 update (1).
-// Thread layout of gj_step's update: rows spread over threads, columns
-// looped inside (computed once per inversion: integer divides).
-struct GjLayout {
-  int rows_per_pass, cgroups, i0, c0;
-  __device__ __forceinline__ explicit GjLayout(int n) {
-    rows_per_pass = blockDim.x >= (unsigned)n ? n : (int)blockDim.x;
-    cgroups = max(1, (int)blockDim.x / rows_per_pass);
-    i0 = threadIdx.x % rows_per_pass;
-    c0 = threadIdx.x / rows_per_pass;
-  }
-};
-
-__device__ __forceinline__ int gj_step(double2* P, int n, int w, int j, int jj, double2* f, double2* rowj,
-                                    InvScratch& s, int* info, const GjLayout& lay) {
-  const double2* colj = P + (size_t)jj * n;
-  int p = cta_pivot(colj, j, n, s);
-  if (p >= n) p = j;
-  // Read-only capture: f = pivot column after the exchange of rows j and p,
-  // rowj = new row j (old row p), rowo = new row p (old row j).
-  double2* rowo = rowj + w;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int src = (i == j) ? p : ((i == p) ? j : i);
-    f[i] = colj[src];
-  }
-  for (int c = threadIdx.x; c < w; c += blockDim.x) {
-    rowj[c] = P[p + (size_t)c * n];
-    rowo[c] = P[j + (size_t)c * n];
-  }
-  // one thread forms the reciprocal of the pivot (three divides), published
-  // by the capture barrier: computed by every thread it was most of a step
-  if (threadIdx.x == 0) rowj[2 * w] = crecip(colj[p]);
-  __syncthreads();
-  const double2 piv = f[j];
-  if (piv.x == 0.0 && piv.y == 0.0 && threadIdx.x == 0 && *info == 0) *info = j + 1;
-  const double2 d = rowj[2 * w];
-  const int rows_per_pass = lay.rows_per_pass, cgroups = lay.cgroups, i0 = lay.i0, c0 = lay.c0;
-  if (c0 < cgroups)
-    for (int i = i0; i < n; i += rows_per_pass) {
-      const double2 fi = f[i];
-      const double2 fd = cmul(fi, d);
-      for (int c = c0; c < w; c += cgroups) {
-        double2* el = P + i + (size_t)c * n;
-        double2 v;
-        if (i == j) {
-          v = (c == jj) ? d : cmul(rowj[c], d);
-        } else if (c == jj) {
-          v = make_double2(-fd.x, -fd.y);
-        } else {
-          const double2 base = (i == p) ? rowo[c] : *el;
-          v = csub(base, cmul(fd, rowj[c]));
-        }
-        *el = v;
-      }
-    }
-  __syncthreads();
-  return p;
 }
 
 // Workspace (complex elements) for cta_zinv of order n: two n x n buffers.
@@ -1079,6 +1002,210 @@ __device__ __forceinline__ void gj_reg_steps(double2 (&x)[R][W], int n, int c0, 
   }
 }
 
+// Gauss-Jordan elimination of the columns [c0, c0 + w) of a column-major
+// matrix of n <= 32 RL rows, the panel in registers: lane l of every warp
+// holds rows l + 32 r (r < RL) of the CW panel columns wp + 8 c, w <= 8 CW.
+// src / dst point at the panel's first column (they may be the same).  Rows
+// never move between registers: lg[r] is the position a row has after the
+// exchanges so far (every warp keeps it), and the rows go there when the
+// panel is stored.
+//
+// Per step the warp that owns the pivot column searches the pivot alone (max
+// |Re|+|Im| over the positions j.., the lowest position on a tie: izamax),
+// forms its reciprocal d, and publishes both with the column f in shared
+// memory before the step's one barrier.  In every warp the pivot's lane
+// leaves its row in shared memory for the other lanes, and all update their
+// columns, x - (f d) row.  The published column has -1 in the pivot row, and
+// that row restarts from 0, so that it becomes row d by the same update; the
+// pivot column restarts from 0, with 1 in the pivot row, likewise.  The owner
+// of the next column updates that column first and publishes it; its other
+// columns wait until after the barrier, when another warp is the owner.
+//
+// What bounds it: the serial chain of a step (barrier, pivot row, update of
+// RL entries, search, reciprocal) beside 64 FMAs per thread (290 cycles of
+// the FP64 pipe for 8 warps): 1450, 1550 and 2040 cycles a step measured at
+// n = 64, 128 and 256.  One inverse on an otherwise idle GPU took 295, 671
+// and 2170 us before the panels and the teams (rows per thread, every warp's
+// candidates and rows exchanged through memory, two serial divisions per
+// pivot; a panel of n <= 64 kept in shared memory), 70, 258 and 767 us now;
+// 296 of them at n = 256 3.72 -> 3.34 ms.
+// The columns of a warp are unrolled, so a step's code is reused by the 8
+// steps of one slot; with every step unrolled the loop ran out of the
+// instruction cache for a third of the time.
+//
+// WHOLE: the panel is the whole matrix (w = n): the columns also go to their
+// places, so dst gets the inverse.
+struct PanelPivot {
+  double2 d;
+  int lane, slot, pos, pad;
+};
+
+// Compile-time integer arguments of generic lambdas, and a loop over them.
+template <int V>
+struct IntC {
+  static constexpr int value = V;
+};
+template <int I, int N, typename F>
+__device__ __forceinline__ void unroll_steps(F& f) {
+  if constexpr (I < N) {
+    f(IntC<I>());
+    unroll_steps<I + 1, N>(f);
+  }
+}
+
+template <int RL, int CW, bool WHOLE>
+__device__ __forceinline__ void gj_panel(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
+  constexpr int NR = 32 * RL, NW = kThreads / 32;
+  constexpr bool kScaleRow = RL > CW;   // scale the row's CW entries by d, else the column's RL
+  constexpr unsigned kAll = 0xffffffffu;
+  // the CTA's main shared-memory region, named here so that its accesses
+  // compile to shared-memory instructions
+  extern __shared__ __align__(16) char smem_raw[];
+  double2* const colb = reinterpret_cast<double2*>(smem_raw);             // [3][NR]
+  double2* const rowb = colb + 3 * NR;                                    // [NW][CW]
+  PanelPivot* const pivs = reinterpret_cast<PanelPivot*>(rowb + NW * CW); // [2]
+  int* const piv = s.piv;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  double2* const prow = rowb + wp * CW;
+  double2 x[RL][CW];
+  int lg[RL];
+#pragma unroll
+  for (int r = 0; r < RL; ++r) {
+    const int row = lane + 32 * r;
+    lg[r] = row < n ? row : -1;
+#pragma unroll
+    for (int c = 0; c < CW; ++c) {
+      const int k = wp + c * NW;
+      x[r][c] = (row < n && k < w) ? src[row + (size_t)k * n] : make_double2(0.0, 0.0);
+    }
+  }
+  // one entry of the next pivot column: a candidate from position j on (NaN
+  // never wins; the lowest position on a tie); at = 32 position + slot
+  auto candidate = [](double2 v, int at, int j, double& ba, int& best) {
+    const double a = cabs1(v);
+    if (at >= 32 * j && (a > ba || (a == ba && at < best))) {
+      ba = a;
+      best = at;
+    }
+  };
+  // Stores column slot C as the pivot column JJ in col and publishes its
+  // pivot.  Each lane forms the reciprocal of its own best candidate beside
+  // the warp's reductions, and the winner publishes its own.
+  auto publish = [&](auto c_c, int JJ, double2* col, PanelPivot* out) {
+    constexpr int C = decltype(c_c)::value;
+    const int j = c0 + JJ;
+    double ba = -1.0;
+    int best = 0;
+#pragma unroll
+    for (int r = 0; r < RL; ++r) {
+      col[lane + 32 * r] = x[r][C];
+      candidate(x[r][C], 32 * lg[r] + r, j, ba, best);
+    }
+    double2 pv = col[lane + 32 * (best & 31)];
+    double2 d = crecip_scaled(pv);
+    // the bits of a value >= 0 order like it; + 1: 0 = no candidate
+    const unsigned long long key = ba >= 0.0 ? (unsigned long long)__double_as_longlong(ba) + 1ull : 0ull;
+    const unsigned hi = (unsigned)(key >> 32);
+    const unsigned mhi = __reduce_max_sync(kAll, hi);
+    unsigned who = __ballot_sync(kAll, hi == mhi);
+    if (__popc(who) > 1) {   // decided by the low words, then by the position
+      const unsigned lo = hi == mhi ? (unsigned)key : 0u;
+      const unsigned mlo = __reduce_max_sync(kAll, lo);
+      const bool cand = hi == mhi && lo == mlo && key != 0ull;
+      const unsigned mi = __reduce_min_sync(kAll, cand ? (unsigned)best : 0xffffffffu);
+      who = __ballot_sync(kAll, cand && (unsigned)best == mi);
+      if (who == 0u) {   // every entry is NaN: the row at position j
+        bool here = false;
+#pragma unroll
+        for (int r = 0; r < RL; ++r)
+          if (lg[r] == j) { here = true; best = j * 32 + r; }
+        pv = col[lane + 32 * (best & 31)];
+        d = crecip_scaled(pv);
+        who = __ballot_sync(kAll, here);
+      }
+    }
+    const int winner = __ffs(who) - 1;
+    if (lane == winner) {
+      *out = PanelPivot{d, lane, best & 31, best >> 5, 0};
+      col[lane + 32 * (best & 31)] = make_double2(-1.0, 0.0);
+      piv[j] = best >> 5;
+      if (pv.x == 0.0 && pv.y == 0.0 && *s.flag == 0) *s.flag = j + 1;
+    }
+#pragma unroll
+    for (int r = 0; r < RL; ++r) x[r][C] = make_double2(lane == winner && r == (best & 31) ? 1.0 : 0.0, 0.0);
+  };
+  if (wp == 0) publish(IntC<0>(), 0, colb, pivs);
+  __syncthreads();
+  int b = 0;   // step mod 3
+  // the steps JJ = JN - 1 whose next column JN is slot c of its warp
+  auto slot_steps = [&](auto c_c) {
+    constexpr int c = decltype(c_c)::value;
+#pragma unroll 1
+    for (int q = (c == 0 ? 1 : 0); q < NW + (c == CW - 1 ? 1 : 0); ++q) {   // (the last step has no next column)
+      const int JN = c * NW + q, JJ = JN - 1, j = c0 + JJ, bn = b == 2 ? 0 : b + 1;
+      if (JJ >= w) return;
+      const PanelPivot pv = pivs[JJ & 1];
+      const double2* const col = colb + b * NR + lane;
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+        if (r == pv.slot && lane == pv.lane) {
+#pragma unroll
+          for (int k = 0; k < CW; ++k) {
+            prow[k] = x[r][k];
+            x[r][k] = make_double2(0.0, 0.0);
+          }
+        }
+#pragma unroll
+      for (int r = 0; r < RL; ++r)   // the exchange of positions j and pos
+        lg[r] = (lane == pv.lane && r == pv.slot) ? j : (lg[r] == j ? pv.pos : lg[r]);
+      double2 f[kScaleRow ? 1 : RL];
+      if constexpr (!kScaleRow) {
+#pragma unroll
+        for (int r = 0; r < RL; ++r) f[r] = cmul(col[32 * r], pv.d);
+      }
+      __syncwarp();
+      auto update = [&](auto k_c) {
+        constexpr int k = decltype(k_c)::value;
+        double2 p = prow[k];
+        if constexpr (kScaleRow) p = cmul(p, pv.d);
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+          const double2 fr = kScaleRow ? col[32 * r] : f[kScaleRow ? 0 : r];
+          x[r][k].x = fma(-fr.x, p.x, fma(fr.y, p.y, x[r][k].x));
+          x[r][k].y = fma(-fr.x, p.y, fma(-fr.y, p.x, x[r][k].y));
+        }
+      };
+      auto others = [&](auto k_c) {
+        if constexpr (decltype(k_c)::value != c) update(k_c);
+      };
+      const bool next = wp == q && JN < w;
+      update(c_c);
+      if (next) publish(c_c, JN, colb + bn * NR, pivs + (JN & 1));
+      else unroll_steps<0, CW>(others);
+      __syncthreads();
+      if (next) {
+        unroll_steps<0, CW>(others);
+        __syncwarp();   // prow is read before the next step's pivot lane writes it
+      }
+      b = bn;
+    }
+  };
+  unroll_steps<0, CW>(slot_steps);
+  int* const dest = s.cperm;
+  if constexpr (WHOLE) gj_block_perm(dest, piv, n, 0, n);   // internal column k is output column dest[k]
+#pragma unroll
+  for (int c = 0; c < CW; ++c) {
+    const int k = wp + c * NW;
+    if (k < w) {
+      double2* out = dst + (size_t)(WHOLE ? dest[k] : k) * n;
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+        if (lg[r] >= 0) out[lg[r]] = x[r][c];
+    }
+  }
+  __syncthreads();
+}
+
 // Delayed update of the tree's lowest levels done inside a leaf, rows in
 // registers: y(i, c) = [i outside the pivot rows [k0, k0+kw)] T(perm[i], c)
 // + sum_k Wc(i, k) T(perm[k0+k], c), c < tw.  Wc (kw columns, kw <= KW)
@@ -1136,7 +1263,7 @@ __device__ __forceinline__ void leaf_apply(double2 (&y)[R][W], const double2* Wc
 // columns) and b: factorise a; apply a's pivots to b; factorise b; apply
 // b's pivots to a.  That is the lowest node of the delayed-update tree,
 // done without a GEMM call (whose 64 x 64 tile would be mostly empty at
-// K <= 8).  The arithmetic per element of a pivot step is that of gj_step.
+// K <= 8).
 // `sh` holds a LeafShared<W>.  Pivots go to s.piv[c0 + jj]; a zero pivot
 // sets *s.flag.  Rows i >= n of the register panel hold zeros and take part
 // in nothing.
@@ -1352,11 +1479,14 @@ __device__ __forceinline__ void gj_rows_update_team(const double2* X, double2* Y
   }
 }
 
-// gj_leaf4 for 1, 2 and 4 rows per thread, each compiled out of line in
-// leaf_dev.cu (see gemm_run); gj_rows_update likewise (rows_run_*: n <= 128
+// The panels and gj_leaf4, each compiled out of line in leaf_dev.cu (see
+// gemm_run); gj_rows_update likewise (rows_run_*: n <= 128
 // two threads per row, n <= 256 one, n <= 512 two rows per thread, n <= 1024
 // four).
-__device__ void leaf_run_r1(double2* X, int n, int c0, int w, double2* sh, InvScratch& s);
+__device__ void panel_run_w32(const double2* A, double2* X, int n, int c0, int w, InvScratch& s);
+__device__ void panel_run_w64(const double2* A, double2* X, int n, int c0, int w, InvScratch& s);
+__device__ void panel_run_4(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s);
+__device__ void panel_run_8(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s);
 __device__ void leaf_run_r2(double2* X, int n, int c0, int w, double2* sh, InvScratch& s);
 __device__ void leaf_run_r4(double2* X, int n, int c0, int w, double2* sh, InvScratch& s);
 __device__ void rows_run_t2(const double2* X, double2* Y, const double2* Wm, int n, int N, int k0, int K,
@@ -1375,9 +1505,9 @@ __device__ void rows_run_team(const double2* X, double2* Y, const double2* Wm, i
 // zinv_ws_elems(n) elements.  `smem` holds kSmemMain bytes.
 //
 // n <= kSmallInvMax: Gauss-Jordan with partial pivoting on the whole matrix
-// in shared memory.  Larger n: the same elimination with delayed updates
-// over a perfect binary tree of 2^d column leaves.  A leaf (up to 32
-// columns, gj_leaf4, panel in registers, its own two lowest nodes inside)
+// in one register panel.  Larger n: the same elimination with delayed
+// updates over a perfect binary tree of 2^d column leaves.  A leaf (32 or 16
+// columns, gj_panel; above kPanelMax 16 or 8, gj_leaf4)
 // is factorised once every earlier pivot has been applied to it; after the
 // left half of a node is done, its pivots are applied to the right half,
 // and after the right half, the right half's pivots to the left half, each
@@ -1407,7 +1537,8 @@ struct InvProg {
   int n, d, nl, k, l, phase, rpt;
   int leaf_open;            // a leaf was handed out: its pivots are still to be shared with the team
   int flip_ta, flip_half;   // parity flip owed by the last update
-  double2* X;               // leaf step: panel base, first column, width
+  const double2* src;       // leaf step: matrix read, matrix written, first column, width
+  double2* X;
   int c0, w;
   long long t0;
   // row-owner update step: Y(:, 0:N) from X, Wm, pivot rows [rk0, rk0 + rK)
@@ -1419,46 +1550,25 @@ struct InvProg {
 
 enum InvStep : int { INV_DONE = 0, INV_LEAF = 1, INV_APPLY = 2, INV_ROWS = 3 };
 
-// Small orders entirely; larger ones: set up the tree.  No copy of A: a
+// Sets up one whole-matrix panel (small orders) or the tree.  No copy of A: a
 // leaf's columns are read from A by the first update that targets them (or,
-// for leaf 0, copied out before its factorisation).  Returns 1 when the
-// inversion is already complete.
-static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* A, double2* out, double2* ws, double2* smem,
+// for leaf 0, by its factorisation).
+static __device__ __noinline__ void inv_begin(InvProg& ip, int n, const double2* A, double2* out, double2* ws, double2* smem,
                                       InvScratch& s) {
   if (threadIdx.x == 0) *s.flag = 0;
   __syncthreads();
   ip.A = A; ip.out = out; ip.n = n;
-  if (n <= kSmallInvMax) {
-    if (team_rank() != 0) {   // one CTA holds the whole matrix; the others take over its info
-      team_sync();
-      if (threadIdx.x == 0) *s.flag = team_ld_int(s.flag, 0);
-      __syncthreads();
-      return 1;
-    }
-    double2* P = smem;
-    double2* f = smem + (size_t)n * n;
-    double2* rowj = f + n;
-    long long t0 = s.tr.start();
-    cta_copy(P, A, n * n);
-    __syncthreads();
-    const GjLayout lay(n);
-    for (int j = 0; j < n; ++j) {
-      int p = gj_step(P, n, n, j, j, f, rowj, s, s.flag, lay);
-      if (threadIdx.x == 0) s.piv[j] = p;
-    }
-    __syncthreads();
-    s.tr.stop(TR_INV_PANEL, t0);
-    t0 = s.tr.start();
-    gj_col_perm(s.cperm, s.piv, n);
-    copy_colperm(out, P, n, s.cperm, threadIdx.x, blockDim.x);
-    team_sync();
-    s.tr.stop(TR_INV_OTHER, t0);
-    return 1;
+  ip.k = 0; ip.l = 0; ip.phase = 0; ip.flip_half = 0; ip.leaf_open = 0;
+  if (n <= kSmallInvMax) {   // one panel, no tree
+    ip.d = ip.nl = 0;
+    ip.src = A; ip.X = out; ip.c0 = 0; ip.w = n;
+    return;
   }
-  // leaves are factorised in registers: rpt rows per thread, four sub-leaves
-  // of 8/rpt columns
+  // leaf width: the register panels hold 4 or 8 rows per lane and 4 or 2
+  // columns per warp; above kPanelMax gj_leaf4 with rpt rows per thread and
+  // four sub-leaves of 8 / rpt columns
   const int rpt = (n + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int wmax = rpt <= 1 ? 32 : (rpt <= 2 ? 16 : 8);
+  const int wmax = n <= 128 ? 32 : (n <= kPanelMax ? 16 : (rpt == 2 ? 16 : 8));
   int d = 0;
   while ((n + (1 << d) - 1) >> d > wmax) ++d;
   ip.rpt = rpt <= 1 ? 1 : (rpt <= 2 ? 2 : 4);
@@ -1466,12 +1576,10 @@ static __device__ __noinline__ int inv_begin(InvProg& ip, int n, const double2* 
   ip.nl = 1 << d;
   ip.buf[0] = ws;
   ip.buf[1] = ws + (size_t)n * n;
-  ip.k = 0; ip.l = 0; ip.phase = 0; ip.flip_half = 0; ip.leaf_open = 0;
   // per-leaf location (nl <= n): 0 / 1 = buffer, kInA = still only in A (read in place, never written)
   unsigned char* par = reinterpret_cast<unsigned char*>(s.cperm);
   for (int k = threadIdx.x; k < ip.nl; k += blockDim.x) par[k] = kInA;
   __syncthreads();
-  return 0;
 }
 
 // Next step of the tree: INV_LEAF (ip.X, ip.c0, ip.w set), INV_APPLY (GEMM
@@ -1484,11 +1592,19 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
     if (team_size() > 1) {
       team_sync();
       if (team_rank() != 0) {
-        for (int j = threadIdx.x; j < ip.w; j += blockDim.x) s.piv[ip.c0 + j] = team_ld_int(s.piv + ip.c0 + j, 0);
+        if (ip.nl > 0)
+          for (int j = threadIdx.x; j < ip.w; j += blockDim.x)
+            s.piv[ip.c0 + j] = team_ld_int(s.piv + ip.c0 + j, 0);
         if (threadIdx.x == 0) *s.flag = team_ld_int(s.flag, 0);
       }
       __syncthreads();
     }
+  }
+  if (ip.nl == 0) {   // one panel
+    if (ip.phase) return INV_DONE;
+    ip.phase = 1;
+    ip.leaf_open = 1;
+    return INV_LEAF;
   }
   if (ip.flip_half) {   // the update just run moved its target leaves to the other buffer
     for (int q = threadIdx.x; q < ip.flip_half; q += blockDim.x) {
@@ -1505,14 +1621,18 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
       const int k = ip.k;
       ip.c0 = (k * n) >> d;
       ip.w = (((k + 1) * n) >> d) - ip.c0;
+      ip.src = ip.buf[par[k] == kInA ? 0 : par[k]];
       if (par[k] == kInA) {   // only leaf 0: every later leaf is the target of an update first
-        const long long t0 = s.tr.start();
-        // CTA 0 alone reads it before the next team_sync
-        if (team_rank() == 0) cta_copy(ip.buf[0] + (size_t)ip.c0 * n, ip.A + (size_t)ip.c0 * n, n * ip.w);
+        if (n <= kPanelMax) {
+          ip.src = ip.A;
+        } else {              // gj_leaf4 works in place; CTA 0 alone reads the copy before the next team_sync
+          const long long t0 = s.tr.start();
+          if (team_rank() == 0) cta_copy(ip.buf[0] + (size_t)ip.c0 * n, ip.A + (size_t)ip.c0 * n, n * ip.w);
+          s.tr.stop(TR_INV_OTHER, t0);
+        }
         __syncthreads();
         if (threadIdx.x == 0) par[k] = 0;
         __syncthreads();
-        s.tr.stop(TR_INV_OTHER, t0);
       }
       ip.X = ip.buf[par[k]];
       ip.phase = 1;
@@ -1561,6 +1681,7 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
 // Final column unscramble; returns info.
 static __device__ __noinline__ int inv_end(InvProg& ip, InvScratch& s) {
   const int n = ip.n;
+  if (ip.nl == 0) return 0;   // the panel wrote the inverse
   unsigned char* par = reinterpret_cast<unsigned char*>(s.cperm);
   // every leaf went through one update per level: all sit in buf[par[0]]
   long long t0 = s.tr.start();
@@ -1576,7 +1697,10 @@ static __device__ __noinline__ int inv_end(InvProg& ip, InvScratch& s) {
 // The leaf step of ip (INV_LEAF): CTA 0 of the team.
 __device__ __forceinline__ void leaf_run(const InvProg& ip, double2* smem, InvScratch& s) {
   if (team_rank() != 0) return;
-  if (ip.rpt == 1) leaf_run_r1(ip.X, ip.n, ip.c0, ip.w, smem, s);
+  if (ip.n <= 32) panel_run_w32(ip.src, ip.X, ip.n, ip.c0, ip.w, s);
+  else if (ip.n <= kSmallInvMax) panel_run_w64(ip.src, ip.X, ip.n, ip.c0, ip.w, s);
+  else if (ip.n <= 128) panel_run_4(ip.src, ip.X, ip.n, ip.c0, ip.w, s);
+  else if (ip.n <= kPanelMax) panel_run_8(ip.src, ip.X, ip.n, ip.c0, ip.w, s);
   else if (ip.rpt == 2) leaf_run_r2(ip.X, ip.n, ip.c0, ip.w, smem, s);
   else leaf_run_r4(ip.X, ip.n, ip.c0, ip.w, smem, s);
 }
@@ -1598,22 +1722,21 @@ __device__ __forceinline__ void rows_run(const InvProg& ip, double2* smem, const
 __device__ __forceinline__ int cta_zinv(int n, const double2* A, double2* out, double2* ws, double2* smem,
                                         InvScratch& s) {
   InvProg ip;
-  if (!inv_begin(ip, n, A, out, ws, smem, s)) {
-    for (;;) {
-      const int step = inv_next(ip, smem, s);
-      if (step == INV_DONE) break;
-      if (step == INV_LEAF) {
-        const long long t0 = s.tr.start();
-        leaf_run(ip, smem, s);
-        s.tr.stop(TR_INV_PANEL, t0);
-      } else if (step == INV_ROWS) {
-        rows_run(ip, smem, s);
-      } else {
-        gemm_run(reinterpret_cast<const GemmDesc*>(smem + kGemmDescOffset), smem);
-      }
+  inv_begin(ip, n, A, out, ws, smem, s);
+  for (;;) {
+    const int step = inv_next(ip, smem, s);
+    if (step == INV_DONE) break;
+    if (step == INV_LEAF) {
+      const long long t0 = s.tr.start();
+      leaf_run(ip, smem, s);
+      s.tr.stop(TR_INV_PANEL, t0);
+    } else if (step == INV_ROWS) {
+      rows_run(ip, smem, s);
+    } else {
+      gemm_run(reinterpret_cast<const GemmDesc*>(smem + kGemmDescOffset), smem);
     }
-    inv_end(ip, s);
   }
+  inv_end(ip, s);
   const int info = *s.flag;
   __syncthreads();
   return info;

@@ -1,12 +1,21 @@
-// Gauss-Jordan leaf factorisations (gj_leaf4) and row-owner node updates
+// Gauss-Jordan panels (gj_panel, gj_leaf4) and row-owner node updates
 // (gj_rows_update), compiled in a translation
 // unit of their own (see gemm_run in cta_ops.cuh).
 #include "cta_ops.cuh"
 
 namespace negf {
 
-__device__ void leaf_run_r1(double2* X, int n, int c0, int w, double2* sh, InvScratch& s) {
-  gj_leaf4<1, 8>(X, n, c0, w, sh, s);
+__device__ void panel_run_w32(const double2* A, double2* X, int n, int c0, int w, InvScratch& s) {
+  gj_panel<1, 4, true>(A, X, n, c0, w, s);
+}
+__device__ void panel_run_w64(const double2* A, double2* X, int n, int c0, int w, InvScratch& s) {
+  gj_panel<2, 8, true>(A, X, n, c0, w, s);
+}
+__device__ void panel_run_4(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
+  gj_panel<4, 4, false>(src + (size_t)c0 * n, dst + (size_t)c0 * n, n, c0, w, s);
+}
+__device__ void panel_run_8(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
+  gj_panel<8, 2, false>(src + (size_t)c0 * n, dst + (size_t)c0 * n, n, c0, w, s);
 }
 __device__ void leaf_run_r2(double2* X, int n, int c0, int w, double2* sh, InvScratch& s) {
   gj_leaf4<2, 4>(X, n, c0, w, sh, s);

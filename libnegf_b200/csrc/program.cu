@@ -49,12 +49,8 @@ __device__ int engine_step(const EngineArgs& a, EngineCtl& c, SmemMap& sm) {
       return STEP_GEMM;
     }
     if (o.kind == K_ZINV) {
-      if (inv_begin(c.ip, o.m, o.A, o.C, w.inv(), sm.main, sm.inv)) {   // small order: done
-        if (tid == 0) sm.ires[0] = *sm.inv.flag;
-        __syncthreads();
-      } else {
-        c.in_inv = 1;
-      }
+      inv_begin(c.ip, o.m, o.A, o.C, w.inv(), sm.main, sm.inv);
+      c.in_inv = 1;
       continue;
     }
     exec_light(o, sm);

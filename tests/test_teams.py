@@ -87,3 +87,63 @@ def test_split_products(m, n, k, batch, dagger):
     bound = 4 * (k + 2) * 2.0 ** -53 * (a.abs() @ b.abs())
     torch.cuda.synchronize()
     assert bool((err <= bound).all())
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 128, 129, 255, 256, 257, 511, 512, 513])
+def test_inverse_at_the_panel_edges(n):
+    """Against LAPACK on well-conditioned matrices: the residual A X - I of
+    Gauss-Jordan with partial pivoting is within c(n) u kappa(A), with c(n)
+    at most 8 n (n terms per entry, a few roundings each); rows in reverse
+    order make every pivot an exchange, equal rows up to sign make ties."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.randn((3, n, n), dtype=torch.complex128, device="cuda", generator=g) / max(1.0, n ** 0.5)
+    A = A + 4.0 * torch.eye(n, dtype=A.dtype, device="cuda")
+    A[1] = A[1].flip(1)                                            # column major: rows reversed
+    if n > 2:
+        A[2] = torch.eye(n, dtype=A.dtype, device="cuda").flip(1) * 2.0
+        A[2, :, 0] = 1.0                                           # a row of ties with the entries below
+        A[2, 0, :] = 1.0
+        A[2] += 3.0 * torch.eye(n, dtype=A.dtype, device="cuda")
+    X = torch.zeros_like(A)
+    info = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.negf_b200_zinv_work_bytes(3, n), dtype=torch.uint8, device="cuda")
+    assert L.negf_b200_zinv_batched(3, n, _dp(A), _dp(X), _ip(info), ctypes.c_void_p(work.data_ptr()),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    assert int(info.abs().max()) == 0
+    for q in range(3):
+        a = A[q].cpu().numpy().T
+        x = X[q].cpu().numpy().T
+        k = np.linalg.cond(a)
+        assert np.abs(a @ x - np.eye(n)).max() <= 8 * n * 2.0 ** -53 * max(k, 1.0)
+
+
+@pytest.mark.parametrize("n", [20, 50, 100, 200, 400])
+def test_inverse_of_non_finite_matrices(n):
+    """NaN never wins a pivot search and reaches the result; an infinite
+    diagonal entry is a pivot whose reciprocal is 0: its row and column of
+    the inverse vanish and the rest is the inverse without them."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 4 * np.sqrt(n) * np.eye(n)
+    A = np.stack([a, a])
+    A[0, n // 2, n // 3] = np.nan
+    A[1, n // 2, n // 2] = np.inf
+    dA = torch.from_numpy(np.ascontiguousarray(A.transpose(0, 2, 1))).cuda()
+    X = torch.zeros_like(dA)
+    info = torch.zeros(2, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.negf_b200_zinv_work_bytes(2, n), dtype=torch.uint8, device="cuda")
+    assert L.negf_b200_zinv_batched(2, n, _dp(dA), _dp(X), _ip(info), ctypes.c_void_p(work.data_ptr()),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    x = X.cpu().numpy().transpose(0, 2, 1)
+    assert np.isnan(x[0]).any()
+    keep = np.arange(n) != n // 2
+    ref = np.linalg.inv(a[np.ix_(keep, keep)])
+    if np.isfinite(x[1]).all():                                    # (n > 64: products with Inf make NaN)
+        assert np.abs(x[1][np.ix_(keep, keep)] - ref).max() <= 1e-12
+    else:
+        assert n > 64
