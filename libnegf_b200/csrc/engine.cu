@@ -155,7 +155,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_engine(EngineArgs a) {
     const int st = engine_step(a, c, smap);
     if (st == STEP_DONE) break;
     if (st == STEP_GEMM) {
-      cta_gemm_body<OP_RT, OP_RT, EPI_RT>(reinterpret_cast<const GemmDesc*>(smap.main + kGemmDescOffset), smap.main);
+      const GemmDesc* d = reinterpret_cast<const GemmDesc*>(smap.main + kGemmDescOffset);
+      if (d->tile == kTile) cta_gemm_body<OP_RT, OP_RT, EPI_RT, kTile>(d, smap.main);
+      else gemm_run_small(d, smap.main);
     } else if (st == STEP_ROWS) {
       rows_run(c.ip, smap.main, smap.inv);
     } else {
@@ -249,29 +251,52 @@ static int resident_teams(int team) {
   return known[dev][lg] - 1;
 }
 
-// A team of G CTAs speeds up a problem's products by its output tiles over G;
-// the elimination's leaves stay with one CTA.  So few problems take large
-// teams (T of n = 384, 6 layers, 12 points: 825 -> 194 ms in teams of 16;
-// n = 97, 48 points: 47 -> 33 ms in teams of 4), a full GPU takes one CTA per
-// problem (n = 256, 296 points: teams of 2 lose the overlap of two problems'
-// phases on an SM), and a call just above a whole number of waves takes a team size
-// that splits its last wave (n = 256, 320 points with DOS: 773 -> 693 ms).
-// The cost: waves x time of a point, with the share of an SM that a second CTA
-// costs the first (measured 1.7 for two products at n >= 256).
+// The team size whose measured cost for `work` problems is least.  Three
+// figures make up the cost (T solves of orders 32 .. 384, 1 .. 400 points,
+// every team size timed):
+//  - the time of one problem alone, relative to one CTA.  Products and
+//    updates split over the team, the elimination's panels do not: order 256
+//    takes 0.58, 0.33, 0.23, 0.18 of the time in teams of 2, 4, 8, 16 (171 ->
+//    29 ms for a point of 3 layers), order 128 0.64 .. 0.32, order 64 0.71 at
+//    best (one panel, four output tiles), order 32 nothing;
+//  - the slowdown when the teams share SMs.  Two CTAs on an SM run 1.6 times
+//    as long as one, as soon as any SM has two; teams of 4 and more leave the
+//    FP64 pipe less idle time to share (2.05 times with every SM holding two)
+//    and are placed two to an SM before every SM has one;
+//  - the waves.  One or two CTAs per problem wait for the last wave; larger
+//    teams drift apart over the waves and lose less.
+// Examples (us per call, one CTA per problem -> chosen): n = 384, 12 points
+// 825000 -> 195000 (16); n = 97, 48 points 28200 -> 16050 (4); n = 256, 320
+// points 400000 -> 362000 (2); 296 points stay with one CTA (278000; 304000
+// in teams of 2).
 TeamShape team_shape(int work, int n, int max_ctas, int sms) {
+  static const double kAlone[3][5] = {{1.0, 0.90, 0.71, 0.70, 0.70},    // n <= 80
+                                      {1.0, 0.64, 0.45, 0.385, 0.32},   // n <= 150
+                                      {1.0, 0.58, 0.33, 0.225, 0.18}};
+  const double* alone = kAlone[n <= 80 ? 0 : (n <= 150 ? 1 : 2)];
   TeamShape best{1, std::max(1, std::min(work, max_ctas))};
-  const int tile = (n + TM - 1) / TM, tiles = tile * tile;
   double best_cost = 0.0;
-  for (int team = 1; team <= 16; team *= 2) {
-    if (team > 1 && team > tiles) break;
+  for (int lg = 0; lg <= 4; ++lg) {
+    const int team = 1 << lg;
+    if (team > 1 && n <= 40) break;
     int teams = std::min(max_ctas / team, team > 1 ? resident_teams(team) : max_ctas);
     if (teams < 1) break;
+    const double waves = (double)work / teams;
     teams = std::min(teams, std::max(1, work));
-    const double share = teams * team <= sms ? 1.0 : 1.0 + 0.7 * (std::min(teams * team, 2 * sms) - sms) / sms;
-    const double serial = n <= 64 ? 0.6 : 0.15;
-    const double point = serial + (1.0 - serial) * ((tiles + team - 1) / team) / tiles;
-    const double cost = (double)((work + teams - 1) / teams) * share * point;
-    if (team == 1 || cost < 0.95 * best_cost) {
+    const double c = 148.0 * teams * team / sms;   // CTAs per 148 SMs
+    double share = 1.0, w = 1.0;
+    if (team <= 2) {
+      if (c > 148.0) share = 1.6;
+      const double whole = (double)(int)waves, frac = waves - whole;
+      if (waves > 1.0) w = whole + (frac > 0.0 ? (team == 1 ? 0.4 + 0.45 * frac : 0.3 + 0.55 * frac) : 0.0);
+    } else {
+      if (c > 192.0) share = 1.42 + 0.63 * (c - 192.0) / 104.0;
+      else if (c > 148.0) share = 1.35 + 0.07 * (c - 148.0) / 44.0;
+      else if (c > 100.0) share = 1.0 + 0.35 * (c - 100.0) / 48.0;
+      if (waves > 1.0) w = 0.35 + 0.68 * waves;
+    }
+    const double cost = alone[lg] * share * w;
+    if (lg == 0 || cost < best_cost) {
       best = TeamShape{team, teams};
       best_cost = cost;
     }
@@ -292,7 +317,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   Operand Bo = (dagger == 2) ? opC(B + b * sB, n) : opN(B + b * sB, k);
   const GemmDesc* d = gemm_desc_publish(m, n, k, Ao, Bo, epi_store(C + b * sC, m, alpha, beta), sm.main, blockIdx.x,
                                         gridDim.x);
-  cta_gemm_body<OP_RT, OP_RT, EPI_RT>(d, sm.main);
+  if (d->tile == kTile) cta_gemm_body<OP_RT, OP_RT, EPI_RT, kTile>(d, sm.main);
+  else gemm_run_small(d, sm.main);
 }
 
 // SMs of the current device, asked once per device.
@@ -318,8 +344,9 @@ cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, 
   // 1604 -> 111 us); with 1184 products and more one CTA runs through all
   // tiles of a product, loading the next tile's operands behind this one's
   // epilogue.
-  const int64_t tiles = (int64_t)((m + TM - 1) / TM) * ((n + TN - 1) / TN);
   const int64_t want = (8LL * device_sms() + batch - 1) / batch;
+  const int T = gemm_tile(m, n, (int)std::min<int64_t>(want, 1 << 20));
+  const int64_t tiles = (int64_t)((m + T - 1) / T) * ((n + T - 1) / T);
   const int split = (int)std::max<int64_t>(1, std::min(tiles, want));
   for (int b0 = 0; b0 < batch; b0 += 65535) {   // gridDim.y limit
     const int nb = std::min(65535, batch - b0);
