@@ -258,33 +258,69 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
                                                 std::to_string(negf::kMaxOrder));
   int st = sync_descs(ctx);
   if (st) return st;
-  negf::TeamShape ts = negf::team_shape(a.npts, sh.nmax, max_ctas(ctx), std::max(1, ctx->sms));
-  const int64_t per = negf::engine_ws_elems(a.mode, sh.nbl_max, sh.ncont_max, sh.nmax);
-  if (ctx->ws_limit > 0) {
-    // fewer resident teams when the workspace would exceed the limit (the persistent
-    // kernel still runs every point); not even one: refuse
-    const size_t per_bytes = (size_t)per * sizeof(double2);
-    const size_t fit = ctx->ws_limit > 256 ? (ctx->ws_limit - 256) / per_bytes : 0;
-    if (fit < 1)
-      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(per_bytes) +
-                                                    " bytes) exceeds the workspace limit");
-    if ((size_t)ts.teams > fit) ts = negf::team_shape((int)fit, sh.nmax, max_ctas(ctx), std::max(1, ctx->sms));
-  }
-  // counter lives at the start of the workspace allocation
-  const size_t need = 256 + (size_t)ts.teams * per * sizeof(double2);
-  st = grow(ctx, &ctx->ws, &ctx->ws_bytes, need);
-  if (st) return st;
-  a.counter = reinterpret_cast<int*>(ctx->ws);
-  a.ws = reinterpret_cast<double2*>(reinterpret_cast<char*>(ctx->ws) + 256);
-  a.ws_per_team = per;
   a.Q = (int64_t)sh.nmax * sh.nmax;
   a.nmax = sh.nmax;
   a.nbl_max = sh.nbl_max;
   a.ncont_max = sh.ncont_max;
   a.devs = ctx->d_descs;
   a.trace = ctx->trace ? ctx->d_trace : nullptr;
-  CK(cudaMemsetAsync(a.counter, 0, sizeof(int), s));
-  cudaError_t e = negf::launch_engine(a, ts.teams, ts.team, s);
+  const int sms = std::max(1, ctx->sms), ctas = max_ctas(ctx);
+  const size_t per = (size_t)negf::engine_ws_elems(a.mode, sh.nbl_max, sh.ncont_max, sh.nmax) * sizeof(double2);
+  const size_t per_c = (size_t)negf::engine_contact_elems(sh.nmax) * sizeof(double2);
+  negf::TeamShape ts = negf::team_shape(a.npts, sh.nmax, ctas, sms);
+  // A call whose (point, contact) pairs do not fill the GPU many times over is
+  // split: the contacts are independent of one another and most of a point's
+  // time, and two launches give each part its own number of teams (n = 384, 12
+  // points: 201 -> 144 ms; n = 256, 320 points with DOS: 692 -> 634).  The pairs' self-energies (and kept surface GFs) live in
+  // the workspace between the launches.
+  const int64_t pairs = (int64_t)a.npts * sh.ncont_max;
+  const size_t blocks = (size_t)pairs * a.Q * sizeof(double2) * (a.acc_lc ? 2 : 1);
+  const size_t ints = (2 * (size_t)pairs * sizeof(int) + 255) / 256 * 256;
+  bool split = sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && blocks <= (size_t(4) << 30);
+  negf::TeamShape tc{1, 1};
+  if (split) tc = negf::team_shape((int)pairs, sh.nmax, ctas, sms);
+  if (ctx->ws_limit > 0) {
+    // fewer resident teams when the workspace would exceed the limit (the persistent
+    // kernel still runs every point); not even one: refuse
+    const size_t room = ctx->ws_limit > 256 ? ctx->ws_limit - 256 : 0;
+    if (split && room < ints + blocks + std::max(per, per_c)) split = false;
+    const size_t rest = split ? room - ints - blocks : room;
+    const size_t fit = rest / per;
+    if (fit < 1)
+      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(per) +
+                                                    " bytes) exceeds the workspace limit");
+    if ((size_t)ts.teams > fit) ts = negf::team_shape((int)fit, sh.nmax, ctas, sms);
+    if (split && (size_t)tc.teams > rest / per_c) tc = negf::team_shape((int)(rest / per_c), sh.nmax, ctas, sms);
+  }
+  // the queue heads lie at the start of the workspace allocation
+  size_t need = (size_t)ts.teams * per;
+  if (split) need = std::max(need, (size_t)tc.teams * per_c) + ints + blocks;
+  st = grow(ctx, &ctx->ws, &ctx->ws_bytes, 256 + need);
+  if (st) return st;
+  char* p = reinterpret_cast<char*>(ctx->ws);
+  CK(cudaMemsetAsync(p, 0, 2 * sizeof(int), s));
+  a.counter = reinterpret_cast<int*>(p);
+  p += 256;
+  cudaError_t e = cudaSuccess;
+  if (split) {
+    a.ncyc_pc = reinterpret_cast<int*>(p);
+    a.st_pc = a.ncyc_pc + pairs;
+    p += ints;
+    a.sig_pc = reinterpret_cast<double2*>(p);
+    a.gs_pc = a.acc_lc ? a.sig_pc + pairs * a.Q : nullptr;
+    p += blocks;
+    a.ws = reinterpret_cast<double2*>(p);
+    a.part = negf::PART_CONTACTS;
+    a.ws_per_team = (int64_t)(per_c / sizeof(double2));
+    e = negf::launch_engine(a, tc.teams, tc.team, s);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
+    ++ctx->launches;
+    a.part = negf::PART_SWEEPS;
+    a.counter += 1;
+  }
+  a.ws = reinterpret_cast<double2*>(p);
+  a.ws_per_team = (int64_t)(per / sizeof(double2));
+  e = negf::launch_engine(a, ts.teams, ts.team, s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
   ++ctx->launches;
   return NEGF_B200_OK;

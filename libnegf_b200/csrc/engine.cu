@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_engine(EngineArgs a) {
   const long long t_all = a.trace ? clock64() : 0;
   EngineCtl c;
   c.prog.pc = 0;
+  c.prog.p = 0;
   c.in_inv = 0;
   c.open = -1;
   for (;;) {
@@ -171,6 +172,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_engine(EngineArgs a) {
     if (threadIdx.x < TR_NPHASE) atomicAdd(a.trace + threadIdx.x, (unsigned long long)smap.tr.acc[threadIdx.x]);
   }
 }
+
+int64_t engine_contact_elems(int nmax) { return (int64_t)S_SIG * nmax * nmax; }
 
 int64_t engine_slots(int mode, int nbl_max, int ncont_max) {
   int64_t s = S_SIG + ncont_max;
@@ -415,6 +418,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   w.base = work + (int64_t)b * dec_work_elems(n);
   w.Q = nn;
   w.ncont = 0;
+  w.sigp = w.gsp = nullptr;
   team_copy(w.slot(0), Ao + b * nn, (int)nn);
   team_copy(w.slot(2), Bo + b * nn, (int)nn);
   team_copy(w.slot(3), Co + b * nn, (int)nn);

@@ -53,8 +53,19 @@ struct DevDesc {
   int has_ss, pad3;
 };
 
+// What an engine launch does of its points: everything, or the two launches
+// of a split call: the contacts (an item of the queue is one contact of one
+// point: its surface GF and self-energy, left in sig_pc / gs_pc with the
+// iteration count and the status), then the rest of every point.
+enum Part : int { PART_ALL = 0, PART_CONTACTS = 1, PART_SWEEPS = 2 };
+
 struct EngineArgs {
   int mode;
+  int part;
+  double2* sig_pc;               // npts x ncont_max slots of Q elements (split calls)
+  double2* gs_pc;                // the same for the kept surface GFs, or null
+  int* ncyc_pc;                  // npts x ncont_max
+  int* st_pc;
   int npts;
   const int* dev_id;
   const double* energy;
@@ -106,6 +117,7 @@ struct EngineArgs {
 // Workspace slot counts of the engine for a launch
 int64_t engine_slots(int mode, int nbl_max, int ncont_max);
 int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax);
+int64_t engine_contact_elems(int nmax);   // workspace of a team in a PART_CONTACTS launch
 size_t engine_smem_bytes(int nmax);
 
 // `teams` teams of `team` CTAs (a thread-block cluster; 1, 2, 4, 8 or 16), one

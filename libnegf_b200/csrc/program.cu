@@ -17,6 +17,7 @@ __device__ int engine_step(const EngineArgs& a, EngineCtl& c, SmemMap& sm) {
   w.Q = a.Q;
   w.ncont = a.ncont_max;
   w.nbl_max = a.nbl_max;
+  bind_point(a, w, c.prog.p);
   for (;;) {
     if (c.in_inv) {
       const int st = inv_next(c.ip, sm.main, sm.inv);

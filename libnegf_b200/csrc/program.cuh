@@ -75,19 +75,21 @@ enum : int { S_INV = 12, S_SIG = 15 };
 
 struct Ws {
   double2* base;
+  double2* sigp;   // the current point's contact self-energies, a slot each
+  double2* gsp;    // its kept surface GFs where they live outside the team's slots (split calls), or null
   int64_t Q;
   int ncont;
   int nbl_max;
   __device__ double2* slot(int k) const { return base + (int64_t)k * Q; }
   __device__ double2* inv() const { return slot(S_INV); }
-  __device__ double2* sig(int c) const { return slot(S_SIG + c); }
+  __device__ double2* sig(int c) const { return sigp + (int64_t)c * Q; }
   __device__ double2* layer(int arr, int i, int nbl) const { return slot(S_SIG + ncont + arr * nbl + i); }
   // T / DOS: Gr(cb,cb) kept at the block of contact c during the forward sweep
   __device__ double2* keep(int c) const { return slot(S_SIG + ncont + nbl_max + c); }
   // density: the surface GF of contact c, kept for the outer blocks
-  __device__ double2* gskeep(int c) const { return slot(S_SIG + 2 * ncont + nbl_max + c); }
+  __device__ double2* gskeep(int c) const { return gsp ? gsp + (int64_t)c * Q : slot(S_SIG + 2 * ncont + nbl_max + c); }
   // GN: the same, after the eight layer arrays
-  __device__ double2* gnkeep(int c) const { return slot(S_SIG + ncont + 8 * nbl_max + c); }
+  __device__ double2* gnkeep(int c) const { return gsp ? gsp + (int64_t)c * Q : slot(S_SIG + ncont + 8 * nbl_max + c); }
 };
 
 // ---------------------------------------------------------------- ops
@@ -385,6 +387,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
 struct Prog {
   int pc;
   int p;                // current point
+  int cend;             // contacts of this item end here
   const DevDesc* d;
   double E;
   int st, ncyc;
@@ -479,12 +482,23 @@ __device__ __forceinline__ const unsigned char* tun_mask_of(const DevDesc* d, in
   return d->tun_mask ? d->tun_mask + d->pstart[bl - 1] : nullptr;
 }
 
+// Where point p's contact blocks live: in the team's slots, or (split calls)
+// in the call's own array.
+__device__ __forceinline__ void bind_point(const EngineArgs& a, Ws& w, int p) {
+  w.sigp = w.slot(S_SIG);
+  w.gsp = nullptr;
+  if (a.part != PART_ALL) {
+    w.sigp = a.sig_pc + (int64_t)p * a.ncont_max * a.Q;
+    if (a.gs_pc) w.gsp = a.gs_pc + (int64_t)p * a.ncont_max * a.Q;
+  }
+}
+
 // the thread that writes a point's results
 __device__ __forceinline__ bool lead() { return threadIdx.x == 0 && team_rank() == 0; }
 
 // Fills `o` with the next block operation of this team and returns true, or
 // returns false when the work queue is exhausted.
-__device__ __forceinline__ bool next_op(const EngineArgs& a, Prog& s, SmemMap& sm, const Ws& w, Op& o) {
+__device__ __forceinline__ bool next_op(const EngineArgs& a, Prog& s, SmemMap& sm, Ws& w, Op& o) {
   const double2 one = cz(1, 0), zero = cz(0, 0), mone = cz(-1, 0);
   double mx;
 dispatch:
@@ -496,7 +510,13 @@ dispatch:
       team_sync();
       s.p = team_ld_int(sm.item, 0);
       team_sync();
+      s.c = 0;
+      if (a.part == PART_CONTACTS) {   // an item is one contact of a point
+        s.c = s.p % a.ncont_max;
+        s.p /= a.ncont_max;
+      }
       if (s.p >= a.npts) break;
+      bind_point(a, w, s.p);
       s.d = a.devs + a.dev_id[s.p];
       s.E = a.energy[s.p];
       s.st = ST_OK;
@@ -508,10 +528,12 @@ dispatch:
         s.ec = cz(s.E, a.energy_im[s.p]);
         s.ecs = s.ec;
       }
-      if (lead() && sm.tr.acc) sm.tr.acc[TR_POINTS] += 1;
+      if (lead() && sm.tr.acc && a.part != PART_CONTACTS) sm.tr.acc[TR_POINTS] += 1;
 
       // ------------------------------------------ contacts (compute_contacts_dns)
-      for (s.c = 0; s.c < s.d->ncont; ++s.c) {
+      if (a.part == PART_CONTACTS && s.c >= s.d->ncont) continue;   // this device has fewer contacts
+      s.cend = (a.part == PART_CONTACTS) ? s.c + 1 : (a.part == PART_SWEEPS ? 0 : s.d->ncont);
+      for (; s.c < s.cend; ++s.c) {
         s.L = s.d->L[s.c];
         s.ncb = s.d->pl[s.d->cblk[s.c] - 1];
         if (a.sgf_in && a.sgf_in[(int64_t)s.p * a.ncont_max + s.c] >= 0) {
@@ -651,6 +673,19 @@ dispatch:
         set_gemm(o, s.ncb, s.ncb, s.L, w.slot(2), s.ncb, OP_N, w.slot(1), s.L, OP_N, w.sig(s.c), s.ncb, one, zero);
         PT_EMIT(s);
       }
+
+      if (a.part == PART_CONTACTS) {
+        if (lead()) {
+          a.ncyc_pc[(int64_t)s.p * a.ncont_max + s.cend - 1] = s.ncyc;
+          a.st_pc[(int64_t)s.p * a.ncont_max + s.cend - 1] = s.st;
+        }
+        continue;
+      }
+      if (a.part == PART_SWEEPS)
+        for (s.c = 0; s.c < s.d->ncont; ++s.c) {
+          s.ncyc += a.ncyc_pc[(int64_t)s.p * a.ncont_max + s.c];
+          put_status(s.st, a.st_pc[(int64_t)s.p * a.ncont_max + s.c]);
+        }
 
       // ------------------------------------------------ transmission bookkeeping
       // calculate_transmissions (src/iterative.F90:1669-1780): the 2-contact

@@ -147,3 +147,54 @@ def test_inverse_of_non_finite_matrices(n):
         assert np.abs(x[1][np.ix_(keep, keep)] - ref).max() <= 1e-12
     else:
         assert n > 64
+
+
+def test_split_calls_match_one_launch(gpu_ctx):
+    """Calls with few points run the contacts of all points first, then their
+    sweeps (two launches); a workspace limit that leaves no room for the
+    contacts' blocks keeps them in one.  The same bits, for devices with
+    different numbers of contacts in one call, terminals, dephasing and the
+    density matrix with its outer blocks."""
+    d2, d3 = G.transport_c0(nbl=4, n=20, seed=5), G.uneven([20, 12, 33, 20], seed=6, cblk=[1, 3, 4])
+    d1 = G.transport_c0(nbl=3, n=20, seed=7, cblk=[1])
+    hs = [gpu_ctx.upload(d) for d in (d2, d3, d1)]
+    ids = np.tile(np.asarray(hs, dtype=np.int32), 5)
+    E = np.linspace(-1.2, 1.2, ids.size)
+    z, w = np.array([0.1 + 0.3j, -0.4 + 0.1j]), np.array([0.5 + 0.1j, 0.2 - 0.3j])
+    frm = np.stack([np.linspace(1, 0, 5), np.linspace(0, 1, 5)], axis=1)
+
+    def solve():
+        out = [gpu_ctx.transmission_dos(hs[1], E, eta=1e-3, dos_delta=1e-3),
+               gpu_ctx.transmissions(hs[1], E, [(1, 2), (2, 3)], eta=1e-3)]
+        mw = gpu_ctx.meir_wingreen(hs[0], E[:5], frm, coupling=0.1, eta=1e-3)
+        (d, u, l), (dc, cd), nc, st = gpu_ctx.density_neq(hs[0], E[:1], [1.0], frm[:1], eta=1e-3)
+        (rd, ru, rl), (rdc, rcd), rnc, rst = gpu_ctx.density(hs[0], z[:1], w[:1])
+        flat = [x for o in out for x in o if x is not None] + [mw[k] for k in sorted(mw)]
+        return flat + d + u + l + dc + cd + [nc, st] + rd + ru + rl + rdc + rcd + [rnc, rst]
+
+    try:
+        gpu_ctx.set_options(schedule=1, scba_niter=3)
+        n0 = gpu_ctx.launch_count()
+        a = solve()
+        split = gpu_ctx.launch_count() - n0
+        # one team's slots of the largest call (the lesser sweeps: 15 + 2 + 8 x 4 + 2 slots of order 33)
+        gpu_ctx.set_workspace_limit(256 + 17 * 53 * 33 * 33)
+        n0 = gpu_ctx.launch_count()
+        b = solve()
+        assert gpu_ctx.launch_count() - n0 < split
+        assert len(a) == len(b) and all(np.array_equal(x, y) for x, y in zip(a, b))
+        gpu_ctx.set_workspace_limit(0)
+        # 1, 2 and 3 contacts in one call
+        T, dos, nc, st = gpu_ctx.transmission_dos(ids[ids != hs[2]], E[ids != hs[2]], eta=1e-3, dos_delta=1e-3)
+        for h in hs[:2]:
+            k = ids[ids != hs[2]] == h
+            T1, dos1, nc1, st1 = gpu_ctx.transmission_dos(h, E[ids == h], eta=1e-3, dos_delta=1e-3)
+            assert np.array_equal(T[k], T1) and np.array_equal(dos[k][:, :dos1.shape[1]], dos1)
+            assert np.array_equal(nc[k], nc1) and np.array_equal(st[k], st1)
+        T3, dos3, nc3, st3 = gpu_ctx.transmission_dos(hs[2], E, eta=1e-3, dos_delta=1e-3, ni=1, nf=1)
+        assert np.all(T3 == 0.0) and np.all(st3 == 0) and np.all(nc3 > 0)
+    finally:
+        gpu_ctx.set_workspace_limit(0)
+        gpu_ctx.set_options()
+        for h in hs:
+            gpu_ctx.release(h)
