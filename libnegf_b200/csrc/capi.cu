@@ -251,12 +251,63 @@ int max_ctas(negf_b200_ctx* ctx) {
   return std::max(1, per_sm * ctx->sms);
 }
 
-// Runs one launch with device-resident inputs/outputs (all pointers device).
-int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cudaStream_t s) {
+// The launches of an engine call and its workspace.
+struct EnginePlan {
+  negf::TeamShape ts, tc;        // whole points (or their sweeps); contacts
+  bool split;                    // two launches: contacts, then sweeps
+  size_t per, per_c;             // bytes of a team's slots in each
+  size_t ints, blocks;           // bytes kept between the two launches
+  size_t need;                   // of the whole workspace
+};
+
+int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, bool outer, EnginePlan& pl) {
   if (sh.nmax > negf::kMaxOrder)
     return fail(ctx, NEGF_B200_ERR_BAD_ARG, "block order " + std::to_string(sh.nmax) + " exceeds " +
                                                 std::to_string(negf::kMaxOrder));
-  int st = sync_descs(ctx);
+  const int sms = std::max(1, ctx->sms), ctas = max_ctas(ctx);
+  pl.per = (size_t)negf::engine_ws_elems(mode, sh.nbl_max, sh.ncont_max, sh.nmax) * sizeof(double2);
+  pl.per_c = (size_t)negf::engine_contact_elems(sh.nmax) * sizeof(double2);
+  pl.ts = negf::team_shape(npts, sh.nmax, ctas, sms);
+  // A call whose (point, contact) pairs do not fill the GPU many times over is
+  // split: the contacts are independent of one another and most of a point's
+  // time, and two launches give each part its own number of teams (n = 384, 12
+  // points: 201 -> 144 ms; n = 256, 320 points with DOS: 692 -> 634).  The
+  // pairs' self-energies (and kept surface GFs) live in the workspace between
+  // the launches.
+  const int64_t pairs = (int64_t)npts * sh.ncont_max;
+  pl.blocks = (size_t)pairs * sh.nmax * sh.nmax * sizeof(double2) * (outer ? 2 : 1);
+  pl.ints = (2 * (size_t)pairs * sizeof(int) + 255) / 256 * 256;
+  pl.split = sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && pl.blocks <= (size_t(4) << 30);
+  pl.tc = negf::TeamShape{1, 1};
+  if (pl.split) pl.tc = negf::team_shape((int)pairs, sh.nmax, ctas, sms);
+  if (ctx->ws_limit > 0) {
+    // fewer resident teams when the workspace would exceed the limit (the persistent
+    // kernel still runs every point); not even one: refuse
+    const size_t room = ctx->ws_limit > 256 ? ctx->ws_limit - 256 : 0;
+    if (pl.split && room < pl.ints + pl.blocks + std::max(pl.per, pl.per_c)) pl.split = false;
+    const size_t rest = pl.split ? room - pl.ints - pl.blocks : room;
+    const size_t fit = rest / pl.per;
+    if (fit < 1)
+      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(pl.per) +
+                                                    " bytes) exceeds the workspace limit");
+    if ((size_t)pl.ts.teams > fit) pl.ts = negf::team_shape((int)fit, sh.nmax, ctas, sms);
+    if (pl.split && (size_t)pl.tc.teams > rest / pl.per_c)
+      pl.tc = negf::team_shape((int)(rest / pl.per_c), sh.nmax, ctas, sms);
+  }
+  pl.need = (size_t)pl.ts.teams * pl.per;
+  if (pl.split) pl.need = std::max(pl.need, (size_t)pl.tc.teams * pl.per_c) + pl.ints + pl.blocks;
+  pl.need += 256;
+  return NEGF_B200_OK;
+}
+
+// Runs one call with device-resident inputs/outputs (all pointers device).
+int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cudaStream_t s) {
+  EnginePlan pl;
+  int st = plan_engine(ctx, a.mode, a.npts, sh, a.acc_lc != nullptr, pl);
+  if (st) return st;
+  st = sync_descs(ctx);
+  if (st) return st;
+  st = grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
   if (st) return st;
   a.Q = (int64_t)sh.nmax * sh.nmax;
   a.nmax = sh.nmax;
@@ -264,63 +315,31 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
   a.ncont_max = sh.ncont_max;
   a.devs = ctx->d_descs;
   a.trace = ctx->trace ? ctx->d_trace : nullptr;
-  const int sms = std::max(1, ctx->sms), ctas = max_ctas(ctx);
-  const size_t per = (size_t)negf::engine_ws_elems(a.mode, sh.nbl_max, sh.ncont_max, sh.nmax) * sizeof(double2);
-  const size_t per_c = (size_t)negf::engine_contact_elems(sh.nmax) * sizeof(double2);
-  negf::TeamShape ts = negf::team_shape(a.npts, sh.nmax, ctas, sms);
-  // A call whose (point, contact) pairs do not fill the GPU many times over is
-  // split: the contacts are independent of one another and most of a point's
-  // time, and two launches give each part its own number of teams (n = 384, 12
-  // points: 201 -> 144 ms; n = 256, 320 points with DOS: 692 -> 634).  The pairs' self-energies (and kept surface GFs) live in
-  // the workspace between the launches.
-  const int64_t pairs = (int64_t)a.npts * sh.ncont_max;
-  const size_t blocks = (size_t)pairs * a.Q * sizeof(double2) * (a.acc_lc ? 2 : 1);
-  const size_t ints = (2 * (size_t)pairs * sizeof(int) + 255) / 256 * 256;
-  bool split = sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && blocks <= (size_t(4) << 30);
-  negf::TeamShape tc{1, 1};
-  if (split) tc = negf::team_shape((int)pairs, sh.nmax, ctas, sms);
-  if (ctx->ws_limit > 0) {
-    // fewer resident teams when the workspace would exceed the limit (the persistent
-    // kernel still runs every point); not even one: refuse
-    const size_t room = ctx->ws_limit > 256 ? ctx->ws_limit - 256 : 0;
-    if (split && room < ints + blocks + std::max(per, per_c)) split = false;
-    const size_t rest = split ? room - ints - blocks : room;
-    const size_t fit = rest / per;
-    if (fit < 1)
-      return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(per) +
-                                                    " bytes) exceeds the workspace limit");
-    if ((size_t)ts.teams > fit) ts = negf::team_shape((int)fit, sh.nmax, ctas, sms);
-    if (split && (size_t)tc.teams > rest / per_c) tc = negf::team_shape((int)(rest / per_c), sh.nmax, ctas, sms);
-  }
-  // the queue heads lie at the start of the workspace allocation
-  size_t need = (size_t)ts.teams * per;
-  if (split) need = std::max(need, (size_t)tc.teams * per_c) + ints + blocks;
-  st = grow(ctx, &ctx->ws, &ctx->ws_bytes, 256 + need);
-  if (st) return st;
+  // the queue heads lie at the start of the workspace
   char* p = reinterpret_cast<char*>(ctx->ws);
   CK(cudaMemsetAsync(p, 0, 2 * sizeof(int), s));
   a.counter = reinterpret_cast<int*>(p);
   p += 256;
   cudaError_t e = cudaSuccess;
-  if (split) {
+  if (pl.split) {
     a.ncyc_pc = reinterpret_cast<int*>(p);
-    a.st_pc = a.ncyc_pc + pairs;
-    p += ints;
+    a.st_pc = a.ncyc_pc + (int64_t)a.npts * sh.ncont_max;
+    p += pl.ints;
     a.sig_pc = reinterpret_cast<double2*>(p);
-    a.gs_pc = a.acc_lc ? a.sig_pc + pairs * a.Q : nullptr;
-    p += blocks;
+    a.gs_pc = a.acc_lc ? a.sig_pc + (int64_t)a.npts * sh.ncont_max * a.Q : nullptr;
+    p += pl.blocks;
     a.ws = reinterpret_cast<double2*>(p);
     a.part = negf::PART_CONTACTS;
-    a.ws_per_team = (int64_t)(per_c / sizeof(double2));
-    e = negf::launch_engine(a, tc.teams, tc.team, s);
+    a.ws_per_team = (int64_t)(pl.per_c / sizeof(double2));
+    e = negf::launch_engine(a, pl.tc.teams, pl.tc.team, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
     ++ctx->launches;
     a.part = negf::PART_SWEEPS;
     a.counter += 1;
   }
   a.ws = reinterpret_cast<double2*>(p);
-  a.ws_per_team = (int64_t)(per / sizeof(double2));
-  e = negf::launch_engine(a, ts.teams, ts.team, s);
+  a.ws_per_team = (int64_t)(pl.per / sizeof(double2));
+  e = negf::launch_engine(a, pl.ts.teams, pl.ts.team, s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
   ++ctx->launches;
   return NEGF_B200_OK;
@@ -1166,9 +1185,27 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
   int st = sync_descs(ctx);
   if (st) return st;
   const int n = sh.n;
-  // the mixed form: two full waves of the inversion (one CTA per matrix, two
-  // per SM: 592 on a B200); the small form: the whole call at once up to 8192
-  int batch = std::min<int>(npts, slices ? 4 * std::max(ctx->sms, 1) : 8192);
+  negf::MixedArgs a;
+  a.npts = npts; a.d_ids = d_ids; a.d_E = d_E; a.eta = eta; a.d_descs = ctx->d_descs;
+  a.n = n; a.nbl = sh.nbl; a.left = sh.left; a.right = sh.right;
+  a.sgf_tol = ctx->opt.sgf_tol; a.sgf_max_iter = ctx->opt.sgf_max_iter; a.slices = slices;
+  a.d_T = d_T; a.d_ncyc = d_ncyc; a.d_status = d_status;
+  a.launches = &ctx->launches;
+  if (slices == 0) {   // small orders: one launch, no workspace (a limit below one point's blocks refuses as ever)
+    if (ctx->ws_limit && ctx->ws_limit < (size_t)14 * n * n * sizeof(double2))
+      return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
+    // the engine runs the same call under stream capture, where nothing can be
+    // allocated: leave its workspace in place (where it fits)
+    LaunchShape es;
+    es.nmax = n; es.nbl_max = sh.nbl; es.ncont_max = 2;
+    EnginePlan pl;
+    if (plan_engine(ctx, negf::MODE_T, npts, es, false, pl) == NEGF_B200_OK)
+      grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
+    const cudaError_t e = negf::launch_small_points(a, s);
+    return e == cudaSuccess ? NEGF_B200_OK : cuda_fail(ctx, e, "lock step");
+  }
+  // two full waves of the inversion (two CTAs per SM: 592 points on a B200)
+  int batch = std::min<int>(npts, 4 * std::max(ctx->sms, 1));
   if (ctx->ws_limit) batch = std::min(batch, negf::mixed_batch_for(ctx->ws_limit, n, slices));
   if (batch < 1) return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
   for (;;) {
@@ -1177,15 +1214,9 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
     if (batch == 1) return st;
     batch = (batch + 1) / 2;
   }
-  negf::MixedArgs a;
-  a.npts = npts; a.d_ids = d_ids; a.d_E = d_E; a.eta = eta; a.d_descs = ctx->d_descs;
-  a.n = n; a.nbl = sh.nbl; a.left = sh.left; a.right = sh.right;
-  a.sgf_tol = ctx->opt.sgf_tol; a.sgf_max_iter = ctx->opt.sgf_max_iter; a.slices = slices;
-  a.d_T = d_T; a.d_ncyc = d_ncyc; a.d_status = d_status;
-  a.launches = &ctx->launches;
   std::string msg;
   st = negf::mixed_run(a, ctx->ws, batch, s, &msg);
-  if (st) return fail(ctx, st, (slices ? "mixed form: " : "lock step: ") + msg);
+  if (st) return fail(ctx, st, "mixed form: " + msg);
   return NEGF_B200_OK;
 }
 

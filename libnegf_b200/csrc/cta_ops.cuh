@@ -1076,7 +1076,9 @@ __device__ __forceinline__ void gj_reg_steps(double2 (&x)[R][W], int n, int c0, 
 // instruction cache for a third of the time.
 //
 // WHOLE: the panel is the whole matrix (w = n): the columns also go to their
-// places, so dst gets the inverse.
+// places, so dst gets the inverse.  scratch: 3 * 32 RL + 8 CW + 4 elements of
+// shared memory (a pointer the compiler can trace to it: with generic
+// accesses a step's stores and loads wait for one another).
 struct PanelPivot {
   double2 d;
   int lane, slot, pos, pad;
@@ -1096,14 +1098,12 @@ __device__ __forceinline__ void unroll_steps(F& f) {
 }
 
 template <int RL, int CW, bool WHOLE>
-__device__ __forceinline__ void gj_panel(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
+__device__ __forceinline__ void gj_panel(const double2* src, int lds, double2* dst, int ldd, int n, int c0, int w,
+                                         double2* scratch, InvScratch& s) {
   constexpr int NR = 32 * RL, NW = kThreads / 32;
   constexpr bool kScaleRow = RL > CW;   // scale the row's CW entries by d, else the column's RL
   constexpr unsigned kAll = 0xffffffffu;
-  // the CTA's main shared-memory region, named here so that its accesses
-  // compile to shared-memory instructions
-  extern __shared__ __align__(16) char smem_raw[];
-  double2* const colb = reinterpret_cast<double2*>(smem_raw);             // [3][NR]
+  double2* const colb = scratch;                                          // [3][NR]
   double2* const rowb = colb + 3 * NR;                                    // [NW][CW]
   PanelPivot* const pivs = reinterpret_cast<PanelPivot*>(rowb + NW * CW); // [2]
   int* const piv = s.piv;
@@ -1118,7 +1118,7 @@ __device__ __forceinline__ void gj_panel(const double2* src, double2* dst, int n
 #pragma unroll
     for (int c = 0; c < CW; ++c) {
       const int k = wp + c * NW;
-      x[r][c] = (row < n && k < w) ? src[row + (size_t)k * n] : make_double2(0.0, 0.0);
+      x[r][c] = (row < n && k < w) ? src[row + (size_t)k * lds] : make_double2(0.0, 0.0);
     }
   }
   // one entry of the next pivot column: a candidate from position j on (NaN
@@ -1143,7 +1143,7 @@ __device__ __forceinline__ void gj_panel(const double2* src, double2* dst, int n
       col[lane + 32 * r] = x[r][C];
       candidate(x[r][C], 32 * lg[r] + r, j, ba, best);
     }
-    double2 pv = col[lane + 32 * (best & 31)];
+    double2 pv = RL == 1 ? x[0][C] : col[lane + 32 * (best & 31)];
     double2 d = crecip_scaled(pv);
     // the bits of a value >= 0 order like it; + 1: 0 = no candidate
     const unsigned long long key = ba >= 0.0 ? (unsigned long long)__double_as_longlong(ba) + 1ull : 0ull;
@@ -1240,7 +1240,7 @@ __device__ __forceinline__ void gj_panel(const double2* src, double2* dst, int n
   for (int c = 0; c < CW; ++c) {
     const int k = wp + c * NW;
     if (k < w) {
-      double2* out = dst + (size_t)(WHOLE ? dest[k] : k) * n;
+      double2* out = dst + (size_t)(WHOLE ? dest[k] : k) * ldd;
 #pragma unroll
       for (int r = 0; r < RL; ++r)
         if (lg[r] >= 0) out[lg[r]] = x[r][c];

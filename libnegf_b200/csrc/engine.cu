@@ -190,10 +190,7 @@ int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax) {
   return e;
 }
 
-// Raises a team kernel's shared-memory limit to that of the largest block
-// order and allows clusters of 16, once per device (not per launch), so that
-// a launch is a stream operation only and can be captured into a CUDA graph.
-cudaError_t team_opt_in(const void* kernel) {
+cudaError_t team_opt_in(const void* kernel, size_t smem) {
   static std::mutex mu;
   static std::set<std::pair<const void*, int>> done;
   int dev = 0;
@@ -201,7 +198,8 @@ cudaError_t team_opt_in(const void* kernel) {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lk(mu);
   if (done.count({kernel, dev})) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)engine_smem_bytes(kMaxOrder));
+  if (smem == 0) smem = engine_smem_bytes(kMaxOrder);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess) done.insert({kernel, dev});
   return e;

@@ -120,6 +120,12 @@ int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax);
 int64_t engine_contact_elems(int nmax);   // workspace of a team in a PART_CONTACTS launch
 size_t engine_smem_bytes(int nmax);
 
+// Raises a kernel's dynamic shared-memory limit (0: to what the team kernels
+// need for the largest block order) and allows clusters of 16, once per
+// kernel and device (not per launch), so that a launch is a stream operation
+// only and can be captured into a CUDA graph.
+cudaError_t team_opt_in(const void* kernel, size_t smem = 0);
+
 // `teams` teams of `team` CTAs (a thread-block cluster; 1, 2, 4, 8 or 16), one
 // point at a time each
 cudaError_t launch_engine(const EngineArgs& a, int teams, int team, cudaStream_t s);

@@ -6,16 +6,22 @@
 namespace negf {
 
 __device__ void panel_run_w32(const double2* A, double2* X, int n, int c0, int w, InvScratch& s) {
-  gj_panel<1, 4, true>(A, X, n, c0, w, s);
+  extern __shared__ __align__(16) char smem_raw[];
+  gj_panel<1, 4, true>(A, n, X, n, n, c0, w, reinterpret_cast<double2*>(smem_raw), s);
 }
 __device__ void panel_run_w64(const double2* A, double2* X, int n, int c0, int w, InvScratch& s) {
-  gj_panel<2, 8, true>(A, X, n, c0, w, s);
+  extern __shared__ __align__(16) char smem_raw[];
+  gj_panel<2, 8, true>(A, n, X, n, n, c0, w, reinterpret_cast<double2*>(smem_raw), s);
 }
 __device__ void panel_run_4(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
-  gj_panel<4, 4, false>(src + (size_t)c0 * n, dst + (size_t)c0 * n, n, c0, w, s);
+  extern __shared__ __align__(16) char smem_raw[];
+  gj_panel<4, 4, false>(src + (size_t)c0 * n, n, dst + (size_t)c0 * n, n, n, c0, w,
+                        reinterpret_cast<double2*>(smem_raw), s);
 }
 __device__ void panel_run_8(const double2* src, double2* dst, int n, int c0, int w, InvScratch& s) {
-  gj_panel<8, 2, false>(src + (size_t)c0 * n, dst + (size_t)c0 * n, n, c0, w, s);
+  extern __shared__ __align__(16) char smem_raw[];
+  gj_panel<8, 2, false>(src + (size_t)c0 * n, n, dst + (size_t)c0 * n, n, n, c0, w,
+                        reinterpret_cast<double2*>(smem_raw), s);
 }
 __device__ void leaf_run_r2(double2* X, int n, int c0, int w, double2* sh, InvScratch& s) {
   gj_leaf4<2, 4>(X, n, c0, w, sh, s);

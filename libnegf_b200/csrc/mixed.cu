@@ -23,7 +23,6 @@
 #include "../../include/negf_b200.h"
 #include "mixed.cuh"
 #include "ozaki.cuh"
-#include "small.cuh"
 
 namespace negf {
 namespace {
@@ -65,11 +64,9 @@ __global__ void k_lead_init(int n, int c, const int* ids, const double* E, doubl
   }
 }
 
-// Ao -= Self, Aos -= Self for the points of the list (its first *count
-// entries when count is given)
-__global__ void k_sub_self(int64_t nn, const int* list, const int* count, const double2* Self, double2* Ao,
+// Ao -= Self, Aos -= Self for the points of the list
+__global__ void k_sub_self(int64_t nn, const int* list, const double2* Self, double2* Ao,
                            double2* Aos, int64_t Q) {
-  if (count && (int)blockIdx.y >= *count) return;
   const int p = list[blockIdx.y];
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nn; q += (int64_t)gridDim.x * blockDim.x) {
     const double2 s = Self[p * Q + q];
@@ -83,12 +80,10 @@ __global__ void k_sub_self(int64_t nn, const int* list, const int* count, const 
 
 // The CPU convergence rule (src/contselfenergy.F90:300-310): a point is done
 // on its second consecutive max|C1| <= tol.  Builds the list of the points
-// that go on (and zeroes their max for the next iteration).  One CTA.  The
-// list's length is na, or *count when count is given.
-__global__ void k_dec_check(int na, const int* count, const int* list, double* mx, int* ok, int* ncyc_c, double tol,
+// that go on (and zeroes their max for the next iteration).  One CTA.
+__global__ void k_dec_check(int na, const int* list, double* mx, int* ok, int* ncyc_c, double tol,
                             int it, int* next, int* next_count, int* redo) {
   __shared__ int cnt;
-  if (count) na = *count;
   if (threadIdx.x == 0) cnt = 0;
   __syncthreads();
   for (int b = threadIdx.x; b < na; b += blockDim.x) {
@@ -117,8 +112,7 @@ __global__ void k_dec_check(int na, const int* count, const int* list, double* m
   if (threadIdx.x == 0) *next_count = cnt;
 }
 
-__global__ void k_info_to_status(int nb, const int* count, const int* list, const int* info, int* status, int code) {
-  if (count) nb = min(nb, *count);
+__global__ void k_info_to_status(int nb, const int* list, const int* info, int* status, int code) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
     const int p = list ? list[b] : b;
     if (info[p] != 0 && status[p] == 0) status[p] = code;
@@ -295,10 +289,8 @@ __global__ void k_retarded_check(int n, const double2* gs, int64_t Q, const int*
 }
 
 // Start of a decimation for the points map[b], b < nsub (map null: b):
-// ok = 0, max = 0, ncyc = 0, sensitivity 0, the active list = the points,
-// its count.
-__global__ void k_dec_start(int nsub, const int* map, int* ok, double* mx, int* ncyc_c, int* list, int* count,
-                            int* sens) {
+// ok = 0, max = 0, ncyc = 0, sensitivity 0, the active list = the points.
+__global__ void k_dec_start(int nsub, const int* map, int* ok, double* mx, int* ncyc_c, int* list, int* sens) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nsub; b += gridDim.x * blockDim.x) {
     const int p = map ? map[b] : b;
     ok[p] = 0;
@@ -307,7 +299,6 @@ __global__ void k_dec_start(int nsub, const int* map, int* ok, double* mx, int* 
     ncyc_c[p] = 0;
     list[b] = p;
   }
-  if (count && blockIdx.x == 0 && threadIdx.x == 0) *count = nsub;
 }
 
 // kept_p = gs_p for the points map[b], b < nsub; one CTA per point.
@@ -391,9 +382,8 @@ Ws carve(void* base, int P, int n, int slices, size_t* total) {
   w.sub = c.take<int>(P);
   w.sens = c.take<int>(P);
   w.agree = c.take<int>(P);
-  const bool small = slices == 0;        // the lock-step FP64 form: one-warp kernels, no splitting
-  w.zwork = c.take<double2>(small ? 1 : (size_t)P * zinv_batched_work_elems(n) + 1);
-  w.oz = small ? nullptr : c.take<uint8_t>(ozaki_layout(P, n, n, n, slices).total);
+  w.zwork = c.take<double2>((size_t)P * zinv_batched_work_elems(n) + 1);
+  w.oz = c.take<uint8_t>(ozaki_layout(P, n, n, n, slices).total);
   *total = c.off + 256;
   return w;
 }
@@ -408,8 +398,7 @@ __global__ void k_finish(int P, const int* ncl, const int* ncr, const int* pst, 
   }
 }
 
-__global__ void k_not_converged(int na, const int* count, const int* list, int* ncyc_c, int* pst, int max_iter) {
-  if (count) na = min(na, *count);
+__global__ void k_not_converged(int na, const int* list, int* ncyc_c, int* pst, int max_iter) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < na; b += gridDim.x * blockDim.x) {
     const int p = list[b];
     ncyc_c[p] = max_iter + 1;
@@ -438,7 +427,6 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
   const int n = a.n;
   const int64_t Q = (int64_t)n * n;
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0), mone = make_double2(-1, 0);
-  const bool small = a.slices == 0;
   size_t tot = 0;
   Ws w = carve(ws, batch, n, a.slices, &tot);
   double2** B = w.blk;
@@ -454,38 +442,22 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
     int r_ = ck((x), what);      \
     if (r_) return r_;           \
   } while (0)
-  // products and inverses of the problems map[b], b < nb (or b < *count)
+  // products and inverses of the problems map[b], b < nb
   uint64_t nl = 0;                 // kernels launched (reported through a.launches)
-  auto prod = [&](int nb, const int* map, const int* count, double2 alpha, const double2* A, const double2* Bm,
-                  double2 beta, double2* C, double* maxabs) -> cudaError_t {
-    if (small) {
-      ++nl;
-      return launch_small_zgemm(nb, n, alpha, A, Bm, beta, C, Q, map, count, maxabs, s);
-    }
+  auto prod = [&](int nb, const int* map, double2 alpha, const double2* A, const double2* Bm, double2 beta, double2* C,
+                  double* maxabs) -> cudaError_t {
     nl += 3;                       // digit split of A, of B, the product
     return launch_ozaki_zgemm(nb, n, n, n, alpha, A, Q, Bm, Q, beta, C, Q, a.slices, w.oz, maxabs, w.pst, s, map);
   };
-  auto inv = [&](int nb, const int* map, const int* count, const double2* A, double2* X) -> cudaError_t {
+  auto inv = [&](int nb, const int* map, const double2* A, double2* X) -> cudaError_t {
     ++nl;
-    if (small) {
-      // the one-warp inversion, then its residual probe and Newton steps where needed
-      cudaError_t e = launch_small_zinv(nb, n, A, X, Q, map, count, w.info, w.pst, NEGF_B200_ERR_SINGULAR, s);
-      if (e != cudaSuccess) return e;
-      ++nl;
-      return launch_small_refine(nb, n, A, X, Q, map, count, s, w.sens);
-    }
     return launch_zinv_mapped(nb, n, A, Q, X, Q, map, w.info, w.zwork, s, w.sens);   // probe and refinement inside
   };
-  // FP64 products of the trace (the one-warp kernel at small orders, else the DMMA product)
+  // FP64 products of the trace
   auto prod64 = [&](int nb, const double2* A, const double2* Bm, double2* C) -> cudaError_t {
     ++nl;
-    if (small) return launch_small_zgemm(nb, n, one, A, Bm, zero, C, Q, nullptr, nullptr, nullptr, s);
     return launch_zgemm_batched(nb, n, n, n, one, A, Q, Bm, Q, zero, C, Q, 0, s);
   };
-  // the small form runs the decimation without a host round trip per
-  // iteration: the kernels read the active count on the device, and the host
-  // looks at it every kPoll iterations
-  constexpr int kPoll = 8;
 
   for (int p0 = 0; p0 < a.npts; p0 += batch) {
     const int P = std::min(batch, a.npts - p0);
@@ -504,39 +476,20 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
       k_lead_init<<<dim3(gx, nsub), eb, 0, s>>>(n, c, ids, E, a.eta, scale, sub, a.d_descs, Ao, Aos, Bo, Co, Q);
       ++nl;
       MCK(cudaGetLastError(), "lead init");
-      int* cnt_cur = small ? w.count : nullptr;        // device active counts (small form)
-      int* cnt_nxt = small ? w.count + 1 : nullptr;
-      k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, ncyc_c, w.list0, cnt_cur, w.sens);
+      k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, ncyc_c, w.list0, w.sens);
       ++nl;
       int na = nsub;                                   // host bound of the active list
       int* cur = w.list0;
       int* nxt = w.list1;
       int it = 1;
       for (; it <= a.sgf_max_iter && na > 0; ++it) {
-        MCK(inv(na, cur, cnt_cur, Ao, Go), "zinv");
-        if (small) {
-          // the rest of the iteration in one fused launch, one CTA per point
-          MCK(cudaMemsetAsync(cnt_nxt, 0, sizeof(int), s), "memset count");
-          MCK(launch_small_dec(na, n, cur, cnt_cur, Go, Co, Bo, C1, B1, Ao, Aos, Q, w.ok, ncyc_c, a.sgf_tol, it,
-                               nxt, cnt_nxt, w.redo, s), "decimation");
-          ++nl;
-          std::swap(cur, nxt);
-          std::swap(cnt_cur, cnt_nxt);
-          std::swap(B[2], B[8]);
-          std::swap(B[3], B[6]);
-          Bo = B[2]; Co = B[3]; B1 = B[8]; C1 = B[6];
-          if (it % kPoll == 0) {
-            MCK(cudaMemcpyAsync(&na, cnt_cur, sizeof(int), cudaMemcpyDeviceToHost, s), "count");
-            MCK(cudaStreamSynchronize(s), "sync");
-          }
-          continue;
-        }
-        // the mixed form: one batched product per step, the active list compacted on the host
-        k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, nullptr, cur, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
+        // one batched product per step, the active list compacted on the host
+        MCK(inv(na, cur, Ao, Go), "zinv");
+        k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
         ++nl;
-        MCK(prod(na, cur, nullptr, one, Go, Co, zero, X, nullptr), "GoXCo");
-        MCK(prod(na, cur, nullptr, one, Co, X, zero, C1, w.mx), "C1");
-        k_dec_check<<<1, 1024, 0, s>>>(na, nullptr, cur, w.mx, w.ok, ncyc_c, a.sgf_tol, it, nxt, w.count, w.redo);
+        MCK(prod(na, cur, one, Go, Co, zero, X, nullptr), "GoXCo");
+        MCK(prod(na, cur, one, Co, X, zero, C1, w.mx), "C1");
+        k_dec_check<<<1, 1024, 0, s>>>(na, cur, w.mx, w.ok, ncyc_c, a.sgf_tol, it, nxt, w.count, w.redo);
         ++nl;
         MCK(cudaGetLastError(), "check");
         std::swap(cur, nxt);
@@ -547,30 +500,24 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
           na = h_count;
           if (na == 0) break;
         }
-        MCK(prod(na, cur, nullptr, one, Bo, X, zero, B1, nullptr), "Self");
-        k_sub_self<<<dim3(gx, na), eb, 0, s>>>(Q, cur, nullptr, B1, Ao, Aos, Q); ++nl;
-        MCK(prod(na, cur, nullptr, one, Go, Bo, zero, Y, nullptr), "GoXBo");
-        MCK(prod(na, cur, nullptr, one, Bo, Y, zero, B1, nullptr), "B1");
-        MCK(prod(na, cur, nullptr, mone, Co, Y, one, Ao, nullptr), "Ao update");
+        MCK(prod(na, cur, one, Bo, X, zero, B1, nullptr), "Self");
+        k_sub_self<<<dim3(gx, na), eb, 0, s>>>(Q, cur, B1, Ao, Aos, Q); ++nl;
+        MCK(prod(na, cur, one, Go, Bo, zero, Y, nullptr), "GoXBo");
+        MCK(prod(na, cur, one, Bo, Y, zero, B1, nullptr), "B1");
+        MCK(prod(na, cur, mone, Co, Y, one, Ao, nullptr), "Ao update");
         // Bo = B1, Co = C1 for every point still iterating (the others are done with them)
         std::swap(B[2], B[8]);
         std::swap(B[3], B[6]);
         Bo = B[2]; Co = B[3]; B1 = B[8]; C1 = B[6];
       }
-      if (small && na > 0) {         // the loop ran to the cap: how many are left
-        MCK(cudaMemcpyAsync(&na, cnt_cur, sizeof(int), cudaMemcpyDeviceToHost, s), "count");
-        MCK(cudaStreamSynchronize(s), "sync");
-      }
       if (na > 0) {
-        k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cnt_cur, cur, ncyc_c, w.pst, a.sgf_max_iter);
+        k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cur, ncyc_c, w.pst, a.sgf_max_iter);
         ++nl;
       }
-      MCK(inv(nsub, sub, nullptr, Aos, B[9 + side]), "gs");
-      if (!small) {
-        k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, nullptr, sub, w.info, w.pst,
-                                                              NEGF_B200_ERR_SINGULAR);
-        ++nl;
-      }
+      MCK(inv(nsub, sub, Aos, B[9 + side]), "gs");
+      k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, w.pst,
+                                                            NEGF_B200_ERR_SINGULAR);
+      ++nl;
       if (a.eta > 0.0) {
         k_retarded_check<<<nsub, 128, 0, s>>>(n, B[9 + side], Q, sub, w.redo);
         ++nl;
@@ -638,28 +585,24 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
       const int c = side == 0 ? a.left : a.right;
       k_tlc<<<dim3(gx, P), eb, 0, s>>>(n, c, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;
       MCK(cudaGetLastError(), "tlc");
-      MCK(prod(P, nullptr, nullptr, one, B[0], B[9 + side], zero, B[2], nullptr), "Tlc gs");
-      MCK(prod(P, nullptr, nullptr, one, B[2], B[1], zero, B[11 + side], nullptr), "Sigma");
+      MCK(prod(P, nullptr, one, B[0], B[9 + side], zero, B[2], nullptr), "Tlc gs");
+      MCK(prod(P, nullptr, one, B[2], B[1], zero, B[11 + side], nullptr), "Sigma");
     }
     // ---- gsmr sweep from block nbl down to 2, then Gr(1,1)
     double2 *g = B[4], *X = B[5], *W = B[6], *U = B[7], *Lb = B[8];
     k_esh<<<dim3(gx, P), eb, 0, s>>>(n, 0, a.nbl - 1, ids, E, a.d_descs, B[12], W, Q); ++nl;
-    MCK(inv(P, nullptr, nullptr, W, g), "gsmr N");
-    if (!small) {
-      k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
-      ++nl;
-    }
+    MCK(inv(P, nullptr, W, g), "gsmr N");
+    k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
+    ++nl;
     for (int i = a.nbl - 2; i >= 0; --i) {
       // W = ESH(i,i) - ESH(i,i+1) gsmr(i+1) ESH(i+1,i)  (block i 0-based; Sigma_left on block 0)
       k_esh_step<<<dim3(gx, P), eb, 0, s>>>(n, i, ids, E, a.d_descs, i == 0 ? B[11] : nullptr, U, Lb, W, Q); ++nl;
       MCK(cudaGetLastError(), "esh");
-      MCK(prod(P, nullptr, nullptr, one, U, g, zero, X, nullptr), "U g");
-      MCK(prod(P, nullptr, nullptr, mone, X, Lb, one, W, nullptr), "W");
-      MCK(inv(P, nullptr, nullptr, W, g), "gsmr");
-      if (!small) {
-        k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
-        ++nl;
-      }
+      MCK(prod(P, nullptr, one, U, g, zero, X, nullptr), "U g");
+      MCK(prod(P, nullptr, mone, X, Lb, one, W, nullptr), "W");
+      MCK(inv(P, nullptr, W, g), "gsmr");
+      k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
+      ++nl;
     }
     // g = Gr(1,1).  Trace with Gamma of the contact on block 1 (FP64 products)
     k_gamma<<<dim3(gx, P), eb, 0, s>>>(n, B[11], B[0], Q); ++nl;

@@ -1,576 +1,467 @@
-// Small-order block operations for the lock-step FP64 form (small.cuh): one
-// CTA per product (operands staged in shared memory), one warp per
-// inversion (lane i holding row i).  Reference operations replaced: the zgemm of prealloc_mult
-// (src/sparsekit_drv.F90:1896-2081) and zinv = zgetrf + zgetrs against the
-// identity (src/inversions.F90:807-839), at orders n <= 32.
+// Small-order transmission (small.cuh): the 2-contact Caroli solve of a point
+// of block order n <= 32 by one CTA, following the reference routine by
+// routine:
+//   surface_green + decimation   src/contselfenergy.F90:184-210, 271-340
+//   compute_contacts             src/contselfenergy.F90:445-491, 552-566
+//   build_ESH (real E)           src/iterative.F90:1956-1982
+//   gsmr sweep, Gr(1,1)          src/iterative_cpu.F90:51-170
+//   Caroli trace                 src/iterative_cpu.F90:399-470
+//
+// At these orders a product is 2000 cycles of an SM's FP64 pipe and an
+// inversion a chain of 32 dependent steps; what a point costs is latency.
+// With every point through one launch per block operation (the form before
+// this one: about 280 launches a call, operands through memory each time) a
+// launch was 10 to 25 us of mostly fixed latency.  Here a point's blocks
+// never leave the SM between operations: one energy of a 20-layer device of
+// order 32 takes 1.30 ms (3.10 before), 512 energies 3.34 ms (6.07).
 #include <cuda_runtime.h>
 
-#include <mutex>
-
+#include "../../include/negf_b200.h"
 #include "cta_ops.cuh"
 #include "small.cuh"
 
 namespace negf {
 namespace {
 
-constexpr int kWarps = 4;                  // problems per CTA
+// Blocks lie in shared memory column major with 34 rows per column: 2 modulo
+// 8 elements, so that the eight lanes of a 128-byte phase of a fragment load
+// hit different banks, for the left operand with lane (g, t) on row g of
+// column t and for the right one with columns taken in the order of ncol().
+constexpr int kLd = 34, kBlk = 32 * kLd;
+constexpr int kBlocks = 6;
 constexpr unsigned kFull = 0xffffffffu;
 
-__device__ __forceinline__ int batch_limit(int batch, const int* count) {
-  return count ? min(*count, batch) : batch;
+struct SmallShared {
+  InvScratch inv;
+  int piv[32], perm[32], cperm[32], flag;
+  double red[3][8];
+  double2 y[32];
+};
+constexpr size_t kScratchElems = 3 * 32 + 8 * 4 + 4;   // gj_panel<1, 4>
+constexpr size_t kSmallSmem = (kBlocks * kBlk + kScratchElems) * sizeof(double2) + sizeof(SmallShared);
+
+// The dynamic shared memory, named wherever it is used so that accesses
+// compile to shared-memory instructions: blocks, panel scratch, the rest.
+extern __shared__ __align__(16) char smem_raw[];
+enum Block : int { B_AO = 0, B_BO = 1, B_CO = 2, B_GO = 3, B_X = 4, B_SL = 5 };
+__device__ __forceinline__ double2* block(int b) { return reinterpret_cast<double2*>(smem_raw) + b * kBlk; }
+__device__ __forceinline__ SmallShared& shared() {
+  return *reinterpret_cast<SmallShared*>(reinterpret_cast<double2*>(smem_raw) + kBlocks * kBlk + kScratchElems);
 }
 
-// One CTA (4 warps) per problem: A and B staged in shared memory by
-// coalesced loads (one memory latency per operand), then warp w computes
-// columns [w CW, (w + 1) CW) of C and lane i row i: A's column k is read
-// conflict-free, B's row k by broadcast.
-template <int N>
-__global__ void __launch_bounds__(kWarps * 32)
-    k_small_zgemm(int batch, int n, double2 alpha, const double2* __restrict__ A, const double2* __restrict__ B,
-                  double2 beta, double2* C, int64_t Q, const int* map, const int* count, double* maxabs) {
-  constexpr int CW = N / kWarps;   // columns per warp
-  __shared__ double2 sA[N * N], sB[N * N];
-  __shared__ double smx[kWarps];
-  __shared__ int sbad[kWarps];
-  const int b = blockIdx.x;
-  if (b >= batch_limit(batch, count)) return;
-  const int p = map ? map[b] : b;
-  const int nn = n * n;
-  const double2* Ap = A + p * Q;
-  const double2* Bp = B + p * Q;
-  {
-    constexpr int R = (N * N + kWarps * 32 - 1) / (kWarps * 32);
-    double2 va[R], vb[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int q = threadIdx.x + i * kWarps * 32;
-      if (q < nn) {
-        va[i] = __ldg(Ap + q);
-        vb[i] = __ldg(Bp + q);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int q = threadIdx.x + i * kWarps * 32;
-      if (q < nn) {
-        sA[q] = va[i];
-        sB[q] = vb[i];
-      }
+__device__ __forceinline__ int ncol(int g) { return (g & 4) | ((g & 1) << 1) | ((g & 2) >> 1); }
+
+// A thread's four elements of a 32 x 32 product (the fragment layout of
+// dmma_16x8x4): element q at (row(q), col(q)); rows and columns from n on
+// are not part of the block.
+struct Frag {
+  double2 v[4];
+};
+struct Lane {
+  int n, g, t, m0, n0;
+  __device__ __forceinline__ explicit Lane(int order) : n(order) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    g = lane >> 2;
+    t = lane & 3;
+    m0 = (w >> 2) * 16;
+    n0 = (((w & 3) + 2 * (w >> 2)) & 3) * 8;   // tiles of n <= 16 on all four schedulers
+  }
+  __device__ __forceinline__ int row(int q) const { return m0 + g + ((q >> 1) << 3); }
+  __device__ __forceinline__ int col(int q) const { return n0 + ncol(2 * t + (q & 1)); }
+  __device__ __forceinline__ bool in(int q) const { return row(q) < n && col(q) < n; }
+  __device__ __forceinline__ int at(int q) const { return row(q) + col(q) * kLd; }
+};
+
+// A B, on the FP64 tensor pipe; entries of A and B from n on are zero.
+__device__ __forceinline__ Frag mm(const Lane& L, const double2* A, const double2* B) {
+  double re[4] = {0.0, 0.0, 0.0, 0.0}, im[4] = {0.0, 0.0, 0.0, 0.0};
+  if (L.m0 < L.n && L.n0 < L.n) {
+    const double2* pa = A + L.t * kLd + L.m0 + L.g;
+    const double2* pb = B + (L.n0 + ncol(L.g)) * kLd + L.t;
+#pragma unroll 4
+    for (int k = 0; k < L.n; k += 4) {
+      const double2 a0 = pa[k * kLd], a1 = pa[k * kLd + 8], b = pb[k];
+      dmma_16x8x4(re, a0.x, a1.x, b.x);
+      dmma_16x8x4(im, a0.x, a1.x, b.y);
+      dmma_16x8x4(re, a0.y, a1.y, -b.y);
+      dmma_16x8x4(im, a0.y, a1.y, b.x);
     }
   }
-  __syncthreads();
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j0 = w * CW;
-  double2 acc[CW];
+  Frag f;
 #pragma unroll
-  for (int jj = 0; jj < CW; ++jj) acc[jj] = make_double2(0.0, 0.0);
-  if (lane < n) {
-    for (int k = 0; k < n; ++k) {
-      const double2 a = sA[lane + k * n];
+  for (int q = 0; q < 4; ++q) f.v[q] = make_double2(re[q], im[q]);
+  return f;
+}
+__device__ __forceinline__ void put(const Lane& L, double2* D, const Frag& f) {
 #pragma unroll
-      for (int jj = 0; jj < CW; ++jj) {
-        const int j = j0 + jj;
-        if (j < n) {
-          const double2 bv = sB[k + j * n];
-          acc[jj].x = fma(a.x, bv.x, acc[jj].x);
-          acc[jj].x = fma(-a.y, bv.y, acc[jj].x);
-          acc[jj].y = fma(a.x, bv.y, acc[jj].y);
-          acc[jj].y = fma(a.y, bv.x, acc[jj].y);
-        }
-      }
-    }
-  }
-  const bool use_beta = beta.x != 0.0 || beta.y != 0.0;
-  double mx = 0.0;
-  bool bad = false;
-  if (lane < n) {
-    double2* Cp = C + p * Q;
+  for (int q = 0; q < 4; ++q)
+    if (L.in(q)) D[L.at(q)] = f.v[q];
+}
+__device__ __forceinline__ Frag get(const Lane& L, const double2* S) {
+  Frag f;
 #pragma unroll
-    for (int jj = 0; jj < CW; ++jj) {
-      const int j = j0 + jj;
-      if (j < n) {
-        double2* el = Cp + lane + (int64_t)j * n;
-        double2 v = cmul(alpha, acc[jj]);
-        if (use_beta) v = cadd(v, cmul(beta, *el));
-        *el = v;
-        const double h = hypot(v.x, v.y);
-        mx = fmax(mx, h);
-        bad |= !(h <= 1.7976931348623157e308);   // NaN or Inf
-      }
-    }
-  }
-  if (maxabs) {
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(kFull, mx, o));
-    bad = __any_sync(kFull, bad);
-    if (lane == 0) {
-      smx[w] = mx;
-      sbad[w] = bad;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      bool any = false;
-      for (int q = 0; q < kWarps; ++q) {
-        mx = fmax(mx, smx[q]);
-        any |= sbad[q] != 0;
-      }
-      // a non-finite element makes the maximum NaN (fmax would drop it): the
-      // positive quiet NaN is above every finite bit pattern, so it stays
-      if (any) mx = __longlong_as_double(0x7ff8000000000000LL);
-      atomicMax(reinterpret_cast<unsigned long long*>(maxabs + p), (unsigned long long)__double_as_longlong(mx));
-    }
-  }
+  for (int q = 0; q < 4; ++q) f.v[q] = L.in(q) ? S[L.at(q)] : make_double2(0.0, 0.0);
+  return f;
+}
+__device__ __forceinline__ void sub_from(const Lane& L, double2* D, const Frag& f) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (L.in(q)) D[L.at(q)] = csub(D[L.at(q)], f.v[q]);
 }
 
-// In-place Gauss-Jordan, one CTA (4 warps) per matrix: lane i holds row i,
-// warp w the columns [w CW, (w + 1) CW).  Rows never move between lanes:
-// each lane carries the logical (pivot-order) index of its row, identical in
-// every warp.  Per step the warp owning column k picks the pivot (the unused
-// row with the largest |Re|+|Im|, lowest logical index on a tie: izamax) by
-// integer warp reductions on the bit pattern and publishes column k and the
-// pivot's lane in shared memory (double-buffered by step parity: one barrier
-// per step); every warp then updates its columns, taking the pivot row's
-// entries from the pivot lane by shuffle.  The pivot row becomes row * d
-// (d = 1 / pivot, entry k = d), every other row r - (r_k d) * row (entry
-// k = -(r_k d)), the update order of the engine's Gauss-Jordan.  The column
-// interchanges that undo the row order are applied to the store addresses.
-template <int N>
-__global__ void __launch_bounds__(kWarps * 32)
-    k_small_zinv(int batch, int n, const double2* A, double2* X, int64_t Q, const int* map, const int* count,
-                 int* info, int* status, int singular_code) {
-  constexpr int CW = N / kWarps;
-  __shared__ double2 colk[2][32];  // one entry per lane: rows >= N exist as lanes too
-  __shared__ int sbl[2];
-  __shared__ int sidx[N];
-  __shared__ int scm[N];
-  const int b = blockIdx.x;
-  if (b >= batch_limit(batch, count)) return;
-  const int p = map ? map[b] : b;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double2* Ap = A + p * Q;
-  double2 r[CW];
+// Maximum of v over the CTA (NaN in any thread: NaN); red: 8 doubles.  Ends
+// with a barrier before red is next written (the callers' own barriers).
+__device__ __forceinline__ double cta_max_nan(double v, double* red) {
+  bool bad = !(v <= 1.7976931348623157e308);
 #pragma unroll
-  for (int cc = 0; cc < CW; ++cc) {
-    const int c = w * CW + cc;
-    r[cc] = (lane < n && c < n) ? Ap[lane + (int64_t)c * n] : make_double2(0.0, 0.0);
-  }
-  int lg = lane;
-  bool used = lane >= n;
-  int inf = 0;
-  for (int k = 0; k < n; ++k) {
-    const int ow = k / CW, ck = k % CW, par = k & 1;
-    if (w == ow) {
-      double2 rk = r[0];
-#pragma unroll
-      for (int cc = 1; cc < CW; ++cc)
-        if (cc == ck) rk = r[cc];
-      // |Re|+|Im| orders as its bit pattern; + 1 puts an unused row with a zero entry
-      // above the used rows (key 0); NaN ranks highest so all lanes see one order
-      double v = cabs1(rk);
-      if (v != v) v = __longlong_as_double(0x7ff0000000000000LL);
-      const unsigned long long key = used ? 0ull : (unsigned long long)__double_as_longlong(v) + 1ull;
-      const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-      const unsigned mhi = __reduce_max_sync(kFull, hi);
-      const unsigned mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-      const bool cand = hi == mhi && lo == mlo;
-      const int blg = (int)__reduce_min_sync(kFull, cand ? (unsigned)lg : 0xffffffffu);
-      const int bl = __ffs(__ballot_sync(kFull, cand && lg == blg)) - 1;
-      colk[par][lane] = rk;
-      if (lane == 0) {
-        sbl[par] = bl;
-        sidx[k] = blg;
-      }
-    }
-    __syncthreads();
-    const int bl = sbl[par];
-    const int blg = sidx[k];
-    const double2 pv = colk[par][bl];
-    if (pv.x == 0.0 && pv.y == 0.0 && inf == 0) inf = k + 1;
-    const double2 d = crecip(pv);
-    const double2 fd = cmul(colk[par][lane], d);
-    // both candidate values for every lane, then selects: no divergent path for the pivot lane
-    const bool isp = lane == bl;
-#pragma unroll
-    for (int cc = 0; cc < CW; ++cc) {
-      const int c = w * CW + cc;
-      double2 pc;
-      pc.x = __shfl_sync(kFull, r[cc].x, bl);
-      pc.y = __shfl_sync(kFull, r[cc].y, bl);
-      const double2 prow = cmul(pc, d);
-      const double2 upd = csub(r[cc], cmul(fd, pc));
-      double2 v = isp ? prow : (c < n ? upd : r[cc]);
-      if (c == k) v = isp ? d : make_double2(-fd.x, -fd.y);
-      r[cc] = v;
-    }
-    if (lg == k) lg = blg;
-    if (lane == bl) {
-      lg = k;
-      used = true;
-    }
-  }
-  // column interchanges in reverse pivot order: output column dest[c] takes internal column c
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kFull, v, o));
+  bad = __any_sync(kFull, bad);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = bad ? __longlong_as_double(0x7ff8000000000000LL) : v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < n; ++j) scm[j] = j;
-    for (int l = n - 1; l >= 0; --l) {
-      const int il = sidx[l];
-      if (il != l) {
-        const int t = scm[il];
-        scm[il] = scm[l];
-        scm[l] = t;
-      }
-    }
-    for (int j = 0; j < n; ++j) sidx[scm[j]] = j;
-  }
-  __syncthreads();
-  if (lane < n) {
-    double2* Xp = X + p * Q;
+  double m = red[0];
 #pragma unroll
-    for (int cc = 0; cc < CW; ++cc) {
-      const int c = w * CW + cc;
-      if (c < n) Xp[lg + (int64_t)sidx[c] * n] = r[cc];
-    }
-  }
-  if (threadIdx.x == 0) {
-    if (info) info[p] = inf;
-    if (status && inf != 0 && status[p] == 0) status[p] = singular_code;
-  }
+  for (int w = 1; w < kThreads / 32; ++w) m = (m != m || red[w] != red[w]) ? m + red[w] : fmax(m, red[w]);
+  return m;
 }
 
-// ---------------------------------------------------------------- decimation steps
-// Row `lane` of columns [w CW, (w + 1) CW) of A B, A and B n x n in shared
-// memory (the product of k_small_zgemm, for the fused decimation iteration below).
-template <int N>
-__device__ __forceinline__ void mm_rows(int n, const double2* sA, const double2* sB, double2 (&acc)[N / kWarps]) {
-  constexpr int CW = N / kWarps;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int jj = 0; jj < CW; ++jj) acc[jj] = make_double2(0.0, 0.0);
-  if (lane >= n) return;
-  for (int k = 0; k < n; ++k) {
-    const double2 a = sA[lane + k * n];
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj) {
-      const int j = w * CW + jj;
-      if (j < n) {
-        const double2 bv = sB[k + j * n];
-        acc[jj].x = fma(a.x, bv.x, acc[jj].x);
-        acc[jj].x = fma(-a.y, bv.y, acc[jj].x);
-        acc[jj].y = fma(a.x, bv.y, acc[jj].y);
-        acc[jj].y = fma(a.y, bv.x, acc[jj].y);
-      }
-    }
-  }
-}
-
-// Three n x n operands into shared memory: every thread issues all of its
-// global loads before its first shared store (one memory latency, not three).
-template <int N>
-__device__ __forceinline__ void stage3(int n, double2* d0, const double2* s0, double2* d1, const double2* s1,
-                                       double2* d2, const double2* s2) {
-  constexpr int R = (N * N + kWarps * 32 - 1) / (kWarps * 32);
-  const int nn = n * n;
-  double2 v0[R], v1[R], v2[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int q = threadIdx.x + i * kWarps * 32;
-    if (q < nn) {
-      v0[i] = __ldg(s0 + q);
-      v1[i] = __ldg(s1 + q);
-      v2[i] = __ldg(s2 + q);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int q = threadIdx.x + i * kWarps * 32;
-    if (q < nn) {
-      d0[q] = v0[i];
-      d1[q] = v1[i];
-      d2[q] = v2[i];
-    }
-  }
-}
-
-// One decimation iteration (src/contselfenergy.F90:271-340) for the points
-// list[b], b < *count, one CTA each, with Go, Co and Bo staged in shared
-// memory once: X = Go Co, C1 = Co X, the CPU convergence rule on max|C1| (a
-// point is done on its second consecutive max|C1| <= tol: ncyc = it; the
-// others go on to next[]), and for the points that go on Self = Bo X,
-// Ao -= Self, Aos -= Self, then Y = Go Bo (in X's place), B1 = Bo Y,
-// Ao -= Co Y.
-template <int N>
-__global__ void __launch_bounds__(kWarps * 32)
-    k_small_dec(int n, const int* list, const int* count, int P, const double2* Go, const double2* Co,
-                const double2* Bo, double2* C1, double2* B1, double2* Ao, double2* Aos, int64_t Q, int* ok,
-                int* ncyc_c, double tol, int it, int* next, int* next_count, int* redo) {
-  constexpr int CW = N / kWarps;
-  extern __shared__ __align__(16) double2 sdec[];
-  double2* sG = sdec;
-  double2* sC = sG + N * N;
-  double2* sB = sC + N * N;
-  double2* sX = sB + N * N;
-  __shared__ double smx[kWarps];
-  __shared__ int sgo;
-  const int b = blockIdx.x;
-  if (b >= min(*count, P)) return;
-  const int p = list[b];
-  const int64_t o = p * Q;
-  stage3<N>(n, sG, Go + o, sC, Co + o, sB, Bo + o);
+// Go = Ao^-1 (Ao kept), the residual probe and up to two Newton steps
+// Go + Go (I - Ao Go) where it exceeds kInvProbeTol (in the X block).
+// Returns 1 for an exactly zero pivot, + 2 where the condition estimate of Ao
+// exceeds kSensitiveCond.
+__device__ __noinline__ int small_inverse(int n) {
+  const Lane L(n);
+  const double2* const A = block(B_AO);
+  double2* const X = block(B_GO);
+  double2* const R = block(B_X);
+  SmallShared& sh = shared();
+  bool sens = false;
+  if (threadIdx.x == 0) sh.flag = 0;
   __syncthreads();
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2 acc[CW];
-  mm_rows<N>(n, sG, sC, acc);                      // X = Go Co
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj)
-      if (w * CW + jj < n) sX[lane + (w * CW + jj) * n] = acc[jj];
-  __syncthreads();
-  mm_rows<N>(n, sC, sX, acc);                      // C1 = Co X
-  double mx = 0.0;
-  bool bad = false;
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj) {
-      const int j = w * CW + jj;
-      if (j < n) {
-        C1[o + lane + j * n] = acc[jj];
-        const double h = hypot(acc[jj].x, acc[jj].y);
-        mx = fmax(mx, h);
-        bad |= !(h <= 1.7976931348623157e308);
-      }
-    }
-  for (int s = 16; s > 0; s >>= 1) mx = fmax(mx, __shfl_xor_sync(kFull, mx, s));
-  if (__any_sync(kFull, bad)) mx = __longlong_as_double(0x7ff8000000000000LL);
-  if (lane == 0) smx[w] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = smx[0];
-    for (int q = 1; q < kWarps; ++q) m = (m != m || smx[q] != smx[q]) ? m + smx[q] : fmax(m, smx[q]);
-    bool go = true;
-    if (!(m <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge; run it again
-      go = false;
-      ncyc_c[p] = it;
-      if (redo) redo[p] = 1;
-    } else if (m <= tol) {
-      if (ok[p]) {
-        go = false;
-        ncyc_c[p] = it;
-      }
-      ok[p] = 1;
-    } else {
-      ok[p] = 0;
-    }
-    if (go) next[atomicAdd(next_count, 1)] = p;
-    sgo = go;
-  }
-  __syncthreads();
-  if (!sgo) return;
-  mm_rows<N>(n, sB, sX, acc);                      // Self = Bo X
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj) {
-      const int j = w * CW + jj;
-      if (j < n) {
-        const int64_t q = o + lane + j * n;
-        Ao[q] = csub(Ao[q], acc[jj]);
-        Aos[q] = csub(Aos[q], acc[jj]);
-      }
-    }
-  __syncthreads();                                 // X is read; Y takes its place
-  mm_rows<N>(n, sG, sB, acc);                      // Y = Go Bo
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj)
-      if (w * CW + jj < n) sX[lane + (w * CW + jj) * n] = acc[jj];
-  __syncthreads();
-  mm_rows<N>(n, sB, sX, acc);                      // B1 = Bo Y
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj)
-      if (w * CW + jj < n) B1[o + lane + (w * CW + jj) * n] = acc[jj];
-  mm_rows<N>(n, sC, sX, acc);                      // Ao -= Co Y
-  if (lane < n)
-#pragma unroll
-    for (int jj = 0; jj < CW; ++jj) {
-      const int j = w * CW + jj;
-      if (j < n) Ao[o + lane + j * n] = csub(Ao[o + lane + j * n], acc[jj]);
-    }
-}
-
-// Dynamic shared memory above the 48 KB default needs an opt-in per device.
-template <typename K>
-cudaError_t opt_in(K kernel, size_t smem, bool (&done)[64], std::mutex& mu) {
-  if (smem <= 48 * 1024) return cudaSuccess;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
-  return e;
-}
-
-// Residual probe of the inverse X of A and up to two Newton steps
-// X <- X + X (I - A X) where it exceeds kInvProbeTol (cta_inv_probe, the
-// engine's refine block), one CTA per problem with A, X and I - A X staged
-// in shared memory.  A problem whose probe passes costs two matrix-vector
-// products and leaves X untouched.
-template <int N>
-__global__ void __launch_bounds__(kWarps * 32)
-    k_small_refine(int batch, int n, const double2* A, double2* X, int64_t Q, const int* map, const int* count,
-                   int* sens) {
-  extern __shared__ __align__(16) double2 sref[];
-  double2* sA = sref;
-  double2* sX = sA + N * N;
-  double2* sR = sX + N * N;
-  double2* y = sR + N * N;
-  __shared__ double red[kWarps], redk[kWarps];
-  const int b = blockIdx.x;
-  if (b >= batch_limit(batch, count)) return;
-  const int p = map ? map[b] : b;
-  const int nn = n * n;
-  const double2* Ap = A + p * Q;
-  double2* Xp = X + p * Q;
-  for (int q = threadIdx.x; q < nn; q += kWarps * 32) {
-    sA[q] = Ap[q];
-    sX[q] = Xp[q];
-  }
-  __syncthreads();
-  bool changed = false;
+  gj_panel<1, 4, true>(A, kLd, X, kLd, n, 0, n, block(kBlocks), sh.inv);
+  const int info = sh.flag != 0 ? 1 : 0;
+  // probe: threads (row, group of columns) = (tid / 8, tid mod 8)
+  const int r = threadIdx.x >> 3, grp = threadIdx.x & 7;
   for (int round = 0; round < 2; ++round) {
-    // probe: y = X v, then max |A y - v|
-    for (int r = threadIdx.x; r < n; r += kWarps * 32) {
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < n; ++c) acc = cadd(acc, cmul(sX[r + c * n], probe_v(c)));
-      y[r] = acc;
+    double2 acc = make_double2(0.0, 0.0);
+    if (r < n)
+      for (int c = grp; c < n; c += 8) acc = cadd(acc, cmul(X[r + c * kLd], probe_v(c)));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      acc.x += __shfl_xor_sync(kFull, acc.x, o);
+      acc.y += __shfl_xor_sync(kFull, acc.y, o);
     }
+    if (grp == 0 && r < n) sh.y[r] = acc;
     __syncthreads();
-    double e = 0.0, kap = 0.0;
-    for (int r = threadIdx.x; r < n; r += kWarps * 32) {
-      double2 acc = make_double2(0.0, 0.0);
-      double sa = 0.0;
-      for (int c = 0; c < n; ++c) {
-        acc = cadd(acc, cmul(sA[r + c * n], y[c]));
-        sa += cabs1(sA[r + c * n]) * cabs1(y[c]);
+    acc = make_double2(0.0, 0.0);
+    double sa = 0.0;
+    if (r < n)
+      for (int c = grp; c < n; c += 8) {
+        const double2 a = A[r + c * kLd], y = sh.y[c];
+        acc = cadd(acc, cmul(a, y));
+        sa += cabs1(a) * cabs1(y);
       }
-      const double d = cabs(csub(acc, probe_v(r)));
-      e = (d <= 1.7976931348623157e308) ? fmax(e, d) : __longlong_as_double(0x7ff0000000000000LL);
-      kap = fmax(kap, sa);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      acc.x += __shfl_xor_sync(kFull, acc.x, o);
+      acc.y += __shfl_xor_sync(kFull, acc.y, o);
+      sa += __shfl_xor_sync(kFull, sa, o);
     }
+    double e = 0.0;
+    if (r < n) {
+      const double2 d = csub(acc, probe_v(r));
+      e = cabs1(d);   // an upper bound of |d| within sqrt 2
+      if (!(e <= 1.7976931348623157e308)) e = __longlong_as_double(0x7ff0000000000000LL);
+      else if (e > kInvProbeTol) e = cabs(d);
+    } else {
+      sa = 0.0;
+    }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       e = fmax(e, __shfl_xor_sync(kFull, e, o));
-      kap = fmax(kap, __shfl_xor_sync(kFull, kap, o));
+      sa = fmax(sa, __shfl_xor_sync(kFull, sa, o));
     }
     if ((threadIdx.x & 31) == 0) {
-      red[threadIdx.x >> 5] = e;
-      redk[threadIdx.x >> 5] = kap;
+      sh.red[0][threadIdx.x >> 5] = e;
+      sh.red[1][threadIdx.x >> 5] = sa;
     }
     __syncthreads();
     double em = 0.0, km = 0.0;
-    for (int q = 0; q < kWarps; ++q) {
-      em = fmax(em, red[q]);
-      km = fmax(km, redk[q]);
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+      em = fmax(em, sh.red[0][w]);
+      km = fmax(km, sh.red[1][w]);
     }
-    __syncthreads();
-    // the condition estimate of the unrefined inverse marks a nearly singular matrix
-    if (round == 0 && km > kSensitiveCond && sens && threadIdx.x == 0) sens[p] = 1;
+    if (round == 0 && km > kSensitiveCond) sens = true;
     if (!(em > kInvProbeTol) || !(em <= 1.7976931348623157e308)) break;
-    // R = I - A X
-    for (int q = threadIdx.x; q < nn; q += kWarps * 32) {
-      const int i = q % n, j = q / n;
-      double2 acc = make_double2(i == j ? 1.0 : 0.0, 0.0);
-      for (int k = 0; k < n; ++k) acc = csub(acc, cmul(sA[i + k * n], sX[k + j * n]));
-      sR[q] = acc;
-    }
+    Frag p = mm(L, A, X);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      p.v[q] = csub(make_double2(L.row(q) == L.col(q) ? 1.0 : 0.0, 0.0), p.v[q]);
+    put(L, R, p);
     __syncthreads();
-    // X + X R, element by element into registers, then back into sX
-    double2 nx[N * N / (kWarps * 32) + 1];
-    int cnt = 0;
-    for (int q = threadIdx.x; q < nn; q += kWarps * 32, ++cnt) {
-      const int i = q % n, j = q / n;
-      double2 acc = sX[q];
-      for (int k = 0; k < n; ++k) acc = cadd(acc, cmul(sX[i + k * n], sR[k + j * n]));
-      nx[cnt] = acc;
-    }
+    p = mm(L, X, R);
     __syncthreads();
-    cnt = 0;
-    for (int q = threadIdx.x; q < nn; q += kWarps * 32, ++cnt) sX[q] = nx[cnt];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (L.in(q)) X[L.at(q)] = cadd(X[L.at(q)], p.v[q]);
     __syncthreads();
-    changed = true;
   }
-  if (changed)
-    for (int q = threadIdx.x; q < nn; q += kWarps * 32) Xp[q] = sX[q];
+  return info + (sens ? 2 : 0);
+}
+
+// D = z S - H (S null: the identity if diag, else zero) for an n x n block
+// in memory; with dag its conjugate transpose.
+__device__ __forceinline__ void load_esh(int n, double2* D, const double2* H, const double2* S, double2 z, bool diag,
+                                         bool dag) {
+  for (int q = threadIdx.x; q < n * n; q += kThreads) {
+    const int i = q % n, j = q / n;
+    const double2 s = S ? S[q] : make_double2(diag && i == j ? 1.0 : 0.0, 0.0);
+    const double2 v = csub(cmul(z, s), H[q]);
+    if (dag) D[j + i * kLd] = cconj(v);
+    else D[i + j * kLd] = v;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
+  double2* const Ao = block(B_AO);
+  double2* const Bo = block(B_BO);
+  double2* const Co = block(B_CO);
+  double2* const Go = block(B_GO);
+  double2* const X = block(B_X);
+  double2* const SL = block(B_SL);               // the left self-energy
+  SmallShared& sh = shared();
+  const int p = blockIdx.x, n = a.n;
+  const Lane L(n);
+  if (threadIdx.x == 0) {
+    sh.inv.piv = sh.piv;
+    sh.inv.perm = sh.perm;
+    sh.inv.cperm = sh.cperm;
+    sh.inv.flag = &sh.flag;
+    sh.inv.redv = nullptr;
+    sh.inv.redi = nullptr;
+    sh.inv.tr.acc = nullptr;
+  }
+  for (int q = threadIdx.x; q < kBlocks * kBlk; q += kThreads) Ao[q] = make_double2(0.0, 0.0);
+  __syncthreads();
+  const DevDesc& d = a.d_descs[a.d_ids[p]];
+  const double E = a.d_E[p];
+  int st = NEGF_B200_OK, ncyc = 0;
+  auto put_st = [&](int code) { if (st == NEGF_B200_OK) st = code; };
+
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const int c = side == 0 ? a.left : a.right;
+    const double2* h00 = d.h00 + d.olead[c];
+    const double2* h01 = d.h01 + d.olead[c];
+    const double2* s00 = d.has_s00 ? d.s00 + d.olead[c] : nullptr;
+    const double2* s01 = d.has_s01 ? d.s01 + d.olead[c] : nullptr;
+    int cyc = 0;
+    bool have = false;                           // a sensitive attempt's gs is kept for comparison
+    Frag kept;
+#pragma unroll 1
+    for (int att = 0;; ++att) {
+      // ---- decimation from the contact energy times 1 + att 2^-50 (see kDecRetries)
+      const double scale = 1.0 + att * 0x1p-50;
+      const double2 ec = make_double2(E * scale, a.eta * scale);
+      load_esh(n, Ao, h00, s00, ec, true, false);
+      load_esh(n, Bo, h01, s01, ec, false, false);
+      load_esh(n, Co, h01, s01, cconj(ec), false, true);
+      __syncthreads();
+      Frag Aos = get(L, Ao);
+      bool ok = false, done = false, sens = false, redo = false;
+      cyc = 0;
+      int it = 1;
+#pragma unroll 1
+      for (; it <= a.sgf_max_iter; ++it) {
+        const int bad_inv = small_inverse(n);
+        if (bad_inv & 1) put_st(NEGF_B200_ERR_SINGULAR);
+        sens |= (bad_inv & 2) != 0;
+        __syncthreads();
+        put(L, X, mm(L, Go, Co));
+        __syncthreads();
+        const Frag C1 = mm(L, Co, X);
+        double mx = 0.0;
+        bool bad = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (L.in(q)) {
+            const double h = hypot(C1.v[q].x, C1.v[q].y);
+            mx = fmax(mx, h);
+            bad |= !(h <= 1.7976931348623157e308);
+          }
+        mx = cta_max_nan(bad ? __longlong_as_double(0x7ff8000000000000LL) : mx, sh.red[2]);
+        if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge; run it again
+          redo = done = true;
+        } else if (mx <= a.sgf_tol) {
+          done = ok;
+          ok = true;
+        } else {
+          ok = false;
+        }
+        if (done) {
+          cyc = it;
+          break;
+        }
+        Frag f = mm(L, Bo, X);                   // Self
+#pragma unroll
+        for (int q = 0; q < 4; ++q) Aos.v[q] = csub(Aos.v[q], f.v[q]);
+        sub_from(L, Ao, f);
+        __syncthreads();                         // X is read; Y takes its place
+        put(L, X, mm(L, Go, Bo));
+        __syncthreads();
+        const Frag B1 = mm(L, Bo, X);
+        f = mm(L, Co, X);
+        sub_from(L, Ao, f);
+        __syncthreads();
+        put(L, Bo, B1);
+        put(L, Co, C1);
+        __syncthreads();
+      }
+      if (!done) {
+        cyc = a.sgf_max_iter + 1;
+        put_st(NEGF_B200_ERR_NOT_CONVERGED);
+      }
+      __syncthreads();
+      put(L, Ao, Aos);
+      __syncthreads();
+      const int bad_gs = small_inverse(n);       // gs in Go
+      if (bad_gs & 1) put_st(NEGF_B200_ERR_SINGULAR);
+      sens |= (bad_gs & 2) != 0;
+      __syncthreads();
+      if (!(a.eta > 0.0)) break;
+      // the retarded branch has -Im gs_ii >= 0 up to 1e-6 of the largest |gs_ii|
+      double lo = 1.7976931348623157e308, hi = 0.0;
+      for (int i = 0; i < n; ++i) {
+        const double2 g = Go[i * (kLd + 1)];
+        const double h = cabs(g);
+        if (!(h <= 1.7976931348623157e308)) redo = true;
+        else {
+          lo = fmin(lo, -g.y);
+          hi = fmax(hi, h);
+        }
+      }
+      if (hi > 0.0 && lo < -1e-6 * hi) redo = true;
+      if (!redo && !sens) break;
+      if (!redo) {   // sensitive: accepted once two attempts reach the same gs
+        const Frag gs = get(L, Go);
+        if (have) {
+          double df = 0.0, mk = 0.0;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            df = fmax(df, cabs(csub(gs.v[q], kept.v[q])));
+            mk = fmax(mk, cabs(kept.v[q]));
+          }
+          df = cta_max_nan(df, sh.red[0]);
+          mk = cta_max_nan(mk, sh.red[1]);
+          __syncthreads();
+          if (df <= 1e-2 * mk) break;
+        }
+        if (att < kDecRetries) {
+          kept = gs;
+          have = true;
+        }
+      }
+      if (att >= kDecRetries) {
+        cyc = a.sgf_max_iter + 1;
+        put_st(NEGF_B200_ERR_NOT_CONVERGED);
+        break;
+      }
+      __syncthreads();
+    }
+    ncyc += cyc;
+    // ---- Sigma = Tlc gs Tcl
+    const double2 ec = make_double2(E, a.eta);
+    const double2* hmc = d.hmc + d.omc[c];
+    const double2* smc = d.has_smc ? d.smc + d.omc[c] : nullptr;
+    load_esh(n, Bo, hmc, smc, ec, false, false);
+    load_esh(n, Co, hmc, smc, cconj(ec), false, true);
+    __syncthreads();
+    put(L, X, mm(L, Bo, Go));
+    __syncthreads();
+    const Frag sig = mm(L, X, Co);
+    if (side == 0) {
+      put(L, SL, sig);
+    } else {
+      // W = ESH(nbl, nbl) - Sigma_right
+      load_esh(n, Ao, d.hd + d.od[a.nbl - 1], d.has_s ? d.sd + d.od[a.nbl - 1] : nullptr, make_double2(E, 0.0), true,
+               false);
+      __syncthreads();
+      sub_from(L, Ao, sig);
+    }
+    __syncthreads();
+  }
+  // ---- gsmr sweep down to Gr(1,1): g in Go
+  if (small_inverse(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
+#pragma unroll 1
+  for (int i = a.nbl - 2; i >= 0; --i) {
+    const double2 e = make_double2(E, 0.0);
+    __syncthreads();
+    load_esh(n, Bo, d.hu + d.oo[i], d.has_s ? d.su + d.oo[i] : nullptr, e, false, false);
+    load_esh(n, Co, d.hl + d.oo[i], d.has_s ? d.sl + d.oo[i] : nullptr, e, false, false);
+    load_esh(n, Ao, d.hd + d.od[i], d.has_s ? d.sd + d.od[i] : nullptr, e, true, false);
+    __syncthreads();
+    put(L, X, mm(L, Bo, Go));
+    if (i == 0) sub_from(L, Ao, get(L, SL));
+    __syncthreads();
+    sub_from(L, Ao, mm(L, X, Co));
+    __syncthreads();
+    if (small_inverse(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
+  }
+  __syncthreads();
+  // ---- Gamma = i (Sigma - Sigma^dag) of the left contact, then the trace
+  //   T = |Re Tr[Gam i(G - G^dag)] - Re Tr[Gam G Gam G^dag]|,
+  //   Tr[Gam G Gam G^dag] = sum (Gam G)_ij conj(G Gam)_ij
+  double t1 = 0.0, t2 = 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (L.in(q)) {
+      const int i = L.row(q), j = L.col(q);
+      const double2 s = SL[i + j * kLd], u = SL[j + i * kLd];
+      const double2 gam = make_double2(-(s.y + u.y), s.x - u.x);
+      Bo[i + j * kLd] = gam;
+      const double2 gji = Go[j + i * kLd], gij = Go[i + j * kLd];
+      t1 += gam.x * -(gji.y + gij.y) - gam.y * (gji.x - gij.x);   // Re(Gam_ij i (G_ji - conj G_ij))
+    }
+  __syncthreads();
+  const Frag M = mm(L, Bo, Go), N = mm(L, Go, Bo);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (L.in(q)) t2 += M.v[q].x * N.v[q].x + M.v[q].y * N.v[q].y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t1 += __shfl_xor_sync(kFull, t1, o);
+    t2 += __shfl_xor_sync(kFull, t2, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh.red[0][threadIdx.x >> 5] = t1;
+    sh.red[1][threadIdx.x >> 5] = t2;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t1 = t2 = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      t1 += sh.red[0][w];
+      t2 += sh.red[1][w];
+    }
+    const double T = fabs(t1 - t2);
+    a.d_T[p] = T;
+    if (a.d_ncyc) a.d_ncyc[p] = ncyc;
+    // a non-finite T that no step flagged (NaN in the device blocks) is reported as such
+    if (a.d_status) a.d_status[p] = (st == NEGF_B200_OK && !isfinite(T)) ? NEGF_B200_ERR_NONFINITE : st;
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_small_refine(int batch, int n, const double2* A, double2* X, int64_t Q, const int* map,
-                                const int* count, cudaStream_t s, int* sens) {
-  if (batch <= 0) return cudaSuccess;
-  if (n < 1 || n > kSmallMax) return cudaErrorInvalidValue;
-  if (n <= 16) {
-    const size_t smem = (3 * 16 * 16 + 16) * sizeof(double2);
-    k_small_refine<16><<<batch, kWarps * 32, smem, s>>>(batch, n, A, X, Q, map, count, sens);
-  } else {
-    const size_t smem = (3 * 32 * 32 + 32) * sizeof(double2);   // above the 48 KB default: opt in per device
-    static std::mutex mu;
-    static bool attr[64] = {false};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(mu);
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(k_small_refine<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
-    k_small_refine<32><<<batch, kWarps * 32, smem, s>>>(batch, n, A, X, Q, map, count, sens);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_small_dec(int P, int n, const int* list, const int* count, const double2* Go, const double2* Co,
-                             const double2* Bo, double2* C1, double2* B1, double2* Ao, double2* Aos, int64_t Q, int* ok,
-                             int* ncyc_c, double tol, int it, int* next, int* next_count, int* redo, cudaStream_t s) {
-  if (P <= 0) return cudaSuccess;
-  if (n < 1 || n > kSmallMax) return cudaErrorInvalidValue;
-  static std::mutex mu;
-  static bool done16[64] = {false}, done32[64] = {false};
-  if (n <= 16) {
-    const size_t smem = 4 * 16 * 16 * sizeof(double2);
-    cudaError_t e = opt_in(k_small_dec<16>, smem, done16, mu);
-    if (e != cudaSuccess) return e;
-    k_small_dec<16><<<P, kWarps * 32, smem, s>>>(n, list, count, P, Go, Co, Bo, C1, B1, Ao, Aos, Q, ok, ncyc_c, tol,
-                                                 it, next, next_count, redo);
-  } else {
-    const size_t smem = 4 * 32 * 32 * sizeof(double2);
-    cudaError_t e = opt_in(k_small_dec<32>, smem, done32, mu);
-    if (e != cudaSuccess) return e;
-    k_small_dec<32><<<P, kWarps * 32, smem, s>>>(n, list, count, P, Go, Co, Bo, C1, B1, Ao, Aos, Q, ok, ncyc_c, tol,
-                                                 it, next, next_count, redo);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_small_zgemm(int batch, int n, double2 alpha, const double2* A, const double2* B, double2 beta,
-                               double2* C, int64_t Q, const int* map, const int* count, double* maxabs,
-                               cudaStream_t s) {
-  if (batch <= 0) return cudaSuccess;
-  if (n < 1 || n > kSmallMax) return cudaErrorInvalidValue;
-  if (n <= 16)
-    k_small_zgemm<16><<<batch, kWarps * 32, 0, s>>>(batch, n, alpha, A, B, beta, C, Q, map, count, maxabs);
-  else
-    k_small_zgemm<32><<<batch, kWarps * 32, 0, s>>>(batch, n, alpha, A, B, beta, C, Q, map, count, maxabs);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_small_zinv(int batch, int n, const double2* A, double2* X, int64_t Q, const int* map,
-                              const int* count, int* info, int* status, int singular_code, cudaStream_t s) {
-  if (batch <= 0) return cudaSuccess;
-  if (n < 1 || n > kSmallMax) return cudaErrorInvalidValue;
-  if (n <= 16)
-    k_small_zinv<16><<<batch, kWarps * 32, 0, s>>>(batch, n, A, X, Q, map, count, info, status, singular_code);
-  else
-    k_small_zinv<32><<<batch, kWarps * 32, 0, s>>>(batch, n, A, X, Q, map, count, info, status, singular_code);
-  return cudaGetLastError();
+cudaError_t launch_small_points(const MixedArgs& a, cudaStream_t s) {
+  if (a.npts <= 0) return cudaSuccess;
+  if (a.n < 1 || a.n > kSmallMax) return cudaErrorInvalidValue;
+  cudaError_t e = team_opt_in((const void*)k_small_point, kSmallSmem);
+  if (e != cudaSuccess) return e;
+  k_small_point<<<a.npts, kThreads, kSmallSmem, s>>>(a);
+  e = cudaGetLastError();
+  if (e == cudaSuccess && a.launches) ++*a.launches;
+  return e;
 }
 
 }  // namespace negf
