@@ -1204,8 +1204,8 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
     const cudaError_t e = negf::launch_small_points(a, s);
     return e == cudaSuccess ? NEGF_B200_OK : cuda_fail(ctx, e, "lock step");
   }
-  // two full waves of the inversion (two CTAs per SM: 592 points on a B200)
-  int batch = std::min<int>(npts, 4 * std::max(ctx->sms, 1));
+  // the contacts of a batch fill two waves of the inversion (two CTAs per SM: 296 points on a B200)
+  int batch = std::min<int>(npts, 2 * std::max(ctx->sms, 1));
   if (ctx->ws_limit) batch = std::min(batch, negf::mixed_batch_for(ctx->ws_limit, n, slices));
   if (batch < 1) return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
   for (;;) {
@@ -1745,7 +1745,7 @@ int negf_b200_zgemm_batched(int32_t batch, int32_t m, int32_t n, int32_t k, cons
 size_t negf_b200_zgemm_i8_work_bytes(int32_t batch, int32_t m, int32_t n, int32_t k, int32_t slices) {
   if (batch <= 0 || m <= 0 || n <= 0 || k <= 0 || slices < negf::kOzMinSlices || slices > negf::kOzMaxSlices)
     return 0;
-  return negf::ozaki_layout(batch, m, n, k, slices).total + 256;
+  return negf::ozaki_work_bytes(batch, m, n, k, slices) + 256;
 }
 
 int negf_b200_zgemm_batched_i8(int32_t batch, int32_t m, int32_t n, int32_t k, const double* alpha,

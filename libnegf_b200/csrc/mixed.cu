@@ -8,7 +8,8 @@
 // decimation's convergence test on max|C1|, the inverses, and the Caroli
 // trace (whose two products are FP64 tensor-core products).
 //
-// Steps per batch, following the reference routine by routine:
+// Steps per batch, following the reference routine by routine (the contacts
+// of every point are problems of their own in the first two):
 //   surface_green + decimation      src/contselfenergy.F90:184-210, 271-340
 //     (lock step over the points still iterating; a point leaves the active
 //     set on its second consecutive max|C1| <= SGFACC, as the CPU rule)
@@ -27,7 +28,7 @@
 namespace negf {
 namespace {
 
-constexpr int kBlocks = 14;   // n x n complex work blocks per point (the 14th: a kept surface GF)
+constexpr int kBlocks = 11;   // n x n complex work blocks per problem (contact of a point)
 
 __device__ __forceinline__ double2 cmulm(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -35,12 +36,15 @@ __device__ __forceinline__ double2 cmulm(double2 a, double2 b) {
 __device__ __forceinline__ double2 conjm(double2 a) { return make_double2(a.x, -a.y); }
 
 // Ao = Ec S00 - H00, Aos = Ao, Bo = Ec S01 - H01, Co = (conj(Ec) S01 - H01)^dag,
-// Ec = (E + i eta) scale, for the points map[b] (map null: b)
-__global__ void k_lead_init(int n, int c, const int* ids, const double* E, double eta, double scale, const int* map,
-                            const DevDesc* descs, double2* Ao, double2* Aos, double2* Bo, double2* Co, int64_t Q) {
+// Ec = (E + i eta) scale, for the problems map[b] (map null: b); problem p <
+// P is contact `left` of point p, problem P + p contact `right`
+__global__ void k_lead_init(int n, int P, int left, int right, const int* ids, const double* E, double eta,
+                            double scale, const int* map, const DevDesc* descs, double2* Ao, double2* Aos, double2* Bo,
+                            double2* Co, int64_t Q) {
   const int p = map ? map[blockIdx.y] : blockIdx.y;
-  const DevDesc& d = descs[ids[p]];
-  const double2 ec = make_double2(E[p] * scale, eta * scale);
+  const int pt = p < P ? p : p - P, c = p < P ? left : right;
+  const DevDesc& d = descs[ids[pt]];
+  const double2 ec = make_double2(E[pt] * scale, eta * scale);
   const int64_t ol = d.olead[c], nn = (int64_t)n * n;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nn; q += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(q % n), j = (int)(q / n);
@@ -119,12 +123,14 @@ __global__ void k_info_to_status(int nb, const int* list, const int* info, int* 
   }
 }
 
-// Tlc = Ec SMC - HMC (n x L), Tcl = (conj(Ec) SMC - HMC)^dag (L x n); here L = n
-__global__ void k_tlc(int n, int c, const int* ids, const double* E, double eta, const DevDesc* descs,
-                      double2* Tlc, double2* Tcl, int64_t Q) {
+// Tlc = Ec SMC - HMC (n x L), Tcl = (conj(Ec) SMC - HMC)^dag (L x n); here L =
+// n.  Problems as in k_lead_init.
+__global__ void k_tlc(int n, int P, int left, int right, const int* ids, const double* E, double eta,
+                      const DevDesc* descs, double2* Tlc, double2* Tcl, int64_t Q) {
   const int p = blockIdx.y;
-  const DevDesc& d = descs[ids[p]];
-  const double2 ec = make_double2(E[p], eta);
+  const int pt = p < P ? p : p - P, c = p < P ? left : right;
+  const DevDesc& d = descs[ids[pt]];
+  const double2 ec = make_double2(E[pt], eta);
   const int64_t om = d.omc[c], nn = (int64_t)n * n;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nn; q += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(q % n), j = (int)(q / n);
@@ -357,35 +363,51 @@ struct Carver {
 struct Ws {
   double2* blk[kBlocks];
   double* mx;
-  int *ok, *ncl, *ncr, *list0, *list1, *count, *info, *pst, *redo, *sub, *sens, *agree;
+  int *ok, *nc, *list0, *list1, *count, *info, *pst, *pst2, *redo, *sub, *sens, *agree;
   double* tb;
   double2* zwork;
-  void* oz;
+  OzakiSet rows[3], cols;      // digits of three left operands and a right one
+  double* t0;
 };
 
 Ws carve(void* base, int P, int n, int slices, size_t* total) {
   Carver c{static_cast<char*>(base)};
   Ws w;
-  const size_t Q = (size_t)n * n;
-  for (int b = 0; b < kBlocks; ++b) w.blk[b] = c.take<double2>((size_t)P * Q);
-  w.mx = c.take<double>(P);
-  w.ok = c.take<int>(P);
-  w.ncl = c.take<int>(P);
-  w.ncr = c.take<int>(P);
-  w.list0 = c.take<int>(P);
-  w.list1 = c.take<int>(P);
+  const size_t Q = (size_t)n * n, N = 2 * (size_t)P;   // problems: the contacts of every point
+  for (int b = 0; b < kBlocks; ++b) w.blk[b] = c.take<double2>(N * Q);
+  w.mx = c.take<double>(N);
+  w.ok = c.take<int>(N);
+  w.nc = c.take<int>(N);
+  w.list0 = c.take<int>(N);
+  w.list1 = c.take<int>(N);
   w.count = c.take<int>(4);
-  w.info = c.take<int>(P);
+  w.info = c.take<int>(N);
   w.pst = c.take<int>(P);
+  w.pst2 = c.take<int>(N);
   w.tb = c.take<double>(P);
-  w.redo = c.take<int>(P);
-  w.sub = c.take<int>(P);
-  w.sens = c.take<int>(P);
-  w.agree = c.take<int>(P);
-  w.zwork = c.take<double2>((size_t)P * zinv_batched_work_elems(n) + 1);
-  w.oz = c.take<uint8_t>(ozaki_layout(P, n, n, n, slices).total);
+  w.redo = c.take<int>(N);
+  w.sub = c.take<int>(N);
+  w.sens = c.take<int>(N);
+  w.agree = c.take<int>(N);
+  w.zwork = c.take<double2>(N * zinv_batched_work_elems(n) + 1);
+  for (int i = 0; i < 3; ++i) {
+    uint8_t* q = c.take<uint8_t>(ozaki_rows_bytes((int)N, n, n, slices));
+    if (base) w.rows[i] = ozaki_rows_at(q, (int)N, n, n, slices);
+  }
+  uint8_t* q = c.take<uint8_t>(ozaki_cols_bytes((int)N, n, n, slices));
+  if (base) w.cols = ozaki_cols_at(q, (int)N, n, n, slices);
+  w.t0 = c.take<double>(N * Q);
   *total = c.off + 256;
   return w;
+}
+
+// The status of a point after its two decimations: a product's code (3, 7) of
+// the right one, else the left one's, else the right one's.
+__global__ void k_merge_status(int P, const int* both, int* pst) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
+    const int l = both[p], r = both[P + p];
+    pst[p] = (r == NEGF_B200_ERR_NONFINITE || r == NEGF_B200_ERR_TIMEOUT || l == 0) ? r : l;
+  }
 }
 
 __global__ void k_finish(int P, const int* ncl, const int* ncr, const int* pst, const double* Tb, double* T,
@@ -442,12 +464,23 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
     int r_ = ck((x), what);      \
     if (r_) return r_;           \
   } while (0)
-  // products and inverses of the problems map[b], b < nb
+  // Products and inverses of the problems map[b], b < nb.  An operand is split
+  // into digits once for all the products it takes part in: of a decimation
+  // iteration's six products, three left and four right operands.
   uint64_t nl = 0;                 // kernels launched (reported through a.launches)
-  auto prod = [&](int nb, const int* map, double2 alpha, const double2* A, const double2* Bm, double2 beta, double2* C,
-                  double* maxabs) -> cudaError_t {
-    nl += 3;                       // digit split of A, of B, the product
-    return launch_ozaki_zgemm(nb, n, n, n, alpha, A, Q, Bm, Q, beta, C, Q, a.slices, w.oz, maxabs, w.pst, s, map);
+  auto rows = [&](int nb, const int* map, const double2* A, int set) -> cudaError_t {
+    ++nl;
+    return launch_ozaki_rows(nb, n, n, A, Q, a.slices, w.rows[set], s, map);
+  };
+  auto cols = [&](int nb, const int* map, const double2* Bm) -> cudaError_t {
+    ++nl;
+    return launch_ozaki_cols(nb, n, n, Bm, Q, a.slices, w.cols, s, map);
+  };
+  auto prod = [&](int nb, const int* map, double2 alpha, int set, double2 beta, double2* C, double* maxabs,
+                  int* status) -> cudaError_t {
+    ++nl;
+    return launch_ozaki_product(nb, n, n, n, alpha, w.rows[set], w.cols, beta, C, Q, a.slices, w.t0, maxabs, status,
+                                s, map);
   };
   auto inv = [&](int nb, const int* map, const double2* A, double2* X) -> cudaError_t {
     ++nl;
@@ -458,25 +491,26 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
     ++nl;
     return launch_zgemm_batched(nb, n, n, n, one, A, Q, Bm, Q, zero, C, Q, 0, s);
   };
+  double2 *gs = B[9], *sig = B[10], *kept_gs = B[10];   // (a kept gs is done with before the self-energies)
 
   for (int p0 = 0; p0 < a.npts; p0 += batch) {
-    const int P = std::min(batch, a.npts - p0);
+    const int P = std::min(batch, a.npts - p0), N = 2 * P;
     const int* ids = a.d_ids + p0;
     const double* E = a.d_E + p0;
-    MCK(cudaMemsetAsync(w.pst, 0, sizeof(int) * P, s), "memset status");
-    // ---- surface Green's function of each contact (B9 left, B10 right)
-    // decimation of contact `side` for the points sub[b], b < nsub (sub null:
-    // all P), the contact energy scaled by `scale`; then gs = Aos^-1 and the
+    MCK(cudaMemsetAsync(w.pst2, 0, sizeof(int) * N, s), "memset status");
+    // ---- surface Green's functions of both contacts of every point (problem
+    // p: left contact of point p, P + p: right), all in lock step.
+    // Decimation of the problems sub[b], b < nsub (sub null: all N), the
+    // contact energy scaled by `scale`; then gs = Aos^-1 and the
     // retarded-branch check (redo[p] = 1 where it fails)
-    auto decimate = [&](int side, const int* sub, int nsub, double scale) -> int {
-      const int c = side == 0 ? a.left : a.right;
-      int* ncyc_c = side == 0 ? w.ncl : w.ncr;
+    auto decimate = [&](const int* sub, int nsub, double scale) -> int {
       double2 *Ao = B[0], *Aos = B[1], *Bo = B[2], *Co = B[3], *Go = B[4], *X = B[5], *C1 = B[6], *Y = B[7],
               *B1 = B[8];
-      k_lead_init<<<dim3(gx, nsub), eb, 0, s>>>(n, c, ids, E, a.eta, scale, sub, a.d_descs, Ao, Aos, Bo, Co, Q);
+      k_lead_init<<<dim3(gx, nsub), eb, 0, s>>>(n, P, a.left, a.right, ids, E, a.eta, scale, sub, a.d_descs, Ao, Aos,
+                                                Bo, Co, Q);
       ++nl;
       MCK(cudaGetLastError(), "lead init");
-      k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, ncyc_c, w.list0, w.sens);
+      k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, w.nc, w.list0, w.sens);
       ++nl;
       int na = nsub;                                   // host bound of the active list
       int* cur = w.list0;
@@ -485,11 +519,15 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
       for (; it <= a.sgf_max_iter && na > 0; ++it) {
         // one batched product per step, the active list compacted on the host
         MCK(inv(na, cur, Ao, Go), "zinv");
-        k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
+        k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.info, w.pst2, NEGF_B200_ERR_SINGULAR);
         ++nl;
-        MCK(prod(na, cur, one, Go, Co, zero, X, nullptr), "GoXCo");
-        MCK(prod(na, cur, one, Co, X, zero, C1, w.mx), "C1");
-        k_dec_check<<<1, 1024, 0, s>>>(na, cur, w.mx, w.ok, ncyc_c, a.sgf_tol, it, nxt, w.count, w.redo);
+        MCK(rows(na, cur, Go, 0), "split Go");
+        MCK(cols(na, cur, Co), "split Co");
+        MCK(prod(na, cur, one, 0, zero, X, nullptr, w.pst2), "GoXCo");
+        MCK(rows(na, cur, Co, 1), "split Co");
+        MCK(cols(na, cur, X), "split X");
+        MCK(prod(na, cur, one, 1, zero, C1, w.mx, w.pst2), "C1");
+        k_dec_check<<<1, 1024, 0, s>>>(na, cur, w.mx, w.ok, w.nc, a.sgf_tol, it, nxt, w.count, w.redo);
         ++nl;
         MCK(cudaGetLastError(), "check");
         std::swap(cur, nxt);
@@ -500,53 +538,53 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
           na = h_count;
           if (na == 0) break;
         }
-        MCK(prod(na, cur, one, Bo, X, zero, B1, nullptr), "Self");
+        MCK(rows(na, cur, Bo, 2), "split Bo");
+        MCK(prod(na, cur, one, 2, zero, B1, nullptr, w.pst2), "Self");
         k_sub_self<<<dim3(gx, na), eb, 0, s>>>(Q, cur, B1, Ao, Aos, Q); ++nl;
-        MCK(prod(na, cur, one, Go, Bo, zero, Y, nullptr), "GoXBo");
-        MCK(prod(na, cur, one, Bo, Y, zero, B1, nullptr), "B1");
-        MCK(prod(na, cur, mone, Co, Y, one, Ao, nullptr), "Ao update");
-        // Bo = B1, Co = C1 for every point still iterating (the others are done with them)
+        MCK(cols(na, cur, Bo), "split Bo");
+        MCK(prod(na, cur, one, 0, zero, Y, nullptr, w.pst2), "GoXBo");
+        MCK(cols(na, cur, Y), "split Y");
+        MCK(prod(na, cur, one, 2, zero, B1, nullptr, w.pst2), "B1");
+        MCK(prod(na, cur, mone, 1, one, Ao, nullptr, w.pst2), "Ao update");
+        // Bo = B1, Co = C1 for every problem still iterating (the others are done with them)
         std::swap(B[2], B[8]);
         std::swap(B[3], B[6]);
         Bo = B[2]; Co = B[3]; B1 = B[8]; C1 = B[6];
       }
       if (na > 0) {
-        k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cur, ncyc_c, w.pst, a.sgf_max_iter);
+        k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.nc, w.pst2, a.sgf_max_iter);
         ++nl;
       }
-      MCK(inv(nsub, sub, Aos, B[9 + side]), "gs");
-      k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, w.pst,
-                                                            NEGF_B200_ERR_SINGULAR);
+      MCK(inv(nsub, sub, Aos, gs), "gs");
+      k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, w.pst2, NEGF_B200_ERR_SINGULAR);
       ++nl;
       if (a.eta > 0.0) {
-        k_retarded_check<<<nsub, 128, 0, s>>>(n, B[9 + side], Q, sub, w.redo);
+        k_retarded_check<<<nsub, 128, 0, s>>>(n, gs, Q, sub, w.redo);
         ++nl;
       }
       return 0;
     };
-    for (int side = 0; side < 2; ++side) {
-      MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * P, s), "memset redo");
-      if (int r = decimate(side, nullptr, P, 1.0)) return r;
-      if (!(a.eta > 0.0)) continue;
+    MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
+    if (int r = decimate(nullptr, N, 1.0)) return r;
+    if (a.eta > 0.0) {
       // Decimations that reached another fixed point (or ran off to Inf / NaN) run
-      // again, in lock step over just those points, from the contact energy times
+      // again, in lock step over just those problems, from the contact energy times
       // 1 + k 2^-50.  A sensitive decimation (one of its inverses needed a Newton
       // step: a nearly singular Ao) is accepted once two attempts reach the same gs.
-      std::vector<int> hredo(P), hsens(P), hagree(P), kept(P, 0), done(P, 0), cur_sub, again, cmp, keep;
-      cur_sub.resize(P);
-      for (int p = 0; p < P; ++p) cur_sub[p] = p;
-      double2* gs = B[9 + side];
+      std::vector<int> hredo(N), hsens(N), hagree(N), kept(N, 0), cur_sub, again, cmp, keep;
+      cur_sub.resize(N);
+      for (int p = 0; p < N; ++p) cur_sub[p] = p;
       for (int att = 1;; ++att) {
-        MCK(cudaMemcpyAsync(hredo.data(), w.redo, sizeof(int) * P, cudaMemcpyDeviceToHost, s), "redo");
-        MCK(cudaMemcpyAsync(hsens.data(), w.sens, sizeof(int) * P, cudaMemcpyDeviceToHost, s), "sens");
+        MCK(cudaMemcpyAsync(hredo.data(), w.redo, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "redo");
+        MCK(cudaMemcpyAsync(hsens.data(), w.sens, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "sens");
         MCK(cudaStreamSynchronize(s), "sync");
         cmp.clear();
         for (int p : cur_sub)
           if (!hredo[p] && hsens[p] && kept[p]) cmp.push_back(p);
         if (!cmp.empty()) {
           MCK(cudaMemcpyAsync(w.sub, cmp.data(), sizeof(int) * cmp.size(), cudaMemcpyHostToDevice, s), "cmp");
-          k_agree<<<(int)cmp.size(), 256, 0, s>>>(Q, w.sub, gs, B[13], Q, 1e-2, w.agree); ++nl;
-          MCK(cudaMemcpyAsync(hagree.data(), w.agree, sizeof(int) * P, cudaMemcpyDeviceToHost, s), "agree");
+          k_agree<<<(int)cmp.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q, 1e-2, w.agree); ++nl;
+          MCK(cudaMemcpyAsync(hagree.data(), w.agree, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "agree");
           MCK(cudaStreamSynchronize(s), "sync");
         }
         again.clear();
@@ -561,56 +599,62 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
         if (again.empty()) break;
         if (att > kDecRetries) {
           for (int p : again) hredo[p] = 1;
-          MCK(cudaMemcpyAsync(w.redo, hredo.data(), sizeof(int) * P, cudaMemcpyHostToDevice, s), "redo");
-          k_flag_unresolved<<<(P + 255) / 256, 256, 0, s>>>(P, w.redo, side == 0 ? w.ncl : w.ncr, w.pst,
-                                                              a.sgf_max_iter);
+          MCK(cudaMemcpyAsync(w.redo, hredo.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s), "redo");
+          k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, w.nc, w.pst2, a.sgf_max_iter);
           ++nl;
           MCK(cudaStreamSynchronize(s), "sync");
           break;
         }
         if (!keep.empty()) {
           MCK(cudaMemcpyAsync(w.sub, keep.data(), sizeof(int) * keep.size(), cudaMemcpyHostToDevice, s), "keep");
-          k_keep<<<(int)keep.size(), 256, 0, s>>>(Q, w.sub, gs, B[13], Q); ++nl;
+          k_keep<<<(int)keep.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q); ++nl;
           for (int p : keep) kept[p] = 1;
         }
         MCK(cudaMemcpyAsync(w.sub, again.data(), sizeof(int) * again.size(), cudaMemcpyHostToDevice, s), "sub");
-        MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * P, s), "memset redo");
-        if (int r = decimate(side, w.sub, (int)again.size(), 1.0 + att * 0x1p-50)) return r;
+        MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
+        if (int r = decimate(w.sub, (int)again.size(), 1.0 + att * 0x1p-50)) return r;
         cur_sub = again;
         MCK(cudaStreamSynchronize(s), "sync");   // the host vectors above are reused next round
       }
     }
-    // ---- self-energies Sigma_c = Tlc gs Tcl (B11 left, B12 right)
-    for (int side = 0; side < 2; ++side) {
-      const int c = side == 0 ? a.left : a.right;
-      k_tlc<<<dim3(gx, P), eb, 0, s>>>(n, c, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;
-      MCK(cudaGetLastError(), "tlc");
-      MCK(prod(P, nullptr, one, B[0], B[9 + side], zero, B[2], nullptr), "Tlc gs");
-      MCK(prod(P, nullptr, one, B[2], B[1], zero, B[11 + side], nullptr), "Sigma");
-    }
+    // ---- self-energies Sigma_c = Tlc gs Tcl of both contacts
+    k_tlc<<<dim3(gx, N), eb, 0, s>>>(n, P, a.left, a.right, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;
+    MCK(cudaGetLastError(), "tlc");
+    MCK(rows(N, nullptr, B[0], 0), "split Tlc");
+    MCK(cols(N, nullptr, gs), "split gs");
+    MCK(prod(N, nullptr, one, 0, zero, B[2], nullptr, w.pst2), "Tlc gs");
+    MCK(rows(N, nullptr, B[2], 0), "split Tlc gs");
+    MCK(cols(N, nullptr, B[1]), "split Tcl");
+    MCK(prod(N, nullptr, one, 0, zero, sig, nullptr, w.pst2), "Sigma");
+    k_merge_status<<<(P + 255) / 256, 256, 0, s>>>(P, w.pst2, w.pst); ++nl;
+    const double2 *sig_l = sig, *sig_r = sig + (int64_t)P * Q;
     // ---- gsmr sweep from block nbl down to 2, then Gr(1,1)
     double2 *g = B[4], *X = B[5], *W = B[6], *U = B[7], *Lb = B[8];
-    k_esh<<<dim3(gx, P), eb, 0, s>>>(n, 0, a.nbl - 1, ids, E, a.d_descs, B[12], W, Q); ++nl;
+    k_esh<<<dim3(gx, P), eb, 0, s>>>(n, 0, a.nbl - 1, ids, E, a.d_descs, sig_r, W, Q); ++nl;
     MCK(inv(P, nullptr, W, g), "gsmr N");
     k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
     ++nl;
     for (int i = a.nbl - 2; i >= 0; --i) {
       // W = ESH(i,i) - ESH(i,i+1) gsmr(i+1) ESH(i+1,i)  (block i 0-based; Sigma_left on block 0)
-      k_esh_step<<<dim3(gx, P), eb, 0, s>>>(n, i, ids, E, a.d_descs, i == 0 ? B[11] : nullptr, U, Lb, W, Q); ++nl;
+      k_esh_step<<<dim3(gx, P), eb, 0, s>>>(n, i, ids, E, a.d_descs, i == 0 ? sig_l : nullptr, U, Lb, W, Q); ++nl;
       MCK(cudaGetLastError(), "esh");
-      MCK(prod(P, nullptr, one, U, g, zero, X, nullptr), "U g");
-      MCK(prod(P, nullptr, mone, X, Lb, one, W, nullptr), "W");
+      MCK(rows(P, nullptr, U, 0), "split U");
+      MCK(cols(P, nullptr, g), "split g");
+      MCK(prod(P, nullptr, one, 0, zero, X, nullptr, w.pst), "U g");
+      MCK(rows(P, nullptr, X, 0), "split U g");
+      MCK(cols(P, nullptr, Lb), "split L");
+      MCK(prod(P, nullptr, mone, 0, one, W, nullptr, w.pst), "W");
       MCK(inv(P, nullptr, W, g), "gsmr");
       k_info_to_status<<<(P + 255) / 256, 256, 0, s>>>(P, nullptr, w.info, w.pst, NEGF_B200_ERR_SINGULAR);
       ++nl;
     }
     // g = Gr(1,1).  Trace with Gamma of the contact on block 1 (FP64 products)
-    k_gamma<<<dim3(gx, P), eb, 0, s>>>(n, B[11], B[0], Q); ++nl;
+    k_gamma<<<dim3(gx, P), eb, 0, s>>>(n, sig_l, B[0], Q); ++nl;
     MCK(prod64(P, B[0], g, B[1]), "Gam G");
     MCK(prod64(P, g, B[0], B[2]), "G Gam");
     k_trace<<<P, 512, 0, s>>>(n, B[0], g, B[1], B[2], w.tb, Q); ++nl;
     MCK(cudaGetLastError(), "trace");
-    k_finish<<<(P + 255) / 256, 256, 0, s>>>(P, w.ncl, w.ncr, w.pst, w.tb, a.d_T + p0,
+    k_finish<<<(P + 255) / 256, 256, 0, s>>>(P, w.nc, w.nc + P, w.pst, w.tb, a.d_T + p0,
                                              a.d_ncyc ? a.d_ncyc + p0 : nullptr,
                                              a.d_status ? a.d_status + p0 : nullptr); ++nl;
     MCK(cudaGetLastError(), "finish");

@@ -134,105 +134,117 @@ constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(k
 // 2^(-12-7(t+u)), exact as a double.
 __device__ __forceinline__ double level_weight(int l) { return __longlong_as_double((long long)(1023 - 12 - 7 * l) << 52); }
 
-template <int S>
-__device__ __forceinline__ void digits(double x, int8_t (&d)[S]) {
-  double y = x * 64.0;
-  double r = rint(y);
-  d[0] = (int8_t)r;
-  x = y - r;
+// The digit t of N values held as remainders x[], packed four to a word (N a
+// multiple of 4), and the next remainders.  Rounding by adding and
+// subtracting 1.5 2^52: the sum's low word is the rounded integer, with no
+// conversion instruction (16 per cycle and SM).
+template <int N>
+__device__ __forceinline__ void digit_words(int t, double (&x)[N], uint32_t (&w)[N / 4]) {
+  constexpr double kRound = 6755399441055744.0;
 #pragma unroll
-  for (int t = 1; t < S; ++t) {
-    y = x * 128.0;
-    r = rint(y);
-    d[t] = (int8_t)r;
-    x = y - r;
+  for (int i = 0; i < N; i += 4) {
+    uint32_t d[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double y = x[i + j] * (t == 0 ? 64.0 : 128.0);
+      const double s = y + kRound;
+      d[j] = (uint32_t)__double2loint(s);
+      x[i + j] = y - (s - kRound);
+    }
+    w[i / 4] = __byte_perm(__byte_perm(d[0], d[1], 0x0040), __byte_perm(d[2], d[3], 0x0040), 0x5410);
   }
+}
+
+// v 2^-e
+__device__ __forceinline__ double scale_down(double v, int e) {
+  return (e > -1000 && e < 1000) ? v * __longlong_as_double((long long)(1023 - e) << 52) : ldexp(v, -e);
 }
 
 // levels kept: digit pairs (t, u) with t + u < levels(S); one TMEM accumulator each
 __host__ __device__ constexpr int oz_levels(int S) { return S + 1 < 8 ? S + 1 : 8; }
 
 // Rows of A (M x K, column major, lda = M): exponent per row, digit planes
-// of Ar, Ai, -Ai with K contiguous (row pitch kp bytes).  Block: 32 rows.
+// of Ar, Ai, -Ai with K contiguous (row pitch kp bytes), stored at the
+// problem's place.  Block: 32 rows; a warp 16 rows x 32 K: lane (row, half)
+// holds 16 consecutive K of its row in registers and writes 16 bytes per
+// plane, two lanes a whole sector.  (Through shared memory byte by byte it
+// took 134 us for 64 matrices of order 256 and 8 digits: 40 us now; 190 MB
+// read and written.)
 template <int S>
-__global__ void __launch_bounds__(256) k_split_rows(int m, int k, int kp, const double2* A, int64_t sA, int8_t* qa,
+__global__ void __launch_bounds__(256, 2) k_split_rows(int m, int k, int kp, const double2* A, int64_t sA, int8_t* qa,
                                                    int* ea, int* flag, const int* item_map) {
   __shared__ double smax[8][32];
   __shared__ int sexp[32];
-  __shared__ int sbad;
-  __shared__ __align__(16) int8_t sq[3][S][32][32];
-  const int item = blockIdx.y;
+  const int64_t prob = item_map ? item_map[blockIdx.y] : blockIdx.y;
   const int m0 = blockIdx.x * 32;
-  const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const double2* Ab = A + (int64_t)(item_map ? item_map[item] : item) * sA;
-  if (threadIdx.x == 0) sbad = 0;
-  __syncthreads();
+  const double2* Ab = A + prob * sA;
   double mx = 0.0;
   bool bad = false;
-  if (m0 + r < m)
-    for (int kk = g; kk < k; kk += 8) {
-      const double2 v = Ab[(int64_t)(m0 + r) + (int64_t)kk * m];
-      bad |= !(isfinite(v.x) && isfinite(v.y));
-      mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
-    }
-  smax[g][r] = mx;
-  if (bad) sbad = 1;
-  __syncthreads();
-  if (g == 0) {
-    double t = smax[0][r];
+  {
+    const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
+    if (m0 + r < m)
+#pragma unroll 8
+      for (int kk = g; kk < k; kk += 8) {
+        const double2 v = Ab[(int64_t)(m0 + r) + (int64_t)kk * m];
+        bad |= !(isfinite(v.x) && isfinite(v.y));
+        mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+      }
+    smax[g][r] = mx;
+    bad = __syncthreads_or(bad);
+    if (g == 0) {
+      double t = smax[0][r];
 #pragma unroll
-    for (int q = 1; q < 8; ++q) t = fmax(t, smax[q][r]);
-    int e = 0;
-    if (t > 0.0 && isfinite(t)) frexp(t, &e);   // t = f 2^e, f in [0.5, 1): |row| < 2^e
-    sexp[r] = e;
-    if (m0 + r < m) ea[(int64_t)item * m + m0 + r] = e;
+      for (int q = 1; q < 8; ++q) t = fmax(t, smax[q][r]);
+      int e = 0;
+      if (t > 0.0 && isfinite(t)) frexp(t, &e);   // t = f 2^e, f in [0.5, 1): |row| < 2^e
+      sexp[r] = e;
+      if (m0 + r < m) ea[prob * m + m0 + r] = e;
+    }
+    if (bad && threadIdx.x == 0) atomicOr(flag + prob, 1);
+    __syncthreads();
   }
-  __syncthreads();
-  if (sbad && threadIdx.x == 0) atomicOr(flag + item, 1);
-  const int e = sexp[r];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rl = 16 * (warp & 1) + (lane >> 1), row = m0 + rl;
+  if (row >= m) return;
+  const int e = sexp[rl];
   const int64_t plane = (int64_t)m * kp;
-  for (int k0 = 0; k0 < kp; k0 += 32) {
+  int8_t* q0 = qa + prob * 3 * S * plane + (int64_t)row * kp;
+  for (int k0 = 32 * (warp >> 1) + 16 * (lane & 1); k0 < kp; k0 += 128) {
+    double re[16], im[16];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int kk = k0 + 4 * g + j;
+    for (int i = 0; i < 16; ++i) {
       double2 v = make_double2(0.0, 0.0);
-      if (m0 + r < m && kk < k) v = Ab[(int64_t)(m0 + r) + (int64_t)kk * m];
-      int8_t dr[S], di[S];
-      digits<S>(ldexp(v.x, -e), dr);
-      digits<S>(ldexp(v.y, -e), di);
+      if (k0 + i < k) v = Ab[(int64_t)row + (int64_t)(k0 + i) * m];
+      re[i] = scale_down(v.x, e);
+      im[i] = scale_down(v.y, e);
+    }
 #pragma unroll
-      for (int t = 0; t < S; ++t) {
-        sq[0][t][r][4 * g + j] = dr[t];
-        sq[1][t][r][4 * g + j] = di[t];
-        sq[2][t][r][4 * g + j] = (int8_t)(-di[t]);
-      }
+    for (int t = 0; t < S; ++t) {
+      uint32_t w[4];
+      digit_words<16>(t, re, w);
+      *reinterpret_cast<uint4*>(q0 + (int64_t)t * plane + k0) = make_uint4(w[0], w[1], w[2], w[3]);
+      digit_words<16>(t, im, w);
+      *reinterpret_cast<uint4*>(q0 + (int64_t)(S + t) * plane + k0) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(q0 + (int64_t)(2 * S + t) * plane + k0) =
+          make_uint4(__vneg4(w[0]), __vneg4(w[1]), __vneg4(w[2]), __vneg4(w[3]));
     }
-    __syncthreads();
-    // 3 * S planes x 32 rows x 2 segments of 16 bytes
-    for (int idx = threadIdx.x; idx < 3 * S * 64; idx += 256) {
-      const int seg = idx & 1, row = (idx >> 1) & 31, pt = idx >> 6;   // pt = arr * S + t
-      const int arr = pt / S, t = pt % S;
-      if (m0 + row < m && k0 + 16 * seg < kp) {
-        int8_t* dst = qa + ((int64_t)(item * 3 + arr) * S + t) * plane + (int64_t)(m0 + row) * kp + k0 + 16 * seg;
-        *reinterpret_cast<int4*>(dst) = *reinterpret_cast<const int4*>(&sq[arr][t][row][16 * seg]);
-      }
-    }
-    __syncthreads();
   }
 }
 
 // Columns of B (K x N, column major, ldb = K): exponent per column, digit
-// planes of Br, Bi with K contiguous.  One warp per column.
+// planes of Br, Bi with K contiguous, at the problem's place.  One warp per
+// column, four consecutive K per lane.
 template <int S>
 __global__ void __launch_bounds__(256) k_split_cols(int k, int n, int kp, const double2* B, int64_t sB, int8_t* qb,
                                                    int* eb, int* flag, const int* item_map) {
-  const int item = blockIdx.y;
+  const int64_t prob = item_map ? item_map[blockIdx.y] : blockIdx.y;
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (c >= n) return;
-  const double2* col = B + (int64_t)(item_map ? item_map[item] : item) * sB + (int64_t)c * k;
+  const double2* col = B + prob * sB + (int64_t)c * k;
   double mx = 0.0;
   bool bad = false;
+#pragma unroll 4
   for (int kk = lane; kk < k; kk += 32) {
     const double2 v = col[kk];
     bad |= !(isfinite(v.x) && isfinite(v.y));
@@ -244,21 +256,27 @@ __global__ void __launch_bounds__(256) k_split_cols(int k, int n, int kp, const 
   int e = 0;
   if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
   if (lane == 0) {
-    eb[(int64_t)item * n + c] = e;
-    if (bad) atomicOr(flag + item, 1);
+    eb[prob * n + c] = e;
+    if (bad) atomicOr(flag + prob, 1);
   }
   const int64_t plane = (int64_t)n * kp;
-  int8_t* q0 = qb + (int64_t)(item * 2) * S * plane + (int64_t)c * kp;
-  for (int kk = lane; kk < kp; kk += 32) {
-    double2 v = make_double2(0.0, 0.0);
-    if (kk < k) v = col[kk];
-    int8_t dr[S], di[S];
-    digits<S>(ldexp(v.x, -e), dr);
-    digits<S>(ldexp(v.y, -e), di);
+  int8_t* q0 = qb + prob * 2 * S * plane + (int64_t)c * kp;
+  for (int k0 = 4 * lane; k0 < kp; k0 += 128) {
+    double re[4], im[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      double2 v = make_double2(0.0, 0.0);
+      if (k0 + i < k) v = col[k0 + i];
+      re[i] = scale_down(v.x, e);
+      im[i] = scale_down(v.y, e);
+    }
 #pragma unroll
     for (int t = 0; t < S; ++t) {
-      q0[(int64_t)t * plane + kk] = dr[t];
-      q0[(int64_t)(S + t) * plane + kk] = di[t];
+      uint32_t w[1];
+      digit_words<4>(t, re, w);
+      *reinterpret_cast<uint32_t*>(q0 + (int64_t)t * plane + k0) = w[0];
+      digit_words<4>(t, im, w);
+      *reinterpret_cast<uint32_t*>(q0 + (int64_t)(S + t) * plane + k0) = w[0];
     }
   }
 }
@@ -271,9 +289,10 @@ struct OzArgs {
   double2* C;
   int64_t sC;
   const int* item_map;   // launch item -> problem index for C / maxabs / status (null = identity)
-  const int* ea;
+  const int* ea;         // exponents, flags and digit planes by problem
   const int* eb;
-  const int* flag;
+  const int* fa;
+  const int* fb;
   double* t0;            // FP64 real part of C, m x n per launch item (read back for the final combine)
   double* maxabs;
   int* status;
@@ -347,6 +366,7 @@ __global__ void __launch_bounds__(kOzWarps * 32, 1)
       int g = 0;
       for (int tile = blockIdx.x; tile < ntiles && !fail; tile += gridDim.x) {
         const int item = tile / per_item, tt = tile % per_item;
+        const int prob = a.item_map ? a.item_map[item] : item;
         const int m0 = (tt / tiles_n) * kOzTileM, n0 = (tt % tiles_n) * kOzTileN;
         for (int mi = 0; mi < 4 && !fail; ++mi) {
           const int part = mi >> 1, grp = mi & 1;
@@ -362,8 +382,8 @@ __global__ void __launch_bounds__(kOzWarps * 32, 1)
             const int arr_a = (part == 0) ? (h == 0 ? 0 : 2) : (h == 0 ? 1 : 0);
             mbar_arrive_tx(&full[st], (uint32_t)(2 * np * kPlaneBytes));
             for (int t = 0; t < np; ++t) {
-              tma_load_3d(sa + t * kPlaneBytes, &tA, &full[st], k0, m0, (item * 3 + arr_a) * S + t);
-              tma_load_3d(sb + t * kPlaneBytes, &tB, &full[st], k0, n0, (item * 2 + h) * S + t);
+              tma_load_3d(sa + t * kPlaneBytes, &tA, &full[st], k0, m0, (prob * 3 + arr_a) * S + t);
+              tma_load_3d(sb + t * kPlaneBytes, &tB, &full[st], k0, n0, (prob * 2 + h) * S + t);
             }
             issued[st] = use + 1;
           }
@@ -419,13 +439,13 @@ __global__ void __launch_bounds__(kOzWarps * 32, 1)
       const int m0 = (tt / tiles_n) * kOzTileM, n0 = (tt % tiles_n) * kOzTileN;
       const int r = m0 + 32 * quarter + lane;
       const bool row_ok = r < a.m;
-      const double rs = row_ok ? pow2(a.ea[(int64_t)item * a.m + r]) : 0.0;
-      const bool nonfinite = a.flag[item] != 0;
+      const double rs = row_ok ? pow2(a.ea[(int64_t)prob * a.m + r]) : 0.0;
+      const bool nonfinite = (a.fa[prob] | a.fb[prob]) != 0;
       // column scales of this tile (the epilogue warps' named barrier 1)
       asm volatile("bar.sync 1, %0;" ::"n"(kOzEpiWarps * 32));
       if (threadIdx.x < kOzTileN) {
         const int c = n0 + threadIdx.x;
-        col_scale[threadIdx.x] = (c < a.n) ? pow2(a.eb[(int64_t)item * a.n + c]) : 0.0;
+        col_scale[threadIdx.x] = (c < a.n) ? pow2(a.eb[(int64_t)prob * a.n + c]) : 0.0;
       }
       asm volatile("bar.sync 1, %0;" ::"n"(kOzEpiWarps * 32));
       double* T0 = a.t0 + (int64_t)item * a.m * a.n;
@@ -602,28 +622,20 @@ int num_sms() {
 }
 
 template <int S>
-cudaError_t run(const OzakiLayout& L, double2 alpha, const double2* A, int64_t sA, const double2* B, int64_t sB,
-                double2 beta, double2* C, int64_t sC, uint8_t* w, double* maxabs, int* status, cudaStream_t s,
-                const int* item_map) {
-  int8_t* qa = reinterpret_cast<int8_t*>(w + L.qa_off);
-  int8_t* qb = reinterpret_cast<int8_t*>(w + L.qb_off);
-  int* ea = reinterpret_cast<int*>(w + L.ea_off);
-  int* eb = reinterpret_cast<int*>(w + L.eb_off);
-  int* flag = reinterpret_cast<int*>(w + L.flag_off);
-  cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int) * (size_t)L.batch, s);
-  if (e != cudaSuccess) return e;
-  k_split_rows<S><<<dim3((L.m + 31) / 32, L.batch), 256, 0, s>>>(L.m, L.k, L.kp, A, sA, qa, ea, flag, item_map);
-  k_split_cols<S><<<dim3((L.n + 7) / 8, L.batch), 256, 0, s>>>(L.k, L.n, L.kp, B, sB, qb, eb, flag, item_map);
+cudaError_t product(int batch, int m, int n, int k, double2 alpha, const OzakiSet& A, const OzakiSet& B, double2 beta,
+                    double2* C, int64_t sC, double* t0, double* maxabs, int* status, cudaStream_t s,
+                    const int* item_map) {
+  const int kp = (k + 15) & ~15;
   CUtensorMap ta, tb;
-  if (!make_map(&ta, qa, L.k, L.m, L.kp, L.batch * 3 * S, kOzTileM) ||
-      !make_map(&tb, qb, L.k, L.n, L.kp, L.batch * 2 * S, kOzTileN))
+  if (!make_map(&ta, A.q, k, m, kp, A.problems * 3 * S, kOzTileM) ||
+      !make_map(&tb, B.q, k, n, kp, B.problems * 2 * S, kOzTileN))
     return cudaErrorInvalidValue;
   OzArgs a;
-  a.m = L.m; a.n = L.n; a.k = L.k; a.nkc = (L.k + kOzKChunk - 1) / kOzKChunk;
-  a.batch = L.batch;
+  a.m = m; a.n = n; a.k = k; a.nkc = (k + kOzKChunk - 1) / kOzKChunk;
+  a.batch = batch;
   a.alpha = alpha; a.beta = beta; a.C = C; a.sC = sC; a.item_map = item_map;
-  a.ea = ea; a.eb = eb; a.flag = flag;
-  a.t0 = reinterpret_cast<double*>(w + L.t0_off);
+  a.ea = A.e; a.eb = B.e; a.fa = A.flag; a.fb = B.flag;
+  a.t0 = t0;
   a.maxabs = maxabs; a.status = status;
   const size_t smem = (size_t)kOzStages * 2 * S * kPlaneBytes + 1024;
   static std::mutex mu;
@@ -633,50 +645,116 @@ cudaError_t run(const OzakiLayout& L, double2 alpha, const double2* A, int64_t s
   {
     std::lock_guard<std::mutex> lk(mu);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-      e = cudaFuncSetAttribute(k_ozaki<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(k_ozaki<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
   }
-  const long long tiles = (long long)((L.m + kOzTileM - 1) / kOzTileM) * ((L.n + kOzTileN - 1) / kOzTileN) * L.batch;
+  const long long tiles = (long long)((m + kOzTileM - 1) / kOzTileM) * ((n + kOzTileN - 1) / kOzTileN) * batch;
   const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
   k_ozaki<S><<<grid, kOzWarps * 32, smem, s>>>(ta, tb, a);
   return cudaGetLastError();
 }
 
+OzakiSet carve_set(uint8_t*& p, int problems, size_t rows, int kp, int arrays, int slices) {
+  OzakiSet r;
+  r.problems = problems;
+  r.q = reinterpret_cast<int8_t*>(p); p += align256((size_t)problems * arrays * slices * rows * kp);
+  r.e = reinterpret_cast<int*>(p); p += align256(sizeof(int) * (size_t)problems * rows);
+  r.flag = reinterpret_cast<int*>(p); p += align256(sizeof(int) * (size_t)problems);
+  return r;
+}
+size_t set_bytes(int problems, size_t rows, int kp, int arrays, int slices) {
+  return align256((size_t)problems * arrays * slices * rows * kp) + align256(sizeof(int) * (size_t)problems * rows) +
+         align256(sizeof(int) * (size_t)problems);
+}
+
 }  // namespace
 
-OzakiLayout ozaki_layout(int batch, int m, int n, int k, int slices) {
-  OzakiLayout L;
-  L.batch = batch; L.m = m; L.n = n; L.k = k; L.slices = slices;
-  L.kp = (k + 15) & ~15;
-  size_t off = 0;
-  L.qa_off = off; off = align256(off + (size_t)batch * 3 * slices * m * L.kp);
-  L.qb_off = off; off = align256(off + (size_t)batch * 2 * slices * n * L.kp);
-  L.ea_off = off; off = align256(off + sizeof(int) * (size_t)batch * m);
-  L.eb_off = off; off = align256(off + sizeof(int) * (size_t)batch * n);
-  L.flag_off = off; off = align256(off + sizeof(int) * (size_t)batch);
-  L.t0_off = off; off = align256(off + sizeof(double) * (size_t)batch * m * n);
-  L.total = off;
-  return L;
+size_t ozaki_rows_bytes(int problems, int m, int k, int slices) {
+  return set_bytes(problems, m, (k + 15) & ~15, 3, slices);
+}
+size_t ozaki_cols_bytes(int problems, int k, int n, int slices) {
+  return set_bytes(problems, n, (k + 15) & ~15, 2, slices);
+}
+OzakiSet ozaki_rows_at(void* base, int problems, int m, int k, int slices) {
+  uint8_t* p = static_cast<uint8_t*>(base);
+  return carve_set(p, problems, m, (k + 15) & ~15, 3, slices);
+}
+OzakiSet ozaki_cols_at(void* base, int problems, int k, int n, int slices) {
+  uint8_t* p = static_cast<uint8_t*>(base);
+  return carve_set(p, problems, n, (k + 15) & ~15, 2, slices);
+}
+
+cudaError_t launch_ozaki_rows(int batch, int m, int k, const double2* A, int64_t sA, int slices, const OzakiSet& d,
+                              cudaStream_t s, const int* map) {
+  if (batch <= 0) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(d.flag, 0, sizeof(int) * (size_t)d.problems, s);
+  if (e != cudaSuccess) return e;
+  const int kp = (k + 15) & ~15;
+  const dim3 grid((m + 31) / 32, batch);
+  switch (slices) {
+    case 4: k_split_rows<4><<<grid, 256, 0, s>>>(m, k, kp, A, sA, d.q, d.e, d.flag, map); break;
+    case 5: k_split_rows<5><<<grid, 256, 0, s>>>(m, k, kp, A, sA, d.q, d.e, d.flag, map); break;
+    case 6: k_split_rows<6><<<grid, 256, 0, s>>>(m, k, kp, A, sA, d.q, d.e, d.flag, map); break;
+    case 7: k_split_rows<7><<<grid, 256, 0, s>>>(m, k, kp, A, sA, d.q, d.e, d.flag, map); break;
+    default: k_split_rows<8><<<grid, 256, 0, s>>>(m, k, kp, A, sA, d.q, d.e, d.flag, map); break;
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ozaki_cols(int batch, int k, int n, const double2* B, int64_t sB, int slices, const OzakiSet& d,
+                              cudaStream_t s, const int* map) {
+  if (batch <= 0) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(d.flag, 0, sizeof(int) * (size_t)d.problems, s);
+  if (e != cudaSuccess) return e;
+  const int kp = (k + 15) & ~15;
+  const dim3 grid((n + 7) / 8, batch);
+  switch (slices) {
+    case 4: k_split_cols<4><<<grid, 256, 0, s>>>(k, n, kp, B, sB, d.q, d.e, d.flag, map); break;
+    case 5: k_split_cols<5><<<grid, 256, 0, s>>>(k, n, kp, B, sB, d.q, d.e, d.flag, map); break;
+    case 6: k_split_cols<6><<<grid, 256, 0, s>>>(k, n, kp, B, sB, d.q, d.e, d.flag, map); break;
+    case 7: k_split_cols<7><<<grid, 256, 0, s>>>(k, n, kp, B, sB, d.q, d.e, d.flag, map); break;
+    default: k_split_cols<8><<<grid, 256, 0, s>>>(k, n, kp, B, sB, d.q, d.e, d.flag, map); break;
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ozaki_product(int batch, int m, int n, int k, double2 alpha, const OzakiSet& A, const OzakiSet& B,
+                                 double2 beta, double2* C, int64_t sC, int slices, double* t0, double* maxabs,
+                                 int* status, cudaStream_t s, const int* map) {
+  if (batch <= 0 || m <= 0 || n <= 0) return cudaSuccess;
+  switch (slices) {
+    case 4: return product<4>(batch, m, n, k, alpha, A, B, beta, C, sC, t0, maxabs, status, s, map);
+    case 5: return product<5>(batch, m, n, k, alpha, A, B, beta, C, sC, t0, maxabs, status, s, map);
+    case 6: return product<6>(batch, m, n, k, alpha, A, B, beta, C, sC, t0, maxabs, status, s, map);
+    case 7: return product<7>(batch, m, n, k, alpha, A, B, beta, C, sC, t0, maxabs, status, s, map);
+    default: return product<8>(batch, m, n, k, alpha, A, B, beta, C, sC, t0, maxabs, status, s, map);
+  }
+}
+
+size_t ozaki_work_bytes(int batch, int m, int n, int k, int slices) {
+  return ozaki_rows_bytes(batch, m, k, slices) + ozaki_cols_bytes(batch, k, n, slices) +
+         align256(sizeof(double) * (size_t)batch * m * n);
 }
 
 cudaError_t launch_ozaki_zgemm(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC, int slices,
-                               void* work, double* maxabs, int* status, cudaStream_t s, const int* item_map) {
+                               void* work, double* maxabs, int* status, cudaStream_t s) {
   if (batch <= 0 || m <= 0 || n <= 0) return cudaSuccess;
   if (k <= 0 || k > 1024 || batch > 65535 || slices < kOzMinSlices || slices > kOzMaxSlices || !work ||
       (reinterpret_cast<uintptr_t>(work) & 255))
     return cudaErrorInvalidValue;
-  const OzakiLayout L = ozaki_layout(batch, m, n, k, slices);
   uint8_t* w = static_cast<uint8_t*>(work);
-  switch (slices) {
-    case 4: return run<4>(L, alpha, A, sA, B, sB, beta, C, sC, w, maxabs, status, s, item_map);
-    case 5: return run<5>(L, alpha, A, sA, B, sB, beta, C, sC, w, maxabs, status, s, item_map);
-    case 6: return run<6>(L, alpha, A, sA, B, sB, beta, C, sC, w, maxabs, status, s, item_map);
-    case 7: return run<7>(L, alpha, A, sA, B, sB, beta, C, sC, w, maxabs, status, s, item_map);
-    default: return run<8>(L, alpha, A, sA, B, sB, beta, C, sC, w, maxabs, status, s, item_map);
-  }
+  const OzakiSet da = ozaki_rows_at(w, batch, m, k, slices);
+  w += ozaki_rows_bytes(batch, m, k, slices);
+  const OzakiSet db = ozaki_cols_at(w, batch, k, n, slices);
+  w += ozaki_cols_bytes(batch, k, n, slices);
+  cudaError_t e = launch_ozaki_rows(batch, m, k, A, sA, slices, da, s, nullptr);
+  if (e == cudaSuccess) e = launch_ozaki_cols(batch, k, n, B, sB, slices, db, s, nullptr);
+  if (e != cudaSuccess) return e;
+  return launch_ozaki_product(batch, m, n, k, alpha, da, db, beta, C, sC, slices, reinterpret_cast<double*>(w), maxabs,
+                              status, s, nullptr);
 }
 
 }  // namespace negf

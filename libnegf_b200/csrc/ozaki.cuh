@@ -27,27 +27,44 @@ constexpr int kOzKChunk = 32;       // bytes of K per pipeline stage (one 32-byt
 constexpr int kOzStages = 3;
 constexpr int kOzMinSlices = 4, kOzMaxSlices = 8;
 
-// Workspace of one batched product (bytes), laid out by ozaki_layout():
-// digit planes of A and B, exponents, non-finite flags, an FP64 m x n
-// buffer per item for the real part.
-struct OzakiLayout {
-  int m, n, k, kp, slices, batch;
-  size_t qa_off, qb_off, ea_off, eb_off, flag_off, t0_off, total;
+// The digits of one operand of a batch of problems: planes, an exponent per
+// row (column) and a non-finite flag per problem, all at the problem's index,
+// so that an operand split once serves every product it takes part in, also
+// after problems have left the batch.
+struct OzakiSet {
+  int8_t* q;
+  int* e;
+  int* flag;
+  int problems;
 };
-OzakiLayout ozaki_layout(int batch, int m, int n, int k, int slices);
+size_t ozaki_rows_bytes(int problems, int m, int k, int slices);   // of left operands (m x k)
+size_t ozaki_cols_bytes(int problems, int k, int n, int slices);   // of right operands (k x n)
+OzakiSet ozaki_rows_at(void* base, int problems, int m, int k, int slices);   // base: 256-byte aligned
+OzakiSet ozaki_cols_at(void* base, int problems, int k, int n, int slices);
 
-// C_p = alpha * A_p * B_p + beta * C_p for the problems p = item_map[b],
-// b < batch (item_map null: p = b); complex128, column major, element
-// strides sA/sB/sC in complex elements.  beta == 0: C is not read.  C may
-// alias A or B (the operands are split into the workspace first).  maxabs
-// (optional, one double per problem, non-negative, updated with atomicMax on
-// its bit pattern): max |C_p| over the stored elements, NaN when one of them
-// is NaN or Inf.  status (optional,
-// one int per problem): 3 on a non-finite operand (C is NaN), 7 when a
-// pipeline wait ran out (C is not written).
+// Split the operands A_p (B_p) of the problems p = map[b], b < batch (map
+// null: p = b); complex128, column major, sA / sB complex elements apart.
+cudaError_t launch_ozaki_rows(int batch, int m, int k, const double2* A, int64_t sA, int slices, const OzakiSet& d,
+                              cudaStream_t s, const int* map);
+cudaError_t launch_ozaki_cols(int batch, int k, int n, const double2* B, int64_t sB, int slices, const OzakiSet& d,
+                              cudaStream_t s, const int* map);
+// C_p = alpha * A_p * B_p + beta * C_p from split operands, the same problem
+// selection.  beta == 0: C is not read.  t0: m x n doubles per launch item.
+// maxabs (optional, one double per problem, non-negative, updated with
+// atomicMax on its bit pattern): max |C_p| over the stored elements, NaN when
+// one of them is NaN or Inf.  status (optional, one int per problem): 3 on a
+// non-finite operand (C is NaN), 7 when a pipeline wait ran out (C is not
+// written).
+cudaError_t launch_ozaki_product(int batch, int m, int n, int k, double2 alpha, const OzakiSet& A, const OzakiSet& B,
+                                 double2 beta, double2* C, int64_t sC, int slices, double* t0, double* maxabs,
+                                 int* status, cudaStream_t s, const int* map);
+
+// Both splits and the product of a whole batch, in a workspace of
+// ozaki_work_bytes() (256-byte aligned).  C may alias A or B (the operands are
+// split into the workspace first).
+size_t ozaki_work_bytes(int batch, int m, int n, int k, int slices);
 cudaError_t launch_ozaki_zgemm(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC, int slices,
-                               void* work, double* maxabs, int* status, cudaStream_t s,
-                               const int* item_map = nullptr);
+                               void* work, double* maxabs, int* status, cudaStream_t s);
 
 }  // namespace negf
