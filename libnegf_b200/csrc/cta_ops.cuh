@@ -181,7 +181,6 @@ enum OpMode : int {
   OP_N = 0,       // X(r,c) = p[r + c*ld]
   OP_C = 1,       // X(r,c) = conj(p[c + r*ld])   (conjugate transpose)
   OP_GATHER = 2,  // X(r,c) = p[perm[r] + c*ld]   (row gather, perm in smem)
-  OP_RT = -1,     // template argument only: the mode is read from the descriptor
 };
 
 struct Operand {
@@ -198,7 +197,6 @@ __device__ __forceinline__ Operand opC(const double2* p, int ld) { return Operan
 enum EpiMode : int {
   EPI_STORE = 0,   // C = alpha*acc + beta*C   (beta==0: C not read)
   EPI_GJ = 1,      // Gauss-Jordan delayed update: C = acc + rowmask(X[perm,:]) (see cta_zinv)
-  EPI_RT = -1,     // template argument only: the mode is read from the descriptor
 };
 
 struct Epilogue {
@@ -224,96 +222,7 @@ __device__ __forceinline__ Epilogue epi_store(double2* C, int ldc, double2 alpha
   return e;
 }
 
-// ---------------------------------------------------------------- tile loads
-// A tile: rows [m0, m0+T) x cols [k0, k0+TK) of op(A) (M x K) into sA[k][m]
-template <int MODE, int T>
-__device__ __forceinline__ void load_a_tile(const Operand& A, int M, int K, int m0, int k0, double2* sA) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int j = 0; j < (T * TK) / kThreads; ++j) {
-    int idx = tid + j * kThreads;
-    int m, k;
-    const double2* src;
-    bool ok;
-    if (MODE == OP_C) {
-      k = idx & (TK - 1); m = idx / TK;
-      ok = (m0 + m < M) && (k0 + k < K);
-      src = ok ? A.p + (size_t)(k0 + k) + (size_t)(m0 + m) * A.ld : A.p;
-    } else {
-      m = idx & (T - 1); k = idx / T;
-      ok = (m0 + m < M) && (k0 + k < K);
-      int row = (MODE == OP_GATHER && ok) ? A.perm[m0 + m] : m0 + m;
-      src = ok ? A.p + (size_t)row + (size_t)(k0 + k) * A.ld : A.p;
-    }
-    cp_async16(&sA[k * TileRing<T>::kLda + m], src, ok);
-  }
-}
-
-// B tile: rows [k0, k0+TK) x cols [n0, n0+T) of op(B) (K x N) into sB[n][k]
-template <int MODE, int T>
-__device__ __forceinline__ void load_b_tile(const Operand& B, int K, int N, int k0, int n0, double2* sB) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int j = 0; j < (TK * T) / kThreads; ++j) {
-    int idx = tid + j * kThreads;
-    int k, n;
-    const double2* src;
-    bool ok;
-    if (MODE == OP_C) {
-      n = idx & (T - 1); k = idx / T;
-      ok = (k0 + k < K) && (n0 + n < N);
-      src = ok ? B.p + (size_t)(n0 + n) + (size_t)(k0 + k) * B.ld : B.p;
-    } else {
-      k = idx & (TK - 1); n = idx / TK;
-      ok = (k0 + k < K) && (n0 + n < N);
-      int row = (MODE == OP_GATHER && ok) ? B.perm[k0 + k] : k0 + k;
-      src = ok ? B.p + (size_t)row + (size_t)(n0 + n) * B.ld : B.p;
-    }
-    cp_async16(&sB[n * B_LD + k], src, ok);
-  }
-}
-
-// ---------------------------------------------------------------- epilogue
-// The value the epilogue combines with the product at (r, c): C(r,c) for
-// EPI_STORE with beta != 0, the permuted previous iterate (or the panel) for
-// EPI_GJ.  Loaded for a whole fragment before any store, so that the loads
-// of one fragment are in flight together instead of each waiting behind the
-// previous element's store.
-template <int EMODE>
-__device__ __forceinline__ double2 epi_old(const Epilogue& e, int r, int c, int M, int N) {
-  if (r >= M || c >= N) return make_double2(0.0, 0.0);
-  if (EMODE == EPI_STORE) {
-    if (e.beta.x == 0.0 && e.beta.y == 0.0) return make_double2(0.0, 0.0);
-    return e.C[(size_t)r + (size_t)c * e.ldc];
-  }
-  if (r >= e.k0 && r < e.k0 + e.jb) return make_double2(0.0, 0.0);
-  return e.xcur[(size_t)e.perm[r] + (size_t)c * e.ldx];
-}
-
-template <int EMODE>
-__device__ __forceinline__ void epi_store_one(const Epilogue& e, int r, int c, double re, double im, double2 old,
-                                              int M, int N, double& lmax, bool want_max) {
-  if (r >= M || c >= N) return;
-  double2 out;
-  if (EMODE == EPI_STORE) {
-    out = make_double2(e.alpha.x * re - e.alpha.y * im, e.alpha.x * im + e.alpha.y * re);
-    out = cadd(out, cmul(e.beta, old));
-  } else {
-    out = make_double2(re + old.x, im + old.y);
-  }
-  e.C[(size_t)r + (size_t)c * e.ldc] = out;
-  if (want_max) lmax = fmax(lmax, cabs(out));
-}
-
 // ---------------------------------------------------------------- GEMM
-// C(MxN) = epilogue( op(A)(MxK) * op(B)(KxN) ).  All threads of the CTA must
-// call it.  `smem` must hold kGemmSmemBytes.  Ends with __syncthreads().
-//
-// The operand pipeline runs over the flattened sequence of (output tile,
-// K-tile) steps, so the next output tile's first operands are in flight
-// while the current tile's epilogue runs; K = 16 products (the Gauss-Jordan
-// updates) are as pipelined as long ones.  One specialisation per operand /
-// epilogue combination keeps the live state of the main loop in registers.
 // GEMM parameters, written to shared memory by the caller and re-read by the
 // product loop after each barrier.  Parameters that only sit in memory cost
 // the loop no registers; the accumulators and fragments get them all.
@@ -334,62 +243,54 @@ struct GemmDesc {
 };
 constexpr int kGemmDescOffset = kRingElems;   // in double2 units, after the staging ring
 
-template <int AM, int BM, int T>
-__device__ __forceinline__ void gemm_issue(const GemmDesc* d, int ld_tile, int ld_kt, double2* st) {
-  const int tilesM = d->tilesM;
-  const int m0 = (ld_tile % tilesM) * T, n0 = (ld_tile / tilesM) * T;
-  const Operand A{d->A, d->lda, AM, d->aperm};
-  const Operand B{d->B, d->ldb, BM, d->bperm};
-  if constexpr (AM >= 0) {
-    load_a_tile<AM, T>(A, d->M, d->K, m0, ld_kt * TK, st);
-  } else {
-    const int am = d->amode;
-    if (am == OP_C) load_a_tile<OP_C, T>(A, d->M, d->K, m0, ld_kt * TK, st);
-    else if (am == OP_GATHER) load_a_tile<OP_GATHER, T>(A, d->M, d->K, m0, ld_kt * TK, st);
-    else load_a_tile<OP_N, T>(A, d->M, d->K, m0, ld_kt * TK, st);
+// One operand's tile of a step by asynchronous copies: T entries from t0 of
+// the output dimension (limit tl) by TK from k0 of K.  Lanes run along the
+// dimension that is contiguous in memory (the output dimension if
+// `tile_fast`), so a thread's T TK / kThreads copies are one pointer and one
+// stride; the gathered modes permute that same dimension.  dt and dk are the
+// shared-memory strides of the two dimensions.  One routine for every mode:
+// with a copy of the loop per mode and each element's address formed on its
+// own, issuing a step's loads cost about 2000 cycles beside 4096 of products
+// (296 products of order 512: 9.96 -> 9.52 ms, of order 256: 1.30 -> 1.22; one
+// of order 64 in a team of 4: 17100 -> 13300 cycles).
+template <int T>
+__device__ __forceinline__ void load_tile(const double2* P, int ld, const int* perm, bool tile_fast, int t0, int tl,
+                                          int k0, int K, uint32_t dst, int dt, int dk) {
+  constexpr int J = T * TK / kThreads;
+  int tid;   // read here every time: kept across the product loop it would cost it registers
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+  const int nf = tile_fast ? T : TK;                 // a power of two
+  const int f = tid & (nf - 1), s0 = tile_fast ? tid / T : tid / TK, ss = tile_fast ? kThreads / T : kThreads / TK;
+  const int fb = (tile_fast ? t0 : k0) + f, sb = (tile_fast ? k0 : t0) + s0, sl = tile_fast ? K : tl;
+  const bool fok = fb < (tile_fast ? tl : K);
+  const int row = (perm && fok) ? perm[fb] : fb;
+  const double2* src = P + (size_t)row + (size_t)sb * ld;
+  const int df = tile_fast ? dt : dk, ds = tile_fast ? dk : dt;
+  dst += (uint32_t)(f * df + s0 * ds) * 16u;
+  const uint32_t dstep = (uint32_t)(ss * ds) * 16u;
+  const size_t step = (size_t)ss * ld;
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const bool ok = fok && sb + j * ss < sl;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + j * dstep),
+                 "l"(ok ? src + j * step : P), "r"(ok ? 16 : 0));
   }
-  if constexpr (BM >= 0) {
-    load_b_tile<BM, T>(B, d->K, d->N, ld_kt * TK, n0, st + TK * TileRing<T>::kLda);
-  } else {
-    const int bm = d->bmode;
-    if (bm == OP_C) load_b_tile<OP_C, T>(B, d->K, d->N, ld_kt * TK, n0, st + TK * TileRing<T>::kLda);
-    else if (bm == OP_GATHER) load_b_tile<OP_GATHER, T>(B, d->K, d->N, ld_kt * TK, n0, st + TK * TileRing<T>::kLda);
-    else load_b_tile<OP_N, T>(B, d->K, d->N, ld_kt * TK, n0, st + TK * TileRing<T>::kLda);
-  }
+}
+
+template <int T>
+__device__ __forceinline__ void gemm_issue(const GemmDesc* d, int tm, int tn, int kt, double2* st) {
+  const int am = d->amode, bm = d->bmode, K = d->K;
+  const uint32_t sa = smem_u32(st);
+  load_tile<T>(d->A, d->lda, am == OP_GATHER ? d->aperm : nullptr, am != OP_C, tm * T, d->M, kt * TK, K, sa, 1,
+               TileRing<T>::kLda);
+  load_tile<T>(d->B, d->ldb, bm == OP_GATHER ? d->bperm : nullptr, bm == OP_C, tn * T, d->N, kt * TK, K,
+               sa + TK * TileRing<T>::kLda * 16u, B_LD, 1);
   cp_async_commit();
 }
 
 // x with its sign bit flipped when m == 0x80000000 (integer pipe, no FP64 op)
 __device__ __forceinline__ double flip_sign(double x, unsigned m) {
   return __hiloint2double(__double2hiint(x) ^ (int)m, __double2loint(x));
-}
-
-template <int EMODE>
-__device__ __forceinline__ double2 epi_old_d(const GemmDesc* d, int r, int c) {
-  if (r >= d->M || c >= d->N) return make_double2(0.0, 0.0);
-  if (EMODE == EPI_STORE || (EMODE == EPI_RT && d->emode == EPI_STORE)) {
-    const double2 be = d->beta;
-    if (be.x == 0.0 && be.y == 0.0) return make_double2(0.0, 0.0);
-    return d->C[(size_t)r + (size_t)c * d->ldc];
-  }
-  if (r >= d->k0 && r < d->k0 + d->jb) return make_double2(0.0, 0.0);
-  return d->xcur[(size_t)d->perm[r] + (size_t)c * d->ldx];
-}
-
-template <int EMODE>
-__device__ __forceinline__ void epi_store_d(const GemmDesc* d, int r, int c, double re, double im, double2 old,
-                                            double& lmax) {
-  if (r >= d->M || c >= d->N) return;
-  double2 out;
-  if (EMODE == EPI_STORE || (EMODE == EPI_RT && d->emode == EPI_STORE)) {
-    const double2 al = d->alpha;
-    out = make_double2(al.x * re - al.y * im, al.x * im + al.y * re);
-    out = cadd(out, cmul(d->beta, old));
-  } else {
-    out = make_double2(re + old.x, im + old.y);
-  }
-  d->C[(size_t)r + (size_t)c * d->ldc] = out;
-  if (d->maxabs) lmax = fmax(lmax, cabs(out));
 }
 
 // The product loop.  All threads of the CTA call it after the descriptor at
@@ -401,7 +302,7 @@ __device__ __forceinline__ void epi_store_d(const GemmDesc* d, int r, int c, dou
 // convention and this loop spills (measured: 30 % slower).  cta_gemm_t is the
 // out-of-line copy for the engine's top level; cta_gemm_body is inlined into
 // the inversion.
-template <int AM, int BM, int EM, int T>
+template <int T>
 __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -411,27 +312,32 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
   constexpr int F = T / 32, kStages = TileRing<T>::kStages, kStageElems = TileRing<T>::kElems, A_LD = TileRing<T>::kLda;
   const int wm = warp >> 2, wn = ((warp & 3) + 2 * wm) & 3;
   // sign masks of the imaginary parts (conjugated operands)
-  const unsigned sa = (AM >= 0) ? (AM == OP_C ? 0x80000000u : 0u) : (d->amode == OP_C ? 0x80000000u : 0u);
-  const unsigned sb = (BM >= 0) ? (BM == OP_C ? 0x80000000u : 0u) : (d->bmode == OP_C ? 0x80000000u : 0u);
+  const unsigned sa = d->amode == OP_C ? 0x80000000u : 0u, sb = d->bmode == OP_C ? 0x80000000u : 0u;
   const int total = d->total;
   double lmax = 0.0;
   double accR[F][F][4], accI[F][F][4];
-  const int tile0 = d->tile0;
-  int ld_tile = tile0, ld_kt = 0, ld_step = 0;   // (tile, K-tile) and index of the next step to load
+  // tile row and column and K-tile of the step computed, and of the next one to load
+  int tn = d->tile0 / d->tilesM, tm = d->tile0 - tn * d->tilesM, kt = 0;
+  int ld_tn = tn, ld_tm = tm, ld_kt = 0, ld_step = 0;
+  auto next_tile = [&](int& m, int& n) {
+    for (m += d->tstep; m >= d->tilesM; m -= d->tilesM) ++n;
+  };
+  auto issue = [&](int slot) {
+    gemm_issue<T>(d, ld_tm, ld_tn, ld_kt, smem + slot * kStageElems);
+    if (++ld_kt == d->nk) { ld_kt = 0; next_tile(ld_tm, ld_tn); }
+    ++ld_step;
+  };
 
   // the first kStages - 1 steps in flight (an empty group keeps the count when
   // there are fewer steps)
 #pragma unroll
   for (int q = 0; q < kStages - 1; ++q) {
     if (ld_step < total) {
-      gemm_issue<AM, BM, T>(d, ld_tile, ld_kt, smem + q * kStageElems);
-      if (++ld_kt == d->nk) { ld_kt = 0; ld_tile += d->tstep; }
-      ++ld_step;
+      issue(q);
     } else {
       cp_async_commit();
     }
   }
-  int tile = tile0, kt = 0;
   for (int step = 0; step < total; ++step) {
     if (kt == 0) {
 #pragma unroll
@@ -447,7 +353,7 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
     const double2* sB = sA + TK * A_LD;
     // warps whose block lies outside M x N, and the K steps past K,
     // skip their products (narrow Gauss-Jordan updates: N, K = 16 or 32)
-    const bool wact = ((tile % d->tilesM) * T + wm * 16 * F < d->M) && ((tile / d->tilesM) * T + wn * 8 * F < d->N);
+    const bool wact = (tm * T + wm * 16 * F < d->M) && (tn * T + wn * 8 * F < d->N);
     const int kleft = d->K - kt * TK;
 #pragma unroll
     for (int ks = 0; ks < TK / 4; ++ks) {
@@ -458,9 +364,7 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
         // 10.36 ms there, 10.12 after the first quarter, 9.96 here; of order
         // 256: 1.360, 1.317, 1.302)
         if (ld_step < total) {
-          gemm_issue<AM, BM, T>(d, ld_tile, ld_kt, smem + (ld_step % kStages) * kStageElems);
-          if (++ld_kt == d->nk) { ld_kt = 0; ld_tile += d->tstep; }
-          ++ld_step;
+          issue(ld_step % kStages);
         } else {
           cp_async_commit();
         }
@@ -495,31 +399,60 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
         for (int j = 0; j < F; ++j) dmma_16x8x4(accI[i][j], ai0, ai1, bre[j]);
       }
     }
-    if (kt == d->nk - 1) {
-      const int tilesM = d->tilesM;
-      const int m0 = (tile % tilesM) * T, n0 = (tile / tilesM) * T;
+    if (kt == d->nk - 1 && wact) {
+      // epilogue: the values combined with the product (C for beta != 0, the
+      // permuted previous iterate outside the pivot rows for EPI_GJ) are loaded
+      // for a fragment before its stores, so that they are in flight together.
+      // Descriptor fields are read per fragment: a store would make the compiler
+      // read them again for every element, and kept over the whole epilogue they
+      // take the accumulators' registers.
+      const int r0 = tm * T + wm * 16 * F + g, c0 = tn * T + wn * 8 * F + 2 * t;
 #pragma unroll
-      for (int i = 0; i < F; ++i) {
-        double2 old[F][4];
+      for (int i = 0; i < F; ++i)
 #pragma unroll
-        for (int j = 0; j < F; ++j)
+        for (int j = 0; j < F; ++j) {
+          const int M = d->M, N = d->N;
+          double2 old[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) old[q] = make_double2(0.0, 0.0);
+          const bool gj = d->emode == EPI_GJ;
+          if (gj || d->beta.x != 0.0 || d->beta.y != 0.0) {
+            const double2* const O = gj ? d->xcur : d->C;
+            const int ldo = gj ? d->ldx : d->ldc;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int r = r0 + i * 16 + 8 * h;
+              if (r >= M || (gj && r >= d->k0 && r < d->k0 + d->jb)) continue;
+              const double2* const row = O + (gj ? d->perm[r] : r);
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+                if (c0 + j * 8 + q < N) old[2 * h + q] = row[(size_t)(c0 + j * 8 + q) * ldo];
+            }
+          }
+          if (!gj) {
+            const double2 al = d->alpha, be = d->beta;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const double re = accR[i][j][q], im = accI[i][j][q];
+              old[q] = cadd(make_double2(al.x * re - al.y * im, al.x * im + al.y * re), cmul(be, old[q]));
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) old[q] = make_double2(accR[i][j][q] + old[q].x, accI[i][j][q] + old[q].y);
+          }
+          const bool want_max = d->maxabs != nullptr;
+          double2* const C = d->C;
+          const int ldc = d->ldc;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const int r = m0 + wm * 16 * F + i * 16 + g + ((q >> 1) << 3);
-            const int c = n0 + wn * 8 * F + j * 8 + 2 * t + (q & 1);
-            old[j][q] = epi_old_d<EM>(d, r, c);
+            const int r = r0 + i * 16 + 8 * (q >> 1), c = c0 + j * 8 + (q & 1);
+            if (r >= M || c >= N) continue;
+            C[(size_t)r + (size_t)c * ldc] = old[q];
+            if (want_max) lmax = fmax(lmax, cabs(old[q]));
           }
-#pragma unroll
-        for (int j = 0; j < F; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = m0 + wm * 16 * F + i * 16 + g + ((q >> 1) << 3);
-            const int c = n0 + wn * 8 * F + j * 8 + 2 * t + (q & 1);
-            epi_store_d<EM>(d, r, c, accR[i][j][q], accI[i][j][q], old[j][q], lmax);
-          }
-      }
+        }
     }
-    if (++kt == d->nk) { kt = 0; tile += d->tstep; }
+    if (++kt == d->nk) { kt = 0; next_tile(tm, tn); }
   }
   if (d->maxabs) {
     // warp max then one atomic per warp on the shared accumulator

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_engine(EngineArgs a) {
     if (st == STEP_DONE) break;
     if (st == STEP_GEMM) {
       const GemmDesc* d = reinterpret_cast<const GemmDesc*>(smap.main + kGemmDescOffset);
-      if (d->tile == kTile) cta_gemm_body<OP_RT, OP_RT, EPI_RT, kTile>(d, smap.main);
+      if (d->tile == kTile) cta_gemm_body<kTile>(d, smap.main);
       else gemm_run_small(d, smap.main);
     } else if (st == STEP_ROWS) {
       rows_run(c.ip, smap.main, smap.inv);
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   Operand Bo = (dagger == 2) ? opC(B + b * sB, n) : opN(B + b * sB, k);
   const GemmDesc* d = gemm_desc_publish(m, n, k, Ao, Bo, epi_store(C + b * sC, m, alpha, beta), sm.main, blockIdx.x,
                                         gridDim.x);
-  if (d->tile == kTile) cta_gemm_body<OP_RT, OP_RT, EPI_RT, kTile>(d, sm.main);
+  if (d->tile == kTile) cta_gemm_body<kTile>(d, sm.main);
   else gemm_run_small(d, sm.main);
 }
 

@@ -6,10 +6,10 @@
 
 namespace negf {
 
-__device__ void gemm_run(const GemmDesc* d, double2* smem) { cta_gemm_body<OP_RT, OP_RT, EPI_RT, kTile>(d, smem); }
+__device__ void gemm_run(const GemmDesc* d, double2* smem) { cta_gemm_body<kTile>(d, smem); }
 
 __device__ void gemm_run_small(const GemmDesc* d, double2* smem) {
-  cta_gemm_body<OP_RT, OP_RT, EPI_RT, kSmallTile>(d, smem);
+  cta_gemm_body<kSmallTile>(d, smem);
 }
 
 }  // namespace negf
