@@ -357,12 +357,14 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
     const int kleft = d->K - kt * TK;
 #pragma unroll
     for (int ks = 0; ks < TK / 4; ++ks) {
-      if (ks == TK / 4 - 2) {
-        // refill the buffer of step - 1 with step + kStages - 1, behind half of
-        // the products: right after the barrier every warp would form its
-        // addresses at once with the pipe idle (296 products of order 512:
-        // 10.36 ms there, 10.12 after the first quarter, 9.96 here; of order
-        // 256: 1.360, 1.317, 1.302)
+      if (ks == (warp < 4 ? (TK / 4 - 1) / 2 : TK / 4 - 1)) {
+        // refill the buffer of step - 1 with step + kStages - 1, among the
+        // products: right after the barrier every warp would form its addresses
+        // at once with the pipe idle (296 products of order 512: 10.36 ms there,
+        // 9.96 behind half of the products).  The two warps of a scheduler
+        // (w, w + 4) take different places, so that one computes meanwhile:
+        // 296 of order 512 in 9.53 ms both behind half, 9.48 so; 6 of them
+        // 307 us, 293 so.
         if (ld_step < total) {
           issue(ld_step % kStages);
         } else {
