@@ -253,7 +253,7 @@ int max_ctas(negf_b200_ctx* ctx) {
 
 // The launches of an engine call and its workspace.
 struct EnginePlan {
-  negf::TeamShape ts, tc;        // whole points (or their sweeps); contacts
+  negf::TeamPlan ts, tc;         // whole points (or their sweeps); contacts
   bool split;                    // two launches: contacts, then sweeps
   size_t per, per_c;             // bytes of a team's slots in each
   size_t ints, blocks;           // bytes kept between the two launches
@@ -267,7 +267,7 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
   const int sms = std::max(1, ctx->sms), ctas = max_ctas(ctx);
   pl.per = (size_t)negf::engine_ws_elems(mode, sh.nbl_max, sh.ncont_max, sh.nmax) * sizeof(double2);
   pl.per_c = (size_t)negf::engine_contact_elems(sh.nmax) * sizeof(double2);
-  pl.ts = negf::team_shape(npts, sh.nmax, ctas, sms);
+  pl.ts = negf::team_plan(npts, sh.nmax, ctas, sms);
   // A call whose (point, contact) pairs do not fill the GPU many times over is
   // split: the contacts are independent of one another and most of a point's
   // time, and two launches give each part its own number of teams (n = 384, 12
@@ -278,8 +278,8 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
   pl.blocks = (size_t)pairs * sh.nmax * sh.nmax * sizeof(double2) * (outer ? 2 : 1);
   pl.ints = (2 * (size_t)pairs * sizeof(int) + 255) / 256 * 256;
   pl.split = sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && pl.blocks <= (size_t(4) << 30);
-  pl.tc = negf::TeamShape{1, 1};
-  if (pl.split) pl.tc = negf::team_shape((int)pairs, sh.nmax, ctas, sms);
+  pl.tc = pl.ts;
+  if (pl.split) pl.tc = negf::team_plan((int)pairs, sh.nmax, ctas, sms);
   if (ctx->ws_limit > 0) {
     // fewer resident teams when the workspace would exceed the limit (the persistent
     // kernel still runs every point); not even one: refuse
@@ -290,12 +290,16 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
     if (fit < 1)
       return fail(ctx, NEGF_B200_ERR_ADMISSION, "one point's workspace (" + std::to_string(pl.per) +
                                                     " bytes) exceeds the workspace limit");
-    if ((size_t)pl.ts.teams > fit) pl.ts = negf::team_shape((int)fit, sh.nmax, ctas, sms);
-    if (pl.split && (size_t)pl.tc.teams > rest / pl.per_c)
-      pl.tc = negf::team_shape((int)(rest / pl.per_c), sh.nmax, ctas, sms);
+    auto fewer = [&](negf::TeamPlan& t, int work, size_t teams) {
+      t.parts = 1;
+      t.count[0] = work;
+      t.shape[0] = negf::team_shape((int)teams, sh.nmax, ctas, sms);
+    };
+    if ((size_t)pl.ts.most_teams() > fit) fewer(pl.ts, npts, fit);
+    if (pl.split && (size_t)pl.tc.most_teams() > rest / pl.per_c) fewer(pl.tc, (int)pairs, rest / pl.per_c);
   }
-  pl.need = (size_t)pl.ts.teams * pl.per;
-  if (pl.split) pl.need = std::max(pl.need, (size_t)pl.tc.teams * pl.per_c) + pl.ints + pl.blocks;
+  pl.need = (size_t)pl.ts.most_teams() * pl.per;
+  if (pl.split) pl.need = std::max(pl.need, (size_t)pl.tc.most_teams() * pl.per_c) + pl.ints + pl.blocks;
   pl.need += 256;
   return NEGF_B200_OK;
 }
@@ -317,31 +321,41 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
   a.trace = ctx->trace ? ctx->d_trace : nullptr;
   // the queue heads lie at the start of the workspace
   char* p = reinterpret_cast<char*>(ctx->ws);
-  CK(cudaMemsetAsync(p, 0, 2 * sizeof(int), s));
-  a.counter = reinterpret_cast<int*>(p);
+  CK(cudaMemsetAsync(p, 0, 4 * sizeof(int), s));
+  a.counter = reinterpret_cast<int*>(p);   // one queue head per launch
   p += 256;
+  auto launch = [&](const negf::TeamPlan& t) -> cudaError_t {
+    a.item0 = 0;
+    for (int i = 0; i < t.parts; ++i) {
+      a.item_end = a.item0 + t.count[i];
+      const cudaError_t e = negf::launch_engine(a, t.shape[i].teams, t.shape[i].team, s);
+      if (e != cudaSuccess) return e;
+      ++ctx->launches;
+      ++a.counter;
+      a.item0 = a.item_end;
+    }
+    return cudaSuccess;
+  };
   cudaError_t e = cudaSuccess;
   if (pl.split) {
+    const int64_t pairs = (int64_t)a.npts * sh.ncont_max;
     a.ncyc_pc = reinterpret_cast<int*>(p);
-    a.st_pc = a.ncyc_pc + (int64_t)a.npts * sh.ncont_max;
+    a.st_pc = a.ncyc_pc + pairs;
     p += pl.ints;
     a.sig_pc = reinterpret_cast<double2*>(p);
-    a.gs_pc = a.acc_lc ? a.sig_pc + (int64_t)a.npts * sh.ncont_max * a.Q : nullptr;
+    a.gs_pc = a.acc_lc ? a.sig_pc + pairs * a.Q : nullptr;
     p += pl.blocks;
     a.ws = reinterpret_cast<double2*>(p);
     a.part = negf::PART_CONTACTS;
     a.ws_per_team = (int64_t)(pl.per_c / sizeof(double2));
-    e = negf::launch_engine(a, pl.tc.teams, pl.tc.team, s);
+    e = launch(pl.tc);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
-    ++ctx->launches;
     a.part = negf::PART_SWEEPS;
-    a.counter += 1;
   }
   a.ws = reinterpret_cast<double2*>(p);
   a.ws_per_team = (int64_t)(pl.per / sizeof(double2));
-  e = negf::launch_engine(a, pl.ts.teams, pl.ts.team, s);
+  e = launch(pl.ts);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch_engine");
-  ++ctx->launches;
   return NEGF_B200_OK;
 }
 

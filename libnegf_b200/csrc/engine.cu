@@ -270,39 +270,83 @@ static int resident_teams(int team) {
 // 825000 -> 195000 (16); n = 97, 48 points 28200 -> 16050 (4); n = 256, 320
 // points 400000 -> 362000 (2); 296 points stay with one CTA (278000; 304000
 // in teams of 2).
-TeamShape team_shape(int work, int n, int max_ctas, int sms) {
+static double team_cost(int work, int n, int max_ctas, int sms, int lg, TeamShape* shape) {
   static const double kAlone[3][5] = {{1.0, 0.90, 0.71, 0.70, 0.70},    // n <= 80
                                       {1.0, 0.64, 0.45, 0.385, 0.32},   // n <= 150
                                       {1.0, 0.58, 0.33, 0.225, 0.18}};
-  const double* alone = kAlone[n <= 80 ? 0 : (n <= 150 ? 1 : 2)];
-  TeamShape best{1, std::max(1, std::min(work, max_ctas))};
-  double best_cost = 0.0;
+  const int team = 1 << lg;
+  if (team > 1 && n <= 40) return -1.0;
+  int teams = std::min(max_ctas / team, team > 1 ? resident_teams(team) : max_ctas);
+  if (teams < 1) return -1.0;
+  const double waves = (double)work / teams;
+  teams = std::min(teams, std::max(1, work));
+  const double c = 148.0 * teams * team / sms;   // CTAs per 148 SMs
+  double share = 1.0, w = 1.0;
+  if (team <= 2) {
+    if (c > 148.0) share = 1.6;
+    const double whole = (double)(int)waves, frac = waves - whole;
+    if (waves > 1.0) w = whole + (frac > 0.0 ? (team == 1 ? 0.4 + 0.45 * frac : 0.3 + 0.55 * frac) : 0.0);
+  } else {
+    if (c > 192.0) share = 1.42 + 0.63 * (c - 192.0) / 104.0;
+    else if (c > 148.0) share = 1.35 + 0.07 * (c - 148.0) / 44.0;
+    else if (c > 100.0) share = 1.0 + 0.35 * (c - 100.0) / 48.0;
+    if (waves > 1.0) w = 0.35 + 0.68 * waves;
+  }
+  *shape = TeamShape{team, teams};
+  return kAlone[n <= 80 ? 0 : (n <= 150 ? 1 : 2)][lg] * share * w;
+}
+
+static double best_team(int work, int n, int max_ctas, int sms, TeamShape* best) {
+  double best_cost = -1.0;
+  *best = TeamShape{1, std::max(1, std::min(work, max_ctas))};
   for (int lg = 0; lg <= 4; ++lg) {
-    const int team = 1 << lg;
-    if (team > 1 && n <= 40) break;
-    int teams = std::min(max_ctas / team, team > 1 ? resident_teams(team) : max_ctas);
-    if (teams < 1) break;
-    const double waves = (double)work / teams;
-    teams = std::min(teams, std::max(1, work));
-    const double c = 148.0 * teams * team / sms;   // CTAs per 148 SMs
-    double share = 1.0, w = 1.0;
-    if (team <= 2) {
-      if (c > 148.0) share = 1.6;
-      const double whole = (double)(int)waves, frac = waves - whole;
-      if (waves > 1.0) w = whole + (frac > 0.0 ? (team == 1 ? 0.4 + 0.45 * frac : 0.3 + 0.55 * frac) : 0.0);
-    } else {
-      if (c > 192.0) share = 1.42 + 0.63 * (c - 192.0) / 104.0;
-      else if (c > 148.0) share = 1.35 + 0.07 * (c - 148.0) / 44.0;
-      else if (c > 100.0) share = 1.0 + 0.35 * (c - 100.0) / 48.0;
-      if (waves > 1.0) w = 0.35 + 0.68 * waves;
-    }
-    const double cost = alone[lg] * share * w;
-    if (lg == 0 || cost < best_cost) {
-      best = TeamShape{team, teams};
-      best_cost = cost;
+    TeamShape t;
+    const double c = team_cost(work, n, max_ctas, sms, lg, &t);
+    if (c >= 0.0 && (best_cost < 0.0 || c < best_cost)) {
+      best_cost = c;
+      *best = t;
     }
   }
-  return best;
+  return best_cost;
+}
+
+TeamShape team_shape(int work, int n, int max_ctas, int sms) {
+  TeamShape t;
+  best_team(work, n, max_ctas, sms, &t);
+  return t;
+}
+
+// Problems a little above one full wave of the best team size leave most CTAs
+// idle in the second wave, although larger teams would finish it sooner: up to
+// two waves, the full one and the rest run as two launches where the costs
+// above say 5 % or more (below that the drain of the first launch takes the
+// gain).  320 points of order 256 with DOS (12 layers): 566 -> 539 ms;
+// 160 points of order 128: 31.6 -> 29.5, of order 97: 27.1 -> 25.7.  Beyond two waves the
+// points' different decimation counts smear the waves and the split gained
+// nothing (600 points of order 128: 88.7 -> 92.6 ms with it).
+TeamPlan team_plan(int work, int n, int max_ctas, int sms) {
+  TeamPlan pl;
+  pl.parts = 1;
+  pl.count[0] = work;
+  pl.count[1] = 0;
+  double cost = 0.95 * best_team(work, n, max_ctas, sms, &pl.shape[0]);
+  pl.shape[1] = pl.shape[0];
+  for (int lg = 0; lg <= 4; ++lg) {
+    TeamShape t, rest;
+    if (team_cost(work, n, max_ctas, sms, lg, &t) < 0.0 || work <= t.teams || work % t.teams == 0) continue;
+    if (work > 2 * t.teams) continue;
+    const int whole = work / t.teams * t.teams;
+    const double c = team_cost(whole, n, max_ctas, sms, lg, &t) + best_team(work - whole, n, max_ctas, sms, &rest);
+    if (c < cost) {
+      cost = c;
+      pl.parts = 2;
+      pl.count[0] = whole;
+      pl.count[1] = work - whole;
+      pl.shape[0] = t;
+      pl.shape[1] = rest;
+    }
+  }
+  return pl;
 }
 
 // ---------------------------------------------------------------- primitives

@@ -61,6 +61,7 @@ enum Part : int { PART_ALL = 0, PART_CONTACTS = 1, PART_SWEEPS = 2 };
 
 struct EngineArgs {
   int mode;
+  int item0, item_end;           // the queue's items of this launch: [item0, item_end)
   int part;
   double2* sig_pc;               // npts x ncont_max slots of Q elements (split calls)
   double2* gs_pc;                // the same for the kept surface GFs, or null
@@ -125,6 +126,8 @@ size_t engine_smem_bytes(int nmax);
 // kernel and device (not per launch), so that a launch is a stream operation
 // only and can be captured into a CUDA graph.
 cudaError_t team_opt_in(const void* kernel, size_t smem = 0);
+// The launch of `teams` clusters of `team` CTAs; attr must live until the launch.
+cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr);
 
 // `teams` teams of `team` CTAs (a thread-block cluster; 1, 2, 4, 8 or 16), one
 // point at a time each
@@ -136,6 +139,16 @@ struct TeamShape {
   int team, teams;
 };
 TeamShape team_shape(int work, int n, int max_ctas, int sms);
+
+// A queue of `work` problems as one or two launches: where the last wave of
+// one team size would leave most CTAs idle, its problems run in a launch of
+// their own with larger teams.
+struct TeamPlan {
+  int parts, count[2];
+  TeamShape shape[2];
+  int most_teams() const { return parts > 1 && shape[1].teams > shape[0].teams ? shape[1].teams : shape[0].teams; }
+};
+TeamPlan team_plan(int work, int n, int max_ctas, int sms);
 
 // CSR -> dense blocks (csr.cu).  Indices 1-based as libNEGF's z_CSR; the
 // outputs are zero-filled staging arrays in the negf_b200_device layout.

@@ -508,14 +508,14 @@ dispatch:
       // ---------------------------------------------------------- next point
       if (lead()) *sm.item = atomicAdd(a.counter, 1);
       team_sync();
-      s.p = team_ld_int(sm.item, 0);
+      s.p = a.item0 + team_ld_int(sm.item, 0);
       team_sync();
+      if (s.p >= a.item_end) break;
       s.c = 0;
       if (a.part == PART_CONTACTS) {   // an item is one contact of a point
         s.c = s.p % a.ncont_max;
         s.p /= a.ncont_max;
       }
-      if (s.p >= a.npts) break;
       bind_point(a, w, s.p);
       s.d = a.devs + a.dev_id[s.p];
       s.E = a.energy[s.p];

@@ -198,3 +198,24 @@ def test_split_calls_match_one_launch(gpu_ctx):
         gpu_ctx.set_options()
         for h in hs:
             gpu_ctx.release(h)
+
+
+@pytest.mark.parametrize("npts", [149, 297])
+def test_last_wave_in_a_launch_of_its_own(gpu_ctx, npts):
+    """149 points have 298 contacts and 297 points as many sweeps: a little
+    over one wave of 296 CTAs, whose rest runs with larger teams.  The same
+    bits as in calls that fit one wave."""
+    h = gpu_ctx.upload(G.transport_c0(nbl=3, n=84, seed=9))
+    E = np.linspace(-1.4, 1.4, npts)
+    try:
+        n0 = gpu_ctx.launch_count()
+        got = gpu_ctx.transmission_dos(h, E, eta=1e-3, dos_delta=1e-3)
+        whole = gpu_ctx.launch_count() - n0
+        n0 = gpu_ctx.launch_count()
+        parts = [gpu_ctx.transmission_dos(h, e, eta=1e-3, dos_delta=1e-3) for e in np.array_split(E, 3)]
+        assert whole == 3 and gpu_ctx.launch_count() - n0 == 6
+        for k, x in enumerate(got):
+            assert np.array_equal(x, np.concatenate([p[k] for p in parts]))
+        assert np.all(got[3] == 0)
+    finally:
+        gpu_ctx.release(h)
