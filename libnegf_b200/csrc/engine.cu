@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 // SMs of the current device, asked once per device.
-static int device_sms() {
+int device_sms() {
   static std::mutex mu;
   static int known[64];
   int dev = 0, n = 0;

@@ -126,6 +126,7 @@ size_t engine_smem_bytes(int nmax);
 // kernel and device (not per launch), so that a launch is a stream operation
 // only and can be captured into a CUDA graph.
 cudaError_t team_opt_in(const void* kernel, size_t smem = 0);
+int device_sms();   // of the current device
 // The launch of `teams` clusters of `team` CTAs; attr must live until the launch.
 cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr);
 

@@ -1,6 +1,6 @@
 // Small-order transmission (small.cuh): the 2-contact Caroli solve of a point
-// of block order n <= 32 by one CTA, following the reference routine by
-// routine:
+// of block order n <= 32 by one CTA, or by two with a contact each, following
+// the reference routine by routine:
 //   surface_green + decimation   src/contselfenergy.F90:184-210, 271-340
 //   compute_contacts             src/contselfenergy.F90:445-491, 552-566
 //   build_ESH (real E)           src/iterative.F90:1956-1982
@@ -13,7 +13,7 @@
 // this one: about 280 launches a call, operands through memory each time) a
 // launch was 10 to 25 us of mostly fixed latency.  Here a point's blocks
 // never leave the SM between operations: one energy of a 20-layer device of
-// order 32 takes 1.30 ms (3.10 before), 512 energies 3.34 ms (6.07).
+// order 32 takes 0.94 ms (3.10 before), 512 energies 3.34 ms (6.07).
 #include <cuda_runtime.h>
 
 #include "../../include/negf_b200.h"
@@ -33,7 +33,7 @@ constexpr unsigned kFull = 0xffffffffu;
 
 struct SmallShared {
   InvScratch inv;
-  int piv[32], perm[32], cperm[32], flag;
+  int piv[32], perm[32], cperm[32], flag, ncyc, st;
   double red[3][8];
   double2 y[32];
 };
@@ -101,6 +101,16 @@ __device__ __forceinline__ Frag get(const Lane& L, const double2* S) {
   Frag f;
 #pragma unroll
   for (int q = 0; q < 4; ++q) f.v[q] = L.in(q) ? S[L.at(q)] : make_double2(0.0, 0.0);
+  return f;
+}
+// get() from the shared memory of another CTA of the cluster
+__device__ __forceinline__ Frag team_get(const Lane& L, const double2* S, int rank) {
+  Frag f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const double* e = reinterpret_cast<const double*>(S + L.at(q));
+    f.v[q] = L.in(q) ? make_double2(team_ld_double(e, rank), team_ld_double(e + 1, rank)) : make_double2(0.0, 0.0);
+  }
   return f;
 }
 __device__ __forceinline__ void sub_from(const Lane& L, double2* D, const Frag& f) {
@@ -230,7 +240,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
   double2* const X = block(B_X);
   double2* const SL = block(B_SL);               // the left self-energy
   SmallShared& sh = shared();
-  const int p = blockIdx.x, n = a.n;
+  const int pair = team_size() == 2, rank = team_rank();
+  const int p = blockIdx.x >> pair, n = a.n;
   const Lane L(n);
   if (threadIdx.x == 0) {
     sh.inv.piv = sh.piv;
@@ -249,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
   auto put_st = [&](int code) { if (st == NEGF_B200_OK) st = code; };
 
 #pragma unroll 1
-  for (int side = 0; side < 2; ++side) {
+  for (int side = rank; side < (pair ? rank + 1 : 2); ++side) {
     const int c = side == 0 ? a.left : a.right;
     const double2* h00 = d.h00 + d.olead[c];
     const double2* h01 = d.h01 + d.olead[c];
@@ -378,10 +389,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     __syncthreads();
     put(L, X, mm(L, Bo, Go));
     __syncthreads();
-    const Frag sig = mm(L, X, Co);
-    if (side == 0) {
-      put(L, SL, sig);
-    } else {
+    Frag sig = mm(L, X, Co);
+    if (side == rank) put(L, SL, sig);
+    if (pair) {
+      // one contact per CTA: CTA 0 goes on with both
+      if (threadIdx.x == 0) {
+        sh.ncyc = ncyc;
+        sh.st = st;
+      }
+      team_sync();
+      if (rank == 0) {
+        sig = team_get(L, SL, 1);
+        ncyc += team_ld_int(&sh.ncyc, 1);
+        put_st(team_ld_int(&sh.st, 1));
+      }
+      team_sync();   // CTA 1's shared memory is read
+      if (rank == 1) return;
+    }
+    if (side == 1 || pair) {
       // W = ESH(nbl, nbl) - Sigma_right
       load_esh(n, Ao, d.hd + d.od[a.nbl - 1], d.has_s ? d.sd + d.od[a.nbl - 1] : nullptr, make_double2(E, 0.0), true,
                false);
@@ -458,8 +483,12 @@ cudaError_t launch_small_points(const MixedArgs& a, cudaStream_t s) {
   if (a.n < 1 || a.n > kSmallMax) return cudaErrorInvalidValue;
   cudaError_t e = team_opt_in((const void*)k_small_point, kSmallSmem);
   if (e != cudaSuccess) return e;
-  k_small_point<<<a.npts, kThreads, kSmallSmem, s>>>(a);
-  e = cudaGetLastError();
+  // Two CTAs per point, a contact each, while they find room at once: order
+  // 32, 74 points: 1.34 ms by one CTA, 0.96 by two; 148 points (two CTAs per
+  // SM): 1.35 and 1.22; 149: 1.71 and 2.00.
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = team_config(a.npts, a.npts <= device_sms() ? 2 : 1, kSmallSmem, s, &attr);
+  e = cudaLaunchKernelEx(&cfg, k_small_point, a);
   if (e == cudaSuccess && a.launches) ++*a.launches;
   return e;
 }

@@ -1,5 +1,5 @@
-// Small-order transmission (n <= 32): one CTA solves one (E, k) point from
-// the lead blocks to the Caroli trace in a single launch, every block in
+// Small-order transmission (n <= 32): one CTA (or two, one per contact) solves one
+// (E, k) point from the lead blocks to the Caroli trace in a single launch, every block in
 // shared memory or registers.
 #pragma once
 #include "mixed.cuh"

@@ -219,3 +219,30 @@ def test_last_wave_in_a_launch_of_its_own(gpu_ctx, npts):
         assert np.all(got[3] == 0)
     finally:
         gpu_ctx.release(h)
+
+
+@pytest.mark.parametrize("n", [1, 7, 16, 31, 32])
+def test_small_orders_by_one_or_two_ctas(gpu_ctx, n):
+    """Up to as many points as SMs two CTAs share a point, a contact each; with
+    more, one CTA does both.  The same bits, cycle counts and statuses, with a
+    non-finite lead on either side and on both."""
+    hs = []
+    for side in (None, 0, 1, 2):
+        dev = G.transport_c0(nbl=3, n=n, seed=11)
+        for c in range(2):
+            if side in (c, 2):
+                dev.lead_h00[c][0, 0] = np.nan
+        hs.append(gpu_ctx.upload(dev))
+    E = np.linspace(-1.1, 1.1, 160)
+    ids = np.asarray(hs, dtype=np.int32)[np.arange(160) % 4]
+    try:
+        one = gpu_ctx.transmission(ids, E, eta=1e-3, check=False)
+        two = [gpu_ctx.transmission(i, e, eta=1e-3, check=False)
+               for i, e in zip(np.array_split(ids, 4), np.array_split(E, 4))]
+        for k, x in enumerate(one):
+            assert np.array_equal(x, np.concatenate([t[k] for t in two]), equal_nan=k == 0)
+        good = ids == hs[0]
+        assert np.all(one[2][good] == 0) and np.all(one[2][~good] != 0)
+    finally:
+        for h in hs:
+            gpu_ctx.release(h)
