@@ -212,6 +212,7 @@ struct Epilogue {
   int k0, jb;           // pivot rows [k0, k0+jb) of the applied block (masked)
   // optional reduction of max |C| over stored elements
   double* maxabs;       // smem accumulator (nullptr = off)
+  bool idle_max = false;   // take part in the team's reduction with 0 (another CTA's product has the maximum)
 };
 
 __device__ __forceinline__ Epilogue epi_store(double2* C, int ldc, double2 alpha, double2 beta) {
@@ -240,6 +241,7 @@ struct GemmDesc {
   int tile0, tstep;   // first output tile of this CTA and the team's size
   int amode, bmode, emode;
   int tile;            // kTile or kSmallTile
+  int want_max;        // the elements stored count for maxabs
 };
 constexpr int kGemmDescOffset = kRingElems;   // in double2 units, after the staging ring
 
@@ -442,7 +444,7 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
 #pragma unroll
             for (int q = 0; q < 4; ++q) old[q] = make_double2(accR[i][j][q] + old[q].x, accI[i][j][q] + old[q].y);
           }
-          const bool want_max = d->maxabs != nullptr;
+          const bool want_max = d->want_max != 0;
           double2* const C = d->C;
           const int ldc = d->ldc;
 #pragma unroll
@@ -510,6 +512,7 @@ __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, cons
     d->C = e.C; d->ldc = e.ldc; d->alpha = e.alpha; d->beta = e.beta;
     d->xcur = e.xcur; d->ldx = e.ldx; d->perm = e.perm; d->k0 = e.k0; d->jb = e.jb;
     d->maxabs = e.maxabs;
+    d->want_max = e.maxabs != nullptr && !e.idle_max;
     d->M = M; d->N = N; d->K = K;
     d->amode = A.mode; d->bmode = B.mode; d->emode = e.mode;
     const int T = gemm_tile(M, N, size);

@@ -42,10 +42,11 @@ __device__ int engine_step(const EngineArgs& a, EngineCtl& c, SmemMap& sm) {
         if (tid == 0) *sm.maxv = 0.0;
         __syncthreads();
         e.maxabs = sm.maxv;
+        e.idle_max = o.flag == 2;
       }
       c.t0 = sm.tr.start();
       gemm_desc_publish(o.m, o.n, o.k, Operand{o.A, o.lda, o.opa, nullptr}, Operand{o.B, o.ldb, o.opb, nullptr}, e,
-                        sm.main);
+                        sm.main, o.rank, o.size);
       c.open = TR_GEMM;
       return STEP_GEMM;
     }

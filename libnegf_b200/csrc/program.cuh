@@ -95,12 +95,12 @@ struct Ws {
 // ---------------------------------------------------------------- ops
 enum OpKind : int {
   K_NONE = 0,
-  K_GEMM,      // C = alpha op(A) op(B) + beta C   (flag: reduce max|C| into sm.maxv)
+  K_GEMM,      // C = alpha op(A) op(B) + beta C   (flag 1: reduce max|C| into sm.maxv; 2: another CTA's product does)
   K_ZINV,      // C = A^-1, order n                 (info -> ires[0])
   K_ESH,       // C (m x n) = s_e S - H - sub - diag(subdiag)   (A = H, X = S, Y = sub, V = subdiag)
   K_COPY,      // C = A, m elements
   K_SUB,       // C -= A, m elements
-  K_DECUPD,    // C -= A and D -= A, m elements (decimation Ao_s, Ao update)
+  K_DECUPD,    // C -= A and D = D - A + B, m elements (decimation Ao_s, Ao update)
   K_SPECTRAL,  // C = i (A - A^dag), order m
   K_TRACE,     // res[slot] = Re Tr(A op(B)), order m (diagonal entries k with mask[k], if mask)
   K_TRACEC,    // res[slot], res[slot+1] = Tr(A op(B)), A m x n
@@ -140,7 +140,8 @@ struct Op {
   int kind;
   int m, n, k;
   int opa, opb, flag, slot;
-  int lda, ldb, ldc, pad;
+  int lda, ldb, ldc;
+  int rank, size;              // K_GEMM: this CTA's place among the CTAs that share its product
   const double2* A;
   const double2* B;
   double2* C;
@@ -161,6 +162,24 @@ __device__ __forceinline__ void set_gemm(Op& o, int M, int N, int K, const doubl
                                          double2 be, int want_max = 0) {
   o.kind = K_GEMM; o.m = M; o.n = N; o.k = K; o.A = A; o.lda = lda; o.opa = opa; o.B = B; o.ldb = ldb;
   o.opb = opb; o.C = C; o.ldc = ldc; o.alpha = al; o.beta = be; o.flag = want_max;
+  o.rank = team_rank(); o.size = team_size();
+}
+
+// Independent products in one step: `of` of them (a power of two, at most the
+// team's size), each by its own part of the team.  A product spread over a
+// whole team is mostly fixed latency (pipeline fill, epilogue, cluster
+// barrier: of 6.6 us for order 64 over four CTAs 2.1 are products), and its
+// tiles rarely divide by the team; side by side these are paid once.  A
+// decimation iteration takes two such steps for six, the forward retarded
+// sweep three for five, a layer of the lesser sweep five for six: SCBA of 32
+// points of order 64 34.8 -> 32.5 ms, 6 points of order 768 131.2 -> 128.
+// The last iteration computes Self, B1 and D in vain; one CTA alone, which
+// would pay for them, does not.
+__device__ __forceinline__ int group_part(int of) { return team_rank() / (team_size() / of); }
+__device__ __forceinline__ int pair_width() { return team_size() > 1 ? 2 : 1; }
+__device__ __forceinline__ void group_gemm(Op& o, int of) {
+  o.size = team_size() / of;
+  o.rank = team_rank() % o.size;
 }
 
 __device__ __forceinline__ void set_esh(Op& o, double2* D, int rows, int cols, const double2* H, const double2* S,
@@ -196,7 +215,7 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
       for (int q = q0; q < o.m; q += qs) {
         const double2 s = o.A[q];
         o.C[q] = csub(o.C[q], s);
-        o.D[q] = csub(o.D[q], s);
+        o.D[q] = cadd(o.B[q], csub(o.D[q], s));
       }
       break;
     case K_SPECTRAL:
@@ -393,7 +412,7 @@ struct Prog {
   int st, ncyc;
   double2 ec, ecs;      // ES-H energy, contact energy
   // contacts / decimation
-  int c, L, ncb, it, ok, done, ib, ix, ic, ic1;
+  int c, L, ncb, it, ok, done, ib, ib1, ic, ic1, gw, gq;
   int att;              // decimation attempt (retarded-branch retries)
   int diverged;         // the attempt's max|C1| went Inf / NaN
   int sens;             // the attempt met a nearly singular Ao (condition estimate above kSensitiveCond)
@@ -463,6 +482,18 @@ __device__ __forceinline__ const double2* esh_lo_op(const DevDesc* d, int i, con
 }
 __device__ __forceinline__ double2 esh_al(const DevDesc* d, double2 a) {
   return d->has_s ? a : make_double2(-a.x, -a.y);
+}
+
+// Product q of a decimation iteration (Ao slot 0, Go 4, X 5, Y 12): 4 X = Go
+// Co, 5 Y = Go Bo; 0 C1 = Co X with max|C1|, 1 Self = Bo X (slot 6), 2 B1 = Bo
+// Y, 3 D = -Co Y (slot 13).
+__device__ __forceinline__ void dec_product(Op& o, const Prog& s, const Ws& w, int q) {
+  const bool left_c = q == 0 || q == 3, of_x = q < 2;
+  const double2* A = w.slot(q >= 4 ? 4 : (left_c ? s.ic : s.ib));
+  const double2* B = w.slot(q >= 4 ? (q == 4 ? s.ic : s.ib) : (of_x ? 5 : 12));
+  double2* C = w.slot(q >= 4 ? (q == 4 ? 5 : 12) : (of_x ? (q == 0 ? s.ic1 : 6) : (q == 2 ? s.ib1 : 13)));
+  set_gemm(o, s.L, s.L, s.L, A, s.L, OP_N, B, s.L, OP_N, C, s.L, make_double2(q == 3 ? -1.0 : 1.0, 0.0),
+           make_double2(0.0, 0.0), q == 0 ? 1 : (q < s.gw ? 2 : 0));
 }
 
 __device__ __forceinline__ void put_status(int& st, int s) { if (st == ST_OK) st = s; }
@@ -560,17 +591,19 @@ dispatch:
         // ---- decimation (src/contselfenergy.F90:271-340): Ao 0, Aos 1, Go 4, Sf 6
         set_simple(o, K_COPY, s.L * s.L, w.slot(0), w.slot(1));
         PT_EMIT(s);
-        s.ok = 0; s.done = 0; s.diverged = 0; s.ib = 2; s.ix = 5; s.ic = 3; s.ic1 = 7;
+        s.gw = min(team_size(), 4);   // products of a step; one CTA keeps the reference's early end
+        s.ok = 0; s.done = 0; s.diverged = 0; s.ib = 2; s.ib1 = 11; s.ic = 3; s.ic1 = 7;
         for (s.it = 1; s.it <= a.sgf_max_iter; ++s.it) {
           o.kind = K_ZINV; o.m = s.L; o.A = w.slot(0); o.C = w.slot(4);
           PT_EMIT(s);
           if (sm.ires[0]) put_status(s.st, ST_SINGULAR);
           PT_REFINE(s, w.slot(0), w.slot(4), s.L);
-          set_gemm(o, s.L, s.L, s.L, w.slot(4), s.L, OP_N, w.slot(s.ic), s.L, OP_N, w.slot(s.ix), s.L, one, zero);
-          PT_EMIT(s);                                                                    // GoXCo
-          set_gemm(o, s.L, s.L, s.L, w.slot(s.ic), s.L, OP_N, w.slot(s.ix), s.L, OP_N, w.slot(s.ic1), s.L, one,
-                   zero, 1);
-          PT_EMIT(s);                                                                    // C1 = Co GoXCo
+          dec_product(o, s, w, s.gw > 1 ? 4 + group_part(2) : 4);                       // X (and Y)
+          if (s.gw > 1) group_gemm(o, 2);
+          PT_EMIT(s);
+          dec_product(o, s, w, group_part(s.gw));                                        // C1 (and Self; B1, D)
+          if (s.gw > 1) group_gemm(o, s.gw);
+          PT_EMIT(s);
           mx = *sm.maxv;
           if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: this iteration will not converge
             s.diverged = 1;
@@ -582,17 +615,18 @@ dispatch:
           } else {
             s.ok = 0;
           }
-          set_gemm(o, s.L, s.L, s.L, w.slot(s.ib), s.L, OP_N, w.slot(s.ix), s.L, OP_N, w.slot(6), s.L, one, zero);
-          PT_EMIT(s);                                                                    // Self = Bo GoXCo
-          o.kind = K_DECUPD; o.m = s.L * s.L; o.A = w.slot(6); o.C = w.slot(1); o.D = w.slot(0);
-          PT_EMIT(s);                                                                    // Ao_s -= Self, Ao -= Self
-          set_gemm(o, s.L, s.L, s.L, w.slot(4), s.L, OP_N, w.slot(s.ib), s.L, OP_N, w.slot(6), s.L, one, zero);
-          PT_EMIT(s);                                                                    // GoXBo
-          set_gemm(o, s.L, s.L, s.L, w.slot(s.ib), s.L, OP_N, w.slot(6), s.L, OP_N, w.slot(s.ix), s.L, one, zero);
-          PT_EMIT(s);                                                                    // B1 = Bo GoXBo
-          set_gemm(o, s.L, s.L, s.L, w.slot(s.ic), s.L, OP_N, w.slot(6), s.L, OP_N, w.slot(0), s.L, mone, one);
-          PT_EMIT(s);                                                                    // Ao -= Co GoXBo
-          { int t = s.ib; s.ib = s.ix; s.ix = t; t = s.ic; s.ic = s.ic1; s.ic1 = t; }   // Bo = B1, Co = C1
+          if (s.gw == 1) {
+            dec_product(o, s, w, 5);
+            PT_EMIT(s);
+          }
+          for (s.gq = s.gw; s.gq < 4; s.gq += s.gw) {                                    // what is left of Self, B1, D
+            dec_product(o, s, w, s.gq + group_part(s.gw));
+            if (s.gw > 1) group_gemm(o, s.gw);
+            PT_EMIT(s);
+          }
+          o.kind = K_DECUPD; o.m = s.L * s.L; o.A = w.slot(6); o.B = w.slot(13); o.C = w.slot(1); o.D = w.slot(0);
+          PT_EMIT(s);                                                                    // Ao_s -= Self, Ao -= Self + Co Y
+          { int t = s.ib; s.ib = s.ib1; s.ib1 = t; t = s.ic; s.ic = s.ic1; s.ic1 = t; }   // Bo = B1, Co = C1
         }
         o.kind = K_ZINV; o.m = s.L; o.A = w.slot(1); o.C = w.slot(4);
         PT_EMIT(s);                                                                      // gs = Ao_s^-1
@@ -806,29 +840,35 @@ dispatch:
               op_esh_lo(o, s.d, s.i - 1, s.ec, w.slot(1));
               PT_EMIT(s);
             }
-            set_gemm(o, s.d->pl[s.i], s.d->pl[s.i - 1], s.d->pl[s.i], w.layer(0, s.i, s.d->nbl), s.d->pl[s.i], OP_N,
-                     esh_lo_op(s.d, s.i - 1, w.slot(1)), s.d->pl[s.i], OP_N, w.slot(2), s.d->pl[s.i],
-                     esh_al(s.d, one), zero);                                                     // gsmr(i) ESH(i,i-1)
-            PT_EMIT(s);
-            set_gemm(o, s.d->pl[s.i], s.d->pl[s.i - 1], s.d->pl[s.i - 1], w.slot(2), s.d->pl[s.i], OP_N,
-                     (a.mode == MODE_GN) ? w.layer(1, s.i - 1, s.d->nbl) : w.slot(11 - s.cur), s.d->pl[s.i - 1], OP_N,
-                     w.slot(6), s.d->pl[s.i], mone, zero);                                         // Gr(i,i-1)
-            PT_EMIT(s);
-            set_gemm(o, s.d->pl[s.i - 1], s.d->pl[s.i], s.d->pl[s.i], esh_up_op(s.d, s.i - 1, w.slot(0)),
-                     s.d->pl[s.i - 1], OP_N, w.layer(0, s.i, s.d->nbl), s.d->pl[s.i], OP_N, w.slot(3),
-                     s.d->pl[s.i - 1], esh_al(s.d, one), zero);                                   // ESH gsmr
-            PT_EMIT(s);
-            if (a.mode == MODE_GN) {
-              set_gemm(o, s.d->pl[s.i - 1], s.d->pl[s.i], s.d->pl[s.i - 1], w.layer(1, s.i - 1, s.d->nbl),
-                       s.d->pl[s.i - 1], OP_N, w.slot(3), s.d->pl[s.i - 1], OP_N, w.layer(2, s.i - 1, s.d->nbl),
-                       s.d->pl[s.i - 1], mone, zero);                                              // Gr(i-1,i)
+            for (s.gq = 0; s.gq < 2; s.gq += pair_width()) {
+              if (s.gq + group_part(pair_width()) == 0)
+                set_gemm(o, s.d->pl[s.i], s.d->pl[s.i - 1], s.d->pl[s.i], w.layer(0, s.i, s.d->nbl), s.d->pl[s.i],
+                         OP_N, esh_lo_op(s.d, s.i - 1, w.slot(1)), s.d->pl[s.i], OP_N, w.slot(2), s.d->pl[s.i],
+                         esh_al(s.d, one), zero);                                                 // gsmr(i) ESH(i,i-1)
+              else
+                set_gemm(o, s.d->pl[s.i - 1], s.d->pl[s.i], s.d->pl[s.i], esh_up_op(s.d, s.i - 1, w.slot(0)),
+                         s.d->pl[s.i - 1], OP_N, w.layer(0, s.i, s.d->nbl), s.d->pl[s.i], OP_N, w.slot(3),
+                         s.d->pl[s.i - 1], esh_al(s.d, one), zero);                               // ESH gsmr
+              group_gemm(o, pair_width());
+              PT_EMIT(s);
+            }
+            // Gr(i,i-1); GN and RHO: Gr(i-1,i) = -Gr(i-1,i-1) ESH(i-1,i) gsmr(i) beside it
+            s.gw = (a.mode == MODE_GN || a.mode == MODE_RHO) ? 2 : 1;
+            for (s.gq = 0; s.gq < s.gw; s.gq += min(s.gw, team_size())) {
+              const int of = min(s.gw, team_size());
+              const double2* const G = (a.mode == MODE_GN) ? w.layer(1, s.i - 1, s.d->nbl) : w.slot(11 - s.cur);
+              if (s.gq + group_part(of) == 0)
+                set_gemm(o, s.d->pl[s.i], s.d->pl[s.i - 1], s.d->pl[s.i - 1], w.slot(2), s.d->pl[s.i], OP_N, G,
+                         s.d->pl[s.i - 1], OP_N, w.slot(6), s.d->pl[s.i], mone, zero);
+              else
+                set_gemm(o, s.d->pl[s.i - 1], s.d->pl[s.i], s.d->pl[s.i - 1], G, s.d->pl[s.i - 1], OP_N, w.slot(3),
+                         s.d->pl[s.i - 1], OP_N, (a.mode == MODE_GN) ? w.layer(2, s.i - 1, s.d->nbl) : w.slot(5),
+                         s.d->pl[s.i - 1], mone, zero);
+              group_gemm(o, of);
               PT_EMIT(s);
             }
             if (a.mode == MODE_RHO) {
-              // Gr(i-1,i) = -Gr(i-1,i-1) ESH(i-1,i) gsmr(i); then w Gr(i,i-1), w Gr(i-1,i) into the sums
-              set_gemm(o, s.d->pl[s.i - 1], s.d->pl[s.i], s.d->pl[s.i - 1], w.slot(11 - s.cur), s.d->pl[s.i - 1],
-                       OP_N, w.slot(3), s.d->pl[s.i - 1], OP_N, w.slot(5), s.d->pl[s.i - 1], mone, zero);
-              PT_EMIT(s);
+              // w Gr(i,i-1), w Gr(i-1,i) into the sums
               set_simple(o, K_ACCUM, s.d->pl[s.i] * s.d->pl[s.i - 1], w.slot(6), a.acc_l + s.d->oo[s.i - 1]);
               o.alpha = a.weight[s.p];
               PT_EMIT(s);
@@ -1045,10 +1085,14 @@ dispatch:
             op_esh_lo(o, s.d, s.i, s.ec, w.slot(9));
             PT_EMIT(s);
           }
-          set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i], s.d->pl[s.i + 1], w.layer(3, s.i + 1, s.d->nbl),
-                   s.d->pl[s.i + 1], OP_N, w.layer(2, s.i, s.d->nbl), s.d->pl[s.i], OP_C, w.slot(7), s.d->pl[s.i + 1],
-                   one, zero);
-          PT_EMIT(s);
+          for (s.gq = 0; s.gq < 2; s.gq += pair_width()) {   // Sigma_n(i+1,i+1) Gr(i,i+1)^dag, .. Gr(i+1,i+1)^dag
+            const int q = s.gq + group_part(pair_width());
+            set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i + q], s.d->pl[s.i + 1], w.layer(3, s.i + 1, s.d->nbl),
+                     s.d->pl[s.i + 1], OP_N, q == 0 ? w.layer(2, s.i, s.d->nbl) : w.layer(1, s.i + 1, s.d->nbl),
+                     s.d->pl[s.i + q], OP_C, w.slot(q == 0 ? 7 : 0), s.d->pl[s.i + 1], one, zero);
+            group_gemm(o, pair_width());
+            PT_EMIT(s);
+          }
           set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i], s.d->pl[s.i], esh_lo_op(s.d, s.i, w.slot(9)), s.d->pl[s.i + 1],
                    OP_N, w.layer(4 + s.par, s.i, s.d->nbl), s.d->pl[s.i], OP_N, w.slot(7), s.d->pl[s.i + 1],
                    esh_al(s.d, mone), one);
@@ -1059,16 +1103,12 @@ dispatch:
           o.kind = K_DAGGER; o.m = s.d->pl[s.i]; o.n = s.d->pl[s.i + 1]; o.A = w.slot(10);
           o.C = w.layer(6 + s.par, s.i, s.d->nbl);
           PT_EMIT(s);
-          set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i + 1], s.d->pl[s.i + 1], w.layer(3, s.i + 1, s.d->nbl),
-                   s.d->pl[s.i + 1], OP_N, w.layer(1, s.i + 1, s.d->nbl), s.d->pl[s.i + 1], OP_C, w.slot(7),
-                   s.d->pl[s.i + 1], one, zero);
-          PT_EMIT(s);
           set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i + 1], s.d->pl[s.i], esh_lo_op(s.d, s.i, w.slot(9)),
-                   s.d->pl[s.i + 1], OP_N, w.layer(6 + s.par, s.i, s.d->nbl), s.d->pl[s.i], OP_N, w.slot(7),
+                   s.d->pl[s.i + 1], OP_N, w.layer(6 + s.par, s.i, s.d->nbl), s.d->pl[s.i], OP_N, w.slot(0),
                    s.d->pl[s.i + 1], esh_al(s.d, mone), one);
           PT_EMIT(s);
           set_gemm(o, s.d->pl[s.i + 1], s.d->pl[s.i + 1], s.d->pl[s.i + 1], w.layer(0, s.i + 1, s.d->nbl),
-                   s.d->pl[s.i + 1], OP_N, w.slot(7), s.d->pl[s.i + 1], OP_N, w.layer(4 + s.par, s.i + 1, s.d->nbl),
+                   s.d->pl[s.i + 1], OP_N, w.slot(0), s.d->pl[s.i + 1], OP_N, w.layer(4 + s.par, s.i + 1, s.d->nbl),
                    s.d->pl[s.i + 1], one, zero);
           PT_EMIT(s);
         }

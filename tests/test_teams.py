@@ -246,3 +246,35 @@ def test_small_orders_by_one_or_two_ctas(gpu_ctx, n):
     finally:
         for h in hs:
             gpu_ctx.release(h)
+
+
+@pytest.mark.parametrize("dev", [
+    lambda: G.uneven([48, 90, 41, 70], seed=3),
+    lambda: G.transport_c1(nbl=3, n=65, seed=2),
+], ids=["uneven", "n65_S"])
+def test_products_side_by_side(gpu_ctx, dev):
+    """Teams run independent products of the sweeps side by side, one CTA one
+    after another: the same bits, in the lesser and SCBA sweeps and in the
+    density matrix (299 further points of weight zero leave the sum alone)."""
+    h = gpu_ctx.upload(dev())
+    E = np.linspace(-1.2, 1.2, 300)
+    frm = np.stack([np.linspace(1, 0, 300), np.linspace(0, 1, 300)], axis=1)
+    z, w = np.full(300, 0.1 + 0.3j), np.zeros(300, dtype=np.complex128)
+    w[0] = 0.5 + 0.1j
+
+    def flat(x):
+        return [x] if isinstance(x, np.ndarray) else [y for v in x for y in flat(v)]
+
+    try:
+        gpu_ctx.set_options(scba_niter=2)
+        one = gpu_ctx.meir_wingreen(h, E, frm, coupling=0.1, eta=1e-3)
+        rho = flat(gpu_ctx.density(h, z, w)[:2])
+        for m in (1, 30, 80):
+            team = gpu_ctx.meir_wingreen(h, E[:m], frm[:m], coupling=0.1, eta=1e-3)
+            for k in sorted(one):
+                assert np.array_equal(team[k], one[k][:m]), k
+            part = flat(gpu_ctx.density(h, z[:m], w[:m])[:2])
+            assert all(np.array_equal(x, y) for x, y in zip(part, rho))
+    finally:
+        gpu_ctx.set_options()
+        gpu_ctx.release(h)
