@@ -7,8 +7,9 @@
 // retarded sweep with the diagonal spectral density, or the elastic
 // dephasing SCBA loop with the lesser sweep, Meir-Wingreen and layer
 // currents.  Teams pull points from a global queue, so all energy x k points
-// of a call (and all SCBA iterations of each point) run in one launch with
-// no host synchronisation; per-point convergence (decimation, SCBA) is
+// of a call (and all SCBA iterations of each point) run in one launch, or in
+// one for the contacts and one for the rest, with no host synchronisation;
+// per-point convergence (decimation, SCBA) is
 // decided on the device.
 //
 // Reference routines (libNEGF): decimation src/contselfenergy.F90:271-340,
@@ -77,6 +78,8 @@ __device__ __noinline__ int zinv_refined(int n, const double2* A, double2* X, do
   return bad;
 }
 
+constexpr unsigned kDecWaveCtas = 296;   // two CTAs on each of a B200's 148 SMs
+
 // Sancho-Rubio decimation (src/contselfenergy.F90:271-340) by one team.
 // In: Ao, Bo, Co in slot 0, 2, 3 (consumed).  Out: surface GF in *go_out
 // (one of the slots).  Returns a status.
@@ -84,23 +87,36 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
                               SmemMap& sm) {
   double2* Ao = w.slot(0);
   double2* Aos = w.slot(1);
-  double2* Bo = w.slot(2);
-  double2* Co = w.slot(3);
   double2* Go = w.slot(4);
-  double2* X = w.slot(5);
   double2* Sf = w.slot(6);
-  double2* C1 = w.slot(7);
+  double2* D = w.slot(13);
   const int nn = L * L;
   int st = ST_OK;
   team_copy(Aos, Ao, nn);
   team_sync();
   bool ok = false, done = false;
   int it;
-  const double2 one = cz(1, 0), zero = cz(0, 0), mone = cz(-1, 0);
+  // the engine's products, side by side in the parts of a team; with more CTAs
+  // than run at once the products in vain would cost more than the latency
+  // (160 of order 256: 82.8 ms one after another, 85.8 side by side)
+  const int gw = gridDim.x > kDecWaveCtas ? 1 : min(team_size(), 4);
+  int ib = 2, ib1 = 11, ic = 3, ic1 = 7;
+  auto run = [&](int first, int of) {
+    const int size = team_size() / of, rank = team_rank();
+    const DecProduct p = dec_product(w, first + rank / size, ib, ib1, ic, ic1, gw);
+    Epilogue e = epi_store(p.C, L, make_double2(p.alpha, 0.0), make_double2(0.0, 0.0));
+    if (p.flag) {
+      if (threadIdx.x == 0) *sm.maxv = 0.0;
+      __syncthreads();
+      e.maxabs = sm.maxv;
+      e.idle_max = p.flag == 2;
+    }
+    gemm_run_any(gemm_desc_publish(L, L, L, opN(p.A, L), opN(p.B, L), e, sm.main, rank % size, size), sm.main);
+  };
   for (it = 1; it <= max_iter; ++it) {
     if (zinv_refined(L, Ao, Go, w.inv(), w.slot(8), w.slot(9), sm)) st = ST_SINGULAR;
-    gemm(L, L, L, opN(Go, L), opN(Co, L), X, L, one, zero, sm);            // GoXCo
-    gemm(L, L, L, opN(Co, L), opN(X, L), C1, L, one, zero, sm, true);      // C1 = Co GoXCo
+    run(4, min(gw, 2));                           // X = Go Co (and Y = Go Bo)
+    run(0, gw);                                   // C1 = Co X (and Self = Bo X; B1 = Bo Y, D = -Co Y)
     const double mx = *sm.maxv;
     if (!(mx <= 1.7976931348623157e308)) break;   // Inf / NaN: will not converge (NOT_CONVERGED)
     if (mx <= tol) {
@@ -109,17 +125,14 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
     } else {
       ok = false;
     }
-    gemm(L, L, L, opN(Bo, L), opN(X, L), Sf, L, one, zero, sm);            // Self = Bo GoXCo
+    if (gw == 1) run(5, 1);
+    for (int q = gw; q < 4; q += gw) run(q, gw);
     for (int q = team_tid(); q < nn; q += team_threads()) {
       Aos[q] = csub(Aos[q], Sf[q]);
-      Ao[q] = csub(Ao[q], Sf[q]);
+      Ao[q] = cadd(D[q], csub(Ao[q], Sf[q]));
     }
     team_sync();
-    gemm(L, L, L, opN(Go, L), opN(Bo, L), Sf, L, one, zero, sm);            // GoXBo
-    gemm(L, L, L, opN(Bo, L), opN(Sf, L), X, L, one, zero, sm);             // B1 = Bo GoXBo
-    gemm(L, L, L, opN(Co, L), opN(Sf, L), Ao, L, mone, one, sm);            // Ao -= Co GoXBo
-    double2* t = Bo; Bo = X; X = t;                                         // Bo = B1
-    t = Co; Co = C1; C1 = t;                                                // Co = C1
+    { int t = ib; ib = ib1; ib1 = t; t = ic; ic = ic1; ic1 = t; }   // Bo = B1, Co = C1
   }
   ncyc = done ? it : max_iter + 1;
   if (!done && st == ST_OK) st = ST_NOT_CONVERGED;

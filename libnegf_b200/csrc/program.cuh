@@ -487,13 +487,26 @@ __device__ __forceinline__ double2 esh_al(const DevDesc* d, double2 a) {
 // Product q of a decimation iteration (Ao slot 0, Go 4, X 5, Y 12): 4 X = Go
 // Co, 5 Y = Go Bo; 0 C1 = Co X with max|C1|, 1 Self = Bo X (slot 6), 2 B1 = Bo
 // Y, 3 D = -Co Y (slot 13).
-__device__ __forceinline__ void dec_product(Op& o, const Prog& s, const Ws& w, int q) {
-  const bool left_c = q == 0 || q == 3, of_x = q < 2;
-  const double2* A = w.slot(q >= 4 ? 4 : (left_c ? s.ic : s.ib));
-  const double2* B = w.slot(q >= 4 ? (q == 4 ? s.ic : s.ib) : (of_x ? 5 : 12));
-  double2* C = w.slot(q >= 4 ? (q == 4 ? 5 : 12) : (of_x ? (q == 0 ? s.ic1 : 6) : (q == 2 ? s.ib1 : 13)));
-  set_gemm(o, s.L, s.L, s.L, A, s.L, OP_N, B, s.L, OP_N, C, s.L, make_double2(q == 3 ? -1.0 : 1.0, 0.0),
-           make_double2(0.0, 0.0), q == 0 ? 1 : (q < s.gw ? 2 : 0));
+struct DecProduct {
+  const double2 *A, *B;
+  double2* C;
+  double alpha;
+  int flag;   // of K_GEMM
+};
+__device__ __forceinline__ DecProduct dec_product(const Ws& w, int q, int ib, int ib1, int ic, int ic1, int gw) {
+  const bool go = q >= 4, left_c = q == 0 || q == 3, of_x = q < 2;
+  DecProduct p;
+  p.A = w.slot(go ? 4 : (left_c ? ic : ib));
+  p.B = w.slot(go ? (q == 4 ? ic : ib) : (of_x ? 5 : 12));
+  p.C = w.slot(go ? (q == 4 ? 5 : 12) : (of_x ? (q == 0 ? ic1 : 6) : (q == 2 ? ib1 : 13)));
+  p.alpha = q == 3 ? -1.0 : 1.0;
+  p.flag = q == 0 ? 1 : (q < gw ? 2 : 0);
+  return p;
+}
+__device__ __forceinline__ void dec_gemm(Op& o, const Prog& s, const Ws& w, int q) {
+  const DecProduct p = dec_product(w, q, s.ib, s.ib1, s.ic, s.ic1, s.gw);
+  set_gemm(o, s.L, s.L, s.L, p.A, s.L, OP_N, p.B, s.L, OP_N, p.C, s.L, make_double2(p.alpha, 0.0),
+           make_double2(0.0, 0.0), p.flag);
 }
 
 __device__ __forceinline__ void put_status(int& st, int s) { if (st == ST_OK) st = s; }
@@ -598,10 +611,10 @@ dispatch:
           PT_EMIT(s);
           if (sm.ires[0]) put_status(s.st, ST_SINGULAR);
           PT_REFINE(s, w.slot(0), w.slot(4), s.L);
-          dec_product(o, s, w, s.gw > 1 ? 4 + group_part(2) : 4);                       // X (and Y)
+          dec_gemm(o, s, w, s.gw > 1 ? 4 + group_part(2) : 4);                       // X (and Y)
           if (s.gw > 1) group_gemm(o, 2);
           PT_EMIT(s);
-          dec_product(o, s, w, group_part(s.gw));                                        // C1 (and Self; B1, D)
+          dec_gemm(o, s, w, group_part(s.gw));                                        // C1 (and Self; B1, D)
           if (s.gw > 1) group_gemm(o, s.gw);
           PT_EMIT(s);
           mx = *sm.maxv;
@@ -616,11 +629,11 @@ dispatch:
             s.ok = 0;
           }
           if (s.gw == 1) {
-            dec_product(o, s, w, 5);
+            dec_gemm(o, s, w, 5);
             PT_EMIT(s);
           }
           for (s.gq = s.gw; s.gq < 4; s.gq += s.gw) {                                    // what is left of Self, B1, D
-            dec_product(o, s, w, s.gq + group_part(s.gw));
+            dec_gemm(o, s, w, s.gq + group_part(s.gw));
             if (s.gw > 1) group_gemm(o, s.gw);
             PT_EMIT(s);
           }
