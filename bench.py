@@ -7,7 +7,7 @@ orbitals, complex128, 10 % random non-zeros, S = I + 0.05 R, 2048 energies in
 outputs T(E,k) and the diagonal spectral density of every orbital.  Seeded
 synthetic data (libNEGF ships no benchmark inputs).
 
-A step is one persistent launch over a batch of (E, k) points of this rank.
+A step is one solve call over a batch of (E, k) points of this rank.
   value  device-resident inputs and outputs (negf_b200_transmission_dos_dev),
          CUDA events on the launching stream, max over ranks.
   e2e    the same batches through the host-buffer C-ABI call
@@ -962,9 +962,9 @@ def main():
             "config": config_of(args, wl, P),
             "e2e": {"value": e2e, "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": gpu_launches,
-            "schedule": ("lock step: every point of a step through each batched block operation at once, one "
-                         "CTA of 4 warps per point and operation (n <= 32)") if gpu_launches > args.steps else
-                        "persistent engine: one launch per step, one CTA per point",
+            "schedule": ("small orders: one launch per step, a point's blocks in the shared memory of one CTA "
+                         "(n <= 32)") if wl["n"] <= 32 and not wl["dos"] and args.schedule != 1 else
+                        "persistent engine: a team of CTAs per point",
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
                          "traffic": dram_bytes_per_launch(wl, P),

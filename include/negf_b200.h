@@ -135,7 +135,9 @@ typedef struct negf_b200_options {
    * neither reads nor fills the SGF cache (a context that keeps one still
    * runs it). */
   int32_t precision;
-  /* Resident CTAs per SM for the persistent point engine (0 = auto). */
+  /* Resident CTAs per SM for the persistent point engine (0 = auto).  The
+   * engine groups them into teams of 1 to 16, one team per point; results do
+   * not depend on the grouping. */
   int32_t ctas_per_sm;
   /* Elastic SCBA mixing and stopping rule.  scba_mix = 1 (default) is the
    * reference: the dephasing self-energies are overwritten by D diag(G)
@@ -149,16 +151,16 @@ typedef struct negf_b200_options {
   int32_t scba_rule;
   /* How the points of a 2-contact transmission solve (negf_b200_transmission,
    * _dev; single pair, no SGF cache) are scheduled under precision = 0:
-   *   1 = the persistent engine: one CTA per point, its whole solve;
-   *   2 = lock step: every point of the call through the same block
-   *       operation at once, one CTA per point and operation (orders
+   *   1 = the persistent engine: a team of CTAs per point, its whole solve;
+   *   2 = the small-order form ("lock step"): one launch for the call, one
+   *       CTA per point, or two with a contact each while the points are
+   *       fewer than the SMs, the point's blocks in shared memory (orders
    *       n <= 32; the call needs the shape rules of the mixed form);
-   *   0 (default) = lock step when the call's points all fit it and n <= 32
-   *       (for _dev calls: every device the context holds) and the stream is
-   *       not capturing, else the engine.
-   * Lock step synchronises its stream a few times per call (the
-   * decimation's active count is read back), so a captured call takes the
-   * engine (schedule 2 under capture: NEGF_B200_ERR_BAD_ARG).
+   *   0 (default) = the small-order form when the call's points all fit it
+   *       and n <= 32 (for _dev calls: every device the context holds) and
+   *       the stream is not capturing, else the engine.
+   * A captured call takes the engine (schedule 2 under capture:
+   * NEGF_B200_ERR_BAD_ARG).
    * Both compute the reference's operation sequence in complex FP64; their
    * last bits differ (summation order).  Under precision != 0 the mixed
    * form runs in lock step whatever this says. */
@@ -181,8 +183,9 @@ int negf_b200_set_options(negf_b200_ctx* ctx, const negf_b200_options* opt);
 /* Last error message of this context (empty if none). */
 const char* negf_b200_last_error(const negf_b200_ctx* ctx);
 /* Kernels launched by this context's solve calls since it was created: one
- * per persistent-engine call, one per batched block operation of lock step
- * (three per product of the mixed form: two digit splits and the product). */
+ * per small-order call, one to four per persistent-engine call (the contacts
+ * and the sweeps, each with the rest above a full wave in a launch of its
+ * own), one per batched block operation of the mixed form. */
 int negf_b200_launch_count(negf_b200_ctx* ctx, uint64_t* count);
 
 /* Uploads a device description to HBM once (H/S blocks, contact blocks) and
@@ -216,7 +219,7 @@ int negf_b200_device_bytes(const negf_b200_ctx* ctx, int32_t device_id,
 
 /* ---- batched per-energy-point solves (host buffers) ----------------------
  * A point is (device_id[p], energy[p]).  All points of one call run in one
- * persistent launch.  `status` (npts) receives a per-point NEGF_B200_* code;
+ * to four persistent launches.  `status` (npts) receives a per-point NEGF_B200_* code;
  * the return value is the first non-OK point status (or a call error).
  * `ncyc` (npts, optional) receives the total decimation iteration count over
  * all contacts at that point (src/integrations.F90:1751 prints the average
@@ -347,8 +350,8 @@ int negf_b200_transmissions(negf_b200_ctx* ctx, int32_t npts,
                             double* ledos, int32_t* ncyc, int32_t* status);
 
 /* Caps the engine workspace of this context at `bytes` (0 = no cap): a launch
- * whose resident CTAs would need more runs with fewer CTAs, and one whose
- * single CTA does not fit returns NEGF_B200_ERR_ADMISSION.  A serving loop
+ * whose resident teams would need more runs with fewer of them, and one whose
+ * single team does not fit returns NEGF_B200_ERR_ADMISSION.  A serving loop
  * admits requests against this budget. */
 int negf_b200_set_workspace_limit(negf_b200_ctx* ctx, size_t bytes);
 
@@ -387,7 +390,7 @@ int negf_b200_sgf_cache_stats(const negf_b200_ctx* ctx, int64_t* hits,
 /* ---- batched solves on device buffers ------------------------------------
  * Same as negf_b200_transmission / _transmission_dos with every per-point
  * array already resident in HBM (device pointers) and no host
- * synchronisation: the launch is enqueued on `stream` (NULL = the context's
+ * synchronisation: the launches are enqueued on `stream` (NULL = the context's
  * stream) and the call returns.  Workspace sizing covers every uploaded
  * device.  `dos_stride` is the row stride of d_dos in doubles. */
 int negf_b200_transmission_dev(negf_b200_ctx* ctx, int32_t npts,

@@ -1,14 +1,14 @@
 """Schedule autotuner for transmission and DOS solves.
 
-The engine's tile shapes are fixed by its register and shared-memory budget
-(64 x 64 product tiles, 16-column inversion leaves); what changes the speed
-for a given device shape is the schedule:
+The engine chooses its product tiles (64 x 64 or 32 x 32) and its teams of
+CTAs by the sizes of a call; what a caller can change is the schedule:
 
 - the persistent engine (options.schedule = 1) with 2 resident CTAs per SM
   (one CTA's latency-bound inversion steps overlap the other's products) or
   1 (a CTA gets the whole L2 share and tensor pipe of an SM);
-- lock step (options.schedule = 2; 2-contact transmission, n <= 32): every
-  point through each batched block operation at once, one CTA per point.
+- the small-order form, "lock step" (options.schedule = 2; 2-contact
+  transmission, n <= 32): one launch, a point's blocks in the shared memory
+  of one CTA, or of two with a contact each.
 
 `tune` times each candidate that the device shape admits on a sample of the
 caller's own points, applies the fastest on top of the caller's other

@@ -1141,8 +1141,8 @@ static bool lockstep_choice(negf_b200_ctx* ctx, int32_t npts, const int32_t* h_i
   if (!mixed && ctx->opt.schedule == 1) return false;
   const bool forced = mixed || ctx->opt.schedule == 2;
   const char* form = mixed ? "the mixed form (precision != 0)" : "lock step (schedule 2)";
-  // lock step reads the decimation's active count back to the host, which a
-  // stream capture cannot hold: the engine takes captured calls
+  // the mixed form reads the decimation's active count back to the host, which a
+  // stream capture cannot hold; the engine takes captured calls at small orders too
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
     cudaGetLastError();

@@ -491,7 +491,7 @@ __device__ __forceinline__ void gemm_run_any(const GemmDesc* d, double2* smem) {
 // of its time goes to its operands); a large tile past the edge of C costs
 // half when C has at most 32 rows or columns (half of the warps have work).
 // One product over many CTAs, n = 64: 20 -> 13 us, n = 128: 33 -> 19, n = 256:
-// 57 -> 29; 6 products of order 300: 110 -> 95.
+// 57 -> 29; 6 products of order 300: 110 -> 95 (82 with the loop's operand issue).
 __host__ __device__ inline int gemm_tile(int M, int N, int size) {
   const int m = (M + kTile - 1) / kTile, n = (N + kTile - 1) / kTile;
   const int sm = (M + kSmallTile - 1) / kSmallTile, sn = (N + kSmallTile - 1) / kSmallTile;
@@ -1013,8 +1013,8 @@ __device__ __forceinline__ void gj_reg_steps(double2 (&x)[R][W], int n, int c0, 
 // n = 64, 128 and 256.  One inverse on an otherwise idle GPU took 295, 671
 // and 2170 us before the panels and the teams (rows per thread, every warp's
 // candidates and rows exchanged through memory, two serial divisions per
-// pivot; a panel of n <= 64 kept in shared memory), 70, 258 and 767 us now;
-// 296 of them at n = 256 3.72 -> 3.34 ms.
+// pivot; a panel of n <= 64 kept in shared memory), 76, 209 and 675 us now;
+// 296 of them at n = 256 3.72 -> 3.01 ms.
 // The columns of a warp are unrolled, so a step's code is reused by the 8
 // steps of one slot; with every step unrolled the loop ran out of the
 // instruction cache for a third of the time.

@@ -172,7 +172,7 @@ __device__ __forceinline__ void set_gemm(Op& o, int M, int N, int K, const doubl
 // tiles rarely divide by the team; side by side these are paid once.  A
 // decimation iteration takes two such steps for six, the forward retarded
 // sweep three for five, a layer of the lesser sweep five for six: SCBA of 32
-// points of order 64 34.8 -> 32.5 ms, 6 points of order 768 131.2 -> 128.
+// points of order 64 34.8 -> 32.5 ms, 12 points of order 384 131.2 -> 127.
 // The last iteration computes Self, B1 and D in vain; one CTA alone, which
 // would pay for them, does not.
 __device__ __forceinline__ int group_part(int of) { return team_rank() / (team_size() / of); }

@@ -8,7 +8,7 @@ solved points in each lane's device cache (the ln_cache counterpart), and
 feeds the GPU from a pool of pending energy points:
 
 - lanes: independent engine contexts on the same GPU, each with its own
-  stream and workspace; a lane runs one persistent launch at a time, and
+  stream and workspace; a lane runs one call's persistent launches at a time, and
   the launches of different lanes run concurrently on the SMs;
 - batching: whenever a lane is free it takes pending points of one solve
   kind (T or T+LDOS, same eta, dos_delta, pairs and precision; for the mixed
