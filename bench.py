@@ -108,14 +108,14 @@ def point_list(wl, seed=11):
     return ids[perm], en[perm]
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the k_engine
-# launch per point, modelled as a + b N for a device of N layers of n = 256
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of a call's
+# k_engine launches per point, modelled as a + b N for a device of N layers of n = 256
 # (T + DOS), from one-pass ncu captures of two small cases of the same kernel
 # ("prof4": N = 4 and "prof": N = 8, 296 points each, a few GB on the device);
-# scaled to a launch by its points.  Measured on B200: prof4 1.2345e12 B,
-# prof 1.3457e12 B per launch -> a = 3.795e9 B (contacts: decimation and
-# self-energies), b = 9.40e7 B per layer.
-DRAM_PER_POINT_MODEL = {256: (3.795e9, 9.40e7)}
+# scaled to a call by its points.  Measured on B200: prof4 1.2781e12 B,
+# prof 1.3840e12 B per call -> a = 3.961e9 B (contacts: decimation and
+# self-energies), b = 8.94e7 B per layer.
+DRAM_PER_POINT_MODEL = {256: (3.961e9, 8.94e7)}
 
 
 def dram_bytes_per_launch(wl, points):
