@@ -210,7 +210,7 @@ struct Epilogue {
   const int* perm;      // smem, full-length row permutation of the applied block
   const double2* W;     // unused
   int k0, jb;           // pivot rows [k0, k0+jb) of the applied block (masked)
-  // optional reduction of max |C| over stored elements
+  // optional reduction of max |C| over stored elements (+Inf when one is NaN)
   double* maxabs;       // smem accumulator (nullptr = off)
   bool idle_max = false;   // take part in the team's reduction with 0 (another CTA's product has the maximum)
 };
@@ -452,7 +452,10 @@ __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) 
             const int r = r0 + i * 16 + 8 * (q >> 1), c = c0 + j * 8 + (q & 1);
             if (r >= M || c >= N) continue;
             C[(size_t)r + (size_t)c * ldc] = old[q];
-            if (want_max) lmax = fmax(lmax, cabs(old[q]));
+            if (want_max) {   // NaN counts as Inf: fmax alone would drop it
+              const double h = cabs(old[q]);
+              if (!(h <= lmax)) lmax = h > lmax ? h : __longlong_as_double(0x7ff0000000000000LL);
+            }
           }
         }
     }

@@ -278,3 +278,30 @@ def test_products_side_by_side(gpu_ctx, dev):
     finally:
         gpu_ctx.set_options()
         gpu_ctx.release(h)
+
+
+@pytest.mark.parametrize("n", [20, 48, 100])
+def test_decimation_that_is_not_finite_counts_as_not_converged(n):
+    """NaN or Inf in a coupling block: max|C1| is not finite, and the count is
+    the cap plus one, with a CTA or with a team per problem; the problems
+    beside it are not touched."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    dev = G.transport_c0(nbl=3, n=n, seed=5)
+    z = (0.3 + 1e-3j) * np.eye(n)
+    blocks = (z - dev.lead_h00[0], -dev.lead_h01[0], -dev.lead_h01[0].conj().T)
+    for batch in (3, 296):
+        A, B, C = (torch.from_numpy(np.ascontiguousarray(x.T)).cuda().expand(batch, n, n).contiguous()
+                   for x in blocks)
+        C[1, n // 2, n // 3] = float("nan")
+        B[2, 0, n - 1] = float("inf")
+        Go = torch.zeros_like(A)
+        nc = torch.zeros(batch, dtype=torch.int32, device="cuda")
+        work = torch.empty(L.negf_b200_decimation_work_bytes(batch, n), dtype=torch.uint8, device="cuda")
+        assert L.negf_b200_decimation_batched(batch, n, _dp(A), _dp(B), _dp(C), _dp(Go), _ip(nc), 1e-9, 50,
+                                              ctypes.c_void_p(work.data_ptr()),
+                                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        k = nc.cpu().numpy()
+        assert k[1] == 51 and k[2] == 51
+        assert 0 < k[0] < 50 and np.all(np.delete(k, [1, 2]) == k[0])
+        assert bool(torch.isfinite(torch.view_as_real(Go[0])).all())
