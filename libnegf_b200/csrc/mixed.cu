@@ -337,7 +337,7 @@ __global__ void k_agree(int64_t nn, const int* map, const double2* gs, const dou
   }
 }
 
-// Points still flagged after the last retry: NOT_CONVERGED, ncyc = cap + 1.
+// Problems still flagged after the last attempt: NOT_CONVERGED, ncyc = cap + 1.
 __global__ void k_flag_unresolved(int P, const int* redo, int* ncyc_c, int* status, int max_iter) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
     if (redo[p]) {
@@ -616,6 +616,9 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
         cur_sub = again;
         MCK(cudaStreamSynchronize(s), "sync");   // the host vectors above are reused next round
       }
+    } else {   // no other branch to try; gs of an iteration broken off (Inf / NaN) means nothing
+      k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, w.nc, w.pst2, a.sgf_max_iter);
+      ++nl;
     }
     // ---- self-energies Sigma_c = Tlc gs Tcl of both contacts
     k_tlc<<<dim3(gx, N), eb, 0, s>>>(n, P, a.left, a.right, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;

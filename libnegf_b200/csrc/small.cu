@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
             bad |= !(h <= 1.7976931348623157e308);
           }
         mx = cta_max_nan(bad ? __longlong_as_double(0x7ff8000000000000LL) : mx, sh.red[2]);
-        if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge; run it again
+        if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge
           redo = done = true;
         } else if (mx <= a.sgf_tol) {
           done = ok;
@@ -339,7 +339,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       if (bad_gs & 1) put_st(NEGF_B200_ERR_SINGULAR);
       sens |= (bad_gs & 2) != 0;
       __syncthreads();
-      if (!(a.eta > 0.0)) break;
+      if (!(a.eta > 0.0)) {   // no other branch to try; gs of an iteration broken off means nothing
+        if (redo) {
+          cyc = a.sgf_max_iter + 1;
+          put_st(NEGF_B200_ERR_NOT_CONVERGED);
+        }
+        break;
+      }
       // the retarded branch has -Im gs_ii >= 0 up to 1e-6 of the largest |gs_ii|
       double lo = 1.7976931348623157e308, hi = 0.0;
       for (int i = 0; i < n; ++i) {

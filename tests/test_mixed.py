@@ -118,3 +118,26 @@ def test_mixed_rejects_what_it_does_not_cover(gpu_ctx):
         gpu_ctx.set_options()
         for h in (d1, d2, ok):
             gpu_ctx.release(h)
+
+
+@pytest.mark.parametrize("eta", [0.0, 1e-3, -1e-3])
+def test_mixed_reports_a_decimation_that_runs_off_at_any_broadening(gpu_ctx, eta):
+    """Products that overflow end the decimation early with finite blocks left:
+    only the status says so, as in the engine."""
+    E = np.linspace(-1.0, 1.0, 6)
+    for side in (0, 1):
+        dev = G.transport_c0(nbl=3, n=16, seed=12)
+        dev.lead_h01[side][0, 0] = 1e200
+        did = gpu_ctx.upload(dev)
+        try:
+            gpu_ctx.set_options(schedule=1)
+            Te, ne, se = gpu_ctx.transmission(did, E, eta=eta, check=False)
+            Tm, nm, sm = _mixed_T(gpu_ctx, did, E, eta)
+            assert np.all(se == native.NOT_CONVERGED) and np.array_equal(sm, se)
+            if eta == 0.0:                                         # in a band at eta = 0 the other contact's count is chaotic
+                assert np.all(nm > 301) and np.all(ne > 301)
+            else:
+                assert np.array_equal(nm, ne)
+        finally:
+            gpu_ctx.set_options()
+            gpu_ctx.release(did)

@@ -197,3 +197,27 @@ def test_lockstep_statuses_match_the_engine(gpu_ctx):
     finally:
         gpu_ctx.release(did)
         gpu_ctx.release(bid)
+
+
+@pytest.mark.parametrize("eta", [0.0, 1e-3, -1e-3])
+def test_a_decimation_that_runs_off_is_reported_at_any_broadening(gpu_ctx, eta):
+    """A coupling block that is not finite, or whose products overflow, ends
+    the decimation early with a finite Ao_s: gs, Sigma and T come out finite,
+    and only the status says that they mean nothing.  The engine's statuses
+    and cycle counts, one CTA per point and two."""
+    E = np.linspace(-1.0, 1.0, 150)
+    for side, val in ((0, np.nan), (1, np.nan), (0, 1e200), (1, 1e200)):
+        dev = G.transport_c0(nbl=3, n=8, seed=12)
+        dev.lead_h01[side][0, 0] = val
+        did = gpu_ctx.upload(dev)
+        try:
+            Te, ne, se = _T(gpu_ctx, did, E, eta, 1)
+            for m in (150, 20):
+                Tl, nl, sl = _T(gpu_ctx, did, E[:m], eta, 2)
+                assert np.all(sl == native.NOT_CONVERGED) and np.array_equal(sl, se[:m])
+                if eta == 0.0:                                     # in a band at eta = 0 the other contact's count is chaotic
+                    assert np.all(nl > 301) and np.all(ne > 301)
+                else:
+                    assert np.array_equal(nl, ne[:m])
+        finally:
+            gpu_ctx.release(did)
