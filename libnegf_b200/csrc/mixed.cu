@@ -257,17 +257,18 @@ __global__ void k_trace(int n, const double2* Gam, const double2* G, const doubl
   }
 }
 
-// Points whose surface Green's function left the retarded solution: the
-// diagonal of -Im gs must be >= 0 (up to 1e-6 of the largest |gs_ii|); a
+// Points whose surface Green's function left the retarded solution (eta > 0,
+// sgn = -1; the advanced one for eta < 0, sgn = 1): the diagonal of sgn Im gs
+// must be >= 0 (up to 1e-6 of the largest |gs_ii|); a
 // converged fixed point of the wrong kind, or one that is not finite, marks
 // the point for the engine (redo[p] = 1).  One CTA per point.
-__global__ void k_retarded_check(int n, const double2* gs, int64_t Q, const int* map, int* redo) {
+__global__ void k_retarded_check(int n, const double2* gs, int64_t Q, double sgn, const int* map, int* redo) {
   const int p = map ? map[blockIdx.x] : blockIdx.x;
   double lo = 1.7976931348623157e308, hi = 0.0;
   int bad = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double2 g = gs[p * Q + (int64_t)i * (n + 1)];
-    const double v = -g.y, h = sqrt(g.x * g.x + g.y * g.y);
+    const double v = sgn * g.y, h = sqrt(g.x * g.x + g.y * g.y);
     if (!(h <= 1.7976931348623157e308)) bad = 1;
     else {
       lo = fmin(lo, v);
@@ -558,15 +559,15 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
       MCK(inv(nsub, sub, Aos, gs), "gs");
       k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, w.pst2, NEGF_B200_ERR_SINGULAR);
       ++nl;
-      if (a.eta > 0.0) {
-        k_retarded_check<<<nsub, 128, 0, s>>>(n, gs, Q, sub, w.redo);
+      if (a.eta != 0.0) {
+        k_retarded_check<<<nsub, 128, 0, s>>>(n, gs, Q, a.eta > 0.0 ? -1.0 : 1.0, sub, w.redo);
         ++nl;
       }
       return 0;
     };
     MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
     if (int r = decimate(nullptr, N, 1.0)) return r;
-    if (a.eta > 0.0) {
+    if (a.eta != 0.0) {
       // Decimations that reached another fixed point (or ran off to Inf / NaN) run
       // again, in lock step over just those problems, from the contact energy times
       // 1 + k 2^-50.  A sensitive decimation (one of its inverses needed a Newton

@@ -339,21 +339,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       if (bad_gs & 1) put_st(NEGF_B200_ERR_SINGULAR);
       sens |= (bad_gs & 2) != 0;
       __syncthreads();
-      if (!(a.eta > 0.0)) {   // no other branch to try; gs of an iteration broken off means nothing
+      if (a.eta == 0.0) {   // no other branch to try; gs of an iteration broken off means nothing
         if (redo) {
           cyc = a.sgf_max_iter + 1;
           put_st(NEGF_B200_ERR_NOT_CONVERGED);
         }
         break;
       }
-      // the retarded branch has -Im gs_ii >= 0 up to 1e-6 of the largest |gs_ii|
+      // the retarded branch (eta > 0) has -Im gs_ii >= 0 up to 1e-6 of the
+      // largest |gs_ii|, the advanced one (eta < 0) Im gs_ii >= 0
+      const double sgn = a.eta > 0.0 ? -1.0 : 1.0;
       double lo = 1.7976931348623157e308, hi = 0.0;
       for (int i = 0; i < n; ++i) {
         const double2 g = Go[i * (kLd + 1)];
         const double h = cabs(g);
         if (!(h <= 1.7976931348623157e308)) redo = true;
         else {
-          lo = fmin(lo, -g.y);
+          lo = fmin(lo, sgn * g.y);
           hi = fmax(hi, h);
         }
       }

@@ -141,3 +141,23 @@ def test_mixed_reports_a_decimation_that_runs_off_at_any_broadening(gpu_ctx, eta
         finally:
             gpu_ctx.set_options()
             gpu_ctx.release(did)
+
+
+@pytest.mark.parametrize("eta", [1e-3, -1e-3])
+def test_mixed_branch_check_follows_the_sign_of_the_broadening(gpu_ctx, eta):
+    """A lead orbital of its own with gain against the broadening's sign is on
+    the wrong branch in every attempt; with loss it is fine."""
+    E = np.linspace(-1.0, 1.0, 6)
+    for sign, bad in ((1.0, True), (-1.0, False)):
+        dev = G.transport_c0(nbl=3, n=16, seed=12)
+        dev.lead_h01[0][0, :] = 0.0
+        dev.lead_h01[0][:, 0] = 0.0
+        dev.lead_h00[0][0, :] = 0.0
+        dev.lead_h00[0][:, 0] = 0.0
+        dev.lead_h00[0][0, 0] = 0.3 + 0.1j * sign * np.sign(eta)
+        did = gpu_ctx.upload(dev)
+        try:
+            Tm, nm, sm = _mixed_T(gpu_ctx, did, E, eta)
+            assert np.all(sm == (native.NOT_CONVERGED if bad else 0))
+        finally:
+            gpu_ctx.release(did)

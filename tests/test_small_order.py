@@ -221,3 +221,26 @@ def test_a_decimation_that_runs_off_is_reported_at_any_broadening(gpu_ctx, eta):
                     assert np.array_equal(nl, ne[:m])
         finally:
             gpu_ctx.release(did)
+
+
+@pytest.mark.parametrize("eta", [1e-3, -1e-3])
+def test_branch_check_follows_the_sign_of_the_broadening(gpu_ctx, eta):
+    """A lead orbital of its own with gain against the broadening's sign: the
+    fixed point lies on the wrong branch for every attempt, NOT_CONVERGED as
+    in the engine; the same orbital with loss is fine."""
+    E = np.linspace(-1.0, 1.0, 20)
+    for sign, bad in ((1.0, True), (-1.0, False)):
+        dev = G.transport_c0(nbl=3, n=8, seed=12)
+        dev.lead_h01[0][0, :] = 0.0
+        dev.lead_h01[0][:, 0] = 0.0
+        dev.lead_h00[0][0, :] = 0.0
+        dev.lead_h00[0][:, 0] = 0.0
+        dev.lead_h00[0][0, 0] = 0.3 + 0.1j * sign * np.sign(eta)
+        did = gpu_ctx.upload(dev)
+        try:
+            Te, ne, se = _T(gpu_ctx, did, E, eta, 1)
+            Tl, nl, sl = _T(gpu_ctx, did, E, eta, 2)
+            assert np.all(se == (native.NOT_CONVERGED if bad else 0))
+            assert np.array_equal(sl, se) and np.array_equal(nl, ne)
+        finally:
+            gpu_ctx.release(did)
