@@ -447,7 +447,9 @@ int negf_b200_get_trace(negf_b200_ctx* ctx, uint64_t* cycles);
 
 /* C = alpha*op(A)*op(B) + beta*C, complex128.  dagger: 0 = (N,N),
  * 1 = (C,N), 2 = (N,C) -- the `dagger` argument of cu_ZmultMat
- * (src/gpuroutines.cu:395-446).  alpha/beta are {re, im}. */
+ * (src/gpuroutines.cu:395-446).  alpha/beta are {re, im}.  C may take the
+ * place of its own problem's A or B for m, n <= 64; above that it must overlap
+ * neither (a product's output tiles are written while others still read). */
 int negf_b200_zgemm_batched(int32_t batch, int32_t m, int32_t n, int32_t k,
                             const double* alpha, const double* A,
                             int64_t strideA, const double* B, int64_t strideB,

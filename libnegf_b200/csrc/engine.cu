@@ -391,6 +391,14 @@ int device_sms() {
   return known[dev] > 0 ? known[dev] : 148;
 }
 
+// Whether some problem's C (nc elements) shares memory with its own operand A (na elements).
+static bool in_place(const double2* A, int64_t sA, int64_t na, const double2* C, int64_t sC, int64_t nc, int batch) {
+  constexpr int64_t kElem = sizeof(double2);
+  const int64_t first = reinterpret_cast<intptr_t>(C) - reinterpret_cast<intptr_t>(A);
+  const int64_t last = first + (int64_t)(batch - 1) * (sC - sA) * kElem;   // of the last problem; linear between
+  return std::min(first, last) < na * kElem && std::max(first, last) > -nc * kElem;
+}
+
 cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                  const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC,
                                  int dagger, cudaStream_t s) {
@@ -402,7 +410,14 @@ cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, 
   // 1604 -> 82 us); with 1184 products and more one CTA runs through all
   // tiles of a product, loading the next tile's operands behind this one's
   // epilogue.
-  const int64_t want = (8LL * device_sms() + batch - 1) / batch;
+  int64_t want = (8LL * device_sms() + batch - 1) / batch;
+  // C in the place of A or B: up to order 64 one CTA holds the whole product in
+  // one tile and has read all operands when it stores (gemm_tile() for one CTA
+  // keeps 64 x 64 in one), so such calls stay with it.
+  if (m <= kTile && n <= kTile &&
+      (in_place(A, sA, (int64_t)m * k, C, sC, (int64_t)m * n, batch) ||
+       in_place(B, sB, (int64_t)k * n, C, sC, (int64_t)m * n, batch)))
+    want = 1;
   const int T = gemm_tile(m, n, (int)std::min<int64_t>(want, 1 << 20));
   const int64_t tiles = (int64_t)((m + T - 1) / T) * ((n + T - 1) / T);
   const int split = (int)std::max<int64_t>(1, std::min(tiles, want));

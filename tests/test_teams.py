@@ -305,3 +305,25 @@ def test_decimation_that_is_not_finite_counts_as_not_converged(n):
         assert k[1] == 51 and k[2] == 51
         assert 0 < k[0] < 50 and np.all(np.delete(k, [1, 2]) == k[0])
         assert bool(torch.isfinite(torch.view_as_real(Go[0])).all())
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64])
+@pytest.mark.parametrize("dagger", [0, 1, 2])
+@pytest.mark.parametrize("place", ["A", "B"])
+def test_product_in_the_place_of_an_operand(n, dagger, place):
+    """Up to order 64 a product may be written over one of its operands: the
+    bits of the product written elsewhere."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    g = torch.Generator(device="cuda").manual_seed(n + dagger)
+    al, be = (ctypes.c_double * 2)(0.5, -1.0), (ctypes.c_double * 2)(0.25, 0.5)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for batch in (1, 7, 300):
+        A, B = (torch.randn((batch, n, n), dtype=torch.complex128, device="cuda", generator=g) for _ in range(2))
+        ref = (A if place == "A" else B).clone()
+        out = A if place == "A" else B
+        for C in (ref, out):
+            assert L.negf_b200_zgemm_batched(batch, n, n, n, al, _dp(A), 2 * n * n, _dp(B), 2 * n * n, be, _dp(C),
+                                             2 * n * n, dagger, s) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
