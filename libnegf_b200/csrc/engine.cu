@@ -203,19 +203,29 @@ int64_t engine_ws_elems(int mode, int nbl_max, int ncont_max, int nmax) {
   return e;
 }
 
+// Kernels whose limits have been raised, by device.
+static std::mutex g_opt_mu;
+static std::set<std::pair<const void*, int>> g_opted;
+
 cudaError_t team_opt_in(const void* kernel, size_t smem) {
-  static std::mutex mu;
-  static std::set<std::pair<const void*, int>> done;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count({kernel, dev})) return cudaSuccess;
+  std::lock_guard<std::mutex> lk(g_opt_mu);
+  if (g_opted.count({kernel, dev})) return cudaSuccess;
   if (smem == 0) smem = engine_smem_bytes(kMaxOrder);
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) done.insert({kernel, dev});
+  if (e == cudaSuccess) g_opted.insert({kernel, dev});
   return e;
+}
+
+void team_opt_out(const void* kernel) {
+  int dev = 0;
+  cudaGetLastError();
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lk(g_opt_mu);
+  g_opted.erase({kernel, dev});
 }
 
 cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
@@ -235,11 +245,8 @@ cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s,
 }
 
 cudaError_t launch_engine(const EngineArgs& a, int teams, int team, cudaStream_t s) {
-  cudaError_t e = team_opt_in((const void*)k_engine);
-  if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = team_config(teams, team, engine_smem_bytes(a.nmax), s, &attr);
-  return cudaLaunchKernelEx(&cfg, k_engine, a);
+  return team_launch(team_config(teams, team, engine_smem_bytes(a.nmax), s, &attr), k_engine, 0, a);
 }
 
 // Clusters of `team` CTAs of the engine that run at once on the current
@@ -402,9 +409,6 @@ static bool in_place(const double2* A, int64_t sA, int64_t na, const double2* C,
 cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                  const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC,
                                  int dagger, cudaStream_t s) {
-  const size_t smem = engine_smem_bytes(1);
-  cudaError_t e = team_opt_in((const void*)k_zgemm_batched);
-  if (e != cudaSuccess) return e;
   // A product's tiles over enough CTAs for four waves of the whole batch: one
   // CTA per product left all but `batch` SMs idle (6 products of order 300:
   // 1604 -> 82 us); with 1184 products and more one CTA runs through all
@@ -423,9 +427,10 @@ cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, 
   const int split = (int)std::max<int64_t>(1, std::min(tiles, want));
   for (int b0 = 0; b0 < batch; b0 += 65535) {   // gridDim.y limit
     const int nb = std::min(65535, batch - b0);
-    k_zgemm_batched<<<dim3(split, nb), kThreads, smem, s>>>(m, n, k, alpha, A + b0 * sA, sA, B + b0 * sB, sB, beta,
-                                                            C + b0 * sC, sC, dagger);
-    e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = team_config(1, 1, engine_smem_bytes(1), s, nullptr);
+    cfg.gridDim = dim3(split, nb);
+    const cudaError_t e = team_launch(cfg, k_zgemm_batched, 0, m, n, k, alpha, A + b0 * sA, sA, B + b0 * sB, sB, beta,
+                                      C + b0 * sC, sC, dagger);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -458,13 +463,11 @@ __global__ void __launch_bounds__(kThreads, 2)
 cudaError_t launch_zinv_mapped(int batch, int n, const double2* A, int64_t sA, double2* X, int64_t sX,
                                const int* map, int* info, double2* work, cudaStream_t s, int* sens) {
   if (batch <= 0) return cudaSuccess;
-  cudaError_t e = team_opt_in((const void*)k_zinv_mapped);
-  if (e != cudaSuccess) return e;
   const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
-  return cudaLaunchKernelEx(&cfg, k_zinv_mapped, n, A, sA, X, sX, map, info, work,
-                            (int64_t)zinv_batched_work_elems(n), sens);
+  return team_launch(cfg, k_zinv_mapped, 0, n, A, sA, X, sX, map, info, work,
+                     (int64_t)zinv_batched_work_elems(n), sens);
 }
 
 cudaError_t launch_zinv_batched(int batch, int n, const double2* A, double2* Ainv, int* info, double2* work,
@@ -504,12 +507,10 @@ __global__ void __launch_bounds__(kThreads, 2)
 cudaError_t launch_decimation_batched(int batch, int n, const double2* Ao, const double2* Bo, const double2* Co,
                                       double2* Go, int* ncyc, double tol, int max_iter, double2* work,
                                       cudaStream_t s) {
-  cudaError_t e = team_opt_in((const void*)k_decimation_batched);
-  if (e != cudaSuccess) return e;
   const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
-  return cudaLaunchKernelEx(&cfg, k_decimation_batched, n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work);
+  return team_launch(cfg, k_decimation_batched, 0, n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work);
 }
 
 }  // namespace negf

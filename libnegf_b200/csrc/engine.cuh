@@ -126,9 +126,25 @@ size_t engine_smem_bytes(int nmax);
 // kernel and device (not per launch), so that a launch is a stream operation
 // only and can be captured into a CUDA graph.
 cudaError_t team_opt_in(const void* kernel, size_t smem = 0);
+void team_opt_out(const void* kernel);   // forgets that, on the current device
 int device_sms();   // of the current device
 // The launch of `teams` clusters of `team` CTAs; attr must live until the launch.
 cudaLaunchConfig_t team_config(int teams, int team, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr);
+// Launches a kernel with its limits raised.  They are attributes of the CUDA
+// context: after a device reset (or a primary context made again) they are
+// back at their defaults and the launch is refused, so a refused launch raises
+// them afresh and tries once more.
+template <typename... P, typename... A>
+cudaError_t team_launch(const cudaLaunchConfig_t& cfg, void (*kernel)(P...), size_t smem_limit, A... args) {
+  cudaError_t e = cudaSuccess;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    e = team_opt_in((const void*)kernel, smem_limit);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e == cudaSuccess) break;
+    team_opt_out((const void*)kernel);
+  }
+  return e;
+}
 
 // `teams` teams of `team` CTAs (a thread-block cluster; 1, 2, 4, 8 or 16), one
 // point at a time each

@@ -35,6 +35,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "engine.cuh"
 #include "ozaki.cuh"
 
 namespace negf {
@@ -638,22 +639,11 @@ cudaError_t product(int batch, int m, int n, int k, double2 alpha, const OzakiSe
   a.t0 = t0;
   a.maxabs = maxabs; a.status = status;
   const size_t smem = (size_t)kOzStages * 2 * S * kPlaneBytes + 1024;
-  static std::mutex mu;
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(k_ozaki<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      if (dev >= 0 && dev < 64) attr_set[dev] = true;
-    }
-  }
   const long long tiles = (long long)((m + kOzTileM - 1) / kOzTileM) * ((n + kOzTileN - 1) / kOzTileN) * batch;
   const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
-  k_ozaki<S><<<grid, kOzWarps * 32, smem, s>>>(ta, tb, a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = team_config(grid, 1, smem, s, nullptr);
+  cfg.blockDim = dim3(kOzWarps * 32);
+  return team_launch(cfg, k_ozaki<S>, smem, ta, tb, a);
 }
 
 OzakiSet carve_set(uint8_t*& p, int problems, size_t rows, int kp, int arrays, int slices) {

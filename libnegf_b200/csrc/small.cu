@@ -489,14 +489,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
 cudaError_t launch_small_points(const MixedArgs& a, cudaStream_t s) {
   if (a.npts <= 0) return cudaSuccess;
   if (a.n < 1 || a.n > kSmallMax) return cudaErrorInvalidValue;
-  cudaError_t e = team_opt_in((const void*)k_small_point, kSmallSmem);
-  if (e != cudaSuccess) return e;
   // Two CTAs per point, a contact each, while they find room at once: order
   // 32, 74 points: 1.34 ms by one CTA, 0.96 by two; 148 points (two CTAs per
   // SM): 1.35 and 1.22; 149: 1.71 and 2.00.
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = team_config(a.npts, a.npts <= device_sms() ? 2 : 1, kSmallSmem, s, &attr);
-  e = cudaLaunchKernelEx(&cfg, k_small_point, a);
+  const cudaError_t e = team_launch(cfg, k_small_point, kSmallSmem, a);
   if (e == cudaSuccess && a.launches) ++*a.launches;
   return e;
 }
