@@ -1221,15 +1221,22 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
   // the contacts of a batch fill two waves of the inversion (two CTAs per SM: 296 points on a B200)
   int batch = std::min<int>(npts, 2 * std::max(ctx->sms, 1));
   if (ctx->ws_limit) batch = std::min(batch, negf::mixed_batch_for(ctx->ws_limit, n, slices));
-  if (batch < 1) return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
+  bool one_contact = false;   // not even one point fits: its contacts one after the other, in half the room
+  if (batch < 1) {
+    if (negf::mixed_ws_bytes(1, n, slices, true) > ctx->ws_limit)
+      return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
+    one_contact = true;
+    batch = 1;
+  }
   for (;;) {
-    st = grow(ctx, &ctx->ws, &ctx->ws_bytes, negf::mixed_ws_bytes(batch, n, slices));
+    st = grow(ctx, &ctx->ws, &ctx->ws_bytes, negf::mixed_ws_bytes(batch, n, slices, one_contact));
     if (st == NEGF_B200_OK) break;
-    if (batch == 1) return st;
-    batch = (batch + 1) / 2;
+    if (batch > 1) batch = (batch + 1) / 2;
+    else if (!one_contact) one_contact = true;
+    else return st;
   }
   std::string msg;
-  st = negf::mixed_run(a, ctx->ws, batch, s, &msg);
+  st = negf::mixed_run(a, ctx->ws, batch, one_contact, s, &msg);
   if (st) return fail(ctx, st, "mixed form: " + msg);
   return NEGF_B200_OK;
 }

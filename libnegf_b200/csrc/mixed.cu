@@ -28,7 +28,9 @@
 namespace negf {
 namespace {
 
-constexpr int kBlocks = 11;   // n x n complex work blocks per problem (contact of a point)
+// n x n complex work blocks per problem (contact of a point); where a point's
+// contacts run one after the other the 12th keeps the left self-energy
+constexpr int kBlocks = 11, kBlocksMax = 12;
 
 __device__ __forceinline__ double2 cmulm(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -362,40 +364,43 @@ struct Carver {
 };
 
 struct Ws {
-  double2* blk[kBlocks];
+  double2* blk[kBlocksMax];
   double* mx;
   int *ok, *nc, *list0, *list1, *count, *info, *pst, *pst2, *redo, *sub, *sens, *agree;
   double* tb;
   double2* zwork;
-  OzakiSet rows[3], cols;      // digits of three left operands and a right one
+  OzakiSet rows[3], cols;      // digits of three left operands (one after the other in the same place
+                               // where the contacts run one by one) and a right one
   double* t0;
 };
 
-Ws carve(void* base, int P, int n, int slices, size_t* total) {
+Ws carve(void* base, int P, int n, int slices, bool one_contact, size_t* total) {
   Carver c{static_cast<char*>(base)};
   Ws w;
-  const size_t Q = (size_t)n * n, N = 2 * (size_t)P;   // problems: the contacts of every point
-  for (int b = 0; b < kBlocks; ++b) w.blk[b] = c.take<double2>(N * Q);
+  // problems at a time: the contacts of every point, or one contact of it
+  const size_t Q = (size_t)n * n, N = (one_contact ? 1 : 2) * (size_t)P;
+  for (int b = 0; b < (one_contact ? kBlocksMax : kBlocks); ++b) w.blk[b] = c.take<double2>(N * Q);
   w.mx = c.take<double>(N);
   w.ok = c.take<int>(N);
-  w.nc = c.take<int>(N);
+  w.nc = c.take<int>(2 * (size_t)P);
   w.list0 = c.take<int>(N);
   w.list1 = c.take<int>(N);
   w.count = c.take<int>(4);
   w.info = c.take<int>(N);
   w.pst = c.take<int>(P);
-  w.pst2 = c.take<int>(N);
+  w.pst2 = c.take<int>(2 * (size_t)P);
   w.tb = c.take<double>(P);
   w.redo = c.take<int>(N);
   w.sub = c.take<int>(N);
   w.sens = c.take<int>(N);
   w.agree = c.take<int>(N);
   w.zwork = c.take<double2>(N * zinv_batched_work_elems(n) + 1);
+  uint8_t* q = nullptr;
   for (int i = 0; i < 3; ++i) {
-    uint8_t* q = c.take<uint8_t>(ozaki_rows_bytes((int)N, n, n, slices));
+    if (i == 0 || !one_contact) q = c.take<uint8_t>(ozaki_rows_bytes((int)N, n, n, slices));
     if (base) w.rows[i] = ozaki_rows_at(q, (int)N, n, n, slices);
   }
-  uint8_t* q = c.take<uint8_t>(ozaki_cols_bytes((int)N, n, n, slices));
+  q = c.take<uint8_t>(ozaki_cols_bytes((int)N, n, n, slices));
   if (base) w.cols = ozaki_cols_at(q, (int)N, n, n, slices);
   w.t0 = c.take<double>(N * Q);
   *total = c.off + 256;
@@ -431,9 +436,9 @@ __global__ void k_not_converged(int na, const int* list, int* ncyc_c, int* pst, 
 
 }  // namespace
 
-size_t mixed_ws_bytes(int batch, int n, int slices) {
+size_t mixed_ws_bytes(int batch, int n, int slices, bool one_contact) {
   size_t t = 0;
-  carve(nullptr, batch, n, slices, &t);
+  carve(nullptr, batch, n, slices, one_contact, &t);
   return t;
 }
 
@@ -441,17 +446,17 @@ int mixed_batch_for(size_t bytes, int n, int slices) {
   int lo = 0, hi = 1 << 14;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
-    if (mixed_ws_bytes(mid, n, slices) <= bytes) lo = mid; else hi = mid - 1;
+    if (mixed_ws_bytes(mid, n, slices, false) <= bytes) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
 
-int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::string* err) {
+int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStream_t s, std::string* err) {
   const int n = a.n;
   const int64_t Q = (int64_t)n * n;
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0), mone = make_double2(-1, 0);
   size_t tot = 0;
-  Ws w = carve(ws, batch, n, a.slices, &tot);
+  Ws w = carve(ws, batch, n, a.slices, one_contact, &tot);
   double2** B = w.blk;
   const dim3 eb(256);
   const int gx = (int)std::min<int64_t>(64, (Q + 255) / 256);
@@ -469,7 +474,16 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
   // into digits once for all the products it takes part in: of a decimation
   // iteration's six products, three left and four right operands.
   uint64_t nl = 0;                 // kernels launched (reported through a.launches)
+  // Where the contacts run one by one the left operands share one place and are
+  // split when a product needs another one than the place holds.
+  const double2* left_of[3] = {nullptr, nullptr, nullptr};
+  int held = -1;
   auto rows = [&](int nb, const int* map, const double2* A, int set) -> cudaError_t {
+    if (one_contact) {
+      left_of[set] = A;
+      if (held == set) held = -1;
+      return cudaSuccess;
+    }
     ++nl;
     return launch_ozaki_rows(nb, n, n, A, Q, a.slices, w.rows[set], s, map);
   };
@@ -479,6 +493,12 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
   };
   auto prod = [&](int nb, const int* map, double2 alpha, int set, double2 beta, double2* C, double* maxabs,
                   int* status) -> cudaError_t {
+    if (one_contact && held != set) {
+      ++nl;
+      const cudaError_t e = launch_ozaki_rows(nb, n, n, left_of[set], Q, a.slices, w.rows[set], s, map);
+      if (e != cudaSuccess) return e;
+      held = set;
+    }
     ++nl;
     return launch_ozaki_product(nb, n, n, n, alpha, w.rows[set], w.cols, beta, C, Q, a.slices, w.t0, maxabs, status,
                                 s, map);
@@ -492,146 +512,152 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::stri
     ++nl;
     return launch_zgemm_batched(nb, n, n, n, one, A, Q, Bm, Q, zero, C, Q, 0, s);
   };
-  double2 *gs = B[9], *sig = B[10], *kept_gs = B[10];   // (a kept gs is done with before the self-energies)
 
   for (int p0 = 0; p0 < a.npts; p0 += batch) {
-    const int P = std::min(batch, a.npts - p0), N = 2 * P;
+    const int P = std::min(batch, a.npts - p0), N = one_contact ? P : 2 * P;
     const int* ids = a.d_ids + p0;
     const double* E = a.d_E + p0;
-    MCK(cudaMemsetAsync(w.pst2, 0, sizeof(int) * N, s), "memset status");
-    // ---- surface Green's functions of both contacts of every point (problem
-    // p: left contact of point p, P + p: right), all in lock step.
-    // Decimation of the problems sub[b], b < nsub (sub null: all N), the
-    // contact energy scaled by `scale`; then gs = Aos^-1 and the
-    // retarded-branch check (redo[p] = 1 where it fails)
-    auto decimate = [&](const int* sub, int nsub, double scale) -> int {
-      double2 *Ao = B[0], *Aos = B[1], *Bo = B[2], *Co = B[3], *Go = B[4], *X = B[5], *C1 = B[6], *Y = B[7],
-              *B1 = B[8];
-      k_lead_init<<<dim3(gx, nsub), eb, 0, s>>>(n, P, a.left, a.right, ids, E, a.eta, scale, sub, a.d_descs, Ao, Aos,
-                                                Bo, Co, Q);
-      ++nl;
-      MCK(cudaGetLastError(), "lead init");
-      k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, w.nc, w.list0, w.sens);
-      ++nl;
-      int na = nsub;                                   // host bound of the active list
-      int* cur = w.list0;
-      int* nxt = w.list1;
-      int it = 1;
-      for (; it <= a.sgf_max_iter && na > 0; ++it) {
-        // one batched product per step, the active list compacted on the host
-        MCK(inv(na, cur, Ao, Go), "zinv");
-        k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.info, w.pst2, NEGF_B200_ERR_SINGULAR);
+    MCK(cudaMemsetAsync(w.pst2, 0, sizeof(int) * 2 * P, s), "memset status");
+    for (int side = 0; side < (one_contact ? 2 : 1); ++side) {
+      const int cl = side == 0 ? a.left : a.right, cr = one_contact ? cl : a.right;
+      int *nc = w.nc + (int64_t)side * P, *pst2 = w.pst2 + (int64_t)side * P;
+      double2 *gs = B[9], *sig = B[10], *kept_gs = B[10];   // (a kept gs is done with before the self-energies)
+      // ---- surface Green's functions of both contacts of every point (problem
+      // p: left contact of point p, P + p: right; or those of one contact), all
+      // in lock step.
+      // Decimation of the problems sub[b], b < nsub (sub null: all N), the
+      // contact energy scaled by `scale`; then gs = Aos^-1 and the
+      // retarded-branch check (redo[p] = 1 where it fails)
+      auto decimate = [&](const int* sub, int nsub, double scale) -> int {
+        double2 *Ao = B[0], *Aos = B[1], *Bo = B[2], *Co = B[3], *Go = B[4], *X = B[5], *C1 = B[6], *Y = B[7],
+                *B1 = B[8];
+        k_lead_init<<<dim3(gx, nsub), eb, 0, s>>>(n, P, cl, cr, ids, E, a.eta, scale, sub, a.d_descs, Ao, Aos,
+                                                  Bo, Co, Q);
         ++nl;
-        MCK(rows(na, cur, Go, 0), "split Go");
-        MCK(cols(na, cur, Co), "split Co");
-        MCK(prod(na, cur, one, 0, zero, X, nullptr, w.pst2), "GoXCo");
-        MCK(rows(na, cur, Co, 1), "split Co");
-        MCK(cols(na, cur, X), "split X");
-        MCK(prod(na, cur, one, 1, zero, C1, w.mx, w.pst2), "C1");
-        k_dec_check<<<1, 1024, 0, s>>>(na, cur, w.mx, w.ok, w.nc, a.sgf_tol, it, nxt, w.count, w.redo);
+        MCK(cudaGetLastError(), "lead init");
+        k_dec_start<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.ok, w.mx, nc, w.list0, w.sens);
         ++nl;
-        MCK(cudaGetLastError(), "check");
-        std::swap(cur, nxt);
-        {
-          int h_count = 0;
-          MCK(cudaMemcpyAsync(&h_count, w.count, sizeof(int), cudaMemcpyDeviceToHost, s), "count");
-          MCK(cudaStreamSynchronize(s), "sync");
-          na = h_count;
-          if (na == 0) break;
-        }
-        MCK(rows(na, cur, Bo, 2), "split Bo");
-        MCK(prod(na, cur, one, 2, zero, B1, nullptr, w.pst2), "Self");
-        k_sub_self<<<dim3(gx, na), eb, 0, s>>>(Q, cur, B1, Ao, Aos, Q); ++nl;
-        MCK(cols(na, cur, Bo), "split Bo");
-        MCK(prod(na, cur, one, 0, zero, Y, nullptr, w.pst2), "GoXBo");
-        MCK(cols(na, cur, Y), "split Y");
-        MCK(prod(na, cur, one, 2, zero, B1, nullptr, w.pst2), "B1");
-        MCK(prod(na, cur, mone, 1, one, Ao, nullptr, w.pst2), "Ao update");
-        // Bo = B1, Co = C1 for every problem still iterating (the others are done with them)
-        std::swap(B[2], B[8]);
-        std::swap(B[3], B[6]);
-        Bo = B[2]; Co = B[3]; B1 = B[8]; C1 = B[6];
-      }
-      if (na > 0) {
-        k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.nc, w.pst2, a.sgf_max_iter);
-        ++nl;
-      }
-      MCK(inv(nsub, sub, Aos, gs), "gs");
-      k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, w.pst2, NEGF_B200_ERR_SINGULAR);
-      ++nl;
-      if (a.eta != 0.0) {
-        k_retarded_check<<<nsub, 128, 0, s>>>(n, gs, Q, a.eta > 0.0 ? -1.0 : 1.0, sub, w.redo);
-        ++nl;
-      }
-      return 0;
-    };
-    MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
-    if (int r = decimate(nullptr, N, 1.0)) return r;
-    if (a.eta != 0.0) {
-      // Decimations that reached another fixed point (or ran off to Inf / NaN) run
-      // again, in lock step over just those problems, from the contact energy times
-      // 1 + k 2^-50.  A sensitive decimation (one of its inverses needed a Newton
-      // step: a nearly singular Ao) is accepted once two attempts reach the same gs.
-      std::vector<int> hredo(N), hsens(N), hagree(N), kept(N, 0), cur_sub, again, cmp, keep;
-      cur_sub.resize(N);
-      for (int p = 0; p < N; ++p) cur_sub[p] = p;
-      for (int att = 1;; ++att) {
-        MCK(cudaMemcpyAsync(hredo.data(), w.redo, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "redo");
-        MCK(cudaMemcpyAsync(hsens.data(), w.sens, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "sens");
-        MCK(cudaStreamSynchronize(s), "sync");
-        cmp.clear();
-        for (int p : cur_sub)
-          if (!hredo[p] && hsens[p] && kept[p]) cmp.push_back(p);
-        if (!cmp.empty()) {
-          MCK(cudaMemcpyAsync(w.sub, cmp.data(), sizeof(int) * cmp.size(), cudaMemcpyHostToDevice, s), "cmp");
-          k_agree<<<(int)cmp.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q, 1e-2, w.agree); ++nl;
-          MCK(cudaMemcpyAsync(hagree.data(), w.agree, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "agree");
-          MCK(cudaStreamSynchronize(s), "sync");
-        }
-        again.clear();
-        keep.clear();
-        for (int p : cur_sub) {
-          if (hredo[p]) { again.push_back(p); continue; }                  // wrong fixed point: run again
-          if (!hsens[p]) continue;                                          // settled
-          if (kept[p] && hagree[p]) continue;                               // two attempts agree
-          keep.push_back(p);                                                // keep this gs, run again
-          again.push_back(p);
-        }
-        if (again.empty()) break;
-        if (att > kDecRetries) {
-          for (int p : again) hredo[p] = 1;
-          MCK(cudaMemcpyAsync(w.redo, hredo.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s), "redo");
-          k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, w.nc, w.pst2, a.sgf_max_iter);
+        int na = nsub;                                   // host bound of the active list
+        int* cur = w.list0;
+        int* nxt = w.list1;
+        int it = 1;
+        for (; it <= a.sgf_max_iter && na > 0; ++it) {
+          // one batched product per step, the active list compacted on the host
+          MCK(inv(na, cur, Ao, Go), "zinv");
+          k_info_to_status<<<(na + 255) / 256, 256, 0, s>>>(na, cur, w.info, pst2, NEGF_B200_ERR_SINGULAR);
           ++nl;
+          MCK(rows(na, cur, Go, 0), "split Go");
+          MCK(cols(na, cur, Co), "split Co");
+          MCK(prod(na, cur, one, 0, zero, X, nullptr, pst2), "GoXCo");
+          MCK(rows(na, cur, Co, 1), "split Co");
+          MCK(cols(na, cur, X), "split X");
+          MCK(prod(na, cur, one, 1, zero, C1, w.mx, pst2), "C1");
+          k_dec_check<<<1, 1024, 0, s>>>(na, cur, w.mx, w.ok, nc, a.sgf_tol, it, nxt, w.count, w.redo);
+          ++nl;
+          MCK(cudaGetLastError(), "check");
+          std::swap(cur, nxt);
+          {
+            int h_count = 0;
+            MCK(cudaMemcpyAsync(&h_count, w.count, sizeof(int), cudaMemcpyDeviceToHost, s), "count");
+            MCK(cudaStreamSynchronize(s), "sync");
+            na = h_count;
+            if (na == 0) break;
+          }
+          MCK(rows(na, cur, Bo, 2), "split Bo");
+          MCK(prod(na, cur, one, 2, zero, B1, nullptr, pst2), "Self");
+          k_sub_self<<<dim3(gx, na), eb, 0, s>>>(Q, cur, B1, Ao, Aos, Q); ++nl;
+          MCK(cols(na, cur, Bo), "split Bo");
+          MCK(prod(na, cur, one, 0, zero, Y, nullptr, pst2), "GoXBo");
+          MCK(cols(na, cur, Y), "split Y");
+          MCK(prod(na, cur, one, 2, zero, B1, nullptr, pst2), "B1");
+          MCK(prod(na, cur, mone, 1, one, Ao, nullptr, pst2), "Ao update");
+          // Bo = B1, Co = C1 for every problem still iterating (the others are done with them)
+          std::swap(B[2], B[8]);
+          std::swap(B[3], B[6]);
+          Bo = B[2]; Co = B[3]; B1 = B[8]; C1 = B[6];
+        }
+        if (na > 0) {
+          k_not_converged<<<(na + 255) / 256, 256, 0, s>>>(na, cur, nc, pst2, a.sgf_max_iter);
+          ++nl;
+        }
+        MCK(inv(nsub, sub, Aos, gs), "gs");
+        k_info_to_status<<<(nsub + 255) / 256, 256, 0, s>>>(nsub, sub, w.info, pst2, NEGF_B200_ERR_SINGULAR);
+        ++nl;
+        if (a.eta != 0.0) {
+          k_retarded_check<<<nsub, 128, 0, s>>>(n, gs, Q, a.eta > 0.0 ? -1.0 : 1.0, sub, w.redo);
+          ++nl;
+        }
+        return 0;
+      };
+      MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
+      if (int r = decimate(nullptr, N, 1.0)) return r;
+      if (a.eta != 0.0) {
+        // Decimations that reached another fixed point (or ran off to Inf / NaN) run
+        // again, in lock step over just those problems, from the contact energy times
+        // 1 + k 2^-50.  A sensitive decimation (one of its inverses needed a Newton
+        // step: a nearly singular Ao) is accepted once two attempts reach the same gs.
+        std::vector<int> hredo(N), hsens(N), hagree(N), kept(N, 0), cur_sub, again, cmp, keep;
+        cur_sub.resize(N);
+        for (int p = 0; p < N; ++p) cur_sub[p] = p;
+        for (int att = 1;; ++att) {
+          MCK(cudaMemcpyAsync(hredo.data(), w.redo, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "redo");
+          MCK(cudaMemcpyAsync(hsens.data(), w.sens, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "sens");
           MCK(cudaStreamSynchronize(s), "sync");
-          break;
+          cmp.clear();
+          for (int p : cur_sub)
+            if (!hredo[p] && hsens[p] && kept[p]) cmp.push_back(p);
+          if (!cmp.empty()) {
+            MCK(cudaMemcpyAsync(w.sub, cmp.data(), sizeof(int) * cmp.size(), cudaMemcpyHostToDevice, s), "cmp");
+            k_agree<<<(int)cmp.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q, 1e-2, w.agree); ++nl;
+            MCK(cudaMemcpyAsync(hagree.data(), w.agree, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "agree");
+            MCK(cudaStreamSynchronize(s), "sync");
+          }
+          again.clear();
+          keep.clear();
+          for (int p : cur_sub) {
+            if (hredo[p]) { again.push_back(p); continue; }                  // wrong fixed point: run again
+            if (!hsens[p]) continue;                                          // settled
+            if (kept[p] && hagree[p]) continue;                               // two attempts agree
+            keep.push_back(p);                                                // keep this gs, run again
+            again.push_back(p);
+          }
+          if (again.empty()) break;
+          if (att > kDecRetries) {
+            for (int p : again) hredo[p] = 1;
+            MCK(cudaMemcpyAsync(w.redo, hredo.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s), "redo");
+            k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, nc, pst2, a.sgf_max_iter);
+            ++nl;
+            MCK(cudaStreamSynchronize(s), "sync");
+            break;
+          }
+          if (!keep.empty()) {
+            MCK(cudaMemcpyAsync(w.sub, keep.data(), sizeof(int) * keep.size(), cudaMemcpyHostToDevice, s), "keep");
+            k_keep<<<(int)keep.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q); ++nl;
+            for (int p : keep) kept[p] = 1;
+          }
+          MCK(cudaMemcpyAsync(w.sub, again.data(), sizeof(int) * again.size(), cudaMemcpyHostToDevice, s), "sub");
+          MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
+          if (int r = decimate(w.sub, (int)again.size(), 1.0 + att * 0x1p-50)) return r;
+          cur_sub = again;
+          MCK(cudaStreamSynchronize(s), "sync");   // the host vectors above are reused next round
         }
-        if (!keep.empty()) {
-          MCK(cudaMemcpyAsync(w.sub, keep.data(), sizeof(int) * keep.size(), cudaMemcpyHostToDevice, s), "keep");
-          k_keep<<<(int)keep.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q); ++nl;
-          for (int p : keep) kept[p] = 1;
-        }
-        MCK(cudaMemcpyAsync(w.sub, again.data(), sizeof(int) * again.size(), cudaMemcpyHostToDevice, s), "sub");
-        MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");
-        if (int r = decimate(w.sub, (int)again.size(), 1.0 + att * 0x1p-50)) return r;
-        cur_sub = again;
-        MCK(cudaStreamSynchronize(s), "sync");   // the host vectors above are reused next round
+      } else {   // no other branch to try; gs of an iteration broken off (Inf / NaN) means nothing
+        k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, nc, pst2, a.sgf_max_iter);
+        ++nl;
       }
-    } else {   // no other branch to try; gs of an iteration broken off (Inf / NaN) means nothing
-      k_flag_unresolved<<<(N + 255) / 256, 256, 0, s>>>(N, w.redo, w.nc, w.pst2, a.sgf_max_iter);
-      ++nl;
+      // ---- self-energies Sigma_c = Tlc gs Tcl of both contacts
+      k_tlc<<<dim3(gx, N), eb, 0, s>>>(n, P, cl, cr, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;
+      MCK(cudaGetLastError(), "tlc");
+      MCK(rows(N, nullptr, B[0], 0), "split Tlc");
+      MCK(cols(N, nullptr, gs), "split gs");
+      MCK(prod(N, nullptr, one, 0, zero, B[2], nullptr, pst2), "Tlc gs");
+      MCK(rows(N, nullptr, B[2], 0), "split Tlc gs");
+      MCK(cols(N, nullptr, B[1]), "split Tcl");
+      MCK(prod(N, nullptr, one, 0, zero, sig, nullptr, pst2), "Sigma");
+      if (one_contact && side == 0) std::swap(B[10], B[11]);
     }
-    // ---- self-energies Sigma_c = Tlc gs Tcl of both contacts
-    k_tlc<<<dim3(gx, N), eb, 0, s>>>(n, P, a.left, a.right, ids, E, a.eta, a.d_descs, B[0], B[1], Q); ++nl;
-    MCK(cudaGetLastError(), "tlc");
-    MCK(rows(N, nullptr, B[0], 0), "split Tlc");
-    MCK(cols(N, nullptr, gs), "split gs");
-    MCK(prod(N, nullptr, one, 0, zero, B[2], nullptr, w.pst2), "Tlc gs");
-    MCK(rows(N, nullptr, B[2], 0), "split Tlc gs");
-    MCK(cols(N, nullptr, B[1]), "split Tcl");
-    MCK(prod(N, nullptr, one, 0, zero, sig, nullptr, w.pst2), "Sigma");
     k_merge_status<<<(P + 255) / 256, 256, 0, s>>>(P, w.pst2, w.pst); ++nl;
-    const double2 *sig_l = sig, *sig_r = sig + (int64_t)P * Q;
+    const double2 *sig_l = one_contact ? B[11] : B[10], *sig_r = one_contact ? B[10] : B[10] + (int64_t)P * Q;
     // ---- gsmr sweep from block nbl down to 2, then Gr(1,1)
     double2 *g = B[4], *X = B[5], *W = B[6], *U = B[7], *Lb = B[8];
     k_esh<<<dim3(gx, P), eb, 0, s>>>(n, 0, a.nbl - 1, ids, E, a.d_descs, sig_r, W, Q); ++nl;

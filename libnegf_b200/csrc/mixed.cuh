@@ -30,14 +30,16 @@ struct MixedArgs {
   uint64_t* launches = nullptr;  // host counter of kernels launched (may be null)
 };
 
-// bytes of workspace for a batch of `batch` points of order n
-size_t mixed_ws_bytes(int batch, int n, int slices);
-// the largest batch that fits `bytes` (0 if none)
+// bytes of workspace for a batch of `batch` points of order n; one_contact: with
+// a point's contacts one after the other instead of side by side (half as much
+// for a point, for calls whose workspace holds no more; the same bits)
+size_t mixed_ws_bytes(int batch, int n, int slices, bool one_contact);
+// the largest batch that fits `bytes` with the contacts side by side (0 if none)
 int mixed_batch_for(size_t bytes, int n, int slices);
 
 // Runs the solve in batches of `batch` points on stream s (synchronises with
 // the host once per decimation iteration to shrink the active set).
 // Returns 0 or a NEGF_B200 status, with a message in *err.
-int mixed_run(const MixedArgs& a, void* ws, int batch, cudaStream_t s, std::string* err);
+int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStream_t s, std::string* err);
 
 }  // namespace negf

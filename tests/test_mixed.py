@@ -161,3 +161,30 @@ def test_mixed_branch_check_follows_the_sign_of_the_broadening(gpu_ctx, eta):
             assert np.all(sm == (native.NOT_CONVERGED if bad else 0))
         finally:
             gpu_ctx.release(did)
+
+
+@pytest.mark.parametrize("n", [1, 16, 48, 96])
+@pytest.mark.parametrize("digits", [4, 8])
+def test_mixed_runs_in_the_workspace_of_one_contact(gpu_ctx, n, digits):
+    """A workspace limit with room for one contact's blocks, not for both at
+    once: the contacts one after the other, the same bits.  The size is 14
+    blocks, the inverse's four, five digit planes and a real block, each
+    array on a 256-byte boundary; a little below it is refused."""
+    up = lambda b: (b + 255) // 256 * 256
+    kp, nn = (n + 15) // 16 * 16, n * n
+    need = (14 * up(16 * nn) + 16 * 256 + up(16 * (4 if n > 64 else 2) * nn + 16)
+            + up(3 * digits * n * kp) + up(2 * digits * n * kp) + 2 * up(4 * n) + up(8 * nn))
+    did = gpu_ctx.upload(G.transport_c0(nbl=3, n=n, seed=2))
+    E = np.linspace(-1.0, 1.0, 5)
+    try:
+        T, nc, st = _mixed_T(gpu_ctx, did, E, 1e-6, digits=digits)
+        gpu_ctx.set_workspace_limit(need)
+        Tk, nk, sk = _mixed_T(gpu_ctx, did, E, 1e-6, digits=digits)
+        assert np.array_equal(Tk, T) and np.array_equal(nk, nc) and np.array_equal(sk, st)
+        gpu_ctx.set_workspace_limit(12 * 16 * nn)
+        with pytest.raises(native.NegfError) as e:
+            _mixed_T(gpu_ctx, did, E, 1e-6, digits=digits)
+        assert e.value.code == native.ADMISSION
+    finally:
+        gpu_ctx.set_workspace_limit(0)
+        gpu_ctx.release(did)
