@@ -163,6 +163,33 @@ def test_mixed_branch_check_follows_the_sign_of_the_broadening(gpu_ctx, eta):
             gpu_ctx.release(did)
 
 
+def test_mixed_batches_do_not_change_a_point(gpu_ctx):
+    """More points than one batch holds (two per SM), and a workspace limit
+    that cuts the call into batches of a few points: the same bits, cycle
+    counts and statuses, with points of two devices and a bad one between."""
+    bad = G.transport_c0(nbl=3, n=16, seed=4)
+    bad.lead_h01[1][0, 0] = np.nan
+    hs = [gpu_ctx.upload(d) for d in (G.transport_c0(nbl=3, n=16, seed=2), G.transport_c0(nbl=3, n=16, seed=3), bad)]
+    E = np.linspace(-2.0, 2.0, 601)
+    ids = np.asarray(hs, dtype=np.int32)[np.arange(E.size) % 3]
+    try:
+        T, nc, st = _mixed_T(gpu_ctx, ids, E, 1e-6)
+        assert np.all(st[ids != hs[2]] == 0) and np.all(st[ids == hs[2]] != 0)
+        for k in (0, 3, 298, 599):
+            s = slice(k, k + 2)
+            Tk, nk, sk = _mixed_T(gpu_ctx, ids[s], E[s], 1e-6)
+            assert np.array_equal(Tk, T[s], equal_nan=True) and np.array_equal(nk, nc[s]) and np.array_equal(sk, st[s])
+        for points in (1, 7):                                      # 42 blocks each, and the small arrays
+            gpu_ctx.set_workspace_limit(points * 42 * 16 * 16 * 16 + 32768)
+            Tk, nk, sk = _mixed_T(gpu_ctx, ids[:40], E[:40], 1e-6)
+            assert np.array_equal(Tk, T[:40], equal_nan=True)
+            assert np.array_equal(nk, nc[:40]) and np.array_equal(sk, st[:40])
+    finally:
+        gpu_ctx.set_workspace_limit(0)
+        for h in hs:
+            gpu_ctx.release(h)
+
+
 @pytest.mark.parametrize("n", [1, 16, 48, 96])
 @pytest.mark.parametrize("digits", [4, 8])
 def test_mixed_runs_in_the_workspace_of_one_contact(gpu_ctx, n, digits):
