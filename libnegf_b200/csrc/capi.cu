@@ -260,7 +260,8 @@ struct EnginePlan {
   size_t need;                   // of the whole workspace
 };
 
-int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, bool outer, EnginePlan& pl) {
+int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, bool outer, EnginePlan& pl,
+                bool may_split = true) {
   if (sh.nmax > negf::kMaxOrder)
     return fail(ctx, NEGF_B200_ERR_BAD_ARG, "block order " + std::to_string(sh.nmax) + " exceeds " +
                                                 std::to_string(negf::kMaxOrder));
@@ -277,7 +278,7 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
   const int64_t pairs = (int64_t)npts * sh.ncont_max;
   pl.blocks = (size_t)pairs * sh.nmax * sh.nmax * sizeof(double2) * (outer ? 2 : 1);
   pl.ints = (2 * (size_t)pairs * sizeof(int) + 255) / 256 * 256;
-  pl.split = sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && pl.blocks <= (size_t(4) << 30);
+  pl.split = may_split && sh.ncont_max > 1 && pairs <= 8 * (int64_t)ctas && pl.blocks <= (size_t(4) << 30);
   pl.tc = pl.ts;
   if (pl.split) pl.tc = negf::team_plan((int)pairs, sh.nmax, ctas, sms);
   if (ctx->ws_limit > 0) {
@@ -311,7 +312,13 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
   if (st) return st;
   st = sync_descs(ctx);
   if (st) return st;
+  const std::string before = ctx->err;
   st = grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
+  if (st && pl.split) {   // whole points in one launch need less: no blocks between launches
+    st = plan_engine(ctx, a.mode, a.npts, sh, a.acc_lc != nullptr, pl, false);
+    if (st == NEGF_B200_OK) st = grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
+    if (st == NEGF_B200_OK) ctx->err = before;
+  }
   if (st) return st;
   a.Q = (int64_t)sh.nmax * sh.nmax;
   a.nmax = sh.nmax;

@@ -1,0 +1,44 @@
+"""The engine's workspace when there is little of it: a limit set by the
+caller, or a device that is nearly full."""
+import numpy as np
+import pytest
+
+from libnegf_b200 import generators as G
+from libnegf_b200 import native
+
+pytestmark = pytest.mark.gpu
+
+
+def _layout(n, nbl, npts):
+    """Bytes of a point's slots, of the blocks kept between the launches of a
+    split call, and of one launch of whole points (at most two CTAs an SM)."""
+    per = (15 + 2 + nbl + 2) * 16 * n * n
+    return per, 2 * npts * 16 * n * n
+
+
+def test_a_call_runs_where_only_its_whole_points_fit():
+    """Without a limit, on a device with room for the slots of whole points but
+    not for the blocks of a split call besides: the call runs as one launch."""
+    torch = pytest.importorskip("torch")
+    n, nbl, npts = 128, 2, 1000
+    per, blocks = _layout(n, nbl, npts)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    whole = 2 * sms * per
+    dev = G.transport_c0(nbl=nbl, n=n, seed=3)
+    E = np.linspace(-1.0, 1.0, npts)
+    with native.Context(0) as ctx:
+        h = ctx.upload(dev)
+        T, nc, st = ctx.transmission(h, E[:20], eta=1e-3)
+    torch.cuda.empty_cache()
+    with native.Context(0) as ctx:
+        h = ctx.upload(dev)
+        free = torch.cuda.mem_get_info()[0]
+        fill = torch.empty(free - whole - blocks // 2, dtype=torch.uint8, device="cuda")
+        try:
+            n0 = ctx.launch_count()
+            Tl, nl, sl = ctx.transmission(h, E, eta=1e-3)
+            assert ctx.launch_count() - n0 == 1
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+    assert np.array_equal(Tl[:20], T) and np.array_equal(nl[:20], nc) and np.all(sl == 0)
