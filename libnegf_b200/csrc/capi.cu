@@ -285,7 +285,10 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
     // fewer resident teams when the workspace would exceed the limit (the persistent
     // kernel still runs every point); not even one: refuse
     const size_t room = ctx->ws_limit > 256 ? ctx->ws_limit - 256 : 0;
-    if (pl.split && room < pl.ints + pl.blocks + std::max(pl.per, pl.per_c)) pl.split = false;
+    // the blocks between the launches must not cost the sweeps a team (1000
+    // points of 2 layers in a limit of 2100 blocks: 4 teams where one launch of
+    // whole points has 100); a contact's slots are the smaller
+    if (pl.split && room < pl.ints + pl.blocks + (size_t)pl.ts.most_teams() * pl.per) pl.split = false;
     const size_t rest = pl.split ? room - pl.ints - pl.blocks : room;
     const size_t fit = rest / pl.per;
     if (fit < 1)

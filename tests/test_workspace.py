@@ -16,6 +16,30 @@ def _layout(n, nbl, npts):
     return per, 2 * npts * 16 * n * n
 
 
+def test_a_tight_limit_keeps_the_teams_of_the_sweeps(gpu_ctx):
+    """The contacts' blocks of a split call count against the limit: where they
+    would leave fewer teams for the points than one launch of whole points
+    has, the call is not split."""
+    n, nbl, npts = 48, 2, 1000
+    per, blocks = _layout(n, nbl, npts)
+    h = gpu_ctx.upload(G.transport_c0(nbl=nbl, n=n, seed=3))
+    E = np.linspace(-1.0, 1.0, npts)
+    try:
+        gpu_ctx.set_options(schedule=1)
+        n0 = gpu_ctx.launch_count()
+        T, nc, st = gpu_ctx.transmission(h, E, eta=1e-3)
+        assert gpu_ctx.launch_count() - n0 >= 2
+        gpu_ctx.set_workspace_limit(blocks + 8 * per)
+        n0 = gpu_ctx.launch_count()
+        Tl, nl, sl = gpu_ctx.transmission(h, E, eta=1e-3)
+        assert gpu_ctx.launch_count() - n0 == 1
+        assert np.array_equal(Tl, T) and np.array_equal(nl, nc) and np.array_equal(sl, st)
+    finally:
+        gpu_ctx.set_workspace_limit(0)
+        gpu_ctx.set_options()
+        gpu_ctx.release(h)
+
+
 def test_a_call_runs_where_only_its_whole_points_fit():
     """Without a limit, on a device with room for the slots of whole points but
     not for the blocks of a split call besides: the call runs as one launch."""
