@@ -308,6 +308,24 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
   return NEGF_B200_OK;
 }
 
+// Makes room for an engine call to come, where it can be had: the workspace
+// in place is given up only for the larger one, and nothing is reported.
+void reserve_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh) {
+  const std::string before = ctx->err;
+  EnginePlan pl;
+  if (plan_engine(ctx, mode, npts, sh, false, pl) == NEGF_B200_OK && pl.need > ctx->ws_bytes) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, pl.need) == cudaSuccess) {
+      if (ctx->ws) cudaFree(ctx->ws);
+      ctx->ws = p;
+      ctx->ws_bytes = pl.need;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  ctx->err = before;
+}
+
 // Runs one call with device-resident inputs/outputs (all pointers device).
 int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cudaStream_t s) {
   EnginePlan pl;
@@ -1222,9 +1240,7 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
     // allocated: leave its workspace in place (where it fits)
     LaunchShape es;
     es.nmax = n; es.nbl_max = sh.nbl; es.ncont_max = 2;
-    EnginePlan pl;
-    if (plan_engine(ctx, negf::MODE_T, npts, es, false, pl) == NEGF_B200_OK)
-      grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
+    reserve_engine(ctx, negf::MODE_T, npts, es);
     const cudaError_t e = negf::launch_small_points(a, s);
     return e == cudaSuccess ? NEGF_B200_OK : cuda_fail(ctx, e, "lock step");
   }

@@ -66,3 +66,13 @@ def test_a_call_runs_where_only_its_whole_points_fit():
             del fill
             torch.cuda.empty_cache()
     assert np.array_equal(Tl[:20], T) and np.array_equal(nl[:20], nc) and np.all(sl == 0)
+
+
+def test_a_call_that_succeeds_leaves_no_message(gpu_ctx):
+    """A small-order call needs no workspace of the engine; a limit that would
+    refuse the engine is none of its errors."""
+    with native.Context(0) as ctx:
+        h = ctx.upload(G.transport_c0(nbl=4, n=8, seed=2))
+        ctx.set_workspace_limit(15 * 16 * 8 * 8)
+        T, nc, st = ctx.transmission(h, np.linspace(-1, 1, 5), eta=1e-3)
+        assert np.all(st == 0) and ctx.last_error() == ""
