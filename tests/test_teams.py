@@ -327,3 +327,71 @@ def test_product_in_the_place_of_an_operand(n, dagger, place):
                                              2 * n * n, dagger, s) == 0
         torch.cuda.synchronize()
         assert torch.equal(out, ref)
+
+
+def _team_of(L, work, n):
+    """The library's own choice of CTAs per problem (its team_shape: two ints
+    in one register), so that a test says which sizes it compares."""
+    f = L["_ZN4negf10team_shapeEiiii"]
+    f.restype, f.argtypes = ctypes.c_uint64, [ctypes.c_int] * 4
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return int(f(work, n, 2 * sms, sms) & 0xffffffff)
+
+
+@pytest.mark.parametrize("n", [64, 65, 96, 127, 129, 256, 257, 512, 513])
+def test_inverse_bits_of_one_cta_and_of_teams(n):
+    """One wave of matrices (a CTA each) against calls small enough for teams
+    of every size the order takes."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    batch = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert _team_of(L, batch, n) == 1
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.randn((batch, n, n), dtype=torch.complex128, device="cuda", generator=g)
+    info = torch.full((batch,), -1, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.negf_b200_zinv_work_bytes(batch, n), dtype=torch.uint8, device="cuda")
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    w = ctypes.c_void_p(work.data_ptr())
+    X = torch.zeros_like(A)
+    assert L.negf_b200_zinv_batched(batch, n, _dp(A), _dp(X), _ip(info), w, s) == 0
+    assert int(info.abs().max()) == 0
+    sizes = {}
+    for m in range(batch - 1, 0, -1):
+        sizes[_team_of(L, m, n)] = m                               # the fewest matrices of each team size
+    sizes.pop(1, None)
+    assert max(sizes) >= (4 if n <= 80 else 16)
+    for team, m in sizes.items():
+        Y = torch.zeros_like(A[:m])
+        assert L.negf_b200_zinv_batched(m, n, _dp(A), _dp(Y), _ip(info), w, s) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(Y, X[:m]), team
+
+
+@pytest.mark.parametrize("batch", [2, 296])
+@pytest.mark.parametrize("n", [65, 100, 200, 300, 600])
+def test_inverse_with_an_infinite_pivot_above_one_panel(n, batch):
+    """An infinite diagonal entry of a matrix with a dominant diagonal is the
+    pivot of its own column, with reciprocal 0: its row and column of the
+    inverse vanish and the rest is the inverse without them, to
+    8 n u kappa |inv| (LAPACK's own error is within it too)."""
+    torch = pytest.importorskip("torch")
+    L = native.load()
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 8 * np.sqrt(n) * np.eye(n)
+    keep = np.arange(n) != n // 2
+    sub = a[np.ix_(keep, keep)]
+    ref = np.linalg.inv(sub)
+    a[n // 2, n // 2] = np.inf
+    dA = torch.from_numpy(np.ascontiguousarray(a.T)).cuda().expand(batch, n, n).contiguous()
+    X = torch.zeros_like(dA)
+    info = torch.zeros(batch, dtype=torch.int32, device="cuda")
+    work = torch.empty(L.negf_b200_zinv_work_bytes(batch, n), dtype=torch.uint8, device="cuda")
+    assert L.negf_b200_zinv_batched(batch, n, _dp(dA), _dp(X), _ip(info), ctypes.c_void_p(work.data_ptr()),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    x = X[batch - 1].cpu().numpy().T
+    assert bool((X == X[0]).all())
+    assert np.all(x[n // 2] == 0) and np.all(x[:, n // 2] == 0)
+    bound = 16 * n * 2.0 ** -53 * np.linalg.cond(sub) * np.linalg.norm(ref, 2)
+    assert np.abs(x[np.ix_(keep, keep)] - ref).max() <= bound
