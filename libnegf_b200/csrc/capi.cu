@@ -1219,8 +1219,8 @@ static int engine_only(negf_b200_ctx* ctx, const char* what) {
   return NEGF_B200_OK;
 }
 
-// Runs a lock-step form on device arrays of ids and energies// Runs a lock-step form on device arrays of ids and energies: sizes the batch
-// to the workspace and calls negf::mixed_run.
+// Runs a lock-step form on device arrays of ids and energies: small orders in
+// one launch, the mixed form in batches sized to the workspace.
 static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, const double* d_E, double eta,
                         double* d_T, int32_t* d_ncyc, int32_t* d_status, cudaStream_t s, const LockShape& sh,
                         int slices) {
@@ -1233,8 +1233,11 @@ static int run_lockstep(negf_b200_ctx* ctx, int32_t npts, const int32_t* d_ids, 
   a.sgf_tol = ctx->opt.sgf_tol; a.sgf_max_iter = ctx->opt.sgf_max_iter; a.slices = slices;
   a.d_T = d_T; a.d_ncyc = d_ncyc; a.d_status = d_status;
   a.launches = &ctx->launches;
-  if (slices == 0) {   // small orders: one launch, no workspace (a limit below one point's blocks refuses as ever)
-    if (ctx->ws_limit && ctx->ws_limit < (size_t)14 * n * n * sizeof(double2))
+  if (slices == 0) {   // small orders: one launch, no workspace
+    // a limit below the blocks of one point, as a form that works in memory has
+    // them, refuses the call like the other forms
+    constexpr size_t kPointBlocks = 14;
+    if (ctx->ws_limit && ctx->ws_limit < kPointBlocks * n * n * sizeof(double2))
       return fail(ctx, NEGF_B200_ERR_ADMISSION, "the workspace limit is below one point of lock step");
     // the engine runs the same call under stream capture, where nothing can be
     // allocated: leave its workspace in place (where it fits)

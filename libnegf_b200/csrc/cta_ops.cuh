@@ -11,8 +11,8 @@
 //             operands staged through shared memory with cp.async.
 //   cta_zinv  in-place-style blocked Gauss-Jordan inversion with partial
 //             pivoting (pivot = max |Re|+|Im|, the izamax rule of zgetrf):
-//             panel factorisation in shared memory, trailing update as a
-//             gathered GEMM on the tensor pipe, out-of-place ping-pong so
+//             panels factorised in registers, updates as gathered products
+//             on the tensor pipe or by row owners, out-of-place ping-pong so
 //             that row interchanges need no in-place hazards.
 //
 // Layout: column-major complex128 (double2 = {re, im}), leading dimension
@@ -160,10 +160,6 @@ __device__ __forceinline__ void team_max(double* v) {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(sdst)),
-               "l"(gsrc), "r"(valid ? 16 : 0));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -208,7 +204,6 @@ struct Epilogue {
   const double2* xcur;  // target columns before the update, read with row permutation
   int ldx;
   const int* perm;      // smem, full-length row permutation of the applied block
-  const double2* W;     // unused
   int k0, jb;           // pivot rows [k0, k0+jb) of the applied block (masked)
   // optional reduction of max |C| over stored elements (+Inf when one is NaN)
   double* maxabs;       // smem accumulator (nullptr = off)
@@ -218,7 +213,7 @@ struct Epilogue {
 __device__ __forceinline__ Epilogue epi_store(double2* C, int ldc, double2 alpha, double2 beta) {
   Epilogue e;
   e.mode = EPI_STORE; e.C = C; e.ldc = ldc; e.alpha = alpha; e.beta = beta;
-  e.xcur = nullptr; e.ldx = 0; e.perm = nullptr; e.W = nullptr; e.k0 = 0; e.jb = 0;
+  e.xcur = nullptr; e.ldx = 0; e.perm = nullptr; e.k0 = 0; e.jb = 0;
   e.maxabs = nullptr;
   return e;
 }
@@ -301,9 +296,9 @@ __device__ __forceinline__ double flip_sign(double x, unsigned m) {
 // Out-of-line device functions here are kept leaves (none calls another
 // out-of-line function): with a call chain of depth two anywhere in a
 // kernel, the compiler gives every callee the full save/restore calling
-// convention and this loop spills (measured: 30 % slower).  cta_gemm_t is the
-// out-of-line copy for the engine's top level; cta_gemm_body is inlined into
-// the inversion.
+// convention and this loop spills (measured: 30 % slower).  gemm_run and
+// gemm_run_small are the out-of-line copies; the engine's kernel inlines the
+// one for large tiles.
 template <int T>
 __device__ __forceinline__ void cta_gemm_body(const GemmDesc* d, double2* smem) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -543,7 +538,7 @@ __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, cons
 // The operand pipeline runs over the flattened sequence of (output tile,
 // K-tile) steps, so the next output tile's first operands are in flight
 // while the current tile's epilogue runs; K = 16 products are as pipelined
-// as long ones.  One specialisation per operand / epilogue combination.
+// as long ones.  One routine per tile size for every operand and epilogue mode.
 __device__ __forceinline__ void cta_gemm(int M, int N, int K, const Operand& A, const Operand& B, const Epilogue& e,
                                          double2* smem) {
   gemm_run_any(gemm_desc_publish(M, N, K, A, B, e, smem), smem);
@@ -684,7 +679,7 @@ __device__ __forceinline__ double cta_max(double v, double* red) {
 #endif
 constexpr double kInvProbeTol = NEGF_INV_PROBE_TOL;
 
-// The fixed probe vector of cta_inv_probe: v_k = (1 + (k mod 7) / 8) - i (k mod 5) / 8.
+// The fixed probe vector of team_inv_probe: v_k = (1 + (k mod 7) / 8) - i (k mod 5) / 8.
 __device__ __forceinline__ double2 probe_v(int k) { return make_double2(1.0 + 0.125 * (k % 7), -0.125 * (k % 5)); }
 
 // Residual probe of a computed inverse X of A (order n, column major):
@@ -823,7 +818,6 @@ struct InvScratch {
   int* piv;    // n
   int* perm;   // n
   int* cperm;  // n
-  double* redv; int* redi;  // >= 32 each
   int* flag;   // info
   Trace tr;
 };
@@ -841,8 +835,7 @@ __device__ __forceinline__ void warp_argmax_key(unsigned long long& key, int& bi
 }
 
 // Workspace (complex elements) for cta_zinv of order n: two n x n buffers.
-__host__ __device__ inline size_t zinv_ws_elems(int n, int smem_bytes) {
-  (void)smem_bytes;
+__host__ __device__ inline size_t zinv_ws_elems(int n) {
   if (n <= kSmallInvMax) return 0;
   return 2 * (size_t)n * n;
 }
@@ -1543,8 +1536,8 @@ enum InvStep : int { INV_DONE = 0, INV_LEAF = 1, INV_APPLY = 2, INV_ROWS = 3 };
 // Sets up one whole-matrix panel (small orders) or the tree.  No copy of A: a
 // leaf's columns are read from A by the first update that targets them (or,
 // for leaf 0, by its factorisation).
-static __device__ __noinline__ void inv_begin(InvProg& ip, int n, const double2* A, double2* out, double2* ws, double2* smem,
-                                      InvScratch& s) {
+static __device__ __noinline__ void inv_begin(InvProg& ip, int n, const double2* A, double2* out, double2* ws,
+                                              InvScratch& s) {
   if (threadIdx.x == 0) *s.flag = 0;
   __syncthreads();
   ip.A = A; ip.out = out; ip.n = n;
@@ -1661,7 +1654,7 @@ static __device__ __noinline__ int inv_next(InvProg& ip, double2* smem, InvScrat
     Operand Bop{X, n, OP_GATHER, s.perm + j0};
     Epilogue e;
     e.mode = EPI_GJ; e.C = Y; e.ldc = n; e.alpha = make_double2(1, 0); e.beta = make_double2(0, 0);
-    e.xcur = X; e.ldx = n; e.perm = s.perm; e.W = nullptr; e.k0 = j0; e.jb = j1 - j0; e.maxabs = nullptr;
+    e.xcur = X; e.ldx = n; e.perm = s.perm; e.k0 = j0; e.jb = j1 - j0; e.maxabs = nullptr;
     gemm_desc_publish(n, a1 - a0, j1 - j0, Aop, Bop, e, smem);
     if (r == half) { ip.phase = 0; ++ip.k; } else { ++ip.l; }
     return INV_APPLY;
@@ -1712,7 +1705,7 @@ __device__ __forceinline__ void rows_run(const InvProg& ip, double2* smem, const
 __device__ __forceinline__ int cta_zinv(int n, const double2* A, double2* out, double2* ws, double2* smem,
                                         InvScratch& s) {
   InvProg ip;
-  inv_begin(ip, n, A, out, ws, smem, s);
+  inv_begin(ip, n, A, out, ws, s);
   for (;;) {
     const int step = inv_next(ip, smem, s);
     if (step == INV_DONE) break;

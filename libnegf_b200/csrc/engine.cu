@@ -78,13 +78,11 @@ __device__ __noinline__ int zinv_refined(int n, const double2* A, double2* X, do
   return bad;
 }
 
-constexpr unsigned kDecWaveCtas = 296;   // two CTAs on each of a B200's 148 SMs
-
 // Sancho-Rubio decimation (src/contselfenergy.F90:271-340) by one team.
 // In: Ao, Bo, Co in slot 0, 2, 3 (consumed).  Out: surface GF in *go_out
-// (one of the slots).  Returns a status.
+// (one of the slots).  wave: CTAs that run at once.  Returns a status.
 __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int max_iter, int& ncyc, double2** go_out,
-                              SmemMap& sm) {
+                              int wave, SmemMap& sm) {
   double2* Ao = w.slot(0);
   double2* Aos = w.slot(1);
   double2* Go = w.slot(4);
@@ -99,7 +97,7 @@ __device__ __noinline__ int cta_decimation(int L, const Ws& w, double tol, int m
   // the engine's products, side by side in the parts of a team; with more CTAs
   // than run at once the products in vain would cost more than the latency
   // (160 of order 256: 82.8 ms one after another, 85.8 side by side)
-  const int gw = gridDim.x > kDecWaveCtas ? 1 : min(team_size(), 4);
+  const int gw = (int)gridDim.x > wave ? 1 : min(team_size(), 4);
   int ib = 2, ib1 = 11, ic = 3, ic1 = 7;
   auto run = [&](int first, int of) {
     const int size = team_size() / of, rank = team_rank();
@@ -283,7 +281,8 @@ static int resident_teams(int team) {
 //  - the slowdown when the teams share SMs.  Two CTAs on an SM run 1.6 times
 //    as long as one, as soon as any SM has two; teams of 4 and more leave the
 //    FP64 pipe less idle time to share (2.05 times with every SM holding two)
-//    and are placed two to an SM before every SM has one;
+//    and are placed two to an SM before every SM has one.  The numbers of CTAs
+//    at which this sets in were measured on 148 SMs and scale with the SMs;
 //  - the waves.  One or two CTAs per problem wait for the last wave; larger
 //    teams drift apart over the waves and lose less.
 // Examples (us per call, one CTA per problem -> chosen): n = 384, 12 points
@@ -437,7 +436,7 @@ cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, 
 }
 
 // per matrix: the inversion's own buffers, then two n x n refinement buffers
-size_t zinv_batched_work_elems(int n) { return zinv_ws_elems(n, kSmemMain) + 2 * (size_t)n * n; }
+size_t zinv_batched_work_elems(int n) { return zinv_ws_elems(n) + 2 * (size_t)n * n; }
 
 // One team per matrix: the inverses of the problems map[b], b < batch (map
 // null: b), matrices sA / sX complex elements apart; work (may be null where
@@ -452,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int b = blockIdx.x / team_size();
   const int64_t p = map ? map[b] : b;
   double2* wb = work ? work + (int64_t)b * wstride : nullptr;
-  double2* R = work ? wb + zinv_ws_elems(n, kSmemMain) : nullptr;
+  double2* R = work ? wb + zinv_ws_elems(n) : nullptr;
   bool near_sing = false;
   int inf = zinv_refined(n, A + p * sA, X + p * sX, wb, R, R ? R + (int64_t)n * n : nullptr, sm, &near_sing);
   if (lead() && info) info[p] = inf;
@@ -481,7 +480,7 @@ size_t decimation_batched_work_elems(int n) { return dec_work_elems(n); }
 
 __global__ void __launch_bounds__(kThreads, 2)
     k_decimation_batched(int n, const double2* Ao, const double2* Bo, const double2* Co, double2* Go, int* ncyc,
-                         double tol, int max_iter, double2* work) {
+                         double tol, int max_iter, double2* work, int wave) {
   extern __shared__ __align__(16) char smem_raw[];
   SmemMap sm = map_smem(smem_raw, n);
   sm.tr.acc = nullptr;
@@ -498,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   team_sync();
   int nc = 0;
   double2* gs = nullptr;
-  cta_decimation(n, w, tol, max_iter, nc, &gs, sm);
+  cta_decimation(n, w, tol, max_iter, nc, &gs, wave, sm);
   team_copy(Go + b * nn, gs, (int)nn);
   if (lead() && ncyc) ncyc[b] = nc;
   team_sync();   // no member's shared memory is read any more
@@ -510,7 +509,8 @@ cudaError_t launch_decimation_batched(int batch, int n, const double2* Ao, const
   const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
-  return team_launch(cfg, k_decimation_batched, 0, n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work);
+  return team_launch(cfg, k_decimation_batched, 0, n, Ao, Bo, Co, Go, ncyc, tol, max_iter, work,
+                     2 * device_sms());
 }
 
 }  // namespace negf

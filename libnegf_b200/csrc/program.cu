@@ -51,7 +51,7 @@ __device__ int engine_step(const EngineArgs& a, EngineCtl& c, SmemMap& sm) {
       return STEP_GEMM;
     }
     if (o.kind == K_ZINV) {
-      inv_begin(c.ip, o.m, o.A, o.C, w.inv(), sm.main, sm.inv);
+      inv_begin(c.ip, o.m, o.A, o.C, w.inv(), sm.inv);
       c.in_inv = 1;
       continue;
     }

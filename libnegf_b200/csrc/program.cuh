@@ -47,8 +47,6 @@ __device__ __forceinline__ SmemMap map_smem(char* base, int nmax) {
   m.red = reinterpret_cast<double*>(p); p += 32 * sizeof(double);
   m.maxv = reinterpret_cast<double*>(p); p += 2 * sizeof(double);
   m.res = reinterpret_cast<double*>(p); p += 12 * sizeof(double);
-  m.inv.redv = reinterpret_cast<double*>(p); p += 32 * sizeof(double);
-  m.inv.redi = reinterpret_cast<int*>(p); p += 32 * sizeof(int);
   m.inv.flag = reinterpret_cast<int*>(p); p += 4 * sizeof(int);
   m.item = reinterpret_cast<int*>(p); p += 4 * sizeof(int);
   m.ires = reinterpret_cast<int*>(p); p += 4 * sizeof(int);
@@ -62,7 +60,7 @@ __device__ __forceinline__ SmemMap map_smem(char* base, int nmax) {
 }
 
 inline size_t smem_bytes_for(int nmax) {
-  return kSmemMain + 32 * 8 + 2 * 8 + 12 * 8 + 32 * 8 + 32 * 4 + 4 * 4 + 4 * 4 + 4 * 4 + 3 * (size_t)nmax * 4 + 8 +
+  return kSmemMain + 32 * 8 + 2 * 8 + 12 * 8 + 4 * 4 + 4 * 4 + 4 * 4 + 3 * (size_t)nmax * 4 + 8 +
          TR_NPHASE * 8;
 }
 
@@ -118,7 +116,7 @@ enum OpKind : int {
   K_LDOS,      // out[k] = sum over LDOS set k of dos[i-1] (A = dos row as doubles, device sets)
   K_ACCUM,     // C[q] += alpha * A[q], q < m (atomic: C is shared by all CTAs)
   K_SUBCOPY,   // C(flag + r, flag + c) = A(r, c), A m x m, C leading dimension ldc
-  K_RESPROBE,  // res[slot] = max_i |(A (B v))_i - v_i|, res[8] = the condition estimate, order m (cta_inv_probe)
+  K_RESPROBE,  // res[slot] = max_i |(A (B v))_i - v_i|, res[8] = the condition estimate, order m (team_inv_probe)
   K_EYE,       // C = identity, order m
   K_RETCHECK,  // res[slot] = min_i s Im A_ii / max_i |A_ii|, order m, s = -sign of the energy's imaginary part
   K_RELDIFF,   // res[slot] = max |A(q) - B(q)| / max |B(q)|, m elements

@@ -248,8 +248,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     sh.inv.perm = sh.perm;
     sh.inv.cperm = sh.cperm;
     sh.inv.flag = &sh.flag;
-    sh.inv.redv = nullptr;
-    sh.inv.redi = nullptr;
     sh.inv.tr.acc = nullptr;
   }
   for (int q = threadIdx.x; q < kBlocks * kBlk; q += kThreads) Ao[q] = make_double2(0.0, 0.0);
