@@ -247,8 +247,10 @@ cudaError_t launch_engine(const EngineArgs& a, int teams, int team, cudaStream_t
   return team_launch(team_config(teams, team, engine_smem_bytes(a.nmax), s, &attr), k_engine, 0, a);
 }
 
-// Clusters of `team` CTAs of the engine that run at once on the current
-// device (0: none), queried once per device and size.
+// Clusters of `team` CTAs that run at once on the current device (0: none),
+// queried once per device and size.  Asked of the engine, and taken for the
+// inverse and the decimation too: all have two CTAs to an SM, of the same
+// threads, registers and shared memory.
 static int resident_teams(int team) {
   static std::mutex mu;
   static int known[64][5];   // count + 1
@@ -257,15 +259,19 @@ static int resident_teams(int team) {
   while ((1 << lg) < team) ++lg;
   std::lock_guard<std::mutex> lk(mu);
   if (known[dev][lg] == 0) {
-    int n = 0;
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = team_config(1, team, engine_smem_bytes(kMaxOrder), nullptr, &attr);
-    if (team_opt_in((const void*)k_engine) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, k_engine, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
+    for (int attempt = 0; attempt < 2; ++attempt) {   // again with the limits raised afresh (see team_launch)
+      int n = 0;
+      cudaError_t e = team_opt_in((const void*)k_engine);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, k_engine, &cfg);
+      if (e == cudaSuccess) {
+        known[dev][lg] = n + 1;
+        break;
+      }
+      team_opt_out((const void*)k_engine);
     }
-    known[dev][lg] = n + 1;
+    if (known[dev][lg] == 0) return 0;   // asked again by the next call
   }
   return known[dev][lg] - 1;
 }
