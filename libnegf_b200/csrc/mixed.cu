@@ -99,7 +99,7 @@ __global__ void k_dec_check(int na, const int* list, double* mx, int* ok, int* n
     if (!(m <= 1.7976931348623157e308)) {   // Inf / NaN: this decimation will not converge; run it again
       go = false;
       ncyc_c[p] = it;
-      redo[p] = 1;
+      redo[p] = 2;
     } else if (m <= tol) {
       if (ok[p]) {
         go = false;
@@ -323,7 +323,8 @@ __global__ void k_agree(int64_t nn, const int* map, const double2* gs, const dou
   double d = 0.0, m = 0.0;
   for (int64_t q = threadIdx.x; q < nn; q += blockDim.x) {
     const double2 a = gs[p * Q + q], b = kept[p * Q + q];
-    d = fmax(d, hypot(a.x - b.x, a.y - b.y));
+    const double h = hypot(a.x - b.x, a.y - b.y);
+    if (!(h <= d)) d = h > d ? h : __longlong_as_double(0x7ff0000000000000LL);   // NaN agrees with nothing
     m = fmax(m, hypot(b.x, b.y));
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -527,7 +528,8 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
       // in lock step.
       // Decimation of the problems sub[b], b < nsub (sub null: all N), the
       // contact energy scaled by `scale`; then gs = Aos^-1 and the
-      // retarded-branch check (redo[p] = 1 where it fails)
+      // retarded-branch check (redo[p] = 1 where it fails, 2 where only the
+      // iteration ran off)
       auto decimate = [&](const int* sub, int nsub, double scale) -> int {
         double2 *Ao = B[0], *Aos = B[1], *Bo = B[2], *Co = B[3], *Go = B[4], *X = B[5], *C1 = B[6], *Y = B[7],
                 *B1 = B[8];
@@ -615,7 +617,13 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
           again.clear();
           keep.clear();
           for (int p : cur_sub) {
-            if (hredo[p]) { again.push_back(p); continue; }                  // wrong fixed point: run again
+            if (hredo[p]) {                                                   // wrong fixed point: run again
+              again.push_back(p);
+              // ran off, with a gs on the right branch: none to accept, but one
+              // that a converged attempt may agree with
+              if (hredo[p] == 2 && !kept[p]) keep.push_back(p);
+              continue;
+            }
             if (!hsens[p]) continue;                                          // settled
             if (kept[p] && hagree[p]) continue;                               // two attempts agree
             keep.push_back(p);                                                // keep this gs, run again

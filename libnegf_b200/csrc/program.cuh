@@ -378,7 +378,8 @@ __device__ __forceinline__ void exec_light(const Op& o, SmemMap& sm) {
     case K_RELDIFF: {
       double d = 0.0, b = 0.0;
       for (int q = tid; q < o.m; q += blockDim.x) {
-        d = fmax(d, cabs(csub(o.A[q], o.B[q])));
+        const double h = cabs(csub(o.A[q], o.B[q]));
+        if (!(h <= d)) d = h > d ? h : __longlong_as_double(0x7ff0000000000000LL);   // NaN agrees with nothing
         b = fmax(b, cabs(o.B[q]));
       }
       d = cta_max(d, sm.red);
@@ -647,9 +648,17 @@ dispatch:
           o.kind = K_RETCHECK; o.m = s.L; o.A = w.slot(4); o.slot = 6; o.scal = (s.ecs.y > 0.0) ? -1.0 : 1.0;
           PT_EMIT(s);
           // a converged fixed point of the wrong kind, or an iteration that ran off to Inf / NaN
-          const bool wrong = (s.done && !(sm.res[6] >= -kRetardedTol)) || s.diverged ||
+          const bool off = !(sm.res[6] >= -kRetardedTol);   // another branch, or not finite
+          const bool wrong = (s.done && off) || s.diverged ||
                              sm.res[6] == -__longlong_as_double(0x7ff0000000000000LL);
           if (wrong && s.att < kDecRetries) {
+            // an iteration that ran off late can leave a gs on the right branch:
+            // none to accept, but one that a converged attempt may agree with
+            if (s.diverged && !off && !s.kept) {
+              set_simple(o, K_COPY, s.L * s.L, w.slot(4), w.slot(10));
+              PT_EMIT(s);
+              s.kept = 1;
+            }
             ++s.att;
             goto decimation_attempt;
           }

@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       load_esh(n, Co, h01, s01, cconj(ec), false, true);
       __syncthreads();
       Frag Aos = get(L, Ao);
-      bool ok = false, done = false, sens = false, redo = false;
+      bool ok = false, done = false, sens = false, diverged = false, off = false;
       cyc = 0;
       int it = 1;
 #pragma unroll 1
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
           }
         mx = cta_max_nan(bad ? __longlong_as_double(0x7ff8000000000000LL) : mx, sh.red[2]);
         if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge
-          redo = done = true;
+          diverged = done = true;
         } else if (mx <= a.sgf_tol) {
           done = ok;
           ok = true;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       sens |= (bad_gs & 2) != 0;
       __syncthreads();
       if (a.eta == 0.0) {   // no other branch to try; gs of an iteration broken off means nothing
-        if (redo) {
+        if (diverged) {
           cyc = a.sgf_max_iter + 1;
           put_st(NEGF_B200_ERR_NOT_CONVERGED);
         }
@@ -351,21 +351,27 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       for (int i = 0; i < n; ++i) {
         const double2 g = Go[i * (kLd + 1)];
         const double h = cabs(g);
-        if (!(h <= 1.7976931348623157e308)) redo = true;
+        if (!(h <= 1.7976931348623157e308)) off = true;
         else {
           lo = fmin(lo, sgn * g.y);
           hi = fmax(hi, h);
         }
       }
-      if (hi > 0.0 && lo < -1e-6 * hi) redo = true;
-      if (!redo && !sens) break;
-      if (!redo) {   // sensitive: accepted once two attempts reach the same gs
+      if (hi > 0.0 && lo < -1e-6 * hi) off = true;
+      if (!diverged && !off && !sens) break;
+      if (diverged) {   // none to accept, but one that a converged attempt may agree with
+        if (!off && !have) {
+          kept = get(L, Go);
+          have = true;
+        }
+      } else if (!off) {   // sensitive: accepted once two attempts reach the same gs
         const Frag gs = get(L, Go);
         if (have) {
           double df = 0.0, mk = 0.0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            df = fmax(df, cabs(csub(gs.v[q], kept.v[q])));
+            const double h = cabs(csub(gs.v[q], kept.v[q]));
+            if (!(h <= df)) df = h > df ? h : __longlong_as_double(0x7ff0000000000000LL);
             mk = fmax(mk, cabs(kept.v[q]));
           }
           df = cta_max_nan(df, sh.red[0]);
