@@ -310,7 +310,7 @@ __global__ void k_dec_start(int nsub, const int* map, int* ok, double* mx, int* 
   }
 }
 
-// kept_p = gs_p for the points map[b], b < nsub; one CTA per point.
+// kept_p = gs_p (or back) for the points map[b], b < nsub; one CTA per point.
 __global__ void k_keep(int64_t nn, const int* map, const double2* gs, double2* kept, int64_t Q) {
   const int p = map[blockIdx.x];
   for (int64_t q = threadIdx.x; q < nn; q += blockDim.x) kept[p * Q + q] = gs[p * Q + q];
@@ -598,16 +598,21 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
         // again, in lock step over just those problems, from the contact energy times
         // 1 + k 2^-50.  A sensitive decimation (one of its inverses needed a Newton
         // step: a nearly singular Ao) is accepted once two attempts reach the same gs.
-        std::vector<int> hredo(N), hsens(N), hagree(N), kept(N, 0), cur_sub, again, cmp, keep;
+        // An attempt that ran off (redo 2) with a gs on the right branch is none to
+        // accept, but one to agree with a converged attempt's, kept before or still
+        // to come.  kept: 1 a converged attempt's gs, of kept_nc iterations, 2 any
+        // other's.
+        std::vector<int> hredo(N), hsens(N), hagree(N), hnc(N), kept(N, 0), kept_nc(N), cur_sub, again, cmp, keep, take;
         cur_sub.resize(N);
         for (int p = 0; p < N; ++p) cur_sub[p] = p;
         for (int att = 1;; ++att) {
           MCK(cudaMemcpyAsync(hredo.data(), w.redo, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "redo");
           MCK(cudaMemcpyAsync(hsens.data(), w.sens, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "sens");
+          MCK(cudaMemcpyAsync(hnc.data(), nc, sizeof(int) * N, cudaMemcpyDeviceToHost, s), "ncyc");
           MCK(cudaStreamSynchronize(s), "sync");
           cmp.clear();
           for (int p : cur_sub)
-            if (!hredo[p] && hsens[p] && kept[p]) cmp.push_back(p);
+            if (kept[p] && ((!hredo[p] && hsens[p]) || (hredo[p] == 2 && kept[p] == 1))) cmp.push_back(p);
           if (!cmp.empty()) {
             MCK(cudaMemcpyAsync(w.sub, cmp.data(), sizeof(int) * cmp.size(), cudaMemcpyHostToDevice, s), "cmp");
             k_agree<<<(int)cmp.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q, 1e-2, w.agree); ++nl;
@@ -616,11 +621,16 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
           }
           again.clear();
           keep.clear();
+          take.clear();
           for (int p : cur_sub) {
+            if (hredo[p] == 2 && kept[p] == 1 && hagree[p]) {                 // the kept gs is accepted
+              take.push_back(p);
+              hredo[p] = 0;
+              hnc[p] = kept_nc[p];
+              continue;
+            }
             if (hredo[p]) {                                                   // wrong fixed point: run again
               again.push_back(p);
-              // ran off, with a gs on the right branch: none to accept, but one
-              // that a converged attempt may agree with
               if (hredo[p] == 2 && !kept[p]) keep.push_back(p);
               continue;
             }
@@ -628,6 +638,12 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
             if (kept[p] && hagree[p]) continue;                               // two attempts agree
             keep.push_back(p);                                                // keep this gs, run again
             again.push_back(p);
+          }
+          if (!take.empty()) {
+            MCK(cudaMemcpyAsync(w.sub, take.data(), sizeof(int) * take.size(), cudaMemcpyHostToDevice, s), "take");
+            k_keep<<<(int)take.size(), 256, 0, s>>>(Q, w.sub, kept_gs, gs, Q); ++nl;
+            MCK(cudaMemcpyAsync(nc, hnc.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s), "ncyc");
+            MCK(cudaStreamSynchronize(s), "sync");
           }
           if (again.empty()) break;
           if (att > kDecRetries) {
@@ -641,7 +657,10 @@ int mixed_run(const MixedArgs& a, void* ws, int batch, bool one_contact, cudaStr
           if (!keep.empty()) {
             MCK(cudaMemcpyAsync(w.sub, keep.data(), sizeof(int) * keep.size(), cudaMemcpyHostToDevice, s), "keep");
             k_keep<<<(int)keep.size(), 256, 0, s>>>(Q, w.sub, gs, kept_gs, Q); ++nl;
-            for (int p : keep) kept[p] = 1;
+            for (int p : keep) {
+              kept[p] = hredo[p] == 2 || hnc[p] > a.sgf_max_iter ? 2 : 1;
+              kept_nc[p] = hnc[p];
+            }
           }
           MCK(cudaMemcpyAsync(w.sub, again.data(), sizeof(int) * again.size(), cudaMemcpyHostToDevice, s), "sub");
           MCK(cudaMemsetAsync(w.redo, 0, sizeof(int) * N, s), "memset redo");

@@ -415,7 +415,9 @@ struct Prog {
   int att;              // decimation attempt (retarded-branch retries)
   int diverged;         // the attempt's max|C1| went Inf / NaN
   int sens;             // the attempt met a nearly singular Ao (condition estimate above kSensitiveCond)
-  int kept;             // a previous sensitive attempt's gs is kept for comparison
+  int kept;             // an attempt's gs is kept for comparison: 1 a sensitive one's that converged, 2 any other's
+  int kit;              // iterations of the kept attempt
+  int off, wrong;       // the attempt's gs is on another branch or not finite; the attempt cannot be accepted
   int in_dec;           // inside a decimation (refinements mark it sensitive)
   double2 ecd;          // contact energy of the attempt
   // inverse refinement (the `refine` block): matrix, its computed inverse, order, return point
@@ -648,25 +650,37 @@ dispatch:
           o.kind = K_RETCHECK; o.m = s.L; o.A = w.slot(4); o.slot = 6; o.scal = (s.ecs.y > 0.0) ? -1.0 : 1.0;
           PT_EMIT(s);
           // a converged fixed point of the wrong kind, or an iteration that ran off to Inf / NaN
-          const bool off = !(sm.res[6] >= -kRetardedTol);   // another branch, or not finite
-          const bool wrong = (s.done && off) || s.diverged ||
-                             sm.res[6] == -__longlong_as_double(0x7ff0000000000000LL);
-          if (wrong && s.att < kDecRetries) {
-            // an iteration that ran off late can leave a gs on the right branch:
-            // none to accept, but one that a converged attempt may agree with
-            if (s.diverged && !off && !s.kept) {
+          s.off = !(sm.res[6] >= -kRetardedTol);   // another branch, or not finite
+          s.wrong = (s.done && s.off) || s.diverged ||
+                    sm.res[6] == -__longlong_as_double(0x7ff0000000000000LL);
+          // an iteration that ran off late can leave a gs on the right branch:
+          // none to accept, but one to agree with a converged attempt's, kept
+          // before or still to come
+          if (s.diverged && !s.off && s.kept == 1) {
+            o.kind = K_RELDIFF; o.m = s.L * s.L; o.A = w.slot(4); o.B = w.slot(10); o.slot = 5;
+            PT_EMIT(s);
+            if (sm.res[5] <= 1e-2) {
+              set_simple(o, K_COPY, s.L * s.L, w.slot(10), w.slot(4));
+              PT_EMIT(s);
+              s.it = s.kit;
+              s.done = 1;
+              goto dec_settled;
+            }
+          }
+          if (s.wrong && s.att < kDecRetries) {
+            if (s.diverged && !s.off && !s.kept) {
               set_simple(o, K_COPY, s.L * s.L, w.slot(4), w.slot(10));
               PT_EMIT(s);
-              s.kept = 1;
+              s.kept = 2;
             }
             ++s.att;
             goto decimation_attempt;
           }
-          if (wrong) s.done = 0;   // no retarded solution reached: NOT_CONVERGED
+          if (s.wrong) s.done = 0;   // no retarded solution reached: NOT_CONVERGED
           // a sensitive decimation (one of its inverses needed refinement) is accepted once
           // two attempts reach the same gs: a fixed point other than the retarded one can
           // pass the diagonal test, and the retarded one is the common outcome
-          if (!wrong && s.sens) {
+          if (!s.wrong && s.sens) {
             if (s.kept) {
               o.kind = K_RELDIFF; o.m = s.L * s.L; o.A = w.slot(4); o.B = w.slot(10); o.slot = 5;
               PT_EMIT(s);
@@ -675,7 +689,8 @@ dispatch:
               if (s.att < kDecRetries) {
                 set_simple(o, K_COPY, s.L * s.L, w.slot(4), w.slot(10));
                 PT_EMIT(s);
-                s.kept = 1;
+                s.kept = s.done ? 1 : 2;
+                s.kit = s.it;
                 ++s.att;
                 goto decimation_attempt;
               }
@@ -683,6 +698,7 @@ dispatch:
             }
           }
         }
+      dec_settled:
         s.in_dec = 0;
         if (!s.done) put_status(s.st, ST_NOT_CONVERGED);
         s.ncyc += s.done ? s.it : a.sgf_max_iter + 1;

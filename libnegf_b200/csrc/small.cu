@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     const double2* s00 = d.has_s00 ? d.s00 + d.olead[c] : nullptr;
     const double2* s01 = d.has_s01 ? d.s01 + d.olead[c] : nullptr;
     int cyc = 0;
-    bool have = false;                           // a sensitive attempt's gs is kept for comparison
+    int have = 0;                                // an attempt's gs is kept: 1 one's that converged, 2 any other's
+    int kept_cyc = 0;
     Frag kept;
 #pragma unroll 1
     for (int att = 0;; ++att) {
@@ -359,14 +360,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       }
       if (hi > 0.0 && lo < -1e-6 * hi) off = true;
       if (!diverged && !off && !sens) break;
-      if (diverged) {   // none to accept, but one that a converged attempt may agree with
-        if (!off && !have) {
-          kept = get(L, Go);
-          have = true;
-        }
-      } else if (!off) {   // sensitive: accepted once two attempts reach the same gs
+      // sensitive: accepted once two attempts reach the same gs.  An attempt that
+      // ran off with a gs on the right branch is none to accept, but one to
+      // agree with a converged attempt's, kept before or still to come
+      if (!off) {
         const Frag gs = get(L, Go);
-        if (have) {
+        if (have == 1 || (have == 2 && !diverged)) {
           double df = 0.0, mk = 0.0;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -377,11 +376,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
           df = cta_max_nan(df, sh.red[0]);
           mk = cta_max_nan(mk, sh.red[1]);
           __syncthreads();
-          if (df <= 1e-2 * mk) break;
+          if (df <= 1e-2 * mk) {
+            if (diverged) {
+              put(L, Go, kept);
+              cyc = kept_cyc;
+            }
+            break;
+          }
         }
-        if (att < kDecRetries) {
+        if (att < kDecRetries && (!diverged || !have)) {
           kept = gs;
-          have = true;
+          have = diverged || !done ? 2 : 1;
+          kept_cyc = cyc;
         }
       }
       if (att >= kDecRetries) {
