@@ -308,6 +308,25 @@ int plan_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh, b
   return NEGF_B200_OK;
 }
 
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Whether the device has `need` bytes with the workspace in place given back.
+bool could_grow(const negf_b200_ctx* ctx, size_t need) {
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return free_bytes + ctx->ws_bytes >= need;
+}
+
 // Makes room for an engine call to come, where it can be had: the workspace
 // in place is given up only for the larger one, and nothing is reported.
 void reserve_engine(negf_b200_ctx* ctx, int mode, int npts, const LaunchShape& sh) {
@@ -334,6 +353,14 @@ int run_device(negf_b200_ctx* ctx, negf::EngineArgs a, const LaunchShape& sh, cu
   st = sync_descs(ctx);
   if (st) return st;
   const std::string before = ctx->err;
+  if (pl.split && pl.need > ctx->ws_bytes) {
+    // a workspace in place that holds whole points is not given up for one that
+    // cannot be had: under stream capture, or with too little free memory
+    EnginePlan whole;
+    if (plan_engine(ctx, a.mode, a.npts, sh, a.acc_lc != nullptr, whole, false) == NEGF_B200_OK &&
+        whole.need <= ctx->ws_bytes && (capturing(s) || !could_grow(ctx, pl.need)))
+      pl = whole;
+  }
   st = grow(ctx, &ctx->ws, &ctx->ws_bytes, pl.need);
   if (st && pl.split) {   // whole points in one launch need less: no blocks between launches
     st = plan_engine(ctx, a.mode, a.npts, sh, a.acc_lc != nullptr, pl, false);
@@ -1171,12 +1198,7 @@ static bool lockstep_choice(negf_b200_ctx* ctx, int32_t npts, const int32_t* h_i
   const char* form = mixed ? "the mixed form (precision != 0)" : "lock step (schedule 2)";
   // the mixed form reads the decimation's active count back to the host, which a
   // stream capture cannot hold; the engine takes captured calls at small orders too
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
-    cudaGetLastError();
-    cap = cudaStreamCaptureStatusNone;
-  }
-  if (cap != cudaStreamCaptureStatusNone) {
+  if (capturing(stream)) {
     if (!forced) return false;
     *st = fail(ctx, NEGF_B200_ERR_BAD_ARG, std::string(form) + " cannot run under stream capture");
     return true;

@@ -1,5 +1,7 @@
 """The engine's workspace when there is little of it: a limit set by the
 caller, or a device that is nearly full."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -66,6 +68,50 @@ def test_a_call_runs_where_only_its_whole_points_fit():
             del fill
             torch.cuda.empty_cache()
     assert np.array_equal(Tl[:20], T) and np.array_equal(nl[:20], nc) and np.all(sl == 0)
+
+
+def test_a_captured_call_takes_the_workspace_in_place():
+    """The same device: after an eager call a captured one, whose split plan
+    would need to grow the workspace, runs whole points in the one in place."""
+    torch = pytest.importorskip("torch")
+    n, nbl, npts = 128, 2, 1000
+    per, blocks = _layout(n, nbl, npts)
+    whole = 2 * torch.cuda.get_device_properties(0).multi_processor_count * per
+    E = np.linspace(-1.0, 1.0, npts)
+    L = native.load()
+    torch.cuda.empty_cache()
+    with native.Context(0) as ctx:
+        h = ctx.upload(G.transport_c0(nbl=nbl, n=n, seed=3))
+        d_ids = torch.full((npts,), h, dtype=torch.int32, device="cuda")
+        d_E = torch.from_numpy(E).cuda()
+        d_T = torch.zeros(npts, dtype=torch.float64, device="cuda")
+        d_nc, d_st = torch.zeros((2, npts), dtype=torch.int32, device="cuda")
+        s = torch.cuda.Stream()
+
+        def call():
+            return L.negf_b200_transmission_dev(ctx.handle, npts, d_ids.data_ptr(), d_E.data_ptr(), 1e-3, 1, 2,
+                                                d_T.data_ptr(), d_nc.data_ptr(), d_st.data_ptr(),
+                                                ctypes.c_void_p(s.cuda_stream))
+
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - whole - blocks // 2, dtype=torch.uint8, device="cuda")
+        try:
+            assert call() == 0
+            s.synchronize()
+            T, nc = d_T.cpu().numpy(), d_nc.cpu().numpy()
+            d_T.zero_()
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                rc = call()
+            assert rc == 0
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(d_T.cpu().numpy(), T) and np.array_equal(d_nc.cpu().numpy(), nc)
+            assert not bool(d_st.any())
+            del g
+        finally:
+            del fill
+            torch.cuda.empty_cache()
 
 
 def test_a_call_that_succeeds_leaves_no_message(gpu_ctx):
