@@ -986,7 +986,8 @@ __device__ __forceinline__ void gj_reg_steps(double2 (&x)[R][W], int n, int c0, 
 
 // Gauss-Jordan elimination of the columns [c0, c0 + w) of a column-major
 // matrix of n <= 32 RL rows, the panel in registers: lane l of every warp
-// holds rows l + 32 r (r < RL) of the CW panel columns wp + 8 c, w <= 8 CW.
+// holds rows l + 32 r (r < RL) of the CW panel columns wp + NW c, w <= NW CW
+// (NW warps in the CTA).
 // src / dst point at the panel's first column (they may be the same).  Rows
 // never move between registers: lg[r] is the position a row has after the
 // exchanges so far (every warp keeps it), and the rows go there when the
@@ -1016,7 +1017,7 @@ __device__ __forceinline__ void gj_reg_steps(double2 (&x)[R][W], int n, int c0, 
 // instruction cache for a third of the time.
 //
 // WHOLE: the panel is the whole matrix (w = n): the columns also go to their
-// places, so dst gets the inverse.  scratch: 3 * 32 RL + 8 CW + 4 elements of
+// places, so dst gets the inverse.  scratch: 3 * 32 RL + NW CW + 4 elements of
 // shared memory (a pointer the compiler can trace to it: with generic
 // accesses a step's stores and loads wait for one another).
 struct PanelPivot {
@@ -1037,10 +1038,10 @@ __device__ __forceinline__ void unroll_steps(F& f) {
   }
 }
 
-template <int RL, int CW, bool WHOLE>
+template <int RL, int CW, bool WHOLE, int NW = kThreads / 32>
 __device__ __forceinline__ void gj_panel(const double2* src, int lds, double2* dst, int ldd, int n, int c0, int w,
                                          double2* scratch, InvScratch& s) {
-  constexpr int NR = 32 * RL, NW = kThreads / 32;
+  constexpr int NR = 32 * RL;
   constexpr bool kScaleRow = RL > CW;   // scale the row's CW entries by d, else the column's RL
   constexpr unsigned kAll = 0xffffffffu;
   double2* const colb = scratch;                                          // [3][NR]

@@ -23,12 +23,25 @@
 namespace negf {
 namespace {
 
-// Blocks lie in shared memory column major with 34 rows per column: 2 modulo
-// 8 elements, so that the eight lanes of a 128-byte phase of a fragment load
-// hit different banks, for the left operand with lane (g, t) on row g of
-// column t and for the right one with columns taken in the order of ncol().
-constexpr int kLd = 34, kBlk = 32 * kLd;
+// The kernel for orders up to M (32 or 16).  Blocks lie in shared memory column
+// major with M + 2 rows per column: 2 modulo 8 elements, so that the eight lanes
+// of a 128-byte phase of a fragment load hit different banks, for the left
+// operand with lane (g, t) on row g of column t and for the right one with
+// columns taken in the order of ncol().  Orders up to 16 have work for two of
+// eight warps in a product and for one row per lane of 16 in a panel, and half
+// the threads let four CTAs share an SM instead of two: 9000 energies of a
+// 10-layer device of order 1, 8 and 16 take 3.8, 6.6 and 12.5 ms (8.3, 12.9 and
+// 20.5 with the shape of order 32; 7.5, 11.9 and 20.6 with one warp per point
+// and block operation, every operation a launch).
 constexpr int kBlocks = 6;
+template <int M>
+struct Shape {
+  static constexpr int kCta = M == 32 ? kThreads : kThreads / 2;   // threads
+  static constexpr int kPerSm = M == 32 ? 2 : 4;                   // CTAs that share an SM
+  static constexpr int kLd = M + 2, kBlk = M * kLd;
+  static constexpr int kWarps = kCta / 32;
+  static constexpr size_t kScratch = 3 * 32 + kWarps * 4 + 4;      // gj_panel<1, 4>
+};
 constexpr unsigned kFull = 0xffffffffu;
 
 struct SmallShared {
@@ -37,27 +50,36 @@ struct SmallShared {
   double red[3][8];
   double2 y[32];
 };
-constexpr size_t kScratchElems = 3 * 32 + 8 * 4 + 4;   // gj_panel<1, 4>
-constexpr size_t kSmallSmem = (kBlocks * kBlk + kScratchElems) * sizeof(double2) + sizeof(SmallShared);
+template <int M>
+constexpr size_t small_smem() {
+  return (kBlocks * Shape<M>::kBlk + Shape<M>::kScratch) * sizeof(double2) + sizeof(SmallShared);
+}
 
 // The dynamic shared memory, named wherever it is used so that accesses
 // compile to shared-memory instructions: blocks, panel scratch, the rest.
 extern __shared__ __align__(16) char smem_raw[];
 enum Block : int { B_AO = 0, B_BO = 1, B_CO = 2, B_GO = 3, B_X = 4, B_SL = 5 };
-__device__ __forceinline__ double2* block(int b) { return reinterpret_cast<double2*>(smem_raw) + b * kBlk; }
+template <int M>
+__device__ __forceinline__ double2* block(int b) {
+  return reinterpret_cast<double2*>(smem_raw) + b * Shape<M>::kBlk;
+}
+template <int M>
 __device__ __forceinline__ SmallShared& shared() {
-  return *reinterpret_cast<SmallShared*>(reinterpret_cast<double2*>(smem_raw) + kBlocks * kBlk + kScratchElems);
+  return *reinterpret_cast<SmallShared*>(reinterpret_cast<double2*>(smem_raw) + kBlocks * Shape<M>::kBlk +
+                                         Shape<M>::kScratch);
 }
 
 __device__ __forceinline__ int ncol(int g) { return (g & 4) | ((g & 1) << 1) | ((g & 2) >> 1); }
 
-// A thread's four elements of a 32 x 32 product (the fragment layout of
+// A thread's four elements of an M x M product (the fragment layout of
 // dmma_16x8x4): element q at (row(q), col(q)); rows and columns from n on
 // are not part of the block.
 struct Frag {
   double2 v[4];
 };
+template <int M>
 struct Lane {
+  static constexpr int kLd = Shape<M>::kLd;
   int n, g, t, m0, n0;
   __device__ __forceinline__ explicit Lane(int order) : n(order) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -73,8 +95,10 @@ struct Lane {
 };
 
 // A B, on the FP64 tensor pipe; entries of A and B from n on are zero.
-__device__ __forceinline__ Frag mm(const Lane& L, const double2* A, const double2* B) {
+template <int M>
+__device__ __forceinline__ Frag mm(const Lane<M>& L, const double2* A, const double2* B) {
   double re[4] = {0.0, 0.0, 0.0, 0.0}, im[4] = {0.0, 0.0, 0.0, 0.0};
+  constexpr int kLd = Shape<M>::kLd;
   if (L.m0 < L.n && L.n0 < L.n) {
     const double2* pa = A + L.t * kLd + L.m0 + L.g;
     const double2* pb = B + (L.n0 + ncol(L.g)) * kLd + L.t;
@@ -92,19 +116,22 @@ __device__ __forceinline__ Frag mm(const Lane& L, const double2* A, const double
   for (int q = 0; q < 4; ++q) f.v[q] = make_double2(re[q], im[q]);
   return f;
 }
-__device__ __forceinline__ void put(const Lane& L, double2* D, const Frag& f) {
+template <int M>
+__device__ __forceinline__ void put(const Lane<M>& L, double2* D, const Frag& f) {
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     if (L.in(q)) D[L.at(q)] = f.v[q];
 }
-__device__ __forceinline__ Frag get(const Lane& L, const double2* S) {
+template <int M>
+__device__ __forceinline__ Frag get(const Lane<M>& L, const double2* S) {
   Frag f;
 #pragma unroll
   for (int q = 0; q < 4; ++q) f.v[q] = L.in(q) ? S[L.at(q)] : make_double2(0.0, 0.0);
   return f;
 }
 // get() from the shared memory of another CTA of the cluster
-__device__ __forceinline__ Frag team_get(const Lane& L, const double2* S, int rank) {
+template <int M>
+__device__ __forceinline__ Frag team_get(const Lane<M>& L, const double2* S, int rank) {
   Frag f;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -113,7 +140,8 @@ __device__ __forceinline__ Frag team_get(const Lane& L, const double2* S, int ra
   }
   return f;
 }
-__device__ __forceinline__ void sub_from(const Lane& L, double2* D, const Frag& f) {
+template <int M>
+__device__ __forceinline__ void sub_from(const Lane<M>& L, double2* D, const Frag& f) {
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     if (L.in(q)) D[L.at(q)] = csub(D[L.at(q)], f.v[q]);
@@ -121,6 +149,7 @@ __device__ __forceinline__ void sub_from(const Lane& L, double2* D, const Frag& 
 
 // Maximum of v over the CTA (NaN in any thread: NaN); red: 8 doubles.  Ends
 // with a barrier before red is next written (the callers' own barriers).
+template <int M>
 __device__ __forceinline__ double cta_max_nan(double v, double* red) {
   bool bad = !(v <= 1.7976931348623157e308);
 #pragma unroll
@@ -130,7 +159,7 @@ __device__ __forceinline__ double cta_max_nan(double v, double* red) {
   __syncthreads();
   double m = red[0];
 #pragma unroll
-  for (int w = 1; w < kThreads / 32; ++w) m = (m != m || red[w] != red[w]) ? m + red[w] : fmax(m, red[w]);
+  for (int w = 1; w < Shape<M>::kWarps; ++w) m = (m != m || red[w] != red[w]) ? m + red[w] : fmax(m, red[w]);
   return m;
 }
 
@@ -138,16 +167,18 @@ __device__ __forceinline__ double cta_max_nan(double v, double* red) {
 // Go + Go (I - Ao Go) where it exceeds kInvProbeTol (in the X block).
 // Returns 1 for an exactly zero pivot, + 2 where the condition estimate of Ao
 // exceeds kSensitiveCond.
+template <int M>
 __device__ __noinline__ int small_inverse(int n) {
-  const Lane L(n);
-  const double2* const A = block(B_AO);
-  double2* const X = block(B_GO);
-  double2* const R = block(B_X);
-  SmallShared& sh = shared();
+  constexpr int kLd = Shape<M>::kLd;
+  const Lane<M> L(n);
+  const double2* const A = block<M>(B_AO);
+  double2* const X = block<M>(B_GO);
+  double2* const R = block<M>(B_X);
+  SmallShared& sh = shared<M>();
   bool sens = false;
   if (threadIdx.x == 0) sh.flag = 0;
   __syncthreads();
-  gj_panel<1, 4, true>(A, kLd, X, kLd, n, 0, n, block(kBlocks), sh.inv);
+  gj_panel<1, 4, true, Shape<M>::kWarps>(A, kLd, X, kLd, n, 0, n, block<M>(kBlocks), sh.inv);
   const int info = sh.flag != 0 ? 1 : 0;
   // probe: threads (row, group of columns) = (tid / 8, tid mod 8)
   const int r = threadIdx.x >> 3, grp = threadIdx.x & 7;
@@ -197,7 +228,7 @@ __device__ __noinline__ int small_inverse(int n) {
     __syncthreads();
     double em = 0.0, km = 0.0;
 #pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) {
+    for (int w = 0; w < Shape<M>::kWarps; ++w) {
       em = fmax(em, sh.red[0][w]);
       km = fmax(km, sh.red[1][w]);
     }
@@ -221,9 +252,11 @@ __device__ __noinline__ int small_inverse(int n) {
 
 // D = z S - H (S null: the identity if diag, else zero) for an n x n block
 // in memory; with dag its conjugate transpose.
+template <int M>
 __device__ __forceinline__ void load_esh(int n, double2* D, const double2* H, const double2* S, double2 z, bool diag,
                                          bool dag) {
-  for (int q = threadIdx.x; q < n * n; q += kThreads) {
+  constexpr int kLd = Shape<M>::kLd;
+  for (int q = threadIdx.x; q < n * n; q += Shape<M>::kCta) {
     const int i = q % n, j = q / n;
     const double2 s = S ? S[q] : make_double2(diag && i == j ? 1.0 : 0.0, 0.0);
     const double2 v = csub(cmul(z, s), H[q]);
@@ -232,17 +265,19 @@ __device__ __forceinline__ void load_esh(int n, double2* D, const double2* H, co
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
-  double2* const Ao = block(B_AO);
-  double2* const Bo = block(B_BO);
-  double2* const Co = block(B_CO);
-  double2* const Go = block(B_GO);
-  double2* const X = block(B_X);
-  double2* const SL = block(B_SL);               // the left self-energy
-  SmallShared& sh = shared();
+template <int M>
+__global__ void __launch_bounds__(Shape<M>::kCta, Shape<M>::kPerSm) k_small_point(MixedArgs a) {
+  constexpr int kLd = Shape<M>::kLd;
+  double2* const Ao = block<M>(B_AO);
+  double2* const Bo = block<M>(B_BO);
+  double2* const Co = block<M>(B_CO);
+  double2* const Go = block<M>(B_GO);
+  double2* const X = block<M>(B_X);
+  double2* const SL = block<M>(B_SL);               // the left self-energy
+  SmallShared& sh = shared<M>();
   const int pair = team_size() == 2, rank = team_rank();
   const int p = blockIdx.x >> pair, n = a.n;
-  const Lane L(n);
+  const Lane<M> L(n);
   if (threadIdx.x == 0) {
     sh.inv.piv = sh.piv;
     sh.inv.perm = sh.perm;
@@ -250,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     sh.inv.flag = &sh.flag;
     sh.inv.tr.acc = nullptr;
   }
-  for (int q = threadIdx.x; q < kBlocks * kBlk; q += kThreads) Ao[q] = make_double2(0.0, 0.0);
+  for (int q = threadIdx.x; q < kBlocks * Shape<M>::kBlk; q += Shape<M>::kCta) Ao[q] = make_double2(0.0, 0.0);
   __syncthreads();
   const DevDesc& d = a.d_descs[a.d_ids[p]];
   const double E = a.d_E[p];
@@ -273,9 +308,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       // ---- decimation from the contact energy times 1 + att 2^-50 (see kDecRetries)
       const double scale = 1.0 + att * 0x1p-50;
       const double2 ec = make_double2(E * scale, a.eta * scale);
-      load_esh(n, Ao, h00, s00, ec, true, false);
-      load_esh(n, Bo, h01, s01, ec, false, false);
-      load_esh(n, Co, h01, s01, cconj(ec), false, true);
+      load_esh<M>(n, Ao, h00, s00, ec, true, false);
+      load_esh<M>(n, Bo, h01, s01, ec, false, false);
+      load_esh<M>(n, Co, h01, s01, cconj(ec), false, true);
       __syncthreads();
       Frag Aos = get(L, Ao);
       bool ok = false, done = false, sens = false, diverged = false, off = false;
@@ -283,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       int it = 1;
 #pragma unroll 1
       for (; it <= a.sgf_max_iter; ++it) {
-        const int bad_inv = small_inverse(n);
+        const int bad_inv = small_inverse<M>(n);
         if (bad_inv & 1) put_st(NEGF_B200_ERR_SINGULAR);
         sens |= (bad_inv & 2) != 0;
         __syncthreads();
@@ -299,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
             mx = fmax(mx, h);
             bad |= !(h <= 1.7976931348623157e308);
           }
-        mx = cta_max_nan(bad ? __longlong_as_double(0x7ff8000000000000LL) : mx, sh.red[2]);
+        mx = cta_max_nan<M>(bad ? __longlong_as_double(0x7ff8000000000000LL) : mx, sh.red[2]);
         if (!(mx <= 1.7976931348623157e308)) {   // Inf / NaN: will not converge
           diverged = done = true;
         } else if (mx <= a.sgf_tol) {
@@ -334,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       __syncthreads();
       put(L, Ao, Aos);
       __syncthreads();
-      const int bad_gs = small_inverse(n);       // gs in Go
+      const int bad_gs = small_inverse<M>(n);       // gs in Go
       if (bad_gs & 1) put_st(NEGF_B200_ERR_SINGULAR);
       sens |= (bad_gs & 2) != 0;
       __syncthreads();
@@ -373,8 +408,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
             if (!(h <= df)) df = h > df ? h : __longlong_as_double(0x7ff0000000000000LL);
             mk = fmax(mk, cabs(kept.v[q]));
           }
-          df = cta_max_nan(df, sh.red[0]);
-          mk = cta_max_nan(mk, sh.red[1]);
+          df = cta_max_nan<M>(df, sh.red[0]);
+          mk = cta_max_nan<M>(mk, sh.red[1]);
           __syncthreads();
           if (df <= 1e-2 * mk) {
             if (diverged) {
@@ -402,8 +437,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     const double2 ec = make_double2(E, a.eta);
     const double2* hmc = d.hmc + d.omc[c];
     const double2* smc = d.has_smc ? d.smc + d.omc[c] : nullptr;
-    load_esh(n, Bo, hmc, smc, ec, false, false);
-    load_esh(n, Co, hmc, smc, cconj(ec), false, true);
+    load_esh<M>(n, Bo, hmc, smc, ec, false, false);
+    load_esh<M>(n, Co, hmc, smc, cconj(ec), false, true);
     __syncthreads();
     put(L, X, mm(L, Bo, Go));
     __syncthreads();
@@ -426,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     }
     if (side == 1 || pair) {
       // W = ESH(nbl, nbl) - Sigma_right
-      load_esh(n, Ao, d.hd + d.od[a.nbl - 1], d.has_s ? d.sd + d.od[a.nbl - 1] : nullptr, make_double2(E, 0.0), true,
+      load_esh<M>(n, Ao, d.hd + d.od[a.nbl - 1], d.has_s ? d.sd + d.od[a.nbl - 1] : nullptr, make_double2(E, 0.0), true,
                false);
       __syncthreads();
       sub_from(L, Ao, sig);
@@ -434,21 +469,21 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
     __syncthreads();
   }
   // ---- gsmr sweep down to Gr(1,1): g in Go
-  if (small_inverse(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
+  if (small_inverse<M>(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
 #pragma unroll 1
   for (int i = a.nbl - 2; i >= 0; --i) {
     const double2 e = make_double2(E, 0.0);
     __syncthreads();
-    load_esh(n, Bo, d.hu + d.oo[i], d.has_s ? d.su + d.oo[i] : nullptr, e, false, false);
-    load_esh(n, Co, d.hl + d.oo[i], d.has_s ? d.sl + d.oo[i] : nullptr, e, false, false);
-    load_esh(n, Ao, d.hd + d.od[i], d.has_s ? d.sd + d.od[i] : nullptr, e, true, false);
+    load_esh<M>(n, Bo, d.hu + d.oo[i], d.has_s ? d.su + d.oo[i] : nullptr, e, false, false);
+    load_esh<M>(n, Co, d.hl + d.oo[i], d.has_s ? d.sl + d.oo[i] : nullptr, e, false, false);
+    load_esh<M>(n, Ao, d.hd + d.od[i], d.has_s ? d.sd + d.od[i] : nullptr, e, true, false);
     __syncthreads();
     put(L, X, mm(L, Bo, Go));
     if (i == 0) sub_from(L, Ao, get(L, SL));
     __syncthreads();
     sub_from(L, Ao, mm(L, X, Co));
     __syncthreads();
-    if (small_inverse(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
+    if (small_inverse<M>(n) & 1) put_st(NEGF_B200_ERR_SINGULAR);
   }
   __syncthreads();
   // ---- Gamma = i (Sigma - Sigma^dag) of the left contact, then the trace
@@ -466,10 +501,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
       t1 += gam.x * -(gji.y + gij.y) - gam.y * (gji.x - gij.x);   // Re(Gam_ij i (G_ji - conj G_ij))
     }
   __syncthreads();
-  const Frag M = mm(L, Bo, Go), N = mm(L, Go, Bo);
+  const Frag gg = mm(L, Bo, Go), hh = mm(L, Go, Bo);
 #pragma unroll
   for (int q = 0; q < 4; ++q)
-    if (L.in(q)) t2 += M.v[q].x * N.v[q].x + M.v[q].y * N.v[q].y;
+    if (L.in(q)) t2 += gg.v[q].x * hh.v[q].x + gg.v[q].y * hh.v[q].y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     t1 += __shfl_xor_sync(kFull, t1, o);
@@ -482,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
   __syncthreads();
   if (threadIdx.x == 0) {
     t1 = t2 = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) {
+    for (int w = 0; w < Shape<M>::kWarps; ++w) {
       t1 += sh.red[0][w];
       t2 += sh.red[1][w];
     }
@@ -494,19 +529,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_small_point(MixedArgs a) {
   }
 }
 
+template <int M>
+cudaError_t launch(const MixedArgs& a, cudaStream_t s) {
+  // Two CTAs per point, a contact each, while they find room at once: order
+  // 32, 74 points: 1.34 ms by one CTA, 0.96 by two; 148 points (two CTAs per
+  // SM): 1.35 and 1.22; 149: 1.71 and 2.00.
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = team_config(a.npts, a.npts <= device_sms() ? 2 : 1, small_smem<M>(), s, &attr);
+  cfg.blockDim = dim3(Shape<M>::kCta);
+  const cudaError_t e = team_launch(cfg, k_small_point<M>, small_smem<M>(), a);
+  if (e == cudaSuccess && a.launches) ++*a.launches;
+  return e;
+}
+
 }  // namespace
 
 cudaError_t launch_small_points(const MixedArgs& a, cudaStream_t s) {
   if (a.npts <= 0) return cudaSuccess;
   if (a.n < 1 || a.n > kSmallMax) return cudaErrorInvalidValue;
-  // Two CTAs per point, a contact each, while they find room at once: order
-  // 32, 74 points: 1.34 ms by one CTA, 0.96 by two; 148 points (two CTAs per
-  // SM): 1.35 and 1.22; 149: 1.71 and 2.00.
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = team_config(a.npts, a.npts <= device_sms() ? 2 : 1, kSmallSmem, s, &attr);
-  const cudaError_t e = team_launch(cfg, k_small_point, kSmallSmem, a);
-  if (e == cudaSuccess && a.launches) ++*a.launches;
-  return e;
+  return a.n <= 16 ? launch<16>(a, s) : launch<32>(a, s);
 }
 
 }  // namespace negf
