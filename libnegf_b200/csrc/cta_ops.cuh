@@ -499,9 +499,11 @@ __host__ __device__ inline int gemm_tile(int M, int N, int size) {
 }
 
 // Publishes the descriptor of one product in shared memory; this CTA takes
-// the output tiles rank, rank + size, ...
+// the output tiles rank, rank + size, ... (of tile x tile elements; 0: the
+// size of gemm_tile()).
 __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, const Operand& A, const Operand& B,
-                                                       const Epilogue& e, double2* smem, int rank, int size) {
+                                                       const Epilogue& e, double2* smem, int rank, int size,
+                                                       int tile = 0) {
   GemmDesc* d = reinterpret_cast<GemmDesc*>(smem + kGemmDescOffset);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -513,7 +515,7 @@ __device__ __forceinline__ GemmDesc* gemm_desc_publish(int M, int N, int K, cons
     d->want_max = e.maxabs != nullptr && !e.idle_max;
     d->M = M; d->N = N; d->K = K;
     d->amode = A.mode; d->bmode = B.mode; d->emode = e.mode;
-    const int T = gemm_tile(M, N, size);
+    const int T = tile ? tile : gemm_tile(M, N, size);
     d->tile = T;
     d->tilesM = (M + T - 1) / T;
     d->nk = max(1, (K + TK - 1) / TK);

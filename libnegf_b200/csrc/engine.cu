@@ -375,10 +375,10 @@ TeamPlan team_plan(int work, int n, int max_ctas, int sms) {
 }
 
 // ---------------------------------------------------------------- primitives
-// CTA (x, b) of the grid: output tiles x, x + gridDim.x, ... of product b.
+// CTA (x, b) of the grid: output tiles (of tile x tile elements) x, x + gridDim.x, ... of product b.
 __global__ void __launch_bounds__(kThreads, 2)
     k_zgemm_batched(int m, int n, int k, double2 alpha, const double2* A, int64_t sA, const double2* B,
-                    int64_t sB, double2 beta, double2* C, int64_t sC, int dagger) {
+                    int64_t sB, double2 beta, double2* C, int64_t sC, int dagger, int tile) {
   extern __shared__ __align__(16) char smem_raw[];
   SmemMap sm = map_smem(smem_raw, 1);
   sm.tr.acc = nullptr;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   Operand Ao = (dagger == 1) ? opC(A + b * sA, k) : opN(A + b * sA, m);
   Operand Bo = (dagger == 2) ? opC(B + b * sB, n) : opN(B + b * sB, k);
   const GemmDesc* d = gemm_desc_publish(m, n, k, Ao, Bo, epi_store(C + b * sC, m, alpha, beta), sm.main, blockIdx.x,
-                                        gridDim.x);
+                                        gridDim.x, tile);
   if (d->tile == kTile) cta_gemm_body<kTile>(d, sm.main);
   else gemm_run_small(d, sm.main);
 }
@@ -411,23 +411,51 @@ static bool in_place(const double2* A, int64_t sA, int64_t na, const double2* C,
   return std::min(first, last) < na * kElem && std::max(first, last) > -nc * kElem;
 }
 
+// The output tile of a batch of m x n products, a tile per CTA.  Small tiles
+// spread few products over more SMs, but cost 0.46 of a large one's time for a
+// quarter of its elements, so they lose as soon as the large ones fill the GPU.
+// Where C has at most 32 rows or columns, half of a large tile's warps idle: it
+// takes 0.66 alone (a small one 0.33), 1.5 times that beside another one, 0.5 in
+// a full GPU.  CTAs that share an SM share its FP64 pipe: 1.95 times the time with
+// two large tiles, 1.7 with two small ones, and in proportion beyond that.  us,
+// small and large tiles, one per CTA: order 64, 74 products 12.9 and 16.8, 148:
+// 22.1 and 16.8, 296: 39.4 and 26.0; order 128, 100: 87.7 and 65.2; order 300, 6:
+// 78.4 and 94.5, 10: 118 and 96.
+static int zgemm_tile(int batch, int m, int n, int sms) {
+  const double big = (double)((m + kTile - 1) / kTile) * ((n + kTile - 1) / kTile);
+  const double small = (double)((m + kSmallTile - 1) / kSmallTile) * ((n + kSmallTile - 1) / kSmallTile);
+  const bool narrow = m <= kSmallTile || n <= kSmallTile;
+  const double work_big = narrow ? 0.66 : 1.0, work_small = narrow ? 0.33 : 0.46;
+  auto time = [&](double ctas, double two) {
+    const double x = ctas * batch / sms;
+    return x <= 1.0 ? 1.0 : (x <= 2.0 ? two : two * (0.5 * x + 0.2));
+  };
+  if (big * batch > 4.0 * sms)   // two waves of large tiles: the work alone decides
+    return (narrow ? 0.5 : 1.0) * big <= 0.46 * small ? kTile : kSmallTile;
+  return work_big * time(big, narrow ? 1.5 : 1.95) <= 0.98 * work_small * time(small, 1.7) ? kTile : kSmallTile;
+}
+
 cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, const double2* A, int64_t sA,
                                  const double2* B, int64_t sB, double2 beta, double2* C, int64_t sC,
                                  int dagger, cudaStream_t s) {
-  // A product's tiles over enough CTAs for four waves of the whole batch: one
-  // CTA per product left all but `batch` SMs idle (6 products of order 300:
-  // 1604 -> 82 us); with 1184 products and more one CTA runs through all
-  // tiles of a product, loading the next tile's operands behind this one's
-  // epilogue.
-  int64_t want = (8LL * device_sms() + batch - 1) / batch;
+  // A tile per CTA (one CTA per product left all but `batch` SMs idle: 6
+  // products of order 300 1604 -> 82 us), up to a number of CTAs per SM beyond
+  // which a CTA runs through several tiles of a product and loads the next
+  // tile's operands behind this one's epilogue: the shorter the product, the
+  // more that counts beside the spread (900 products of 128 x 128: K = 16 103 us
+  // with two tiles per CTA, 122 with one; K = 128 509 and 484).
+  const int sms = device_sms();
+  int T = zgemm_tile(batch, m, n, sms);
+  const int64_t per_sm = std::min(48, 4 * ((k + TK - 1) / TK) + 4);
+  int64_t want = (per_sm * sms + batch - 1) / batch;
   // C in the place of A or B: up to order 64 one CTA holds the whole product in
-  // one tile and has read all operands when it stores (gemm_tile() for one CTA
-  // keeps 64 x 64 in one), so such calls stay with it.
+  // one tile and has read all operands when it stores, so such calls stay with it.
   if (m <= kTile && n <= kTile &&
       (in_place(A, sA, (int64_t)m * k, C, sC, (int64_t)m * n, batch) ||
-       in_place(B, sB, (int64_t)k * n, C, sC, (int64_t)m * n, batch)))
+       in_place(B, sB, (int64_t)k * n, C, sC, (int64_t)m * n, batch))) {
+    T = m <= kSmallTile && n <= kSmallTile ? kSmallTile : kTile;
     want = 1;
-  const int T = gemm_tile(m, n, (int)std::min<int64_t>(want, 1 << 20));
+  }
   const int64_t tiles = (int64_t)((m + T - 1) / T) * ((n + T - 1) / T);
   const int split = (int)std::max<int64_t>(1, std::min(tiles, want));
   for (int b0 = 0; b0 < batch; b0 += 65535) {   // gridDim.y limit
@@ -435,7 +463,7 @@ cudaError_t launch_zgemm_batched(int batch, int m, int n, int k, double2 alpha, 
     cudaLaunchConfig_t cfg = team_config(1, 1, engine_smem_bytes(1), s, nullptr);
     cfg.gridDim = dim3(split, nb);
     const cudaError_t e = team_launch(cfg, k_zgemm_batched, 0, m, n, k, alpha, A + b0 * sA, sA, B + b0 * sB, sB, beta,
-                                      C + b0 * sC, sC, dagger);
+                                      C + b0 * sC, sC, dagger, T);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
