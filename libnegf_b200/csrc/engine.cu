@@ -493,10 +493,24 @@ __global__ void __launch_bounds__(kThreads, 2)
   team_sync();   // no member's shared memory is read any more
 }
 
+// Teams for a batch of inverses alone.  Their panels do not split over a team,
+// so a team's other CTAs mostly wait in the places of other matrices: with more
+// matrices than SMs one CTA each, with more than half as many one (up to order
+// 128, four leaves) or two.  ms by this rule and by the teams that suit a
+// decimation: order 256, 100 matrices 1.88 and 2.36, 250: 2.85 and 3.80, 297: 4.40
+// and 5.82; order 128, 170: 0.49 and 0.68; order 257, 100: 3.3 and 4.7.
+TeamShape zinv_shape(int batch, int n, int max_ctas, int sms) {
+  if (2 * batch > sms) {
+    const int team = batch > sms || n <= 128 ? 1 : 2;
+    if (team == 1 || resident_teams(team) >= 1) return TeamShape{team, std::min(batch, max_ctas / team)};
+  }
+  return team_shape(batch, n, max_ctas, sms);
+}
+
 cudaError_t launch_zinv_mapped(int batch, int n, const double2* A, int64_t sA, double2* X, int64_t sX,
                                const int* map, int* info, double2* work, cudaStream_t s, int* sens) {
   if (batch <= 0) return cudaSuccess;
-  const TeamShape t = team_shape(batch, n, 2 * device_sms(), device_sms());
+  const TeamShape t = zinv_shape(batch, n, 2 * device_sms(), device_sms());
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = team_config(batch, t.team, engine_smem_bytes(n), s, &attr);
   return team_launch(cfg, k_zinv_mapped, 0, n, A, sA, X, sX, map, info, work,

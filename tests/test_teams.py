@@ -330,9 +330,9 @@ def test_product_in_the_place_of_an_operand(n, dagger, place):
 
 
 def _team_of(L, work, n):
-    """The library's own choice of CTAs per problem (its team_shape: two ints
-    in one register), so that a test says which sizes it compares."""
-    f = L["_ZN4negf10team_shapeEiiii"]
+    """The library's own choice of CTAs per matrix (its zinv_shape: two ints in
+    one register), so that a test says which sizes it compares."""
+    f = L["_ZN4negf10zinv_shapeEiiii"]
     f.restype, f.argtypes = ctypes.c_uint64, [ctypes.c_int] * 4
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
